@@ -8,6 +8,7 @@
 #include <numeric>
 #include <vector>
 
+#include "leaf_copy.cuh"
 #include "method_state.hpp"
 #include "sort_reduce.hpp"
 
@@ -301,27 +302,44 @@ __global__ void k_pick(const int* flags, const int* pos, int n, const int4* o_in
     }
 }
 
+// f32 leaves 0..n-1 -> pool slots 0..n-1, one warp per leaf (312k f16 leaves:
+// 552 us one value per thread, 160 us this way, 6.0 TB/s).
 template <typename T>
-__global__ void k_from_f32(const float* in, T* out, size_t n) {
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
-        out[i] = from_f<T>(in[i]);
+__global__ void __launch_bounds__(256) k_from_f32(const float* __restrict__ in, T* __restrict__ out, size_t n) {
+    const int lane = threadIdx.x & 31;
+    const bool vec = aligned16(in);
+    for (size_t i = (blockIdx.x * (size_t)blockDim.x + threadIdx.x) >> 5; i < n;
+         i += ((size_t)gridDim.x * blockDim.x) >> 5)
+        leaf_in(in + i * kLeafVoxels, out + i * kLeafVoxels, vec, lane);
+}
+
+// CTAs of 256 threads for a kernel that gives each leaf one warp: all
+// resident at once (8 per SM), fewer when the leaves are few.
+int leaf_warp_blocks(const vlr_ctx* ctx, size_t n) {
+    return (int)std::max<size_t>(1, std::min<size_t>((n + 7) / 8, (size_t)ctx->sm_count * 8));
 }
 
 __global__ void k_gather_origins(const int* list, int n, const int4* origin, int4* o_out) {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) o_out[i] = origin[list[i]];
 }
 
-// Masks and f32 values of the leaves at list positions sel[0..k) in that
-// order (output order), one CTA per leaf.
+// Mask and f32 values of pool slot s as output record i, by one warp.
 template <typename T>
-__global__ void k_gather_sel(const int* list, const int* sel, int k, const uint64_t* mask, const T* vals,
-                             uint64_t* m_out, float* v_out) {
-    for (int i = blockIdx.x; i < k; i += gridDim.x) {
-        const int s = list[sel[i]];
-        if (threadIdx.x < 8) m_out[(size_t)i * 8 + threadIdx.x] = mask[(size_t)s * 8 + threadIdx.x];
-        for (int t = threadIdx.x; t < kLeafVoxels; t += blockDim.x)
-            v_out[(size_t)i * kLeafVoxels + t] = to_f(vals[(size_t)s * kLeafVoxels + t]);
-    }
+__device__ __forceinline__ void record_out(int s, size_t i, const uint64_t* __restrict__ mask,
+                                           const T* __restrict__ vals, uint64_t* __restrict__ m_out,
+                                           float* __restrict__ v_out, bool vec, int lane) {
+    if (lane < 8) m_out[i * 8 + lane] = mask[(size_t)s * 8 + lane];
+    leaf_out(vals + (size_t)s * kLeafVoxels, v_out + i * kLeafVoxels, vec, lane);
+}
+
+// Masks and f32 values of the leaves at list positions sel[0..k) in that
+// order (output order), one warp per leaf.
+template <typename T>
+__global__ void __launch_bounds__(256) k_gather_sel(const int* list, const int* sel, int k, const uint64_t* mask,
+                                                   const T* vals, uint64_t* m_out, float* v_out) {
+    const bool vec = aligned16(v_out);
+    for (int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < k; i += (gridDim.x * blockDim.x) >> 5)
+        record_out(list[sel[i]], (size_t)i, mask, vals, m_out, v_out, vec, threadIdx.x & 31);
 }
 
 // Output order of a host step without a host round trip: for up to
@@ -374,16 +392,14 @@ __global__ void __launch_bounds__(256) k_rank_scatter(const int* __restrict__ li
 
 // k_gather_sel with the count and the sort status read on the device.
 template <typename T>
-__global__ void k_gather_sel_dev(const int* list, const int* sel, const int* count, const int* status,
-                                 const uint64_t* mask, const T* vals, uint64_t* m_out, float* v_out) {
+__global__ void __launch_bounds__(256) k_gather_sel_dev(const int* list, const int* sel, const int* count,
+                                                       const int* status, const uint64_t* mask, const T* vals,
+                                                       uint64_t* m_out, float* v_out) {
     if (!*status) return;
     const int k = *count;
-    for (int i = blockIdx.x; i < k; i += gridDim.x) {
-        const int s = list[sel[i]];
-        if (threadIdx.x < 8) m_out[(size_t)i * 8 + threadIdx.x] = mask[(size_t)s * 8 + threadIdx.x];
-        for (int t = threadIdx.x; t < kLeafVoxels; t += blockDim.x)
-            v_out[(size_t)i * kLeafVoxels + t] = to_f(vals[(size_t)s * kLeafVoxels + t]);
-    }
+    const bool vec = aligned16(v_out);
+    for (int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < k; i += (gridDim.x * blockDim.x) >> 5)
+        record_out(list[sel[i]], (size_t)i, mask, vals, m_out, v_out, vec, threadIdx.x & 31);
 }
 
 __global__ void k_count_active(const int* list, const int* count_ptr, const uint64_t* mask,
@@ -488,7 +504,7 @@ int upload_enqueue(vlr_ctx* ctx, vlr_level_set* ls, const int32_t* origins, cons
     k_unpack_upload<<<ls->grid_blocks, 256, 0, ctx->stream>>>(o3, (int)n, ls->origin);
     if (ls->precision == VLR_PREC_F16) {
         VLR_CUDA(ctx, cudaMemcpyAsync(tmp, phi, vbytes, cudaMemcpyHostToDevice, ctx->stream));
-        k_from_f32<__half><<<ls->grid_blocks, 256, 0, ctx->stream>>>(tmp, (__half*)ls->vals[0], kLeafVoxels * n);
+        k_from_f32<__half><<<leaf_warp_blocks(ctx, n), 256, 0, ctx->stream>>>(tmp, (__half*)ls->vals[0], n);
     } else {
         VLR_CUDA(ctx, cudaMemcpyAsync(ls->vals[0], phi, vbytes, cudaMemcpyHostToDevice, ctx->stream));
     }
@@ -514,20 +530,21 @@ __global__ void k_upload_dev_origins(const int32_t* o3, int n, int4* origin, uns
 }
 
 // The listed leaves in list order into device buffers (origins i32[3], masks,
-// f32 values), one CTA per leaf.
+// f32 values), one warp per leaf (312k f16 leaves: 466 us one CTA per leaf
+// and one value per thread, 166 us this way, 5.9 TB/s).
 template <typename T>
-__global__ void k_export_dev(const int* list, const int* count, const int4* origin, const uint64_t* mask,
-                             const T* vals, int32_t* o3, uint64_t* m_out, float* v_out) {
-    const int n = *count;
-    for (int i = blockIdx.x; i < n; i += gridDim.x) {
+__global__ void __launch_bounds__(256) k_export_dev(const int* list, const int* count, const int4* origin,
+                                                   const uint64_t* mask, const T* vals, int32_t* o3,
+                                                   uint64_t* m_out, float* v_out) {
+    const int n = *count, lane = threadIdx.x & 31;
+    const bool vec = aligned16(v_out);
+    for (int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < n; i += (gridDim.x * blockDim.x) >> 5) {
         const int s = list[i];
-        if (threadIdx.x < 3) {
+        if (lane < 3) {
             const int4 o = origin[s];
-            o3[3 * i + threadIdx.x] = threadIdx.x == 0 ? o.x : (threadIdx.x == 1 ? o.y : o.z);
+            o3[3 * (size_t)i + lane] = lane == 0 ? o.x : (lane == 1 ? o.y : o.z);
         }
-        if (threadIdx.x < 8) m_out[(size_t)i * 8 + threadIdx.x] = mask[(size_t)s * 8 + threadIdx.x];
-        for (int t = threadIdx.x; t < kLeafVoxels; t += blockDim.x)
-            v_out[(size_t)i * kLeafVoxels + t] = to_f(vals[(size_t)s * kLeafVoxels + t]);
+        record_out(s, (size_t)i, mask, vals, m_out, v_out, vec, lane);
     }
 }
 
@@ -685,7 +702,7 @@ int download_sorted_device(vlr_ctx* ctx, const vlr_level_set* ls, size_t n, int3
     const int* sel = (const int*)v2;
     if (origins) k_sorted_origins<<<B, 256, 0, st>>>(ls->list, v2, nn, ls->origin, o3);
     if (masks || phi) {
-        const int G = (int)std::min<size_t>(n, (size_t)ctx->sm_count * 8);
+        const int G = leaf_warp_blocks(ctx, n);
         if (ls->precision == VLR_PREC_F16)
             k_gather_sel<__half><<<G, 256, 0, st>>>(ls->list, sel, nn, ls->mask, (const __half*)ls->vals[0], mm, v);
         else
@@ -751,7 +768,7 @@ int download_n(vlr_ctx* ctx, const vlr_level_set* ls, size_t n, int grid, int32_
     }
     if (k && (masks || phi)) {
         VLR_CUDA(ctx, cudaMemcpyAsync(dsel, sel.data(), sizeof(int) * k, cudaMemcpyHostToDevice, ctx->stream));
-        const int B = (int)std::min<size_t>(k, (size_t)ctx->sm_count * 8);
+        const int B = leaf_warp_blocks(ctx, k);
         if (ls->precision == VLR_PREC_F16)
             k_gather_sel<__half><<<B, 256, 0, ctx->stream>>>(ls->list, dsel, (int)k, ls->mask,
                                                              (const __half*)ls->vals[0], mm, v);
@@ -821,22 +838,21 @@ __global__ void k_slab_keys(const int* __restrict__ list, const int* __restrict_
 }
 
 // Origins, masks and f32 values of the first min(*kept, room) sorted list
-// positions sel[i], one CTA per leaf.
+// positions sel[i], one warp per leaf.
 template <typename T>
 __global__ void k_gather_slab(const int* __restrict__ list, const unsigned* __restrict__ sel,
                               const int* __restrict__ kept, int room, const int4* __restrict__ origin,
                               const uint64_t* __restrict__ mask, const T* __restrict__ vals, int32_t* __restrict__ o3,
                               uint64_t* __restrict__ m_out, float* __restrict__ v_out) {
-    const int k = min(*kept, room);
-    for (int i = blockIdx.x; i < k; i += gridDim.x) {
+    const int k = min(*kept, room), lane = threadIdx.x & 31;
+    const bool vec = aligned16(v_out);
+    for (int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < k; i += (gridDim.x * blockDim.x) >> 5) {
         const int s = list[sel[i]];
-        if (threadIdx.x < 3) {
+        if (lane < 3) {
             const int4 o = origin[s];
-            o3[3 * i + threadIdx.x] = threadIdx.x == 0 ? o.x : (threadIdx.x == 1 ? o.y : o.z);
+            o3[3 * (size_t)i + lane] = lane == 0 ? o.x : (lane == 1 ? o.y : o.z);
         }
-        if (threadIdx.x < 8) m_out[(size_t)i * 8 + threadIdx.x] = mask[(size_t)s * 8 + threadIdx.x];
-        for (int t = threadIdx.x; t < kLeafVoxels; t += blockDim.x)
-            v_out[(size_t)i * kLeafVoxels + t] = to_f(vals[(size_t)s * kLeafVoxels + t]);
+        record_out(s, (size_t)i, mask, vals, m_out, v_out, vec, lane);
     }
 }
 
@@ -857,7 +873,7 @@ int load_pool(vlr_ctx* ctx, vlr_level_set* ls, const int32_t* o3, const uint64_t
         k_unpack_upload<<<ls->grid_blocks, 256, 0, st>>>(o3, (int)n, ls->origin);
         VLR_CUDA(ctx, cudaMemcpyAsync(ls->mask, masks, 64 * n, cudaMemcpyDeviceToDevice, st));
         if (ls->precision == VLR_PREC_F16)
-            k_from_f32<__half><<<ls->grid_blocks, 256, 0, st>>>(phi, (__half*)ls->vals[0], kLeafVoxels * n);
+            k_from_f32<__half><<<leaf_warp_blocks(ctx, n), 256, 0, st>>>(phi, (__half*)ls->vals[0], n);
         else
             VLR_CUDA(ctx, cudaMemcpyAsync(ls->vals[0], phi, sizeof(float) * kLeafVoxels * n, cudaMemcpyDeviceToDevice,
                                           st));
@@ -1353,8 +1369,8 @@ int vlr_ls_upload_device(vlr_ctx* ctx, vlr_level_set* ls, const int32_t* d_origi
         k_upload_dev_origins<<<ls->grid_blocks, 256, 0, ctx->stream>>>(d_origins, n, ls->origin, ctx->d_errword);
         VLR_CUDA(ctx, cudaMemcpyAsync(ls->mask, d_masks, 64 * n_leaves, cudaMemcpyDeviceToDevice, ctx->stream));
         if (ls->precision == VLR_PREC_F16)
-            k_from_f32<__half><<<ls->grid_blocks, 256, 0, ctx->stream>>>(d_phi, (__half*)ls->vals[0],
-                                                                          kLeafVoxels * n_leaves);
+            k_from_f32<__half><<<leaf_warp_blocks(ctx, n_leaves), 256, 0, ctx->stream>>>(
+                d_phi, (__half*)ls->vals[0], n_leaves);
         else
             VLR_CUDA(ctx, cudaMemcpyAsync(ls->vals[0], d_phi, sizeof(float) * kLeafVoxels * n_leaves,
                                           cudaMemcpyDeviceToDevice, ctx->stream));
@@ -1376,7 +1392,7 @@ int vlr_ls_download_device(vlr_ctx* ctx, const vlr_level_set* ls, int32_t* d_ori
     if (rc) return rc;
     if (n > cap_leaves) return set_error(ctx, VLR_ERR_CAPACITY, "output buffers too small");
     if (n) {
-        const int B = (int)std::min<size_t>(n, (size_t)ctx->sm_count * 8);
+        const int B = leaf_warp_blocks(ctx, n);
         if (ls->precision == VLR_PREC_F16)
             k_export_dev<__half><<<B, 256, 0, ctx->stream>>>(ls->list, ls->scalars, ls->origin, ls->mask,
                                                              (const __half*)ls->vals[0], d_origins, d_masks, d_phi);
