@@ -624,20 +624,23 @@ def full_period(args, ctx, precision, reinit_mode=0):
 # each array counted once per launch (the trilinear corners and the
 # candidates' feet are read through the cache by up to 27 neighbours):
 #   k_adj_forward: band index 4 + displacement 12 + phi_k 4 + phi_k+1 4
-#   k_adj_pack:    band index 4 + displacement 12 + lambda 4 + foot word 4 + weights and lambda 16
-#   k_adj_lambda:  band index 4 + own foot 20 + phi_k 4 + G read and written 24 + lambda out 4
-ADJ_BYTES_PER_BAND_VOXEL = {"k_adj_forward": 24, "k_adj_pack": 40, "k_adj_lambda": 56}
+#   k_adj_pack:    band index 4 + velocity 12 + lambda 4 + foot word 4 + weights and lambda 16
+#   k_adj_lambda:  band index 4 + foot word 4 + weights and lambda 16, and
+#     staggered field: gradient 12 + G read and written 24 + velocity 12 + next foot 20
+#     level set (fixed feet): lambda 4 + lambda out 4
+ADJ_BYTES_PER_BAND_VOXEL = {"k_adj_forward": 24, "k_adj_pack": 40, "k_adj_lambda": 92}
+ADJ_LS_BYTES_PER_BAND_VOXEL = {"k_adj_forward": 24, "k_adj_lambda": 32}
 
 
-def adjoint_roofline(kern, nb, peak, peak_kind):
+def adjoint_roofline(kern, nb, peak, peak_kind, bytes_per_voxel=ADJ_BYTES_PER_BAND_VOXEL):
     """HBM roofline of the adjoint's dominant kernel from a profiled pass:
     kern = {name: (total ms, launches)}."""
-    timed = {k: v for k, v in kern.items() if k in ADJ_BYTES_PER_BAND_VOXEL and v[1] > 0}
+    timed = {k: v for k, v in kern.items() if k in bytes_per_voxel and v[1] > 0}
     if not timed:
         return None
     dom = max(timed, key=lambda k: timed[k][0])
     ms = timed[dom][0] / timed[dom][1]
-    per = ADJ_BYTES_PER_BAND_VOXEL[dom]
+    per = bytes_per_voxel[dom]
     achieved = per * nb / (ms * 1e-3) / 1e9
     return {"bound": "hbm", "kernel": dom, "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
             "peak_kind": peak_kind, "traffic": None, "algorithmic_bytes_per_band_voxel": per,
@@ -767,7 +770,7 @@ def bench_level_set_adjoint(args, ctx, ls, steps=32, chk=6, shift=(4, 0, 0)):
         d_lam.mul_(2.0)
         fn.backward_device(d_lam.data_ptr(), d_g0.data_ptr(), 0)
     ctx.check_device()
-    kern = {k: ctx.kernel_time(k) for k in ("k_adj_forward", "k_adj_pack", "k_adj_lambda")}
+    kern = {k: ctx.kernel_time(k) for k in ("k_adj_forward", "k_adj_lambda")}
     ctx.profile(False)
     fn.close()
     f, b = statistics.median(fw), statistics.median(bw)
@@ -778,7 +781,7 @@ def bench_level_set_adjoint(args, ctx, ls, steps=32, chk=6, shift=(4, 0, 0)):
             "value": nb * steps / ((f + b) * 1e-3), "unit": "band voxel-steps/s (forward + backward)",
             "forward_voxels_per_s": nb * steps / (f * 1e-3),
             "kernels_ms_per_launch": {k: v[0] / max(v[1], 1) for k, v in kern.items()},
-            "roofline": adjoint_roofline(kern, nb, *measured_peaks()),
+            "roofline": adjoint_roofline(kern, nb, *measured_peaks(), ADJ_LS_BYTES_PER_BAND_VOXEL),
             "timing": "device buffers, CUDA events on the library stream (forward_device + backward_device)"}
 
 

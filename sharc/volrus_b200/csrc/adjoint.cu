@@ -14,10 +14,21 @@
 //   G(x)      += lambda_{k+1}(x) (-dt c_k) grad trilinear(phi_k)(p_k(x))
 //   dL/dphi_0 = lambda_0,  dL/dV = upsample^T G
 // The lambda transpose is a gather over the band voxels whose foot cell can
-// hold the corner (a window of (2R+2)^3 voxels, R the per-step reach), summed
-// in a fixed order; upsample^T goes through a stable radix sort and a
-// segmented sum.  No float atomics: deterministic results.  phi_k for the
-// backward pass is recomputed from checkpoints taken every C steps (sqrt(K)).
+// hold the corner (a window of at most (2R+2)^3 voxels, R the per-step reach),
+// summed in a fixed order.  upsample^T depends on the geometry alone: its
+// entries are sorted by node once at creation (stable radix sort) and a
+// backward pass sums each node's entries in that order.  No float atomics:
+// deterministic results.  The trilinear gradient of phi_k at every foot comes
+// from recomputing phi_k between checkpoints taken every C steps (sqrt(K)),
+// by the forward kernel itself, which reads the same eight corners.  A level
+// set's displacement is fixed and its map is linear in lambda with constant
+// feet, so its backward pass needs neither phi_k nor checkpoints.
+//
+// State lives in leaf pools (512 values a leaf); band voxels are listed in
+// leaf order, and the step kernels take the list in chunks of up to 32 voxels
+// of one leaf, one warp a chunk: the leaf's 27 neighbour slots sit in the
+// warp's lanes (one shuffle per lookup instead of a load) and its candidate
+// window is uniform over the warp.
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -49,27 +60,36 @@ struct vlr_adjoint {
     double dt = 0.0, t0 = 0.0, period = 1.0;
     int steps = 0, chk_every = 1;
     float* checkpoints = nullptr;        // (steps / chk_every + 1) x n_band
-    float* segment = nullptr;            // chk_every x n_band (recomputed states)
-    float* lam[2] = {nullptr, nullptr};
+    float3* segment = nullptr;           // chk_every x n_band (gradients of the recomputed states at the feet)
+    float* lam[2] = {nullptr, nullptr};  // band order: [1] lambda_K (and phi_K), [0] lambda_0
     float* lam_final = nullptr;          // lam buffer holding dL/dphi_0 after the last backward pass
     // the forward and backward step loops captured as CUDA graphs (dropped
     // when the velocity, hence the reach, changes)
     cudaGraphExec_t fwd_exec = nullptr, bwd_exec = nullptr;
-    float* bwd_final = nullptr;          // lam buffer the captured backward loop ends in
     float* gvel = nullptr;               // dL/dV, 3 x n^3
     float3* G = nullptr;
     int reach = 1;                       // displacement bound per step, voxels (ceil of dt max|V|)
     int gather = 0;                      // transpose kernel: 0 by band size and reach, 1 windowed, 2 quad
     int disp = 0;                        // 1: ub holds each band voxel's fixed backtrace displacement
                                          // (a level set's time-independent velocity), step factor 1
-    unsigned* foot_pk = nullptr;         // per pool voxel: packed foot offsets of band voxels, 0 elsewhere
-    int* lrange = nullptr;               // per leaf: min and max foot offset per axis of its band voxels (6 ints)
-    int* wrange = nullptr;               // per leaf: candidate window per axis for its corners (6 ints)
-    float4* foot_w = nullptr;            // per pool voxel: (wx, wy, wz, lambda) of band voxels
-    unsigned* keys = nullptr;
-    float* pvals = nullptr;
-    void* scratch = nullptr;
-    size_t n_pairs_cap = 0;
+    int* lstart = nullptr;               // n_leaves + 1: first band index of each leaf
+    int2* chunks = nullptr;              // up to 32 band voxels of one leaf: see load_chunk
+    int n_chunks = 0;
+    float* urange = nullptr;             // per leaf: min and max of ub per axis over its band voxels (6 floats)
+    float* nrange = nullptr;             // the same over the leaf's 27-leaf neighbourhood
+    // feet of the band voxels by pool voxel, ping-pong over the steps (one
+    // buffer for a fixed displacement): packed offsets (0 off the band) and
+    // (wx, wy, wz, lambda); a fixed displacement keeps lambda in lam_pool
+    unsigned* foot_pk[2] = {nullptr, nullptr};
+    float4* foot_w[2] = {nullptr, nullptr};
+    float* lam_pool[2] = {nullptr, nullptr};
+    // upsample^T: entry e adds ent_w[e] G[ent_b[e]] (G as 3 n_band floats) to
+    // node seg_node[j], e in [seg_start[j], seg_start[j + 1])
+    int* ent_b = nullptr;
+    float* ent_w = nullptr;
+    int* seg_start = nullptr;
+    unsigned* seg_node = nullptr;
+    int n_seg = 0;
 };
 
 namespace vlr {
@@ -141,37 +161,132 @@ __device__ __forceinline__ Foot foot_of(float3 u, float s) {
     return f;
 }
 
-// One forward step over the band voxels, one thread each.  Non-band voxels
-// never change, and both state buffers hold phi_0 there (the callers copy it
-// into both), so they are not touched.
-__global__ void k_adj_forward(const int* __restrict__ bvox, int nb, const int* __restrict__ nbr,
-                              const float3* __restrict__ ub, const float* __restrict__ src, float* __restrict__ dst,
-                              float s, float hw, unsigned* err) {
-    for (int b = blockIdx.x * blockDim.x + threadIdx.x; b < nb; b += gridDim.x * blockDim.x) {
-        const int t = bvox[b];
-        const int slot = t >> 9, off = t & 511;
-        Foot f = foot_of(ub[b], s);
-        int x = (off >> 6) + f.fx, y = ((off >> 3) & 7) + f.fy, z = (off & 7) + f.fz;
-        if (x < -8 || y < -8 || z < -8 || x > 14 || y > 14 || z > 14) {
-            atomicOr(err, kErrReach);
-            dst[t] = src[t];
-            continue;
-        }
-        float c000 = adj_read(src, nbr, slot, x, y, z, hw), c100 = adj_read(src, nbr, slot, x + 1, y, z, hw);
-        float c010 = adj_read(src, nbr, slot, x, y + 1, z, hw), c110 = adj_read(src, nbr, slot, x + 1, y + 1, z, hw);
-        float c001 = adj_read(src, nbr, slot, x, y, z + 1, hw), c101 = adj_read(src, nbr, slot, x + 1, y, z + 1, hw);
-        float c011 = adj_read(src, nbr, slot, x, y + 1, z + 1, hw),
-              c111 = adj_read(src, nbr, slot, x + 1, y + 1, z + 1, hw);
-        float c00 = c000 * (1 - f.wx) + c100 * f.wx, c01 = c001 * (1 - f.wx) + c101 * f.wx;
-        float c10 = c010 * (1 - f.wx) + c110 * f.wx, c11 = c011 * (1 - f.wx) + c111 * f.wx;
-        float c0 = c00 * (1 - f.wy) + c10 * f.wy, c1 = c01 * (1 - f.wy) + c11 * f.wy;
-        dst[t] = c0 * (1 - f.wz) + c1 * f.wz;
-    }
+// One warp's chunk of the band list: up to 32 band voxels of one leaf, packed
+// as (leaf << 6 | first chunk of its leaf << 5 | voxels - 1, first band
+// index).  Lanes past the chunk repeat its first voxel (they take part in the
+// shuffles and store nothing); row holds the leaf's neighbour slots, lane d
+// the one at leaf offset d.
+struct Chunk {
+    int leaf, b, off, row;
+    bool on;
+};
+__device__ __forceinline__ Chunk load_chunk(int2 h, const int* __restrict__ bvox, const int* __restrict__ nbr,
+                                            int lane) {
+    Chunk k;
+    k.leaf = h.x >> 6;
+    k.row = lane < kNbr ? __ldg(&nbr[(size_t)k.leaf * kNbr + lane]) : -1;
+    k.on = lane <= (h.x & 31);
+    k.b = k.on ? h.y + lane : h.y;
+    k.off = __ldg(&bvox[k.b]) & 511;
+    return k;
 }
 
-__global__ void k_adj_gather_band(const int* __restrict__ bvox, int nb, const float* __restrict__ phi,
-                                  float* __restrict__ out) {
-    for (int b = blockIdx.x * blockDim.x + threadIdx.x; b < nb; b += gridDim.x * blockDim.x) out[b] = phi[bvox[b]];
+// Resident CTAs of 256 threads per SM of the chunk kernels.
+constexpr int kChunkCtas = 6;
+
+// The chain header -> voxel, foot, neighbour slots -> corners is three trips
+// to memory per chunk, and a band beyond L2 pays DRAM latency for each.  So
+// every warp asks for the lines of the chunk one wave of warps ahead to be
+// brought into L2: its list entries, per-voxel records and neighbour row and,
+// once per leaf, the leaf's part of the pool arrays.
+__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
+
+// Lanes `from` on take the 128-byte lines of [p, p + bytes).
+__device__ __forceinline__ void prefetch_lines(const void* p, int bytes, int lane, int from) {
+    const uintptr_t a = reinterpret_cast<uintptr_t>(p) & ~(uintptr_t)127;
+    const int n = (int)((reinterpret_cast<uintptr_t>(p) + bytes + 127 - a) >> 7);
+    if (lane >= from && lane < from + n) prefetch_l2(reinterpret_cast<const char*>(a) + (lane - from) * 128);
+}
+
+// Leaf offset (0, 1, 2) of local coordinate c in [-8, 15].
+__device__ __forceinline__ int leaf_of(int c) { return (c + 8) >> 3; }
+
+// One forward step over the band voxels, one warp per chunk.  Non-band voxels
+// never change and every state buffer holds phi_0 there from creation, so
+// they are not touched.  chk: the new values in band order (a checkpoint, or
+// phi_K), when not null.  GRAD: the trilinear gradient of src at the foot, in
+// band order (the backward pass's recomputation); dst may then be null.
+//
+// Bound: the latency of header -> voxel, foot, slots -> eight corners (24
+// bytes a voxel from HBM, 28 us at 7.67M band voxels).  One thread per voxel
+// with a neighbour-table load per corner took 121 us there, slots by shuffles
+// 110 us, and 96 us with the next wave's lines prefetched into L2; 2.5 against
+// 3.6 us at 77k voxels (launch-bound).
+template <bool GRAD>
+__global__ void __launch_bounds__(256, kChunkCtas)
+    k_adj_forward(const int2* __restrict__ chunks, int n_chunks, int ahead, const int* __restrict__ bvox,
+                  const int* __restrict__ nbr, const float3* __restrict__ ub, const float* __restrict__ src,
+                  float* __restrict__ dst, float* __restrict__ chk, float3* __restrict__ grad, float s, float hw,
+                  unsigned* err) {
+    const int lane = threadIdx.x & 31;
+    const int c = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    if (c >= n_chunks) return;
+    const Chunk k = load_chunk(__ldg(&chunks[c]), bvox, nbr, lane);
+    const bool more = c + ahead < n_chunks;
+    const int2 ha = more ? __ldg(&chunks[c + ahead]) : make_int2(0, 0);
+    const Foot f = foot_of(ub[k.b], s);
+    int x = (k.off >> 6) + f.fx, y = ((k.off >> 3) & 7) + f.fy, z = (k.off & 7) + f.fz;
+    const bool bad = x < -8 || y < -8 || z < -8 || x > 14 || y > 14 || z > 14;
+    if (bad) x = y = z = 0;
+    const int lx[2] = {leaf_of(x) * 9, leaf_of(x + 1) * 9}, ly[2] = {leaf_of(y) * 3, leaf_of(y + 1) * 3},
+              lz[2] = {leaf_of(z), leaf_of(z + 1)};
+    const int ox[2] = {(x & 7) << 6, ((x + 1) & 7) << 6}, oy[2] = {(y & 7) << 3, ((y + 1) & 7) << 3},
+              oz[2] = {z & 7, (z + 1) & 7};
+    int sl[8];
+    int miss = 0;
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+        sl[q] = __shfl_sync(0xffffffffu, k.row, lx[q >> 2] + ly[(q >> 1) & 1] + lz[q & 1]);
+        miss |= sl[q];
+    }
+    float v[8];
+    if (miss >= 0) {
+#pragma unroll
+        for (int q = 0; q < 8; ++q)
+            v[q] = src[(size_t)sl[q] * kLeafVoxels + (ox[q >> 2] | oy[(q >> 1) & 1] | oz[q & 1])];
+    } else {
+        // a corner in an absent leaf: copysign(hw, the leaf's own value at the clamped position)
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+            if (sl[q] >= 0) {
+                v[q] = src[(size_t)sl[q] * kLeafVoxels + (ox[q >> 2] | oy[(q >> 1) & 1] | oz[q & 1])];
+            } else {
+                const int cx = min(max(x + (q >> 2), 0), 7), cy = min(max(y + ((q >> 1) & 1), 0), 7),
+                          cz = min(max(z + (q & 1), 0), 7);
+                v[q] = copysignf(hw, src[(size_t)k.leaf * kLeafVoxels + ((cx << 6) | (cy << 3) | cz)]);
+            }
+        }
+    }
+    if (more) {
+        const int na = (ha.x & 31) + 1;
+        if (ha.x & 32) prefetch_lines(src + (size_t)(ha.x >> 6) * kLeafVoxels, 2048, lane, 0);
+        prefetch_lines(ub + ha.y, 12 * na, lane, 17);
+        prefetch_lines(bvox + ha.y, 4 * na, lane, 22);
+        prefetch_lines(nbr + (size_t)(ha.x >> 6) * kNbr, 4 * kNbr, lane, 24);
+        if (lane == 31) prefetch_l2(&chunks[min(c + 2 * ahead, n_chunks - 1)]);
+    }
+    const float c00 = v[0] * (1 - f.wx) + v[4] * f.wx, c01 = v[1] * (1 - f.wx) + v[5] * f.wx;
+    const float c10 = v[2] * (1 - f.wx) + v[6] * f.wx, c11 = v[3] * (1 - f.wx) + v[7] * f.wx;
+    const float c0 = c00 * (1 - f.wy) + c10 * f.wy, c1 = c01 * (1 - f.wy) + c11 * f.wy;
+    float val = c0 * (1 - f.wz) + c1 * f.wz;
+    const size_t t = (size_t)k.leaf * kLeafVoxels + k.off;
+    if (bad) {
+        if (k.on) atomicOr(err, kErrReach);
+        val = src[t];
+    }
+    if (!k.on) return;
+    if (dst) dst[t] = val;
+    if (chk) chk[k.b] = val;
+    if constexpr (GRAD) {
+        const float wx[2] = {1 - f.wx, f.wx}, wy[2] = {1 - f.wy, f.wy}, wz[2] = {1 - f.wz, f.wz};
+        grad[k.b] = make_float3(
+            wy[0] * wz[0] * (v[4] - v[0]) + wy[1] * wz[0] * (v[6] - v[2]) + wy[0] * wz[1] * (v[5] - v[1]) +
+                wy[1] * wz[1] * (v[7] - v[3]),
+            wx[0] * wz[0] * (v[2] - v[0]) + wx[1] * wz[0] * (v[6] - v[4]) + wx[0] * wz[1] * (v[3] - v[1]) +
+                wx[1] * wz[1] * (v[7] - v[5]),
+            wx[0] * wy[0] * (v[1] - v[0]) + wx[1] * wy[0] * (v[5] - v[4]) + wx[0] * wy[1] * (v[3] - v[2]) +
+                wx[1] * wy[1] * (v[7] - v[6]));
+    }
 }
 
 __global__ void k_adj_scatter_band(const int* __restrict__ bvox, int nb, const float* __restrict__ in,
@@ -179,290 +294,415 @@ __global__ void k_adj_scatter_band(const int* __restrict__ bvox, int nb, const f
     for (int b = blockIdx.x * blockDim.x + threadIdx.x; b < nb; b += gridDim.x * blockDim.x) phi[bvox[b]] = in[b];
 }
 
-// Band index of the voxel at local (x, y, z) of leaf slot, or n_band (dropped key).
-__device__ __forceinline__ unsigned band_key(const int* __restrict__ nbr, const int* __restrict__ bidx, int slot, int x,
-                                             int y, int z, unsigned nb) {
-    int s = nbr[slot * kNbr + nbx(x) * 9 + nbx(y) * 3 + nbx(z)];
-    if (s < 0) return nb;
-    int b = bidx[(size_t)s * kLeafVoxels + voxel_off(x, y, z)];
-    return b < 0 ? nb : (unsigned)b;
+// A band voxel's foot as the gathers read it: floor offsets packed as three
+// biased 7-bit fields (bit 31 marks a band voxel, other pool voxels hold 0)
+// and the fractions, so a candidate costs one word and a hit one more load,
+// not a chain of band-index, velocity and lambda lookups.
+__device__ __forceinline__ unsigned pack_foot(const Foot& f) {
+    return 0x80000000u | ((unsigned)(f.fx + 64) << 14) | ((unsigned)(f.fy + 64) << 7) | (unsigned)(f.fz + 64);
 }
 
-// Per step k, for every band voxel x: its foot (floor offsets packed as three
-// biased bytes, bit 31 marking a band voxel) and (wx, wy, wz, lambda(x)) in
-// pool order, so the gather below reads one word per candidate instead of a
-// chain of band-index, velocity and lambda lookups.
+// Feet of the band voxels for step factor s; lam (band order) or null: 0.
 __global__ void k_adj_pack(const int* __restrict__ bvox, int nb, const float3* __restrict__ ub,
                            const float* __restrict__ lam, float s, unsigned* __restrict__ foot_pk,
                            float4* __restrict__ foot_w) {
     for (int b = blockIdx.x * blockDim.x + threadIdx.x; b < nb; b += gridDim.x * blockDim.x) {
         const Foot f = foot_of(ub[b], s);
         const int sv = bvox[b];
-        foot_pk[sv] = 0x80000000u | ((unsigned)(f.fx + 64) << 14) | ((unsigned)(f.fy + 64) << 7) |
-                      (unsigned)(f.fz + 64);
-        foot_w[sv] = make_float4(f.wx, f.wy, f.wz, lam[b]);
+        foot_pk[sv] = pack_foot(f);
+        foot_w[sv] = make_float4(f.wx, f.wy, f.wz, lam ? lam[b] : 0.f);
     }
 }
 
-// k_adj_pack for a displacement fixed over the steps (a level set's
-// time-independent velocity): the feet and weights of the first step stand,
-// so later steps write only lambda, the fourth word of each band voxel's
-// foot record.
-__global__ void k_adj_pack_lambda(const int* __restrict__ bvox, int nb, const float* __restrict__ lam,
-                                  float4* __restrict__ foot_w) {
-    float* w = reinterpret_cast<float*>(foot_w);
-    for (int b = blockIdx.x * blockDim.x + threadIdx.x; b < nb; b += gridDim.x * blockDim.x)
-        w[4 * (size_t)bvox[b] + 3] = lam[b];
-}
-
-// Per leaf, the smallest and largest foot offset per axis over its band
-// voxels at this step (empty leaves: min > max).  One warp per leaf.
-__global__ void k_adj_leafrange(const unsigned* __restrict__ foot_pk, int n_leaves, int* __restrict__ lrange) {
+// Per leaf, the smallest and largest velocity (or displacement) component per
+// axis over its band voxels (+inf and -inf without any), one warp per leaf; a
+// NaN counts as 0, the offset its conversion to an integer gives.
+__global__ void k_adj_urange(const float3* __restrict__ ub, const int* __restrict__ lstart, int n_leaves,
+                             float* __restrict__ urange) {
     const int lane = threadIdx.x & 31;
     for (int leaf = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; leaf < n_leaves;
          leaf += (gridDim.x * blockDim.x) >> 5) {
-        int lo[3] = {INT_MAX, INT_MAX, INT_MAX}, hi[3] = {INT_MIN, INT_MIN, INT_MIN};
-        for (int v = lane; v < kLeafVoxels; v += 32) {
-            const unsigned pk = foot_pk[(size_t)leaf * kLeafVoxels + v];
-            if (!(pk >> 31)) continue;
-            const int f[3] = {(int)((pk >> 14) & 127u) - 64, (int)((pk >> 7) & 127u) - 64, (int)(pk & 127u) - 64};
+        float lo[3], hi[3];
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            lo[a] = INFINITY;
+            hi[a] = -INFINITY;
+        }
+        for (int b = lstart[leaf] + lane; b < lstart[leaf + 1]; b += 32) {
+            const float3 u3 = ub[b];
+            const float u[3] = {u3.x, u3.y, u3.z};
 #pragma unroll
             for (int a = 0; a < 3; ++a) {
-                lo[a] = min(lo[a], f[a]);
-                hi[a] = max(hi[a], f[a]);
+                const float v = u[a] == u[a] ? u[a] : 0.f;
+                lo[a] = fminf(lo[a], v);
+                hi[a] = fmaxf(hi[a], v);
             }
         }
 #pragma unroll
-        for (int a = 0; a < 3; ++a) {
-            lo[a] = __reduce_min_sync(0xffffffffu, lo[a]);
-            hi[a] = __reduce_max_sync(0xffffffffu, hi[a]);
-        }
-        if (lane < 3) {
-            lrange[leaf * 6 + lane] = lo[lane];
-            lrange[leaf * 6 + 3 + lane] = hi[lane];
+        for (int a = 0; a < 3; ++a)
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) {
+                lo[a] = fminf(lo[a], __shfl_xor_sync(0xffffffffu, lo[a], o));
+                hi[a] = fmaxf(hi[a], __shfl_xor_sync(0xffffffffu, hi[a], o));
+            }
+        if (lane == 0) {
+#pragma unroll
+            for (int a = 0; a < 3; ++a) {
+                urange[(size_t)leaf * 6 + a] = lo[a];
+                urange[(size_t)leaf * 6 + 3 + a] = hi[a];
+            }
         }
     }
 }
 
-// Per leaf, the window of candidate offsets dx (per axis) for its corners b:
-// a band voxel x = b + dx has b in its foot cell only if dx = -f(x) - {0, 1},
-// f(x) its foot offset; x lies in the 27-leaf neighbourhood (|f| <= R < 8),
-// so dx runs over [-max f - 1, -min f] taken over the neighbourhood's band
-// voxels, within [-1 - R, R].  Empty neighbourhoods get an empty window.
-__global__ void k_adj_window(const int* __restrict__ nbr, const int* __restrict__ lrange, int n_leaves, int R,
-                             int* __restrict__ wrange) {
+// urange folded over each leaf's 27-leaf neighbourhood.
+__global__ void k_adj_nrange(const int* __restrict__ nbr, const float* __restrict__ urange, int n_leaves,
+                             float* __restrict__ nrange) {
     for (int leaf = blockIdx.x * blockDim.x + threadIdx.x; leaf < n_leaves; leaf += gridDim.x * blockDim.x) {
-        int lo[3] = {INT_MAX, INT_MAX, INT_MAX}, hi[3] = {INT_MIN, INT_MIN, INT_MIN};
+        float lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
         for (int d = 0; d < kNbr; ++d) {
             const int s = nbr[(size_t)leaf * kNbr + d];
             if (s < 0) continue;
 #pragma unroll
             for (int a = 0; a < 3; ++a) {
-                lo[a] = min(lo[a], lrange[s * 6 + a]);
-                hi[a] = max(hi[a], lrange[s * 6 + 3 + a]);
+                lo[a] = fminf(lo[a], urange[(size_t)s * 6 + a]);
+                hi[a] = fmaxf(hi[a], urange[(size_t)s * 6 + 3 + a]);
             }
         }
 #pragma unroll
         for (int a = 0; a < 3; ++a) {
-            const bool empty = lo[a] > hi[a];
-            wrange[leaf * 6 + a] = empty ? 1 : max(-hi[a] - 1, -1 - R);
-            wrange[leaf * 6 + 3 + a] = empty ? 0 : min(-lo[a], R);
+            nrange[(size_t)leaf * 6 + a] = lo[a];
+            nrange[(size_t)leaf * 6 + 3 + a] = hi[a];
         }
     }
 }
 
-// Adjoint of step k as a gather, one band voxel b per thread:
-//   G(b)      += lambda(b) s grad trilinear(phi_k)(p(b))      (b's own foot)
+// Candidate offsets [lo, hi] along an axis for the corners of a leaf whose
+// neighbourhood's velocities lie in [ulo, uhi]: a band voxel x = b + dx has b
+// in its foot cell only if dx = -f(x) - {0, 1}, f(x) = floor(s u(x)) its foot
+// offset, and x lies in the 27-leaf neighbourhood (|f| <= R < 8).  Rounding
+// and floor are monotone, so the offsets' extremes are those of s ulo and
+// s uhi.  An empty neighbourhood gives an empty window.
+__device__ __forceinline__ void window_of(float ulo, float uhi, float s, int R, int& lo, int& hi) {
+    if (!(ulo <= uhi)) {
+        lo = 1;
+        hi = 0;
+        return;
+    }
+    const int fa = (int)floorf(s * ulo), fb = (int)floorf(s * uhi);
+    lo = max(-max(fa, fb) - 1, -1 - R);
+    hi = min(-min(fa, fb), R);
+}
+
+// What a step of the backward pass does with lambda_k(b), beyond returning it
+// in band order (out, when not null):
+//   a fixed displacement writes it to the other lam_pool buffer;
+//   a staggered field adds lambda_{k+1}(b) s grad phi_k(p(b)) to G(b) (stores
+//   it on the first step) and packs the feet of the next step (k - 1) into
+//   the other foot buffers.
+struct BackOut {
+    float* out;            // band order, or null
+    float* lam_pool;       // fixed displacement: pool order, or null on the last step
+    const float3* grad;    // staggered: gradient at the feet of this step, band order
+    float3* G;
+    int first;             // staggered: the first step of the backward pass
+    const float3* ub;
+    float s, s_next;
+    unsigned* foot_pk;     // staggered: buffers of the next step, null on the last
+    float4* foot_w;
+};
+
+__device__ __forceinline__ void back_store(const BackOut& o, int b, size_t sv, float lam_own, float lam) {
+    if (o.out) o.out[b] = lam;
+    if (o.lam_pool) o.lam_pool[sv] = lam;
+    if (o.G) {
+        const float3 g = o.grad[b];
+        float3 t = o.first ? make_float3(0.f, 0.f, 0.f) : o.G[b];
+        t.x += lam_own * o.s * g.x;
+        t.y += lam_own * o.s * g.y;
+        t.z += lam_own * o.s * g.z;
+        o.G[b] = t;
+    }
+    if (o.foot_pk) {
+        const Foot f = foot_of(o.ub[b], o.s_next);
+        o.foot_pk[sv] = pack_foot(f);
+        o.foot_w[sv] = make_float4(f.wx, f.wy, f.wz, lam);
+    }
+}
+
+// i, j, k of corner b in candidate x's foot cell as bits 14, 7 and 0, or a
+// word with other bits set when b is no corner of it.  key packs 64 - dx,
+// 64 - dy, 64 - dz like a foot (with bit 31): the difference's fields are
+// b - (x + floor offset), and since they stay within +-14 a field outside
+// {0, 1} leaves some of its bits 1..6 set, borrows included.
+constexpr unsigned kCorner = (1u << 14) | (1u << 7) | 1u;
+__device__ __forceinline__ unsigned cell_key(int dx, int dy, int dz) {
+    return 0x80000000u | ((unsigned)(64 - dx) << 14) | ((unsigned)(64 - dy) << 7) | (unsigned)(64 - dz);
+}
+
+// lambda of the candidate times its weight for the corner, added to acc.
+__device__ __forceinline__ void add_corner(float& acc, unsigned t, const float4& w, float lam) {
+    const float wx = (t >> 14) & 1u ? w.x : 1 - w.x, wy = (t >> 7) & 1u ? w.y : 1 - w.y, wz = t & 1u ? w.z : 1 - w.z;
+    acc += lam * wx * wy * wz;
+}
+
+// Adjoint of step k as a gather:
 //   lambda'(b) = sum over band voxels x of lambda(x) w_b(p(x))  (b as a corner)
 // A step moves a voxel by at most R = reach voxels per axis, so b is a corner
-// of x's foot cell only if x lies in b + [-1-R, R]^3; those candidates are
-// visited in a fixed order (x, then y, then z ascending), each x's foot taken
-// from the same foot_of() as the forward step (through k_adj_pack), so the
-// transpose is exact and the sum order is fixed: deterministic, with no sort
-// and no float atomics.  RT = 1: the whole window [-2, 1]^3, unrolled.  RT =
-// 0: the visit is narrowed to the leaf's window from k_adj_window (offsets
-// outside it cannot hold b as a corner), which keeps the order of the
-// contributing terms, hence the sums, unchanged; smooth fields leave 2-3
-// offsets per axis, against 2R + 2 in the whole window.
-template <int RT>
-__global__ void k_adj_lambda(const int* __restrict__ bvox, int nb, const int* __restrict__ nbr,
-                             const float* __restrict__ phi_k, const unsigned* __restrict__ foot_pk,
-                             const float4* __restrict__ foot_w, float s, float hw, const int* __restrict__ wrange,
-                             float* __restrict__ lam_out, float3* __restrict__ G) {
-    for (int b = blockIdx.x * blockDim.x + threadIdx.x; b < nb; b += gridDim.x * blockDim.x) {
-        const int sv = bvox[b], slot = sv >> 9, off = sv & 511;
-        const int cx = off >> 6, cy = (off >> 3) & 7, cz = off & 7;
-        {
-            const unsigned pk = foot_pk[sv];
-            const float4 w4 = foot_w[sv];
-            const float l = w4.w;
-            const int x = cx + (int)((pk >> 14) & 127u) - 64, y = cy + (int)((pk >> 7) & 127u) - 64,
-                      z = cz + (int)(pk & 127u) - 64;
-            const float wx[2] = {1 - w4.x, w4.x}, wy[2] = {1 - w4.y, w4.y}, wz[2] = {1 - w4.z, w4.z};
-            float c[8];
-#pragma unroll
-            for (int q = 0; q < 8; ++q) c[q] = adj_read(phi_k, nbr, slot, x + (q >> 2), y + ((q >> 1) & 1), z + (q & 1), hw);
-            // c[q] with q = i*4 + j*2 + k
-            float gx = wy[0] * wz[0] * (c[4] - c[0]) + wy[1] * wz[0] * (c[6] - c[2]) + wy[0] * wz[1] * (c[5] - c[1]) +
-                       wy[1] * wz[1] * (c[7] - c[3]);
-            float gy = wx[0] * wz[0] * (c[2] - c[0]) + wx[1] * wz[0] * (c[6] - c[4]) + wx[0] * wz[1] * (c[3] - c[1]) +
-                       wx[1] * wz[1] * (c[7] - c[5]);
-            float gz = wx[0] * wy[0] * (c[1] - c[0]) + wx[1] * wy[0] * (c[5] - c[4]) + wx[0] * wy[1] * (c[3] - c[2]) +
-                       wx[1] * wy[1] * (c[7] - c[6]);
-            float3 g = G[b];
-            g.x += l * s * gx;
-            g.y += l * s * gy;
-            g.z += l * s * gz;
-            G[b] = g;
+// of x's foot cell only if x lies in b + [-1-R, R]^3, and only if it lies in
+// the leaf's window (window_of); those candidates are visited in a fixed order
+// (x, then y, then z ascending, one partial sum per x, added in x order),
+// each x's foot taken from the same foot_of()
+// as the forward step, so the transpose is exact and the sum order fixed:
+// deterministic, with no sort and no float atomics.  Offsets outside the
+// window hold no corner, so the window changes neither the contributing terms
+// nor their order; smooth fields leave 2-3 offsets per axis, against 2R + 2.
+//
+// One warp per chunk of a leaf's band voxels: the window is uniform, a
+// neighbour slot costs a shuffle, and the words of up to three candidates
+// along z are loaded before the first is tested.  Where the neighbourhood has
+// one foot offset (floor(s u) equal at both ends of its range on every axis,
+// the common case of a smooth field), candidate and corner correspond one to
+// one, so no candidate word is read or tested; voxels off the band hold
+// lambda 0 and weight 0 and add nothing.  LAM: lambda read from lam_in (pool
+// order), else from the foot record.
+//
+// Bound: instruction issue and L1 throughput of the 8-27 candidate words and 8
+// hits per voxel (32 bytes a voxel from HBM).  7.67M band voxels of a level
+// set: 373 us one thread per voxel with its own gradient term, 313 us in
+// chunks without it (770 instructions a chunk), 197 us with the untested
+// path, 166 us with the prefetch.
+template <bool LAM>
+__global__ void __launch_bounds__(256, kChunkCtas)
+    k_adj_lambda(const int2* __restrict__ chunks, int n_chunks, int ahead, const int* __restrict__ bvox,
+                 const int* __restrict__ nbr, const float* __restrict__ nrange, const unsigned* __restrict__ foot_pk,
+                 const float4* __restrict__ foot_w, const float* __restrict__ lam_in, int R, BackOut o) {
+    const int lane = threadIdx.x & 31;
+    const int c = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    if (c >= n_chunks) return;
+    const int2 h = __ldg(&chunks[c]);
+    const bool more = c + ahead < n_chunks;
+    const int2 ha = more ? __ldg(&chunks[c + ahead]) : make_int2(0, 0);
+    const Chunk k = load_chunk(h, bvox, nbr, lane);
+    int x0, x1, y0, y1, z0, z1;
+    const float* nr = nrange + (size_t)k.leaf * 6;
+    window_of(__ldg(&nr[0]), __ldg(&nr[3]), o.s, R, x0, x1);
+    window_of(__ldg(&nr[1]), __ldg(&nr[4]), o.s, R, y0, y1);
+    window_of(__ldg(&nr[2]), __ldg(&nr[5]), o.s, R, z0, z1);
+    if (more) {
+        const int na = (ha.x & 31) + 1, leaf = ha.x >> 6;
+        if (ha.x & 32) {
+            const char* w = reinterpret_cast<const char*>(foot_w + (size_t)leaf * kLeafVoxels);
+            prefetch_l2(w + lane * 128);
+            prefetch_l2(w + 4096 + lane * 128);
+            if (LAM) prefetch_lines(lam_in + (size_t)leaf * kLeafVoxels, 2048, lane, 0);
+            prefetch_lines(nrange + (size_t)leaf * 6, 24, lane, 20);
         }
-        const int* nrow = nbr + slot * kNbr;
-        int x0 = -2, y0 = -2, z0 = -2, x1 = 1, y1 = 1, z1 = 1;
-        if (RT == 0) {
-            const int* w6 = wrange + slot * 6;
-            x0 = __ldg(&w6[0]);
-            y0 = __ldg(&w6[1]);
-            z0 = __ldg(&w6[2]);
-            x1 = __ldg(&w6[3]);
-            y1 = __ldg(&w6[4]);
-            z1 = __ldg(&w6[5]);
+        prefetch_lines(bvox + ha.y, 4 * na, lane, 22);
+        prefetch_lines(nbr + (size_t)leaf * kNbr, 4 * kNbr, lane, 24);
+        if (lane == 31) prefetch_l2(&chunks[min(c + 2 * ahead, n_chunks - 1)]);
+    }
+    const int cx = k.off >> 6, cy = (k.off >> 3) & 7, cz = k.off & 7;
+    float acc = 0.f;
+    if (x1 - x0 == 1 && y1 - y0 == 1 && z1 - z0 == 1) {
+        // one foot offset in the neighbourhood: the eight candidates are
+        // the eight corners in order, (1, 1, 1) first
+        unsigned e[8];
+        bool there[8];
+        float plane[2] = {0.f, 0.f};
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+            const int x = cx + x0 + (q >> 2), y = cy + y0 + ((q >> 1) & 1), z = cz + z0 + (q & 1);
+            const int ns = __shfl_sync(0xffffffffu, k.row, leaf_of(x) * 9 + leaf_of(y) * 3 + leaf_of(z));
+            there[q] = ns >= 0;
+            e[q] = (unsigned)ns * kLeafVoxels + (unsigned)voxel_off(x, y, z);
         }
-        float acc = 0.f;
 #pragma unroll
-        for (int dx = x0; dx <= x1; ++dx) {
-            const int x = cx + dx;
+        for (int q = 0; q < 8; ++q) {
+            if (!there[q]) continue;
+            const float4 w = __ldg(&foot_w[e[q]]);
+            const float l = LAM ? __ldg(&lam_in[e[q]]) : w.w;
+            const float wx = q >> 2 ? 1 - w.x : w.x, wy = (q >> 1) & 1 ? 1 - w.y : w.y, wz = q & 1 ? 1 - w.z : w.z;
+            plane[q >> 2] += l * wx * wy * wz;
+        }
+        acc = plane[0] + plane[1];
+        x1 = x0 - 1;  // no candidate left for the general loop
+    }
+    for (int dx = x0; dx <= x1; ++dx) {
+        const int x = cx + dx;
+        float plane = 0.f;
+        for (int dy = y0; dy <= y1; ++dy) {
+            const int y = cy + dy;
+            const int nb2 = leaf_of(x) * 9 + leaf_of(y) * 3;
+            const int o2 = ((x & 7) << 6) | ((y & 7) << 3);
+            for (int dz = z0; dz <= z1; dz += 3) {
+                unsigned t[3], e[3];
 #pragma unroll
-            for (int dy = y0; dy <= y1; ++dy) {
-                const int y = cy + dy;
-                const int nb2 = nbx(x) * 9 + nbx(y) * 3;
-#pragma unroll
-                for (int dz = z0; dz <= z1; ++dz) {
-                    const int z = cz + dz;
-                    const int ns = __ldg(&nrow[nb2 + nbx(z)]);
-                    if (ns < 0) continue;
-                    const size_t e = (size_t)ns * kLeafVoxels + voxel_off(x, y, z);
-                    const unsigned pk = __ldg(&foot_pk[e]);
-                    // corner index of b in x's foot cell: b - (x + floor(offset))
-                    const int i = 64 - dx - (int)((pk >> 14) & 127u), j = 64 - dy - (int)((pk >> 7) & 127u),
-                              k = 64 - dz - (int)(pk & 127u);
-                    if (!(pk >> 31) || (unsigned)i > 1u || (unsigned)j > 1u || (unsigned)k > 1u) continue;
-                    const float4 w4 = __ldg(&foot_w[e]);
-                    const float wx = i ? w4.x : 1 - w4.x, wy = j ? w4.y : 1 - w4.y, wz = k ? w4.z : 1 - w4.z;
-                    acc += w4.w * wx * wy * wz;
+                for (int q = 0; q < 3; ++q) {
+                    const int z = cz + dz + q;
+                    // offsets past the window (up to z1 + 2 <= R + 2 < 9 from the voxel) test nothing
+                    const int ns = __shfl_sync(0xffffffffu, k.row, nb2 + min(leaf_of(z), 2));
+                    e[q] = (unsigned)ns * kLeafVoxels + (unsigned)(o2 | (z & 7));
+                    t[q] = ~0u;
+                    if (ns >= 0 && dz + q <= z1) t[q] = cell_key(dx, dy, dz + q) - __ldg(&foot_pk[e[q]]);
                 }
+#pragma unroll
+                for (int q = 0; q < 3; ++q)
+                    if (!(t[q] & ~kCorner)) {
+                        const float4 w = __ldg(&foot_w[e[q]]);
+                        add_corner(plane, t[q], w, LAM ? __ldg(&lam_in[e[q]]) : w.w);
+                    }
             }
         }
-        lam_out[b] = acc;
+        acc += plane;
     }
+    if (!k.on) return;
+    const size_t sv = (size_t)k.leaf * kLeafVoxels + k.off;
+    back_store(o, k.b, sv, LAM ? 0.f : foot_w[sv].w, acc);
 }
 
-// k_adj_lambda<1> for small bands, four lanes per band voxel: lane q of the
-// quad visits offset dx = q - 2 of the whole window [-2, 1]^3 (dy, dz
-// ascending) and the quad sums its four partial sums in the fixed order
-// ((q0 + q1) + q2) + q3; lane 0 adds b's own gradient term.  Deterministic;
-// the rounding differs from the one-thread order only in how the partial sums
-// associate.  Fills the GPU where one thread per band voxel leaves most warp
-// slots empty.
-__global__ void k_adj_lambda_quad(const int* __restrict__ bvox, int nb, const int* __restrict__ nbr,
-                                  const float* __restrict__ phi_k, const unsigned* __restrict__ foot_pk,
-                                  const float4* __restrict__ foot_w, float s, float hw, float* __restrict__ lam_out,
-                                  float3* __restrict__ G) {
+// k_adj_lambda for small bands and a reach of one voxel, four lanes per band
+// voxel: lane q of the quad visits offset dx = q - 2 of the whole window
+// [-2, 1]^3 (dy, dz ascending) and the quad sums its four partial sums in the
+// fixed order ((q0 + q1) + q2) + q3: k_adj_lambda's sums.  Fills the GPU
+// where one thread per band voxel leaves most warp slots empty; what is left
+// is one chain of loads (voxel, 4 neighbour slots, 16 candidate words, up to
+// 4 foot records), so all of each kind are issued together.
+template <bool LAM>
+__global__ void __launch_bounds__(256) k_adj_lambda_quad(const int* __restrict__ bvox, int nb,
+                                                        const int* __restrict__ nbr,
+                                                        const unsigned* __restrict__ foot_pk,
+                                                        const float4* __restrict__ foot_w,
+                                                        const float* __restrict__ lam_in, BackOut o) {
     const int q = threadIdx.x & 3;
     for (long long gq = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 2; gq < nb;
          gq += ((long long)gridDim.x * blockDim.x) >> 2) {
         const int b = (int)gq;
         const int sv = bvox[b], slot = sv >> 9, off = sv & 511;
-        const int cx = off >> 6, cy = (off >> 3) & 7, cz = off & 7;
-        if (q == 0) {
-            const unsigned pk = foot_pk[sv];
-            const float4 w4 = foot_w[sv];
-            const float l = w4.w;
-            const int x = cx + (int)((pk >> 14) & 127u) - 64, y = cy + (int)((pk >> 7) & 127u) - 64,
-                      z = cz + (int)(pk & 127u) - 64;
-            const float wx[2] = {1 - w4.x, w4.x}, wy[2] = {1 - w4.y, w4.y}, wz[2] = {1 - w4.z, w4.z};
-            float c[8];
+        const int cy = (off >> 3) & 7, cz = off & 7;
+        const int dx = q - 2, x = (off >> 6) + dx;
+        // offsets -2..1 along an axis meet at most two leaves, those of the first and the last
+        const int* nrow = nbr + (size_t)slot * kNbr + leaf_of(x) * 9;
+        const int ya = leaf_of(cy - 2), yb = leaf_of(cy + 1), za = leaf_of(cz - 2), zb = leaf_of(cz + 1);
+        const int s4[4] = {__ldg(&nrow[ya * 3 + za]), __ldg(&nrow[ya * 3 + zb]), __ldg(&nrow[yb * 3 + za]),
+                           __ldg(&nrow[yb * 3 + zb])};
+        unsigned t[16];
 #pragma unroll
-            for (int k = 0; k < 8; ++k) c[k] = adj_read(phi_k, nbr, slot, x + (k >> 2), y + ((k >> 1) & 1), z + (k & 1), hw);
-            float gx = wy[0] * wz[0] * (c[4] - c[0]) + wy[1] * wz[0] * (c[6] - c[2]) + wy[0] * wz[1] * (c[5] - c[1]) +
-                       wy[1] * wz[1] * (c[7] - c[3]);
-            float gy = wx[0] * wz[0] * (c[2] - c[0]) + wx[1] * wz[0] * (c[6] - c[4]) + wx[0] * wz[1] * (c[3] - c[1]) +
-                       wx[1] * wz[1] * (c[7] - c[5]);
-            float gz = wx[0] * wy[0] * (c[1] - c[0]) + wx[1] * wy[0] * (c[5] - c[4]) + wx[0] * wy[1] * (c[3] - c[2]) +
-                       wx[1] * wy[1] * (c[7] - c[6]);
-            float3 g = G[b];
-            g.x += l * s * gx;
-            g.y += l * s * gy;
-            g.z += l * s * gz;
-            G[b] = g;
+        for (int c = 0; c < 16; ++c) {
+            const int dy = (c >> 2) - 2, dz = (c & 3) - 2, y = cy + dy, z = cz + dz;
+            const int u0 = leaf_of(z) == za ? s4[0] : s4[1], u1 = leaf_of(z) == za ? s4[2] : s4[3];
+            const int ns = leaf_of(y) == ya ? u0 : u1;
+            t[c] = ~0u;
+            if (ns >= 0)
+                t[c] = cell_key(dx, dy, dz) - __ldg(&foot_pk[(size_t)ns * kLeafVoxels + voxel_off(x, y, z)]);
         }
-        const int* nrow = nbr + slot * kNbr;
         float acc = 0.f;
-        const int dx = q - 2;
-        const int x = cx + dx;
 #pragma unroll
-        for (int dy = -2; dy <= 1; ++dy) {
-            const int y = cy + dy;
-            const int nb2 = nbx(x) * 9 + nbx(y) * 3;
-#pragma unroll
-            for (int dz = -2; dz <= 1; ++dz) {
-                const int z = cz + dz;
-                const int ns = __ldg(&nrow[nb2 + nbx(z)]);
-                if (ns < 0) continue;
-                const size_t e = (size_t)ns * kLeafVoxels + voxel_off(x, y, z);
-                const unsigned pk = __ldg(&foot_pk[e]);
-                const int i = 64 - dx - (int)((pk >> 14) & 127u), j = 64 - dy - (int)((pk >> 7) & 127u),
-                          k = 64 - dz - (int)(pk & 127u);
-                if (!(pk >> 31) || (unsigned)i > 1u || (unsigned)j > 1u || (unsigned)k > 1u) continue;
-                const float4 w4 = __ldg(&foot_w[e]);
-                const float wx = i ? w4.x : 1 - w4.x, wy = j ? w4.y : 1 - w4.y, wz = k ? w4.z : 1 - w4.z;
-                acc += w4.w * wx * wy * wz;
-            }
+        for (int c = 0; c < 16; ++c) {
+            if (t[c] & ~kCorner) continue;
+            const int y = cy + (c >> 2) - 2, z = cz + (c & 3) - 2;
+            const int u0 = leaf_of(z) == za ? s4[0] : s4[1], u1 = leaf_of(z) == za ? s4[2] : s4[3];
+            const size_t e = (size_t)(leaf_of(y) == ya ? u0 : u1) * kLeafVoxels + voxel_off(x, y, z);
+            const float4 w = __ldg(&foot_w[e]);
+            add_corner(acc, t[c], w, LAM ? __ldg(&lam_in[e]) : w.w);
         }
         // the quad's lanes are consecutive; sum in lane order
         const unsigned qmask = 0xFu << (threadIdx.x & 28);
         const float a1 = __shfl_sync(qmask, acc, (threadIdx.x & 31 & ~3) + 1);
         const float a2 = __shfl_sync(qmask, acc, (threadIdx.x & 31 & ~3) + 2);
         const float a3 = __shfl_sync(qmask, acc, (threadIdx.x & 31 & ~3) + 3);
-        if (q == 0) lam_out[b] = ((acc + a1) + a2) + a3;
+        if (q == 0) back_store(o, b, (size_t)sv, LAM ? 0.f : foot_w[sv].w, ((acc + a1) + a2) + a3);
     }
 }
 
-// Transpose of the upsample: 3 x 8 (node, G_a * weight) pairs per band voxel.
-__global__ void k_adj_emit_vel(const int* __restrict__ bvox, const int4* __restrict__ origin, int nb,
-                               const float3* __restrict__ G, int n, float H, unsigned* __restrict__ keys,
-                               float* __restrict__ vals) {
-    for (int b = blockIdx.x * blockDim.x + threadIdx.x; b < nb; b += gridDim.x * blockDim.x) {
-        const int sv = bvox[b], s = sv >> 9, off = sv & 511;
-        const int4 o = origin[s];
-        const float p[3] = {(float)(o.x + (off >> 6)), (float)(o.y + ((off >> 3) & 7)), (float)(o.z + (off & 7))};
-        const float3 gg = G[b];
-        const float ga[3] = {gg.x, gg.y, gg.z};
-        for (int a = 0; a < 3; ++a) {
-            float g[3] = {p[0] / H, p[1] / H, p[2] / H};
-            for (int q = 0; q < 3; ++q)
-                if (q != a) g[q] -= 0.5f;
-            int i0[3];
-            float w[3];
-            for (int q = 0; q < 3; ++q) {
-                float fl = floorf(g[q]);
-                i0[q] = (int)fl;
-                w[q] = g[q] - fl;
-            }
-            for (int q = 0; q < 8; ++q) {
-                int di = q >> 2, dj = (q >> 1) & 1, dk = q & 1;
-                int i = min(max(i0[0] + di, 0), n - 1), j = min(max(i0[1] + dj, 0), n - 1),
-                    k = min(max(i0[2] + dk, 0), n - 1);
-                float wt = (di ? w[0] : 1 - w[0]) * (dj ? w[1] : 1 - w[1]) * (dk ? w[2] : 1 - w[2]);
-                size_t e = ((size_t)b * 3 + a) * 8 + q;
-                keys[e] = (unsigned)((size_t)a * n * n * n + ((size_t)i * n + j) * n + k);
-                vals[e] = ga[a] * wt;
-            }
+// Transpose of the upsample.  Entry e = (b * 3 + a) * 8 + q is corner q of
+// component a at band voxel b: its node, and its weight there.
+__device__ __forceinline__ unsigned vel_entry(const int* __restrict__ bvox, const int4* __restrict__ origin, int e,
+                                              int n, float H, float* wt) {
+    const int b = e / 24, a = (e >> 3) % 3, q = e & 7;
+    const int sv = bvox[b], off = sv & 511;
+    const int4 o = origin[sv >> 9];
+    float g[3] = {(float)(o.x + (off >> 6)) / H, (float)(o.y + ((off >> 3) & 7)) / H, (float)(o.z + (off & 7)) / H};
+    int node[3];
+    float w = 1.f;
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+        if (c != a) g[c] -= 0.5f;
+        const float fl = floorf(g[c]);
+        const float f = g[c] - fl;
+        const int d = (q >> (2 - c)) & 1;
+        node[c] = min(max((int)fl + d, 0), n - 1);
+        w *= d ? f : 1 - f;
+    }
+    *wt = w;
+    return (unsigned)((size_t)a * n * n * n + ((size_t)node[0] * n + node[1]) * n + node[2]);
+}
+
+__global__ void k_adj_vel_keys(const int* __restrict__ bvox, const int4* __restrict__ origin, int ne, int n, float H,
+                               unsigned* __restrict__ keys, unsigned* __restrict__ ids) {
+    for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < ne; e += gridDim.x * blockDim.x) {
+        float w;
+        keys[e] = vel_entry(bvox, origin, e, n, H, &w);
+        ids[e] = (unsigned)e;
+    }
+}
+
+// Sorted entries -> source (b * 3 + a) and weight; head = 1 where a node starts.
+__global__ void k_adj_vel_entries(const int* __restrict__ bvox, const int4* __restrict__ origin, int ne, int n,
+                                  float H, const unsigned* __restrict__ keys, const unsigned* __restrict__ ids,
+                                  int* __restrict__ ent_b, float* __restrict__ ent_w, int* __restrict__ head) {
+    for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < ne; j += gridDim.x * blockDim.x) {
+        const int e = (int)ids[j];
+        float w;
+        vel_entry(bvox, origin, e, n, H, &w);
+        ent_b[j] = e >> 3;
+        ent_w[j] = w;
+        head[j] = j == 0 || keys[j] != keys[j - 1];
+    }
+}
+
+__global__ void k_adj_vel_segments(const unsigned* __restrict__ keys, const int* __restrict__ head,
+                                   const int* __restrict__ rank, int ne, int* __restrict__ seg_start,
+                                   unsigned* __restrict__ seg_node) {
+    for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < ne; j += gridDim.x * blockDim.x)
+        if (head[j]) {
+            seg_start[rank[j]] = j;
+            seg_node[rank[j]] = keys[j];
         }
+}
+
+// dL/dV: eight lanes per node sum its entries (lane l takes entries l, l + 8,
+// ...; the eight partial sums are folded by xor shuffles): a fixed order.
+__global__ void k_adj_vel_sum(const int* __restrict__ seg_start, const unsigned* __restrict__ seg_node, int n_seg,
+                              const int* __restrict__ ent_b, const float* __restrict__ ent_w,
+                              const float* __restrict__ G, float* __restrict__ out) {
+    const int l = threadIdx.x & 7;
+    for (int base = (blockIdx.x * blockDim.x + threadIdx.x) >> 3; (base & ~3) < n_seg;
+         base += (gridDim.x * blockDim.x) >> 3) {
+        const bool on = base < n_seg;
+        const int e0 = on ? seg_start[base] : 0, e1 = on ? seg_start[base + 1] : 0;
+        float s = 0.f;
+        for (int e = e0 + l; e < e1; e += 8) s += G[ent_b[e]] * ent_w[e];
+#pragma unroll
+        for (int d = 4; d > 0; d >>= 1) s += __shfl_xor_sync(0xffffffffu, s, d);
+        if (on && l == 0) out[seg_node[base]] = s;
     }
 }
 
-__global__ void k_zero3(float3* a, int n) {
+// Chunks of the band list: leaf i's band voxels [lstart[i], lstart[i + 1])
+// in groups of 32; cnt = groups per leaf, pos = their exclusive sum.
+__global__ void k_adj_chunk_count(const int* __restrict__ lstart, int n, int* __restrict__ cnt) {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-        a[i] = make_float3(0.f, 0.f, 0.f);
+        cnt[i] = (lstart[i + 1] - lstart[i] + 31) >> 5;
+}
+
+__global__ void k_adj_chunk_fill(const int* __restrict__ lstart, const int* __restrict__ pos, int n,
+                                 int2* __restrict__ chunks) {
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        int j = pos[i];
+        const int e = lstart[i + 1];
+        for (int b = lstart[i]; b < e; b += 32) chunks[j++] = make_int2(i << 6 | (b == lstart[i] ? 32 : 0) | (min(e - b, 32) - 1), b);
+    }
 }
 
 __global__ void k_adj_hash_insert(const int4* origin, int n, uint64_t* hkey, int* hval, int hcap, long long b0,
@@ -518,8 +758,9 @@ void adj_drop_graphs(vlr_adjoint* a) {
 void adj_free(vlr_adjoint* a) {
     adj_drop_graphs(a);
     void* ptrs[] = {a->origin, a->nbr, a->hkey, a->hval, a->phi[0], a->phi[1], a->phi_init, a->bidx, a->bvox,
-                    a->ub, a->vel, a->checkpoints, a->segment, a->lam[0], a->lam[1], a->G, a->keys, a->pvals,
-                    a->scratch, a->gvel, a->foot_pk, a->foot_w, a->lrange, a->wrange};
+                    a->ub, a->vel, a->checkpoints, a->segment, a->lam[0], a->lam[1], a->G, a->gvel, a->lstart,
+                    a->chunks, a->urange, a->nrange, a->foot_pk[0], a->foot_pk[1], a->foot_w[0], a->foot_w[1],
+                    a->lam_pool[0], a->lam_pool[1], a->ent_b, a->ent_w, a->seg_start, a->seg_node};
     for (void* p : ptrs) cudaFree(p);
 }
 
@@ -539,110 +780,199 @@ float step_factor(const vlr_adjoint* a, int k) {
     return (float)(-a->dt * std::cos(pi * t1 / a->period));
 }
 
-int enqueue_forward_step(vlr_ctx* ctx, vlr_adjoint* a, int k, const float* src, float* dst) {
-    VLR_TIMED(ctx, "k_adj_forward",
-              k_adj_forward<<<blocks_for(ctx, a->n_band), 256, 0, ctx->stream>>>(
-                  a->bvox, a->n_band, a->nbr, a->ub, src, dst, step_factor(a, k), a->hw, ctx->d_errword));
-    VLR_CUDA(ctx, cudaGetLastError());
-    return VLR_OK;
-}
+// CTAs of 256 threads (8 warps) for the chunk kernels, one chunk a warp (a
+// persistent grid with the next chunk's loads held in registers spilled: the
+// forward kernel 150 us against 110), and the chunks of one wave of warps.
+int chunk_blocks(const vlr_adjoint* a) { return (a->n_chunks + 7) / 8; }
+int chunk_wave(const vlr_ctx* ctx) { return ctx->sm_count * kChunkCtas * 8; }
 
-// The forward step loop from the initial state (checkpoints every C steps;
-// phi_K on the band into lam[1]), enqueued without waiting.
-int adj_forward_enqueue(vlr_ctx* ctx, vlr_adjoint* a) {
+// Step k from src into dst (and, in band order, into chk); with grad the
+// gradient of src at the feet too.
+int enqueue_forward_step(vlr_ctx* ctx, vlr_adjoint* a, int k, const float* src, float* dst, float* chk,
+                         float3* grad) {
     cudaStream_t st = ctx->stream;
-    const size_t nb = (size_t)a->n_band;
-    // both state buffers start as phi_0 (the steps rewrite band voxels only)
-    VLR_CUDA(ctx, cudaMemcpyAsync(a->phi[0], a->phi_init, sizeof(float) * 512 * a->n_leaves, cudaMemcpyDeviceToDevice,
-                                  st));
-    VLR_CUDA(ctx, cudaMemcpyAsync(a->phi[1], a->phi_init, sizeof(float) * 512 * a->n_leaves, cudaMemcpyDeviceToDevice,
-                                  st));
-    int cur = 0;
-    for (int k = 0; k < a->steps; ++k) {
-        if (k % a->chk_every == 0)
-            k_adj_gather_band<<<blocks_for(ctx, nb), 256, 0, st>>>(a->bvox, (int)nb, a->phi[cur],
-                                                                   a->checkpoints + (size_t)(k / a->chk_every) * nb);
-        int rc = enqueue_forward_step(ctx, a, k, a->phi[cur], a->phi[1 - cur]);
-        if (rc) return rc;
-        cur = 1 - cur;
-    }
-    k_adj_gather_band<<<blocks_for(ctx, nb), 256, 0, st>>>(a->bvox, (int)nb, a->phi[cur], a->lam[1]);
+    const int B = chunk_blocks(a);
+    if (grad)
+        VLR_TIMED(ctx, "k_adj_forward",
+                  k_adj_forward<true><<<B, 256, 0, st>>>(a->chunks, a->n_chunks, chunk_wave(ctx), a->bvox, a->nbr, a->ub, src,
+                                                         dst, chk, grad, step_factor(a, k), a->hw, ctx->d_errword));
+    else
+        VLR_TIMED(ctx, "k_adj_forward",
+                  k_adj_forward<false><<<B, 256, 0, st>>>(a->chunks, a->n_chunks, chunk_wave(ctx), a->bvox, a->nbr, a->ub,
+                                                          src, dst, chk, nullptr, step_factor(a, k), a->hw,
+                                                          ctx->d_errword));
     VLR_CUDA(ctx, cudaGetLastError());
     return VLR_OK;
 }
 
-// The backward step loop from lambda_K in lam[1] (recompute from checkpoints,
-// gather transpose, G accumulation), enqueued without waiting; records the
-// lam buffer it ends in.
+// The forward step loop from the initial state, enqueued without waiting:
+// phi_K on the band into lam[1], and for a staggered field phi_k at every
+// multiple of C (but 0, which is phi_init) into the checkpoints.  Step 0 reads
+// phi_init; both state buffers hold its non-band values from creation.
+int adj_forward_enqueue(vlr_ctx* ctx, vlr_adjoint* a) {
+    const size_t nb = (size_t)a->n_band;
+    const float* src = a->phi_init;
+    for (int k = 0; k < a->steps; ++k) {
+        float* dst = a->phi[k & 1];
+        float* chk = nullptr;
+        if (k + 1 == a->steps) chk = a->lam[1];
+        else if (!a->disp && (k + 1) % a->chk_every == 0) chk = a->checkpoints + (size_t)((k + 1) / a->chk_every) * nb;
+        int rc = enqueue_forward_step(ctx, a, k, src, dst, chk, nullptr);
+        if (rc) return rc;
+        src = dst;
+    }
+    return VLR_OK;
+}
+
+// One step of the lambda recursion, from foot buffer `cur` (and lam_pool cur).
+int enqueue_lambda_step(vlr_ctx* ctx, vlr_adjoint* a, int cur, const BackOut& o) {
+    cudaStream_t st = ctx->stream;
+    const int nb = a->n_band;
+    const unsigned* pk = a->foot_pk[a->disp ? 0 : cur];
+    const float4* w = a->foot_w[a->disp ? 0 : cur];
+    // The quad wins while its voxels fit one wave (4 CTAs of 64 voxels per SM,
+    // 37,888 here): 10.7 against 14.7 us a launch at 30,368 band voxels, even
+    // at 47,354 (14.5, 14.7), behind from there (16.8, 14.7 at 77,406; 65, 31
+    // at 644,824).  It covers a reach of one voxel only.
+    if (a->gather == 2 || (a->gather == 0 && a->reach == 1 && nb <= ctx->sm_count * 4 * 64)) {
+        const int B = blocks_for(ctx, 4ll * nb);
+        if (a->disp)
+            VLR_TIMED(ctx, "k_adj_lambda", k_adj_lambda_quad<true><<<B, 256, 0, st>>>(a->bvox, nb, a->nbr, pk, w,
+                                                                                      a->lam_pool[cur], o));
+        else
+            VLR_TIMED(ctx, "k_adj_lambda", k_adj_lambda_quad<false><<<B, 256, 0, st>>>(a->bvox, nb, a->nbr, pk, w,
+                                                                                       nullptr, o));
+    } else {
+        const int B = chunk_blocks(a);
+        if (a->disp)
+            VLR_TIMED(ctx, "k_adj_lambda",
+                      k_adj_lambda<true><<<B, 256, 0, st>>>(a->chunks, a->n_chunks, chunk_wave(ctx), a->bvox, a->nbr,
+                                                            a->nrange, pk, w, a->lam_pool[cur], a->reach, o));
+        else
+            VLR_TIMED(ctx, "k_adj_lambda",
+                      k_adj_lambda<false><<<B, 256, 0, st>>>(a->chunks, a->n_chunks, chunk_wave(ctx), a->bvox, a->nbr,
+                                                             a->nrange, pk, w, nullptr, a->reach, o));
+    }
+    VLR_CUDA(ctx, cudaGetLastError());
+    return VLR_OK;
+}
+
+// The backward step loop from lambda_K in lam[1] to lambda_0 in lam[0] (and,
+// for a staggered field, G), enqueued without waiting.
 int adj_backward_enqueue(vlr_ctx* ctx, vlr_adjoint* a) {
     cudaStream_t st = ctx->stream;
-    const size_t nb = (size_t)a->n_band;
-    float* lam = a->lam[1];
-    k_zero3<<<blocks_for(ctx, nb), 256, 0, st>>>(a->G, (int)nb);
-    const int C = a->chk_every;
-    for (int seg = (a->steps - 1) / C; seg >= 0; --seg) {
-        const int k0 = seg * C, k1 = std::min(a->steps, k0 + C);
-        // recompute phi_k0 .. phi_{k1-1} from the checkpoint
-        VLR_CUDA(ctx, cudaMemcpyAsync(a->phi[0], a->phi_init, sizeof(float) * 512 * a->n_leaves,
-                                      cudaMemcpyDeviceToDevice, st));
-        k_adj_scatter_band<<<blocks_for(ctx, nb), 256, 0, st>>>(a->bvox, (int)nb, a->checkpoints + (size_t)seg * nb,
-                                                                a->phi[0]);
-        VLR_CUDA(ctx, cudaMemcpyAsync(a->phi[1], a->phi[0], sizeof(float) * 512 * a->n_leaves,
-                                      cudaMemcpyDeviceToDevice, st));
-        int cur = 0;
-        for (int k = k0; k < k1; ++k) {
-            k_adj_gather_band<<<blocks_for(ctx, nb), 256, 0, st>>>(a->bvox, (int)nb, a->phi[cur],
-                                                                   a->segment + (size_t)(k - k0) * nb);
-            if (k + 1 < k1) {
-                int rc = enqueue_forward_step(ctx, a, k, a->phi[cur], a->phi[1 - cur]);
-                if (rc) return rc;
-                cur = 1 - cur;
-            }
+    const int nb = a->n_band, K = a->steps, C = a->chk_every;
+    int cur = 0;
+    BackOut o = {};
+    if (a->disp) {
+        // fixed feet (packed at creation): the recursion is linear in lambda alone
+        k_adj_scatter_band<<<blocks_for(ctx, nb), 256, 0, st>>>(a->bvox, nb, a->lam[1], a->lam_pool[0]);
+        o.s = 1.0f;
+        for (int k = K - 1; k >= 0; --k, cur ^= 1) {
+            o.out = k == 0 ? a->lam[0] : nullptr;
+            o.lam_pool = k == 0 ? nullptr : a->lam_pool[cur ^ 1];
+            int rc = enqueue_lambda_step(ctx, a, cur, o);
+            if (rc) return rc;
         }
-        // adjoint steps k1-1 .. k0: phi_k from the segment (scattered into a full pool)
-        for (int k = k1 - 1; k >= k0; --k) {
-            k_adj_scatter_band<<<blocks_for(ctx, nb), 256, 0, st>>>(a->bvox, (int)nb,
-                                                                    a->segment + (size_t)(k - k0) * nb, a->phi[0]);
-            float* lam_out = (lam == a->lam[1]) ? a->lam[0] : a->lam[1];
-            const float sk = step_factor(a, k);
-            // a fixed displacement keeps the feet, their weights and the
-            // leaves' windows of the backward pass's first step
-            const bool feet_stand = a->disp && k != a->steps - 1;
-            if (feet_stand)
-                VLR_TIMED(ctx, "k_adj_pack",
-                          k_adj_pack_lambda<<<blocks_for(ctx, nb), 256, 0, st>>>(a->bvox, (int)nb, lam, a->foot_w));
-            else
-                VLR_TIMED(ctx, "k_adj_pack",
-                          k_adj_pack<<<blocks_for(ctx, nb), 256, 0, st>>>(a->bvox, (int)nb, a->ub, lam, sk,
-                                                                          a->foot_pk, a->foot_w));
-            const int gb = blocks_for(ctx, nb);
-            const int nl = a->n_leaves;
-            // the narrowed window pays when the whole window is large (reach >= 2)
-            // or the band is, where its two small per-leaf passes are cheap
-            if (a->gather == 2 || (a->gather == 0 && a->reach == 1 && nb < (1u << 20))) {
-                // small band: a quad of lanes per band voxel fills the GPU
-                VLR_TIMED(ctx, "k_adj_lambda",
-                          k_adj_lambda_quad<<<blocks_for(ctx, 4ll * nb), 256, 0, st>>>(
-                              a->bvox, (int)nb, a->nbr, a->phi[0], a->foot_pk, a->foot_w, sk, a->hw, lam_out, a->G));
-            } else {
-                if (!feet_stand) {
-                    VLR_TIMED(ctx, "k_adj_leafrange",
-                              k_adj_leafrange<<<blocks_for(ctx, 32ll * nl), 256, 0, st>>>(a->foot_pk, nl, a->lrange));
-                    VLR_TIMED(ctx, "k_adj_window",
-                              k_adj_window<<<blocks_for(ctx, nl), 256, 0, st>>>(a->nbr, a->lrange, nl, a->reach,
-                                                                                a->wrange));
-                }
-                VLR_TIMED(ctx, "k_adj_lambda",
-                          k_adj_lambda<0><<<gb, 256, 0, st>>>(a->bvox, (int)nb, a->nbr, a->phi[0], a->foot_pk,
-                                                              a->foot_w, sk, a->hw, a->wrange, lam_out, a->G));
-            }
-            lam = lam_out;
-        }
-        (void)cur;
+        return VLR_OK;
     }
-    VLR_CUDA(ctx, cudaGetLastError());
-    a->bwd_final = lam;
+    VLR_TIMED(ctx, "k_adj_pack",
+              k_adj_pack<<<blocks_for(ctx, nb), 256, 0, st>>>(a->bvox, nb, a->ub, a->lam[1], step_factor(a, K - 1),
+                                                              a->foot_pk[0], a->foot_w[0]));
+    o.G = a->G;
+    o.ub = a->ub;
+    for (int seg = (K - 1) / C; seg >= 0; --seg) {
+        const int k0 = seg * C, k1 = std::min(K, k0 + C);
+        // gradients of phi_k0 .. phi_{k1-1} at the feet, recomputing the states from the checkpoint
+        const float* src = a->phi_init;
+        if (seg) {
+            k_adj_scatter_band<<<blocks_for(ctx, nb), 256, 0, st>>>(a->bvox, nb, a->checkpoints + (size_t)seg * nb,
+                                                                    a->phi[1]);
+            src = a->phi[1];
+        }
+        for (int k = k0; k < k1; ++k) {
+            float* dst = a->phi[(k - k0) & 1];
+            int rc = enqueue_forward_step(ctx, a, k, src, k + 1 < k1 ? dst : nullptr, nullptr,
+                                          a->segment + (size_t)(k - k0) * nb);
+            if (rc) return rc;
+            src = dst;
+        }
+        for (int k = k1 - 1; k >= k0; --k, cur ^= 1) {
+            o.out = k == 0 ? a->lam[0] : nullptr;
+            o.grad = a->segment + (size_t)(k - k0) * nb;
+            o.first = k == K - 1;
+            o.s = step_factor(a, k);
+            o.s_next = k ? step_factor(a, k - 1) : 0.f;
+            o.foot_pk = k ? a->foot_pk[cur ^ 1] : nullptr;
+            o.foot_w = k ? a->foot_w[cur ^ 1] : nullptr;
+            int rc = enqueue_lambda_step(ctx, a, cur, o);
+            if (rc) return rc;
+        }
+    }
     return VLR_OK;
+}
+
+// Velocity ranges of the leaves and of their neighbourhoods, from ub.
+int enqueue_ranges(vlr_ctx* ctx, vlr_adjoint* a) {
+    const int n = a->n_leaves;
+    k_adj_urange<<<blocks_for(ctx, 32ll * n), 256, 0, ctx->stream>>>(a->ub, a->lstart, n, a->urange);
+    k_adj_nrange<<<blocks_for(ctx, n), 256, 0, ctx->stream>>>(a->nbr, a->urange, n, a->nrange);
+    VLR_CUDA(ctx, cudaGetLastError());
+    return VLR_OK;
+}
+
+// The chunk list from lstart (synchronises; allocates a->chunks).
+int make_chunks(vlr_ctx* ctx, vlr_adjoint* a) {
+    const int n = a->n_leaves;
+    int* cnt = nullptr;
+    VLR_CUDA(ctx, cudaMallocFromPoolAsync(&cnt, sizeof(int) * (2 * (size_t)n + 1), ctx->pool, ctx->stream));
+    int* pos = cnt + n;
+    k_adj_chunk_count<<<blocks_for(ctx, n), 256, 0, ctx->stream>>>(a->lstart, n, cnt);
+    int rc = scan_exclusive(ctx, cnt, pos, n, pos + n);
+    if (!rc) rc = read_int(ctx, pos + n, &a->n_chunks);
+    cudaError_t e = rc ? cudaSuccess : cudaMalloc(&a->chunks, sizeof(int2) * std::max(a->n_chunks, 1));
+    if (!rc && e == cudaSuccess) {
+        k_adj_chunk_fill<<<blocks_for(ctx, n), 256, 0, ctx->stream>>>(a->lstart, pos, n, a->chunks);
+        e = cudaGetLastError();
+    }
+    cudaFreeAsync(cnt, ctx->stream);
+    return rc || e == cudaSuccess ? rc : check_cuda(ctx, e, "adjoint chunk list");
+}
+
+// The sorted entries of upsample^T (synchronises; allocates them).
+int make_vel_entries(vlr_ctx* ctx, vlr_adjoint* a) {
+    cudaStream_t st = ctx->stream;
+    const int ne = a->n_band * 24, n = a->n_stag, B = blocks_for(ctx, ne);
+    const float H = (float)a->H;
+    // temporaries in one block of the context's pool
+    const size_t sb = (sort_reduce_scratch_bytes(ne) + 255) & ~(size_t)255;
+    char* blk = nullptr;
+    VLR_CUDA(ctx, cudaMallocFromPoolAsync((void**)&blk, sb + sizeof(int) * (4 * (size_t)ne + 1), ctx->pool, st));
+    unsigned* keys = (unsigned*)(blk + sb);
+    unsigned* ids = keys + ne;
+    int* head = (int*)(ids + ne);
+    int* rank = head + ne;
+    unsigned *ks = nullptr, *is = nullptr;
+    auto make = [&]() -> int {
+        VLR_CUDA(ctx, cudaMalloc(&a->ent_b, sizeof(int) * ne));
+        VLR_CUDA(ctx, cudaMalloc(&a->ent_w, sizeof(float) * ne));
+        k_adj_vel_keys<<<B, 256, 0, st>>>(a->bvox, a->origin, ne, n, H, keys, ids);
+        int rc = radix_sort_pairs(ctx, keys, ids, ne, 3u * n * n * n, blk, &ks, &is);
+        if (rc) return rc;
+        k_adj_vel_entries<<<B, 256, 0, st>>>(a->bvox, a->origin, ne, n, H, ks, is, a->ent_b, a->ent_w, head);
+        rc = scan_exclusive(ctx, head, rank, ne, rank + ne);
+        if (!rc) rc = read_int(ctx, rank + ne, &a->n_seg);
+        if (rc) return rc;
+        VLR_CUDA(ctx, cudaMalloc(&a->seg_start, sizeof(int) * ((size_t)a->n_seg + 1)));
+        VLR_CUDA(ctx, cudaMalloc(&a->seg_node, sizeof(unsigned) * a->n_seg));
+        k_adj_vel_segments<<<B, 256, 0, st>>>(ks, head, rank, ne, a->seg_start, a->seg_node);
+        VLR_CUDA(ctx, cudaMemcpyAsync(a->seg_start + a->n_seg, &ne, sizeof(int), cudaMemcpyHostToDevice, st));
+        VLR_CUDA(ctx, cudaGetLastError());
+        return VLR_OK;
+    };
+    const int rc = make();
+    cudaFreeAsync(blk, st);
+    return rc;
 }
 
 // Run `enqueue` through a CUDA graph captured on first use (or directly while
@@ -783,7 +1113,6 @@ int vlr_adj_create_level_set(vlr_ctx* ctx, vlr_level_set* ls, int steps, int che
         return fail(rc ? rc : set_error(ctx, VLR_ERR_INVALID, "empty band"));
     }
     a->n_band = nb;
-    const int n_chk = steps / checkpoint_every + 1;
     a->hcap = 64;
     while ((size_t)a->hcap < 2 * (size_t)n) a->hcap <<= 1;
     ADJ_MALLOC(a->bvox, sizeof(int) * nb);
@@ -793,17 +1122,23 @@ int vlr_adj_create_level_set(vlr_ctx* ctx, vlr_level_set* ls, int steps, int che
     ADJ_MALLOC(a->phi[0], sizeof(float) * pool);
     ADJ_MALLOC(a->phi[1], sizeof(float) * pool);
     ADJ_MALLOC(a->ub, sizeof(float3) * nb);
-    ADJ_MALLOC(a->checkpoints, sizeof(float) * (size_t)nb * n_chk);
-    ADJ_MALLOC(a->segment, sizeof(float) * (size_t)nb * checkpoint_every);
     ADJ_MALLOC(a->lam[0], sizeof(float) * nb);
     ADJ_MALLOC(a->lam[1], sizeof(float) * nb);
-    ADJ_MALLOC(a->G, sizeof(float3) * nb);
-    ADJ_MALLOC(a->foot_pk, sizeof(unsigned) * pool);
-    ADJ_MALLOC(a->foot_w, sizeof(float4) * pool);
-    ADJ_MALLOC(a->lrange, sizeof(int) * 6 * (size_t)n);
-    ADJ_MALLOC(a->wrange, sizeof(int) * 6 * (size_t)n);
+    ADJ_MALLOC(a->lstart, sizeof(int) * ((size_t)n + 1));
+    ADJ_MALLOC(a->foot_pk[0], sizeof(unsigned) * pool);
+    ADJ_MALLOC(a->foot_w[0], sizeof(float4) * pool);
+    ADJ_MALLOC(a->lam_pool[0], sizeof(float) * pool);
+    ADJ_MALLOC(a->lam_pool[1], sizeof(float) * pool);
+    ADJ_MALLOC(a->urange, sizeof(float) * 6 * (size_t)n);
+    ADJ_MALLOC(a->nrange, sizeof(float) * 6 * (size_t)n);
 #undef ADJ_MALLOC
-    VLR_CUDA(ctx, cudaMemsetAsync(a->foot_pk, 0, sizeof(unsigned) * pool, st));
+    for (float* p : a->phi)
+        VLR_CUDA(ctx, cudaMemcpyAsync(p, a->phi_init, sizeof(float) * pool, cudaMemcpyDeviceToDevice, st));
+    VLR_CUDA(ctx, cudaMemcpyAsync(a->lstart, pos, sizeof(int) * ((size_t)n + 1), cudaMemcpyDeviceToDevice, st));
+    VLR_CUDA(ctx, cudaMemsetAsync(a->foot_pk[0], 0, sizeof(unsigned) * pool, st));
+    // off the band: weight 0, lambda 0
+    VLR_CUDA(ctx, cudaMemsetAsync(a->foot_w[0], 0, sizeof(float4) * pool, st));
+    for (float* p : a->lam_pool) VLR_CUDA(ctx, cudaMemsetAsync(p, 0, sizeof(float) * pool, st));
     VLR_CUDA(ctx, cudaMemsetAsync(a->hkey, 0xFF, sizeof(uint64_t) * a->hcap, st));  // kEmptyKey
     k_adjls_band<<<gb, 512, 0, st>>>(ls->list, n, ls->mask, pos, a->bidx, a->bvox);
     k_adj_hash_insert<<<(n + 255) / 256, 256, 0, st>>>(a->origin, n, a->hkey, a->hval, a->hcap, a->base[0], a->base[1],
@@ -820,6 +1155,14 @@ int vlr_adj_create_level_set(vlr_ctx* ctx, vlr_level_set* ls, int steps, int che
                                                     (float)ls->sp.dt, ls->sp.integrator, a->ub, d_max,
                                                     ctx->d_errword);
     VLR_CUDA(ctx, cudaGetLastError());
+    // the displacement is fixed: its feet, ranges and chunks stand for every pass
+    k_adj_pack<<<blocks_for(ctx, nb), 256, 0, st>>>(a->bvox, nb, a->ub, nullptr, 1.0f, a->foot_pk[0], a->foot_w[0]);
+    rc = enqueue_ranges(ctx, a);
+    if (!rc) rc = make_chunks(ctx, a);
+    if (rc) {
+        cudaFree(cnt);
+        return fail(rc);
+    }
     unsigned mbits = 0;
     VLR_CUDA(ctx, cudaMemcpyAsync(&mbits, d_max, sizeof(unsigned), cudaMemcpyDeviceToHost, st));
     cudaError_t e = cudaStreamSynchronize(st);
@@ -890,13 +1233,16 @@ int vlr_adj_create(vlr_ctx* ctx, const int32_t* origins, const uint64_t* masks, 
     int rc = choose_base(ctx, origins, n_leaves, a->base);
     if (rc) return fail(rc);
     // band: active voxels, in leaf order then ZYX
-    std::vector<int> bidx(n_leaves * 512, -1), bvox;
-    for (size_t i = 0; i < n_leaves; ++i)
+    std::vector<int> bidx(n_leaves * 512, -1), bvox, lstart;
+    for (size_t i = 0; i < n_leaves; ++i) {
+        lstart.push_back((int)bvox.size());
         for (int off = 0; off < 512; ++off)
             if ((masks[8 * i + (off >> 6)] >> (off & 63)) & 1ull) {
                 bidx[i * 512 + off] = (int)bvox.size();
                 bvox.push_back((int)(i * 512 + off));
             }
+    }
+    lstart.push_back((int)bvox.size());
     a->n_band = (int)bvox.size();
     if (a->n_band == 0) return fail(set_error(ctx, VLR_ERR_INVALID, "empty band"));
     const size_t nb = (size_t)a->n_band;
@@ -906,7 +1252,7 @@ int vlr_adj_create(vlr_ctx* ctx, const int32_t* origins, const uint64_t* masks, 
     for (size_t i = 0; i < n_leaves; ++i) o4[i] = make_int4(origins[3 * i], origins[3 * i + 1], origins[3 * i + 2], 0);
     size_t nvel = 3ull * n_stag * n_stag * n_stag;
     int n_chk = steps / checkpoint_every + 1;
-    a->n_pairs_cap = std::max(nb * 8, nb * 24);
+    if (nb > (size_t)INT32_MAX / 24) return fail(set_error(ctx, VLR_ERR_CAPACITY, "band too large for a staggered adjoint"));
 #define ADJ_MALLOC(p, bytes) \
     do { cudaError_t e_ = cudaMalloc(&(p), (bytes)); if (e_ != cudaSuccess) return fail(check_cuda(ctx, e_, "cudaMalloc")); } while (0)
     ADJ_MALLOC(a->origin, sizeof(int4) * n_leaves);
@@ -921,23 +1267,29 @@ int vlr_adj_create(vlr_ctx* ctx, const int32_t* origins, const uint64_t* masks, 
     ADJ_MALLOC(a->ub, sizeof(float3) * nb);
     ADJ_MALLOC(a->vel, sizeof(float) * nvel);
     ADJ_MALLOC(a->checkpoints, sizeof(float) * nb * n_chk);
-    ADJ_MALLOC(a->segment, sizeof(float) * nb * checkpoint_every);
+    ADJ_MALLOC(a->segment, sizeof(float3) * nb * checkpoint_every);
     ADJ_MALLOC(a->lam[0], sizeof(float) * nb);
     ADJ_MALLOC(a->lam[1], sizeof(float) * nb);
     ADJ_MALLOC(a->gvel, sizeof(float) * nvel);
-    ADJ_MALLOC(a->foot_pk, sizeof(unsigned) * 512 * n_leaves);
-    ADJ_MALLOC(a->foot_w, sizeof(float4) * 512 * n_leaves);
-    ADJ_MALLOC(a->lrange, sizeof(int) * 6 * n_leaves);
-    ADJ_MALLOC(a->wrange, sizeof(int) * 6 * n_leaves);
-    VLR_CUDA(ctx, cudaMemsetAsync(a->foot_pk, 0, sizeof(unsigned) * 512 * n_leaves, ctx->stream));
+    for (int q = 0; q < 2; ++q) {
+        ADJ_MALLOC(a->foot_pk[q], sizeof(unsigned) * 512 * n_leaves);
+        ADJ_MALLOC(a->foot_w[q], sizeof(float4) * 512 * n_leaves);
+    }
+    ADJ_MALLOC(a->lstart, sizeof(int) * (n_leaves + 1));
+    ADJ_MALLOC(a->urange, sizeof(float) * 6 * n_leaves);
+    ADJ_MALLOC(a->nrange, sizeof(float) * 6 * n_leaves);
     ADJ_MALLOC(a->G, sizeof(float3) * nb);
-    ADJ_MALLOC(a->keys, sizeof(unsigned) * a->n_pairs_cap);
-    ADJ_MALLOC(a->pvals, sizeof(float) * a->n_pairs_cap);
-    ADJ_MALLOC(a->scratch, sort_reduce_scratch_bytes((int)a->n_pairs_cap));
 #undef ADJ_MALLOC
     cudaStream_t st = ctx->stream;
+    for (int q = 0; q < 2; ++q) {  // off the band: no foot, weight 0, lambda 0
+        VLR_CUDA(ctx, cudaMemsetAsync(a->foot_pk[q], 0, sizeof(unsigned) * 512 * n_leaves, st));
+        VLR_CUDA(ctx, cudaMemsetAsync(a->foot_w[q], 0, sizeof(float4) * 512 * n_leaves, st));
+    }
+    VLR_CUDA(ctx, cudaMemcpyAsync(a->lstart, lstart.data(), sizeof(int) * (n_leaves + 1), cudaMemcpyHostToDevice, st));
     VLR_CUDA(ctx, cudaMemcpyAsync(a->origin, o4.data(), sizeof(int4) * n_leaves, cudaMemcpyHostToDevice, st));
     VLR_CUDA(ctx, cudaMemcpyAsync(a->phi_init, phi, sizeof(float) * 512 * n_leaves, cudaMemcpyHostToDevice, st));
+    for (float* p : a->phi)
+        VLR_CUDA(ctx, cudaMemcpyAsync(p, a->phi_init, sizeof(float) * 512 * n_leaves, cudaMemcpyDeviceToDevice, st));
     VLR_CUDA(ctx, cudaMemcpyAsync(a->bidx, bidx.data(), sizeof(int) * 512 * n_leaves, cudaMemcpyHostToDevice, st));
     VLR_CUDA(ctx, cudaMemcpyAsync(a->bvox, bvox.data(), sizeof(int) * nb, cudaMemcpyHostToDevice, st));
     a->reach = reach_of(vel, nvel, dt);
@@ -952,6 +1304,10 @@ int vlr_adj_create(vlr_ctx* ctx, const int32_t* origins, const uint64_t* masks, 
                                                                     a->base[0], a->base[1], a->base[2], a->nbr);
     k_adj_upsample<<<blocks_for(ctx, nb), 256, 0, st>>>(a->bvox, a->origin, (int)nb, a->vel, n_stag, (float)stag_cell,
                                                         a->ub);
+    rc = enqueue_ranges(ctx, a);
+    if (!rc) rc = make_chunks(ctx, a);
+    if (!rc) rc = make_vel_entries(ctx, a);
+    if (rc) return fail(rc);
     cudaError_t e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) return fail(check_cuda(ctx, e, "adjoint setup"));
     rc = consume_device_errors(ctx, "vlr_adj_create");
@@ -995,6 +1351,8 @@ int vlr_adj_set_inputs(vlr_ctx* ctx, vlr_adjoint* a, const float* phi0_band, con
         VLR_CUDA(ctx, cudaMemcpyAsync(a->vel, vel, sizeof(float) * nvel, cudaMemcpyHostToDevice, st));
         k_adj_upsample<<<blocks_for(ctx, a->n_band), 256, 0, st>>>(a->bvox, a->origin, a->n_band, a->vel, a->n_stag,
                                                                    (float)a->H, a->ub);
+        const int rc = enqueue_ranges(ctx, a);
+        if (rc) return rc;
     }
     VLR_CUDA(ctx, cudaGetLastError());
     VLR_CUDA(ctx, cudaStreamSynchronize(st));
@@ -1035,18 +1393,18 @@ int vlr_adj_backward_device(vlr_ctx* ctx, vlr_adjoint* a, const float* d_grad_ph
         VLR_CUDA(ctx, cudaMemcpyAsync(a->lam[1], d_grad_phik_band, sizeof(float) * nb, cudaMemcpyDeviceToDevice, st));
     int rc = run_captured(ctx, &a->bwd_exec, [&]() { return adj_backward_enqueue(ctx, a); });
     if (rc) return rc;
-    float* lam = a->bwd_final;
+    float* lam = a->lam[0];
     a->lam_final = lam;
     if (d_grad_phi0_band)
         VLR_CUDA(ctx, cudaMemcpyAsync(d_grad_phi0_band, lam, sizeof(float) * nb, cudaMemcpyDeviceToDevice, st));
     if (d_grad_vel) {
         size_t nvel = 3ull * a->n_stag * a->n_stag * a->n_stag;
+        VLR_CUDA(ctx, cudaMemsetAsync(d_grad_vel, 0, sizeof(float) * nvel, st));
         VLR_TIMED(ctx, "k_adj_emit_vel",
-                  k_adj_emit_vel<<<blocks_for(ctx, nb), 256, 0, st>>>(a->bvox, a->origin, (int)nb, a->G, a->n_stag,
-                                                                      (float)a->H, a->keys, a->pvals));
-        rc = sort_reduce(ctx, a->keys, a->pvals, (int)(nb * 24), (unsigned)nvel + 1, d_grad_vel, (unsigned)nvel,
-                         a->scratch);
-        if (rc) return rc;
+                  k_adj_vel_sum<<<blocks_for(ctx, 8ll * a->n_seg), 256, 0, st>>>(
+                      a->seg_start, a->seg_node, a->n_seg, a->ent_b, a->ent_w, reinterpret_cast<const float*>(a->G),
+                      d_grad_vel));
+        VLR_CUDA(ctx, cudaGetLastError());
     }
     return VLR_OK;
 }
