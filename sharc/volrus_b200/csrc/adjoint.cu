@@ -35,6 +35,7 @@
 #include <numeric>
 #include <vector>
 
+#include "box_reduce.cuh"
 #include "method_state.hpp"
 #include "sort_reduce.hpp"
 
@@ -945,7 +946,7 @@ int make_vel_entries(vlr_ctx* ctx, vlr_adjoint* a) {
     const int ne = a->n_band * 24, n = a->n_stag, B = blocks_for(ctx, ne);
     const float H = (float)a->H;
     // temporaries in one block of the context's pool
-    const size_t sb = (sort_reduce_scratch_bytes(ne) + 255) & ~(size_t)255;
+    const size_t sb = (radix_scratch_bytes(ne, 4) + 255) & ~(size_t)255;
     char* blk = nullptr;
     VLR_CUDA(ctx, cudaMallocFromPoolAsync((void**)&blk, sb + sizeof(int) * (4 * (size_t)ne + 1), ctx->pool, st));
     unsigned* keys = (unsigned*)(blk + sb);
@@ -957,7 +958,7 @@ int make_vel_entries(vlr_ctx* ctx, vlr_adjoint* a) {
         VLR_CUDA(ctx, cudaMalloc(&a->ent_b, sizeof(int) * ne));
         VLR_CUDA(ctx, cudaMalloc(&a->ent_w, sizeof(float) * ne));
         k_adj_vel_keys<<<B, 256, 0, st>>>(a->bvox, a->origin, ne, n, H, keys, ids);
-        int rc = radix_sort_pairs(ctx, keys, ids, ne, 3u * n * n * n, blk, &ks, &is);
+        int rc = radix_sort(ctx, keys, ids, ne, bits_for(3ll * n * n * n - 1), blk, &ks, &is);
         if (rc) return rc;
         k_adj_vel_entries<<<B, 256, 0, st>>>(a->bvox, a->origin, ne, n, H, ks, is, a->ent_b, a->ent_w, head);
         rc = scan_exclusive(ctx, head, rank, ne, rank + ne);

@@ -311,74 +311,97 @@ int grid_index(vlr_ctx* ctx, vlr_grid* g) {
 
 // ------------------------------------------------------------------ scan
 
-// Block-wide exclusive scan of one int per thread (blockDim.x == 1024).
-__device__ inline int block_excl_scan(int v, int* warp_sums, int* total) {
-    int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+// Exclusive scan in tiles of 8192 (1024 threads, 8 consecutive values each).
+// More than one tile: k_scan_sums first writes the tiles' sums, and each block
+// of k_scan_tiles adds up the sums of the tiles before its own, so no block
+// waits on another and nothing is allocated per level.  A scan was two
+// launches, five from 1025 values up (about 8 us of launches and gaps); it is
+// one up to 8192 values (2.2 us) and two beyond.
+constexpr int kScanThreads = 1024;
+constexpr int kScanItems = 8;
+constexpr int kScanTile = kScanThreads * kScanItems;
+
+// Block-wide inclusive scan of one int per thread; *total = the block's sum.
+__device__ inline int block_incl_scan(int v, int* warp_sums, int* total) {
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     int x = v;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
-        int y = __shfl_up_sync(0xffffffffu, x, o);
+        const int y = __shfl_up_sync(0xffffffffu, x, o);
         if (lane >= o) x += y;
     }
     if (lane == 31) warp_sums[w] = x;
     __syncthreads();
     if (w == 0) {
-        int s = (lane < (int)(blockDim.x >> 5)) ? warp_sums[lane] : 0;
-        int si = s;
+        int s = warp_sums[lane];
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
-            int y = __shfl_up_sync(0xffffffffu, si, o);
-            if (lane >= o) si += y;
+            const int y = __shfl_up_sync(0xffffffffu, s, o);
+            if (lane >= o) s += y;
         }
-        warp_sums[lane] = si - s;  // exclusive prefix of warp sums
-        if (lane == 31) *total = si;
+        warp_sums[lane] = s;
     }
     __syncthreads();
-    int r = x - v + warp_sums[w];
-    __syncthreads();
-    return r;
+    *total = warp_sums[31];
+    return x + (w ? warp_sums[w - 1] : 0);
 }
 
-__global__ void __launch_bounds__(1024) k_scan_block(const int* in, int* out, int n, int* block_sums) {
+__global__ void __launch_bounds__(kScanThreads) k_scan_sums(const int* __restrict__ in, int n, int* __restrict__ sums) {
     __shared__ int ws[32];
-    __shared__ int tot;
-    int i = blockIdx.x * 1024 + threadIdx.x;
-    int v = (i < n) ? in[i] : 0;
-    int e = block_excl_scan(v, ws, &tot);
-    if (i < n) out[i] = e;
-    if (threadIdx.x == 0) block_sums[blockIdx.x] = tot;
+    const size_t base = (size_t)blockIdx.x * kScanTile;
+    int v = 0;
+#pragma unroll
+    for (int q = 0; q < kScanItems; ++q) {
+        const size_t i = base + q * kScanThreads + threadIdx.x;
+        if (i < (size_t)n) v += in[i];
+    }
+    int tot;
+    block_incl_scan(v, ws, &tot);
+    if (threadIdx.x == 0) sums[blockIdx.x] = tot;
 }
 
-__global__ void k_scan_add(int* out, int n, const int* block_offsets) {
-    int i = blockIdx.x * 1024 + threadIdx.x;
-    if (i < n) out[i] += block_offsets[blockIdx.x];
+__global__ void __launch_bounds__(kScanThreads) k_scan_tiles(const int* in, int* out, int n,
+                                                            const int* __restrict__ sums, int* total) {
+    __shared__ int ws[32];
+    int before = 0;
+    if (blockIdx.x > 0) {  // one tile: sums is null
+        int v = 0;
+        for (int t = threadIdx.x; t < (int)blockIdx.x; t += kScanThreads) v += sums[t];
+        block_incl_scan(v, ws, &before);
+        __syncthreads();
+    }
+    const size_t i0 = (size_t)blockIdx.x * kScanTile + (size_t)threadIdx.x * kScanItems;
+    int v[kScanItems], s = 0;
+#pragma unroll
+    for (int q = 0; q < kScanItems; ++q) {
+        v[q] = i0 + q < (size_t)n ? in[i0 + q] : 0;
+        s += v[q];
+    }
+    int tot;
+    int run = before + block_incl_scan(s, ws, &tot) - s;
+#pragma unroll
+    for (int q = 0; q < kScanItems; ++q) {
+        if (i0 + q < (size_t)n) out[i0 + q] = run;
+        run += v[q];
+    }
+    if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) *total = before + tot;
 }
 
-__global__ void k_scan_total(const int* in, const int* out, int n, int* total) {
-    if (threadIdx.x == 0 && blockIdx.x == 0) *total = (n > 0) ? out[n - 1] + in[n - 1] : 0;
-}
-
-// Scratch layout per level: block sums then their scan.
+// Exclusive scan of n ints on the context stream; *d_total (device) = their sum.
 int scan_exclusive(vlr_ctx* ctx, const int* d_in, int* d_out, int n, int* d_total) {
     if (n <= 0) {
         VLR_CUDA(ctx, cudaMemsetAsync(d_total, 0, sizeof(int), ctx->stream));
         return VLR_OK;
     }
-    int nb = (n + 1023) / 1024;
+    const int nb = (int)(((long long)n + kScanTile - 1) / kScanTile);
     int* sums = nullptr;
-    int* sums_scan = nullptr;
-    VLR_CUDA(ctx, cudaMallocFromPoolAsync(&sums, sizeof(int) * (nb + 1) * 2, ctx->pool, ctx->stream));
-    sums_scan = sums + nb + 1;
-    k_scan_block<<<nb, 1024, 0, ctx->stream>>>(d_in, d_out, n, sums);
     if (nb > 1) {
-        int* dummy_total = sums_scan + nb;
-        int rc = scan_exclusive(ctx, sums, sums_scan, nb, dummy_total);
-        if (rc) return rc;
-        k_scan_add<<<nb, 1024, 0, ctx->stream>>>(d_out, n, sums_scan);
+        VLR_CUDA(ctx, cudaMallocFromPoolAsync(&sums, sizeof(int) * nb, ctx->pool, ctx->stream));
+        k_scan_sums<<<nb, kScanThreads, 0, ctx->stream>>>(d_in, n, sums);
     }
-    k_scan_total<<<1, 32, 0, ctx->stream>>>(d_in, d_out, n, d_total);
+    k_scan_tiles<<<nb, kScanThreads, 0, ctx->stream>>>(d_in, d_out, n, sums, d_total);
     VLR_CUDA(ctx, cudaGetLastError());
-    VLR_CUDA(ctx, cudaFreeAsync(sums, ctx->stream));
+    if (sums) VLR_CUDA(ctx, cudaFreeAsync(sums, ctx->stream));
     return VLR_OK;
 }
 

@@ -157,7 +157,7 @@ struct TileBase {
 };
 
 __global__ void k_mc_cand(const int4* __restrict__ origin, int n, TileBase tb, uint64_t* __restrict__ keys,
-                          unsigned* __restrict__ lo, unsigned* __restrict__ idx, unsigned* __restrict__ err) {
+                          unsigned* __restrict__ idx, unsigned* __restrict__ err) {
     const int d[7][3] = {{0, 0, 0}, {-1, 0, 0}, {1, 0, 0}, {0, -1, 0}, {0, 1, 0}, {0, 0, -1}, {0, 0, 1}};
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < 7ll * n;
          i += (long long)gridDim.x * blockDim.x) {
@@ -167,23 +167,14 @@ __global__ void k_mc_cand(const int4* __restrict__ origin, int n, TileBase tb, u
                               (long long)(o.z >> 3) + d[j][2], tb.b);
         if (k == kBadKey) atomicOr(err, kErrExtent);
         keys[i] = k;
-        lo[i] = (unsigned)k;
         idx[i] = (unsigned)i;
     }
 }
 
-__global__ void k_mc_hi(const uint64_t* __restrict__ keys, const unsigned* __restrict__ idx, int n,
-                        unsigned* __restrict__ hi) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-        hi[i] = (unsigned)(keys[idx[i]] >> 32);
-}
-
-__global__ void k_mc_unique(const uint64_t* __restrict__ keys, const unsigned* __restrict__ idx, int n,
-                            uint64_t* __restrict__ sorted, int* __restrict__ flag) {
+__global__ void k_mc_unique(const uint64_t* __restrict__ sorted, int n, int* __restrict__ flag) {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const uint64_t k = keys[idx[i]];
-        sorted[i] = k;
-        flag[i] = (k != kBadKey && (i == 0 || k != keys[idx[i - 1]])) ? 1 : 0;
+        const uint64_t k = sorted[i];
+        flag[i] = (k != kBadKey && (i == 0 || k != sorted[i - 1])) ? 1 : 0;
     }
 }
 
@@ -461,14 +452,12 @@ int volume_to_mesh(vlr_ctx* ctx, const vlr_grid* g, float iso, double* h_verts, 
     for (int a = 0; a < 3; ++a) tb.b[a] = g->base[a];
     const int thr = 256, blocks = ctx->sm_count * 8;
     // candidates and their sort
-    const size_t sort_bytes = sort_reduce_scratch_bytes(n7);
+    const size_t sort_bytes = radix_scratch_bytes(n7, 8);
     char* buf = nullptr;
-    const size_t cand_bytes = (size_t)n7 * (8 + 4 + 4 + 4 + 8 + 4 + 4) + sort_bytes + 256;
+    const size_t cand_bytes = (size_t)n7 * (8 + 4 + 4 + 4) + sort_bytes + 256;
     VLR_CUDA(ctx, cudaMallocFromPoolAsync((void**)&buf, cand_bytes, ctx->pool, st));
     char* p = buf;
     uint64_t* keys = (uint64_t*)p;  p += (size_t)n7 * 8;
-    uint64_t* sorted = (uint64_t*)p;  p += (size_t)n7 * 8;
-    unsigned* lo = (unsigned*)p;  p += (size_t)n7 * 4;
     unsigned* idx = (unsigned*)p;  p += (size_t)n7 * 4;
     int* flag = (int*)p;  p += (size_t)n7 * 4;
     int* pos = (int*)p;  p += (size_t)n7 * 4 + 16;
@@ -477,22 +466,13 @@ int volume_to_mesh(vlr_ctx* ctx, const vlr_grid* g, float iso, double* h_verts, 
         cudaFreeAsync(buf, st);
         return code;
     };
-    // 63-bit keys sorted as two stable 32-bit passes carrying the candidate index
-    k_mc_cand<<<blocks, thr, 0, st>>>(g->origin, g->n, tb, keys, lo, idx, ctx->d_errword);
-    unsigned *k1, *v1, *k2, *v2;
-    rc = radix_sort_pairs(ctx, lo, idx, n7, 0xffffffffu, scratch, &k1, &v1);
+    // 63-bit keys (a bad key, all ones, sorts last)
+    k_mc_cand<<<blocks, thr, 0, st>>>(g->origin, g->n, tb, keys, idx, ctx->d_errword);
+    uint64_t* sorted;
+    unsigned* order;
+    rc = radix_sort(ctx, keys, idx, n7, 64, scratch, &sorted, &order);
     if (rc) return done(rc);
-    // high words in candidate order of the first pass; the order array moves
-    // out of the scratch (if it ended there) before the second pass reuses it
-    unsigned* hi = (unsigned*)flag;
-    k_mc_hi<<<blocks, thr, 0, st>>>(keys, v1, n7, hi);
-    if (v1 != idx) VLR_CUDA(ctx, cudaMemcpyAsync(idx, v1, (size_t)n7 * 4, cudaMemcpyDeviceToDevice, st));
-    rc = radix_sort_pairs(ctx, hi, idx, n7, 0x7fffffffu, scratch, &k2, &v2);
-    if (rc) return done(rc);
-    (void)k1;
-    (void)k2;
-    // v2 is the final order; flag (the high words) is rewritten here as unique flags
-    k_mc_unique<<<blocks, thr, 0, st>>>(keys, v2, n7, sorted, flag);
+    k_mc_unique<<<blocks, thr, 0, st>>>(sorted, n7, flag);
     rc = scan_exclusive(ctx, flag, pos, n7, pos + n7);
     if (rc) return done(rc);
     int m = 0;

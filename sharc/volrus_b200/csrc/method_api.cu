@@ -8,6 +8,7 @@
 #include <numeric>
 #include <vector>
 
+#include "box_reduce.cuh"
 #include "leaf_copy.cuh"
 #include "method_state.hpp"
 #include "sort_reduce.hpp"
@@ -626,27 +627,33 @@ int enqueue_one_step(vlr_ctx* ctx, vlr_level_set* ls) {
 
 // Leaves of one grid (grid < 0: all) of a level set holding n listed leaves,
 // sorted by (grid, x, y, z), into host buffers.
-// Leaf keys of list positions 0..n-1 of a single grid (leaf coordinates
-// relative to the hash base, `bits` each: key order is the origins'
-// lexicographic order), their low words and the identity permutation.
-__global__ void k_leaf_keys(const int* __restrict__ list, int n, const int4* __restrict__ origin, long long b0,
-                            long long b1, long long b2, int bits, unsigned long long* __restrict__ keys,
-                            unsigned* __restrict__ lo, unsigned* __restrict__ idx) {
+// Bounding box (leaf coordinates) of the listed leaves.
+__global__ void __launch_bounds__(256) k_leaf_box(const int* __restrict__ list, int n, const int4* __restrict__ origin,
+                                                 int* __restrict__ box) {
+    int lo[3] = {INT_MAX, INT_MAX, INT_MAX}, hi[3] = {INT_MIN, INT_MIN, INT_MIN};
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const int4 o = origin[list[i]];
-        const unsigned long long k = ((unsigned long long)((o.x >> 3) - b0) << (2 * bits)) |
-                                     ((unsigned long long)((o.y >> 3) - b1) << bits) |
-                                     (unsigned long long)((o.z >> 3) - b2);
-        keys[i] = k;
-        lo[i] = (unsigned)k;
-        idx[i] = (unsigned)i;
+        const int c[3] = {o.x >> 3, o.y >> 3, o.z >> 3};
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            lo[a] = min(lo[a], c[a]);
+            hi[a] = max(hi[a], c[a]);
+        }
     }
+    block_box(lo, hi, box);
 }
 
-__global__ void k_leaf_keys_hi(const unsigned long long* __restrict__ keys, const unsigned* __restrict__ perm, int n,
-                               unsigned* __restrict__ hi) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-        hi[i] = (unsigned)(keys[perm[i]] >> 32);
+// Leaf keys of list positions 0..n-1 of a single grid (leaf coordinates
+// relative to the box's corner, by and bz bits for y and z: key order is the
+// origins' lexicographic order) and the identity permutation.
+__global__ void k_leaf_keys(const int* __restrict__ list, int n, const int4* __restrict__ origin, int x0, int y0,
+                            int z0, int by, int bz, uint64_t* __restrict__ keys, unsigned* __restrict__ idx) {
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const int4 o = origin[list[i]];
+        keys[i] = ((uint64_t)(unsigned)((o.x >> 3) - x0) << (by + bz)) | ((uint64_t)(unsigned)((o.y >> 3) - y0) << bz) |
+                  (uint64_t)(unsigned)((o.z >> 3) - z0);
+        idx[i] = (unsigned)i;
+    }
 }
 
 // Origins (i32[3]) of the list positions perm[0..n) in that order.
@@ -661,44 +668,50 @@ __global__ void k_sorted_origins(const int* __restrict__ list, const unsigned* _
 }
 
 // The sorted download of all leaves of a single grid with the order made on
-// the device: 64-bit leaf keys sorted by two stable 32-bit radix passes (low
-// word, then high word), then origins, masks and f32 values gathered in that
-// order and copied once into the caller's buffers.
+// the device: the leaves' bounding box, radix sort of keys of just its bits
+// (24 for 256 leaves an axis, against the 63 of hash keys: 3 passes, not 8),
+// then origins, masks and f32 values gathered in that order and copied once
+// into the caller's buffers.
 int download_sorted_device(vlr_ctx* ctx, const vlr_level_set* ls, size_t n, int32_t* origins, uint64_t* masks,
                            float* phi) {
     cudaStream_t st = ctx->stream;
     const int nn = (int)n;
-    const size_t sort_bytes = sort_reduce_scratch_bytes(nn);
+    const size_t sort_bytes = radix_scratch_bytes(nn, 8);
     const size_t vbytes = sizeof(float) * kLeafVoxels * n;
     char* buf = nullptr;
-    VLR_CUDA(ctx, cudaMallocFromPoolAsync((void**)&buf, vbytes + n * (8 + 4 * 3 + 12 + 64) + sort_bytes + 512,
-                                          ctx->pool, st));
+    VLR_CUDA(ctx, cudaMallocFromPoolAsync((void**)&buf, vbytes + n * (8 + 4 + 12 + 64) + sort_bytes + 512, ctx->pool,
+                                          st));
     auto done = [&](int code) {
         cudaFreeAsync(buf, st);
         return code;
     };
     char* q = buf;
     float* v = (float*)q;  q += vbytes;
-    unsigned long long* keys = (unsigned long long*)q;  q += n * 8;
+    uint64_t* keys = (uint64_t*)q;  q += n * 8;
     uint64_t* mm = (uint64_t*)q;  q += n * 64;
-    unsigned* lo = (unsigned*)q;  q += n * 4;
     unsigned* idx = (unsigned*)q;  q += n * 4;
-    unsigned* hi = (unsigned*)q;  q += n * 4;
     int32_t* o3 = (int32_t*)q;  q += n * 12;
     void* scratch = (void*)(((uintptr_t)q + 255) & ~(uintptr_t)255);
-    const vlr::MGridParams& P = ls->h_params[0];
     const int B = ctx->sm_count * 8;
-    k_leaf_keys<<<B, 256, 0, st>>>(ls->list, nn, ls->origin, P.base[0], P.base[1], P.base[2], ls->key_bits, keys, lo,
-                                   idx);
-    unsigned *k1, *v1, *k2, *v2;
-    int rc = radix_sort_pairs(ctx, lo, idx, nn, 0xffffffffu, scratch, &k1, &v1);
+    int* box = (int*)scratch;  // read back before the sort uses its scratch
+    int* hb = static_cast<int*>(ctx->pinned) + 32;
+    auto box_of = [&]() -> int {
+        VLR_CUDA(ctx, cudaMemsetAsync(box, kBoxClear, 6 * sizeof(int), st));
+        k_leaf_box<<<ctx->sm_count, 256, 0, st>>>(ls->list, nn, ls->origin, box);
+        VLR_CUDA(ctx, cudaMemcpyAsync(hb, box, 6 * sizeof(int), cudaMemcpyDeviceToHost, st));
+        VLR_CUDA(ctx, cudaStreamSynchronize(st));
+        return VLR_OK;
+    };
+    int rc = box_of();
     if (rc) return done(rc);
-    k_leaf_keys_hi<<<B, 256, 0, st>>>(keys, v1, nn, hi);
-    if (v1 != idx) VLR_CUDA(ctx, cudaMemcpyAsync(idx, v1, n * 4, cudaMemcpyDeviceToDevice, st));
-    rc = radix_sort_pairs(ctx, hi, idx, nn, 0x7fffffffu, scratch, &k2, &v2);
+    const int lo[3] = {~hb[0], ~hb[1], ~hb[2]};
+    int bits[3];
+    for (int a = 0; a < 3; ++a) bits[a] = bits_for((long long)hb[3 + a] - lo[a]);
+    k_leaf_keys<<<B, 256, 0, st>>>(ls->list, nn, ls->origin, lo[0], lo[1], lo[2], bits[1], bits[2], keys, idx);
+    uint64_t* sorted_keys;
+    unsigned* v2;
+    rc = radix_sort(ctx, keys, idx, nn, bits[0] + bits[1] + bits[2], scratch, &sorted_keys, &v2);
     if (rc) return done(rc);
-    (void)k1;
-    (void)k2;
     const int* sel = (const int*)v2;
     if (origins) k_sorted_origins<<<B, 256, 0, st>>>(ls->list, v2, nn, ls->origin, o3);
     if (masks || phi) {
@@ -810,27 +823,26 @@ int download_n(vlr_ctx* ctx, const vlr_level_set* ls, size_t n, int grid, int32_
 // level set holds the stepped state as after a one-pass host step.
 constexpr int kSlabRing = 16;                   // voxels: two leaves of input beside a slab
 constexpr size_t kSlabLeavesAuto = 1u << 17;    // automatic count: one slab per this many leaves
-constexpr unsigned long long kSlabOther = 0x7fffffffffffffffull;  // key of a leaf the slab does not keep
+constexpr uint64_t kSlabOther = 0x7fffffffffffffffull;  // key of a leaf the slab does not keep
 
-// Keys of the listed leaves (as k_leaf_keys) for those with x in [xlo, xhi),
+// 63-bit keys of the listed leaves (leaf coordinates relative to the hash base) for those with x in [xlo, xhi),
 // kSlabOther for the others (sorted after every kept leaf), and the number
 // of kept leaves added to *kept.
 __global__ void k_slab_keys(const int* __restrict__ list, const int* __restrict__ count,
                             const int4* __restrict__ origin, long long b0, long long b1, long long b2, int bits,
-                            long long xlo, long long xhi, unsigned long long* __restrict__ keys,
-                            unsigned* __restrict__ lo, unsigned* __restrict__ idx, int* __restrict__ kept) {
+                            long long xlo, long long xhi, uint64_t* __restrict__ keys, unsigned* __restrict__ idx,
+                            int* __restrict__ kept) {
     const int n = *count;
     int c = 0;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const int4 o = origin[list[i]];
-        unsigned long long k = kSlabOther;
+        uint64_t k = kSlabOther;
         if (o.x >= xlo && o.x < xhi) {
             k = ((unsigned long long)((o.x >> 3) - b0) << (2 * bits)) |
                 ((unsigned long long)((o.y >> 3) - b1) << bits) | (unsigned long long)((o.z >> 3) - b2);
             ++c;
         }
         keys[i] = k;
-        lo[i] = (unsigned)k;
         idx[i] = (unsigned)i;
     }
     for (int d = 16; d > 0; d >>= 1) c += __shfl_down_sync(0xffffffffu, c, d);
@@ -954,8 +966,8 @@ int step_host_slabs(vlr_ctx* ctx, vlr_level_set* ls, const SlabPlan& P, const in
     const size_t cap_out = std::min(cap_leaves, (size_t)ls->cap);
     const size_t cmax = (size_t)ls->cap;
     const size_t rec = sizeof(float) * kLeafVoxels + 64 + 12;
-    const size_t sort_bytes = sort_reduce_scratch_bytes((int)cmax);
-    const size_t bytes = n * rec + cap_out * rec + cmax * (8 + 12) + sort_bytes + 2 * kHostSlabsMax * sizeof(int) +
+    const size_t sort_bytes = radix_scratch_bytes((int)cmax, 8);
+    const size_t bytes = n * rec + cap_out * rec + cmax * (8 + 4) + sort_bytes + 2 * kHostSlabsMax * sizeof(int) +
                          16 * 256;  // each of the 12 pieces below starts on a 256-byte boundary
     char* buf = nullptr;
     VLR_CUDA(ctx, cudaMallocFromPoolAsync((void**)&buf, bytes, ctx->pool, st));
@@ -971,10 +983,8 @@ int step_host_slabs(vlr_ctx* ctx, vlr_level_set* ls, const SlabPlan& P, const in
     float* out_sv = (float*)take(cap_out * 4 * kLeafVoxels);
     uint64_t* out_sm = (uint64_t*)take(cap_out * 64);
     int32_t* out_so = (int32_t*)take(cap_out * 12);
-    unsigned long long* keys = (unsigned long long*)take(cmax * 8);
-    unsigned* klo = (unsigned*)take(cmax * 4);
+    uint64_t* keys = (uint64_t*)take(cmax * 8);
     unsigned* kidx = (unsigned*)take(cmax * 4);
-    unsigned* khi = (unsigned*)take(cmax * 4);
     // [0, ns) kept per slab, [kHostSlabsMax] step at entry
     int* d_small = (int*)take(2 * kHostSlabsMax * sizeof(int));
     void* scratch = take(sort_bytes);
@@ -1068,17 +1078,10 @@ int step_host_slabs(vlr_ctx* ctx, vlr_level_set* ls, const SlabPlan& P, const in
         offs[s] = off;
         if (c) {
             k_slab_keys<<<B, 256, 0, st>>>(ls->list, ls->scalars, ls->origin, G.base[0], G.base[1], G.base[2],
-                                           ls->key_bits, P.x[s], P.x[s + 1], keys, klo, kidx, d_small + s);
-            unsigned *k1, *v1, *k2, *v2;
-            if ((rc = radix_sort_pairs(ctx, klo, kidx, c, 0xffffffffu, scratch, &k1, &v1))) return finish(rc);
-            k_leaf_keys_hi<<<B, 256, 0, st>>>(keys, v1, c, khi);
-            if (v1 != kidx &&
-                (rc = cuda_rc(ctx, cudaMemcpyAsync(kidx, v1, (size_t)c * 4, cudaMemcpyDeviceToDevice, st),
-                                 "cudaMemcpyAsync")))
-                return finish(rc);
-            if ((rc = radix_sort_pairs(ctx, khi, kidx, c, 0x7fffffffu, scratch, &k2, &v2))) return finish(rc);
-            (void)k1;
-            (void)k2;
+                                           ls->key_bits, P.x[s], P.x[s + 1], keys, kidx, d_small + s);
+            uint64_t* k2;
+            unsigned* v2;
+            if ((rc = radix_sort(ctx, keys, kidx, c, 63, scratch, &k2, &v2))) return finish(rc);
             const size_t o = std::min(off, cap_out);
             const int room = (int)(cap_out - o);
             if (ls->precision == VLR_PREC_F16)

@@ -213,7 +213,7 @@ int vlr_advect_points(vlr_ctx* ctx, const vlr_grid* vx, const vlr_grid* vy, cons
     for (int i = 0; i < 12; ++i) inv.r[i] = world_to_index[i];
     // one stream-ordered block: particles in and out, keys, permutation, flags, ranks, sort scratch
     const size_t pb = sizeof(vlr_particle) * n, wb = sizeof(unsigned) * n;
-    const size_t sb = sort_reduce_scratch_bytes(nn);
+    const size_t sb = radix_scratch_bytes(nn, 4);
     auto al = [](size_t b) { return (b + 255) & ~(size_t)255; };
     const size_t total = 2 * al(pb) + 8 * al(wb) + al(sizeof(int) * 2) + al(sb) + al(sizeof(int32_t) * 3 * n) +
                          al(sizeof(uint32_t) * (n + 1));
@@ -256,18 +256,18 @@ int vlr_advect_points(vlr_ctx* ctx, const vlr_grid* vx, const vlr_grid* vy, cons
     // stable sorts by z, then y, then x: lexicographic (x, y, z), ties in input
     // order.  A sort may leave its result in its scratch, which the next sort
     // reuses, so each pass's permutation is first moved to pbuf.
-    const unsigned lim = (1u << 29) - 1u;
+    const int bits = 29;
     unsigned *ko = nullptr, *perm = nullptr;
     if (cudaMemcpyAsync(kbuf, kz, wb, cudaMemcpyDeviceToDevice, st) != cudaSuccess)
         return fail(check_cuda(ctx, cudaGetLastError(), "key copy"));
-    rc = radix_sort_pairs(ctx, kbuf, idx, nn, lim, scratch, &ko, &perm);
+    rc = radix_sort(ctx, kbuf, idx, nn, bits, scratch, &ko, &perm);
     if (rc) return fail(rc);
     const unsigned* axis_keys[2] = {ky, kx};
     for (int pass = 0; pass < 2; ++pass) {
         if (perm != pbuf && cudaMemcpyAsync(pbuf, perm, wb, cudaMemcpyDeviceToDevice, st) != cudaSuccess)
             return fail(check_cuda(ctx, cudaGetLastError(), "permutation copy"));
         k_gather_keys<<<blocks, 256, 0, st>>>(axis_keys[pass], pbuf, nn, kbuf);
-        rc = radix_sort_pairs(ctx, kbuf, pbuf, nn, lim, scratch, &ko, &perm);
+        rc = radix_sort(ctx, kbuf, pbuf, nn, bits, scratch, &ko, &perm);
         if (rc) return fail(rc);
     }
     VLR_TIMED(ctx, "k_points_emit",

@@ -443,8 +443,8 @@ static int alloc_cross(vlr_ctx* ctx, int n, CrossBufs& b) {
 }
 
 // Crossing-list sort on the device: the bounding box of the coordinates, then
-// (x, y, z)-major keys of their offsets to it, sorted by two stable 32-bit
-// radix passes (low word, then high word) that carry the list index.
+// (x, y, z)-major keys of their offsets to it, radix-sorted with the list
+// index.
 __global__ void k_cross_box(const int* __restrict__ c, int n, int* __restrict__ box) {
     int lo[3] = {INT_MAX, INT_MAX, INT_MAX}, hi[3] = {INT_MIN, INT_MIN, INT_MIN};
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
@@ -464,20 +464,13 @@ __global__ void k_cross_box(const int* __restrict__ c, int n, int* __restrict__ 
 }
 
 __global__ void k_cross_keys(const int* __restrict__ c, int n, int bx, int by, int bz, int bits,
-                             uint64_t* __restrict__ keys, unsigned* __restrict__ lo, unsigned* __restrict__ idx) {
+                             uint64_t* __restrict__ keys, unsigned* __restrict__ idx) {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const uint64_t k = ((uint64_t)(unsigned)(c[3 * i] - bx) << (2 * bits)) |
                            ((uint64_t)(unsigned)(c[3 * i + 1] - by) << bits) | (uint64_t)(unsigned)(c[3 * i + 2] - bz);
         keys[i] = k;
-        lo[i] = (unsigned)k;
         idx[i] = (unsigned)i;
     }
-}
-
-__global__ void k_cross_hi(const uint64_t* __restrict__ keys, const unsigned* __restrict__ idx, int n,
-                           unsigned* __restrict__ hi) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-        hi[i] = (unsigned)(keys[idx[i]] >> 32);
 }
 
 __global__ void k_cross_gather(const int* __restrict__ c, const unsigned* __restrict__ idx, int n,
@@ -491,7 +484,7 @@ __global__ void k_cross_gather(const int* __restrict__ c, const unsigned* __rest
 static int sort_crossings_device(vlr_ctx* ctx, const int* d_c, int n, int* d_out, bool* sorted) {
     *sorted = false;
     cudaStream_t st = ctx->stream;
-    const size_t sort_bytes = sort_reduce_scratch_bytes(n);
+    const size_t sort_bytes = radix_scratch_bytes(n, 8);
     char* buf = nullptr;
     VLR_CUDA(ctx, cudaMallocFromPoolAsync((void**)&buf, (size_t)n * 20 + sort_bytes + 256, ctx->pool, st));
     auto done = [&](int code) {
@@ -500,9 +493,7 @@ static int sort_crossings_device(vlr_ctx* ctx, const int* d_c, int n, int* d_out
     };
     char* p = buf;
     uint64_t* keys = (uint64_t*)p;  p += (size_t)n * 8;
-    unsigned* lo = (unsigned*)p;  p += (size_t)n * 4;
     unsigned* idx = (unsigned*)p;  p += (size_t)n * 4;
-    unsigned* hi = (unsigned*)p;  p += (size_t)n * 4;
     int* box = (int*)(((uintptr_t)p + 15) & ~(uintptr_t)15);
     void* scratch = (void*)(((uintptr_t)(box + 8) + 15) & ~(uintptr_t)15);
     const int init[6] = {INT_MAX, INT_MAX, INT_MAX, INT_MIN, INT_MIN, INT_MIN};
@@ -519,17 +510,12 @@ static int sort_crossings_device(vlr_ctx* ctx, const int* d_c, int n, int* d_out
         while (bits < 40 && (1ll << bits) <= ext) ++bits;
     }
     if (3 * bits > 63) return done(VLR_OK);
-    k_cross_keys<<<blocks, 256, 0, st>>>(d_c, n, hb[0], hb[1], hb[2], bits, keys, lo, idx);
-    unsigned *k1, *v1, *k2, *v2;
-    int rc = radix_sort_pairs(ctx, lo, idx, n, 0xffffffffu, scratch, &k1, &v1);
+    k_cross_keys<<<blocks, 256, 0, st>>>(d_c, n, hb[0], hb[1], hb[2], bits, keys, idx);
+    uint64_t* sorted_keys;
+    unsigned* order;
+    int rc = radix_sort(ctx, keys, idx, n, 3 * bits, scratch, &sorted_keys, &order);
     if (rc) return done(rc);
-    k_cross_hi<<<blocks, 256, 0, st>>>(keys, v1, n, hi);
-    if (v1 != idx) VLR_CUDA(ctx, cudaMemcpyAsync(idx, v1, (size_t)n * 4, cudaMemcpyDeviceToDevice, st));
-    rc = radix_sort_pairs(ctx, hi, idx, n, 0x7fffffffu, scratch, &k2, &v2);
-    if (rc) return done(rc);
-    (void)k1;
-    (void)k2;
-    k_cross_gather<<<blocks, 256, 0, st>>>(d_c, v2, n, d_out);
+    k_cross_gather<<<blocks, 256, 0, st>>>(d_c, order, n, d_out);
     VLR_CUDA(ctx, cudaGetLastError());
     *sorted = true;
     return done(VLR_OK);
