@@ -894,7 +894,7 @@ def ref_step_leg(args, ctx, ls, flush, stream, clk):
             times.append(e0.elapsed_time(e1))
             out_active = out.active_voxel_count()
             out.close()
-    kern = {kk: ctx.kernel_time(kk) for kk in ("k_advect_ref", "k_crossings", "k_rebuild_window")}
+    kern = {kk: ctx.kernel_time(kk) for kk in ("k_advect_ref", "k_cross_sign", "k_rebuild_window")}
     ctx.profile(False)
     ms = sum(times) / len(times)
     for gg in (g0, *vgrids):
@@ -1279,10 +1279,10 @@ def bench_ref_sphere(args, ctx, peak, peak_kind):
             ctx.synchronize()
             times.append(e0.elapsed_time(e1))
             out.close()
-    kernels = {k: ctx.kernel_time(k) for k in ("k_advect_ref", "k_crossings", "k_rebuild_window")}
+    kernels = {k: ctx.kernel_time(k) for k in ("k_advect_ref", "k_cross_sign", "k_rebuild_window")}
     ctx.profile(False)
     ms = sum(times) / len(times)
-    per_leaf = {"k_advect_ref": 1024 * 4 + 144, "k_crossings": 512 * 4 + 64 + 16 + 64,
+    per_leaf = {"k_advect_ref": 1024 * 4 + 144, "k_cross_sign": 512 * 4 + 4 * 64,
                 "k_rebuild_window": 1024 * 4 + 64 * 3}
     dom = max(kernels, key=lambda k: kernels[k][0])
     dom_ms = kernels[dom][0] / max(kernels[dom][1], 1)

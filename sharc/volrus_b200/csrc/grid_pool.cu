@@ -346,7 +346,7 @@ __device__ inline int block_incl_scan(int v, int* warp_sums, int* total) {
     return x + (w ? warp_sums[w - 1] : 0);
 }
 
-__global__ void __launch_bounds__(kScanThreads) k_scan_sums(const int* __restrict__ in, int n, int* __restrict__ sums) {
+__global__ void __launch_bounds__(kScanThreads) k_scan_sums(const int* __restrict__ in, long long n, int* __restrict__ sums) {
     __shared__ int ws[32];
     const size_t base = (size_t)blockIdx.x * kScanTile;
     int v = 0;
@@ -360,7 +360,7 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_sums(const int* __restric
     if (threadIdx.x == 0) sums[blockIdx.x] = tot;
 }
 
-__global__ void __launch_bounds__(kScanThreads) k_scan_tiles(const int* in, int* out, int n,
+__global__ void __launch_bounds__(kScanThreads) k_scan_tiles(const int* in, int* out, long long n,
                                                             const int* __restrict__ sums, int* total) {
     __shared__ int ws[32];
     int before = 0;
@@ -388,12 +388,12 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_tiles(const int* in, int*
 }
 
 // Exclusive scan of n ints on the context stream; *d_total (device) = their sum.
-int scan_exclusive(vlr_ctx* ctx, const int* d_in, int* d_out, int n, int* d_total) {
+int scan_exclusive(vlr_ctx* ctx, const int* d_in, int* d_out, long long n, int* d_total) {
     if (n <= 0) {
         VLR_CUDA(ctx, cudaMemsetAsync(d_total, 0, sizeof(int), ctx->stream));
         return VLR_OK;
     }
-    const int nb = (int)(((long long)n + kScanTile - 1) / kScanTile);
+    const int nb = (int)((n + kScanTile - 1) / kScanTile);
     int* sums = nullptr;
     if (nb > 1) {
         VLR_CUDA(ctx, cudaMallocFromPoolAsync(&sums, sizeof(int) * nb, ctx->pool, ctx->stream));

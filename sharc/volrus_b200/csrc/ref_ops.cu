@@ -2,7 +2,8 @@
 // leaves, bit-exact with the crate's CPU code.
 //   k_advect_ref      advect_level_set            src/tools/advection.rs:32-56
 //   k_sample_points   sample_trilinear            src/tools/interpolation.rs:11-48
-//   k_crossings       find_zero_crossings         src/tools/level_set_track.rs:14-47
+//   k_cross_sign, k_cross_bits, k_emit_crossings
+//                     find_zero_crossings         src/tools/level_set_track.rs:14-47
 //   k_rebuild_window  rebuild_narrow_band         src/tools/level_set_track.rs:80-114
 //   k_rebuild_brute   (same, any half-width)
 //   k_trim            trim_narrow_band            src/tools/level_set_track.rs:53-68
@@ -15,7 +16,6 @@
 #include <vector>
 
 #include "ref_ops.hpp"
-#include "sort_reduce.hpp"
 
 namespace vlr {
 
@@ -84,74 +84,165 @@ __device__ inline void local_get(const GridView& g, int slot, int x, int y, int 
     on = mask_bit(g.mask + (size_t)s * 8, off);
 }
 
-// 256 threads, voxels tid and tid+256.  Writes the crossing mask (same bit
-// layout as the activity mask) and the per-leaf crossing count.
-__global__ void __launch_bounds__(256) k_crossings(GridView g, uint64_t* __restrict__ xmask, int* __restrict__ xcount,
-                                                  unsigned long long* __restrict__ total) {
-    int slot = blockIdx.x;
-    if (slot >= g.n) return;
-    const uint64_t* m = g.mask + (size_t)slot * 8;
-    int cnt = 0;
-    for (int r = 0; r < 2; ++r) {
-        int off = threadIdx.x + 256 * r;
-        bool cross = false;
-        if (mask_bit(m, off)) {
-            float val = g.values[(size_t)slot * kLeafVoxels + off];
-            if (val == 0.0f) {
-                cross = true;
-            } else {
-                int x = off >> 6, y = (off >> 3) & 7, z = off & 7;
-                const int ddx[6] = {1, -1, 0, 0, 0, 0};
-                const int ddy[6] = {0, 0, 1, -1, 0, 0};
-                const int ddz[6] = {0, 0, 0, 0, 1, -1};
+// find_zero_crossings on bit masks.  A voxel is a crossing if it is active and
+// exactly zero, or if its product with an active 6-neighbour is negative: for
+// products that do not underflow, if their signs differ.  k_cross_sign streams
+// the values once into per-leaf masks of the positive, negative and zero
+// active voxels (NaN is none of them, and its product is not negative);
+// k_cross_bits then compares 64 voxels at a time against the six shifted
+// masks.  A leaf holding a non-zero |v| < 2^-62, whose products may round to
+// zero, is flagged, and its candidates and its neighbours' are decided by the
+// products themselves.
+//
+// Bound: HBM, the one pass over the values (2.2 KB a leaf).  17.5k leaves
+// (L2-resident) take 12 us for the signs and 8 us for the bits; one thread per
+// voxel with a table lookup per neighbour took 83 us.
+constexpr float kTinyValue = 2.16840434497100887e-19f;  // 2^-62
+
+// One warp per leaf: 16 coalesced rows of 32 values, a ballot each, lane w
+// keeping word w.
+__global__ void __launch_bounds__(256) k_cross_sign(const uint64_t* __restrict__ mask, const float* __restrict__ values,
+                                                   int n, unsigned* __restrict__ pos, unsigned* __restrict__ neg,
+                                                   unsigned* __restrict__ zero, unsigned char* __restrict__ tiny) {
+    const int lane = threadIdx.x & 31;
+    for (int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < n; i += (gridDim.x * blockDim.x) >> 5) {
+        const float* v = values + (size_t)i * kLeafVoxels;
+        const unsigned act = lane < 16 ? reinterpret_cast<const unsigned*>(mask)[(size_t)i * 16 + lane] : 0u;
+        float x[16];
 #pragma unroll
-                for (int q = 0; q < 6; ++q) {
-                    float nv;
-                    bool non;
-                    local_get(g, slot, x + ddx[q], y + ddy[q], z + ddz[q], nv, non);
-                    if (non && __fmul_rn(val, nv) < 0.0f) {
-                        cross = true;
-                        break;
-                    }
-                }
+        for (int w = 0; w < 16; ++w) x[w] = v[w * 32 + lane];
+        unsigned p = 0, m = 0, z = 0;
+        bool t = false;
+#pragma unroll
+        for (int w = 0; w < 16; ++w) {
+            const unsigned bp = __ballot_sync(0xffffffffu, x[w] > 0.0f), bm = __ballot_sync(0xffffffffu, x[w] < 0.0f),
+                           bz = __ballot_sync(0xffffffffu, x[w] == 0.0f);
+            const float a = fabsf(x[w]);
+            const bool on = (__shfl_sync(0xffffffffu, act, w) >> lane) & 1u;
+            t |= on && a > 0.0f && a < kTinyValue;
+            if (lane == w) {
+                p = bp & act;
+                m = bm & act;
+                z = bz & act;
             }
         }
-        unsigned b = __ballot_sync(0xffffffffu, cross);
-        if ((threadIdx.x & 31) == 0) {
-            ((unsigned*)xmask)[(size_t)slot * 16 + (off >> 5)] = b;
-            cnt += __popc(b);
+        const bool any = __any_sync(0xffffffffu, t);
+        if (lane < 16) {
+            pos[(size_t)i * 16 + lane] = p;
+            neg[(size_t)i * 16 + lane] = m;
+            zero[(size_t)i * 16 + lane] = z;
         }
-    }
-    __shared__ int s_cnt;
-    if (threadIdx.x == 0) s_cnt = 0;
-    __syncthreads();
-    if ((threadIdx.x & 31) == 0 && cnt) atomicAdd(&s_cnt, cnt);
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        xcount[slot] = s_cnt;
-        if (s_cnt) atomicAdd(total, (unsigned long long)s_cnt);
+        if (lane == 0) tiny[i] = any;
     }
 }
 
-// Write crossing coordinates of each leaf at its scanned position.
-__global__ void __launch_bounds__(512) k_emit_crossings(GridView g, const uint64_t* __restrict__ xmask,
-                                                       const int* __restrict__ pos, int* __restrict__ coords) {
-    int slot = blockIdx.x;
-    if (slot >= g.n) return;
-    int off = threadIdx.x;
-    const uint64_t* xm = xmask + (size_t)slot * 8;
-    bool on = mask_bit(xm, off);
-    // rank of this bit among the leaf's set bits
-    int w = off >> 6, b = off & 63;
-    int rank = 0;
-    for (int q = 0; q < w; ++q) rank += __popcll(xm[q]);
-    rank += __popcll(xm[w] & ((b == 0) ? 0ull : (~0ull >> (64 - b))));
+// The voxels of plane word (leaf, x) that have a 6-neighbour in mask m (bit
+// y * 8 + z); nb: the leaf's face neighbours -x, +x, -y, +y, -z, +z.
+__device__ __forceinline__ uint64_t near6(const uint64_t* __restrict__ m, int leaf, int x, const int* nb) {
+    constexpr uint64_t Z0 = 0x0101010101010101ull, Z7 = 0x8080808080808080ull;
+    const uint64_t c = m[(size_t)leaf * 8 + x];
+    auto word = [&](int s, int w) { return s >= 0 ? m[(size_t)s * 8 + w] : 0ull; };
+    const uint64_t xm = x > 0 ? m[(size_t)leaf * 8 + x - 1] : word(nb[0], 7);
+    const uint64_t xp = x < 7 ? m[(size_t)leaf * 8 + x + 1] : word(nb[1], 0);
+    return xm | xp | (c << 8) | (c >> 8) | (word(nb[2], x) >> 56) | (word(nb[3], x) << 56) | ((c << 1) & ~Z0) |
+           ((c >> 1) & ~Z7) | ((word(nb[4], x) & Z7) >> 7) | ((word(nb[5], x) & Z0) << 7);
+}
+
+// Where a leaf's rows lie in the list's order.  The pool is sorted by (x, y,
+// z) of origin, so the leaves of one origin x are a run [g0, g0 + gn) and
+// those of one (x, y) a run [c0, c0 + cn) in it; in global (x, y, z) order the
+// run's 8 planes follow one another, in a plane the (x, y) runs, in a run its
+// 8 rows y, in a row the leaves: no sort is needed.
+struct RowPlace {
+    int g0, gn, c0, cn;
+};
+__device__ __forceinline__ size_t row_of(const RowPlace& r, int leaf, int x, int y) {
+    return (size_t)r.g0 * 64 + (size_t)x * 8 * r.gn + (size_t)(r.c0 - r.g0) * 8 + (size_t)y * r.cn + (leaf - r.c0);
+}
+
+// Eight lanes per leaf, one plane word each.  xmask: the zero masks on entry,
+// the crossing masks on return; *any is set when there is one.  rows (when
+// not null): the crossings of each row at its place in the list's order,
+// place[leaf] for the pass that writes them.
+__global__ void __launch_bounds__(256) k_cross_bits(GridView g, const uint64_t* __restrict__ pos,
+                                                   const uint64_t* __restrict__ neg,
+                                                   const unsigned char* __restrict__ tiny, uint64_t* __restrict__ xmask,
+                                                   int* __restrict__ any, int* __restrict__ rows,
+                                                   RowPlace* __restrict__ place) {
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    const int leaf = t >> 3, x = t & 7;
+    const bool on = leaf < g.n;
+    uint64_t cross = 0;
     if (on) {
-        int4 o = g.origin[slot];
-        int j = pos[slot] + rank;
-        coords[3 * j] = o.x + (off >> 6);
-        coords[3 * j + 1] = o.y + ((off >> 3) & 7);
-        coords[3 * j + 2] = o.z + (off & 7);
+        const int* row = g.nbr + (size_t)leaf * kNbr;
+        const int nb[6] = {row[4], row[22], row[10], row[16], row[12], row[14]};
+        const uint64_t p = pos[t], m = neg[t], z = xmask[t];
+        cross = z | (p & near6(neg, leaf, x, nb)) | (m & near6(pos, leaf, x, nb));
+        bool exact = tiny[leaf];
+#pragma unroll
+        for (int q = 0; q < 6; ++q) exact |= nb[q] >= 0 && tiny[nb[q]];
+        if (exact) {
+            for (uint64_t w = cross & ~z; w; w &= w - 1) {
+                const int b = __ffsll((long long)w) - 1, y = b >> 3, zz = b & 7;
+                const float val = g.values[(size_t)leaf * kLeafVoxels + x * 64 + b];
+                bool yes = false;
+                for (int q = 0; q < 6; ++q) {
+                    const int s = (q & 1) ? 1 : -1;
+                    float nv;
+                    bool non;
+                    local_get(g, leaf, x + (q >> 1 == 0 ? s : 0), y + (q >> 1 == 1 ? s : 0), zz + (q >> 1 == 2 ? s : 0),
+                              nv, non);
+                    yes |= non && __fmul_rn(val, nv) < 0.0f;
+                }
+                if (!yes) cross &= ~(1ull << b);
+            }
+        }
+        xmask[t] = cross;
+    }
+    if (__any_sync(0xffffffffu, cross != 0ull) && (threadIdx.x & 31) == 0) *any = 1;
+    if (!rows) return;
+    // lane x of a leaf's eight searches one end of its runs: first leaf with
+    // the same x, first with a larger x, and the same for (x, y)
+    int lo = 0;
+    if (on && x < 4) {
+        const int4 o = g.origin[leaf];
+        int hi = g.n;
+        while (lo < hi) {
+            const int mid = lo + ((hi - lo) >> 1);
+            const int4 c = g.origin[mid];
+            const bool less = c.x < o.x || (x >= 2 && c.x == o.x && c.y < o.y);
+            const bool same = c.x == o.x && (x < 2 || c.y == o.y);
+            if (less || ((x & 1) && same)) lo = mid + 1;
+            else hi = mid;
+        }
+    }
+    const int base = threadIdx.x & 24;
+    RowPlace r;
+    r.g0 = __shfl_sync(0xffffffffu, lo, base);
+    r.gn = __shfl_sync(0xffffffffu, lo, base + 1) - r.g0;
+    r.c0 = __shfl_sync(0xffffffffu, lo, base + 2);
+    r.cn = __shfl_sync(0xffffffffu, lo, base + 3) - r.c0;
+    if (!on) return;
+    if (x == 0) place[leaf] = r;
+#pragma unroll
+    for (int y = 0; y < 8; ++y) rows[row_of(r, leaf, x, y)] = __popc((unsigned)(cross >> (8 * y)) & 0xffu);
+}
+
+// The crossings of each row (64 threads per leaf, one row each) at its scanned position.
+__global__ void __launch_bounds__(256) k_emit_crossings(GridView g, const uint64_t* __restrict__ xmask,
+                                                       const int* __restrict__ rows,
+                                                       const RowPlace* __restrict__ place, int* __restrict__ coords) {
+    const int leaf = (blockIdx.x * blockDim.x + threadIdx.x) >> 6, r = threadIdx.x & 63;
+    if (leaf >= g.n) return;
+    unsigned b = reinterpret_cast<const unsigned char*>(xmask)[(size_t)leaf * 64 + r];
+    if (!b) return;
+    const int x = r >> 3, y = r & 7;
+    const int4 o = g.origin[leaf];
+    size_t j = 3 * (size_t)rows[row_of(place[leaf], leaf, x, y)];
+    for (; b; b &= b - 1, j += 3) {
+        coords[j] = o.x + x;
+        coords[j + 1] = o.y + y;
+        coords[j + 2] = o.z + __ffs(b) - 1;
     }
 }
 
@@ -403,159 +494,85 @@ int sample_points(vlr_ctx* ctx, const vlr_grid* g, const double* h_pts, size_t n
     return VLR_OK;
 }
 
-// Crossing masks and counts on the device; *total_out is the crossing count.
-int crossings(vlr_ctx* ctx, const vlr_grid* g, uint64_t* d_xmask, int* d_xcount, unsigned long long* d_total,
-              unsigned long long* total_out) {
-    VLR_CUDA(ctx, cudaMemsetAsync(d_total, 0, sizeof(unsigned long long), ctx->stream));
-    if (g->n > 0)
-        VLR_TIMED(ctx, "k_crossings",
-                  k_crossings<<<g->n, 256, 0, ctx->stream>>>(make_view(g), d_xmask, d_xcount, d_total));
-    VLR_CUDA(ctx, cudaGetLastError());
-    unsigned long long* h = (unsigned long long*)ctx->pinned;
-    VLR_CUDA(ctx, cudaMemcpyAsync(h, d_total, sizeof(unsigned long long), cudaMemcpyDeviceToHost, ctx->stream));
-    VLR_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-    *total_out = *h;
-    return VLR_OK;
-}
-
+// Device buffers of a crossing search over n leaves, in one block.
 struct CrossBufs {
-    uint64_t* xmask = nullptr;
-    int* xcount = nullptr;
-    int* pos = nullptr;
-    unsigned long long* total = nullptr;
-    int* flags = nullptr;
+    char* block = nullptr;
+    uint64_t* xmask = nullptr;  // crossing masks
+    uint64_t* pos = nullptr;
+    uint64_t* neg = nullptr;
+    unsigned char* tiny = nullptr;
+    int* any = nullptr;         // 1 when there is a crossing
+    int* total = nullptr;       // their number (with rows)
+    int* flags = nullptr;       // one int per leaf, for the caller
+    int* rows = nullptr;        // 64 n ints
+    RowPlace* place = nullptr;
 };
 
-static int alloc_cross(vlr_ctx* ctx, int n, CrossBufs& b) {
-    size_t need = sizeof(uint64_t) * 8 * (size_t)n + sizeof(int) * (3 * (size_t)n + 8) + 64;
-    char* p = nullptr;
-    VLR_CUDA(ctx, cudaMallocFromPoolAsync((void**)&p, need, ctx->pool, ctx->stream));
-    b.xmask = (uint64_t*)p;
-    p += sizeof(uint64_t) * 8 * (size_t)n;
-    b.total = (unsigned long long*)p;
-    p += 16;
-    b.xcount = (int*)p;
-    p += sizeof(int) * ((size_t)n + 1);
-    b.pos = (int*)p;
-    p += sizeof(int) * ((size_t)n + 1);
-    b.flags = (int*)p;
+static int alloc_cross(vlr_ctx* ctx, int n, bool rows, CrossBufs& b) {
+    const size_t m = (size_t)n;
+    auto up = [](size_t v) { return (v + 255) & ~(size_t)255; };
+    const size_t need = up(192 * m) + up(m) + 256 + up(4 * m) + (rows ? up(sizeof(RowPlace) * m) + up(256 * m) : 0);
+    VLR_CUDA(ctx, cudaMallocFromPoolAsync((void**)&b.block, need, ctx->pool, ctx->stream));
+    char* p = b.block;
+    auto take = [&](size_t v) {
+        char* r = p;
+        p += up(v);
+        return r;
+    };
+    b.xmask = (uint64_t*)take(192 * m);
+    b.pos = b.xmask + 8 * m;
+    b.neg = b.pos + 8 * m;
+    b.tiny = (unsigned char*)take(m);
+    b.any = (int*)take(8);
+    b.total = b.any + 1;
+    b.flags = (int*)take(4 * m);
+    if (rows) {
+        b.place = (RowPlace*)take(sizeof(RowPlace) * m);
+        b.rows = (int*)take(256 * m);
+    }
     return VLR_OK;
 }
 
-// Crossing-list sort on the device: the bounding box of the coordinates, then
-// (x, y, z)-major keys of their offsets to it, radix-sorted with the list
-// index.
-__global__ void k_cross_box(const int* __restrict__ c, int n, int* __restrict__ box) {
-    int lo[3] = {INT_MAX, INT_MAX, INT_MAX}, hi[3] = {INT_MIN, INT_MIN, INT_MIN};
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-        for (int a = 0; a < 3; ++a) {
-            lo[a] = min(lo[a], c[3 * i + a]);
-            hi[a] = max(hi[a], c[3 * i + a]);
-        }
-    for (int a = 0; a < 3; ++a) {
-        lo[a] = __reduce_min_sync(0xffffffffu, lo[a]);
-        hi[a] = __reduce_max_sync(0xffffffffu, hi[a]);
-    }
-    if ((threadIdx.x & 31) == 0)
-        for (int a = 0; a < 3; ++a) {
-            atomicMin(&box[a], lo[a]);
-            atomicMax(&box[3 + a], hi[a]);
-        }
-}
-
-__global__ void k_cross_keys(const int* __restrict__ c, int n, int bx, int by, int bz, int bits,
-                             uint64_t* __restrict__ keys, unsigned* __restrict__ idx) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const uint64_t k = ((uint64_t)(unsigned)(c[3 * i] - bx) << (2 * bits)) |
-                           ((uint64_t)(unsigned)(c[3 * i + 1] - by) << bits) | (uint64_t)(unsigned)(c[3 * i + 2] - bz);
-        keys[i] = k;
-        idx[i] = (unsigned)i;
-    }
-}
-
-__global__ void k_cross_gather(const int* __restrict__ c, const unsigned* __restrict__ idx, int n,
-                               int* __restrict__ out) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < 3 * n; i += gridDim.x * blockDim.x)
-        out[i] = c[3 * idx[i / 3] + i % 3];
-}
-
-// Sorts the n crossing coordinates d_c into d_out by (x, y, z) on the device;
-// *sorted = false (nothing written) when the box needs keys over 63 bits.
-static int sort_crossings_device(vlr_ctx* ctx, const int* d_c, int n, int* d_out, bool* sorted) {
-    *sorted = false;
+// Crossing masks (and row counts, scanned into positions) on the device, enqueued.
+static int crossings(vlr_ctx* ctx, const vlr_grid* g, CrossBufs& b) {
     cudaStream_t st = ctx->stream;
-    const size_t sort_bytes = radix_scratch_bytes(n, 8);
-    char* buf = nullptr;
-    VLR_CUDA(ctx, cudaMallocFromPoolAsync((void**)&buf, (size_t)n * 20 + sort_bytes + 256, ctx->pool, st));
-    auto done = [&](int code) {
-        cudaFreeAsync(buf, st);
-        return code;
-    };
-    char* p = buf;
-    uint64_t* keys = (uint64_t*)p;  p += (size_t)n * 8;
-    unsigned* idx = (unsigned*)p;  p += (size_t)n * 4;
-    int* box = (int*)(((uintptr_t)p + 15) & ~(uintptr_t)15);
-    void* scratch = (void*)(((uintptr_t)(box + 8) + 15) & ~(uintptr_t)15);
-    const int init[6] = {INT_MAX, INT_MAX, INT_MAX, INT_MIN, INT_MIN, INT_MIN};
-    int* hb = static_cast<int*>(ctx->pinned) + 32;
-    std::memcpy(hb, init, sizeof(init));
-    VLR_CUDA(ctx, cudaMemcpyAsync(box, hb, sizeof(init), cudaMemcpyHostToDevice, st));
-    const int blocks = ctx->sm_count * 8;
-    k_cross_box<<<blocks, 256, 0, st>>>(d_c, n, box);
-    VLR_CUDA(ctx, cudaMemcpyAsync(hb, box, sizeof(init), cudaMemcpyDeviceToHost, st));
-    VLR_CUDA(ctx, cudaStreamSynchronize(st));
-    int bits = 0;
-    for (int a = 0; a < 3; ++a) {
-        const long long ext = (long long)hb[3 + a] - hb[a];
-        while (bits < 40 && (1ll << bits) <= ext) ++bits;
-    }
-    if (3 * bits > 63) return done(VLR_OK);
-    k_cross_keys<<<blocks, 256, 0, st>>>(d_c, n, hb[0], hb[1], hb[2], bits, keys, idx);
-    uint64_t* sorted_keys;
-    unsigned* order;
-    int rc = radix_sort(ctx, keys, idx, n, 3 * bits, scratch, &sorted_keys, &order);
-    if (rc) return done(rc);
-    k_cross_gather<<<blocks, 256, 0, st>>>(d_c, order, n, d_out);
+    VLR_CUDA(ctx, cudaMemsetAsync(b.any, 0, 2 * sizeof(int), st));
+    const int n = g->n;
+    VLR_TIMED(ctx, "k_cross_sign",
+              k_cross_sign<<<std::min((n + 7) / 8, ctx->sm_count * 8), 256, 0, st>>>(
+                  g->mask, (const float*)g->values, n, (unsigned*)b.pos, (unsigned*)b.neg, (unsigned*)b.xmask, b.tiny));
+    VLR_TIMED(ctx, "k_crossings", k_cross_bits<<<(n + 31) / 32, 256, 0, st>>>(make_view(g), b.pos, b.neg, b.tiny,
+                                                                             b.xmask, b.any, b.rows, b.place));
     VLR_CUDA(ctx, cudaGetLastError());
-    *sorted = true;
-    return done(VLR_OK);
+    return b.rows ? scan_exclusive(ctx, b.rows, b.rows, 64ll * n, b.total) : VLR_OK;
 }
 
-int find_zero_crossings(vlr_ctx* ctx, const vlr_grid* g, int32_t* h_coords, size_t cap, size_t* count,
-                        bool* sorted) {
+static void emit_crossings(vlr_ctx* ctx, const vlr_grid* g, const CrossBufs& b, int* d_coords) {
+    k_emit_crossings<<<(g->n + 3) / 4, 256, 0, ctx->stream>>>(make_view(g), b.xmask, b.rows, b.place, d_coords);
+}
+
+int find_zero_crossings(vlr_ctx* ctx, const vlr_grid* g, int32_t* h_coords, size_t cap, size_t* count) {
     *count = 0;
     if (g->n == 0) return VLR_OK;
     CrossBufs b;
-    int rc = alloc_cross(ctx, g->n, b);
-    if (rc) return rc;
-    unsigned long long total = 0;
-    rc = crossings(ctx, g, b.xmask, b.xcount, b.total, &total);
-    if (rc) return rc;
-    *count = (size_t)total;
-    if (total > 0 && h_coords && cap > 0) {
-        rc = scan_exclusive(ctx, b.xcount, b.pos, g->n, b.pos + g->n);
+    int* d_coords = nullptr;
+    auto run = [&]() -> int {
+        int rc = alloc_cross(ctx, g->n, true, b);
+        if (!rc) rc = crossings(ctx, g, b);
+        int total = 0;
+        if (!rc) rc = read_int(ctx, b.total, &total);
         if (rc) return rc;
-        int* d_coords = nullptr;
-        VLR_CUDA(ctx, cudaMallocFromPoolAsync(&d_coords, sizeof(int) * 6 * total, ctx->pool, ctx->stream));
-        k_emit_crossings<<<g->n, 512, 0, ctx->stream>>>(make_view(g), b.xmask, b.pos, d_coords);
+        *count = (size_t)total;
+        if (total == 0 || !h_coords || cap == 0) return VLR_OK;
+        VLR_CUDA(ctx, cudaMallocFromPoolAsync(&d_coords, sizeof(int) * 3 * (size_t)total, ctx->pool, ctx->stream));
+        emit_crossings(ctx, g, b, d_coords);
         VLR_CUDA(ctx, cudaGetLastError());
-        // emitted leaf by leaf (leaves in (x, y, z) order, voxels ZYX), which
-        // is not the global (x, y, z) order: sorted on the device when the
-        // keys fit 63 bits, else by the caller on the host
-        bool dev_sorted = false;
-        if (sorted) {
-            rc = sort_crossings_device(ctx, d_coords, (int)total, d_coords + 3 * total, &dev_sorted);
-            if (rc) return rc;
-        }
-        const int* src = dev_sorted ? d_coords + 3 * total : d_coords;
-        size_t m = std::min<size_t>(cap, total);
-        VLR_CUDA(ctx, cudaMemcpyAsync(h_coords, src, sizeof(int) * 3 * m, cudaMemcpyDeviceToHost, ctx->stream));
-        VLR_CUDA(ctx, cudaFreeAsync(d_coords, ctx->stream));
-        VLR_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-        if (sorted) *sorted = dev_sorted;
-    }
-    VLR_CUDA(ctx, cudaFreeAsync(b.xmask, ctx->stream));
-    return VLR_OK;
+        return d2h_copy(ctx, h_coords, d_coords, sizeof(int) * 3 * std::min<size_t>(cap, (size_t)total));
+    };
+    const int rc = run();
+    if (d_coords) cudaFreeAsync(d_coords, ctx->stream);
+    if (b.block) cudaFreeAsync(b.block, ctx->stream);
+    return rc;
 }
 
 int trim_narrow_band(vlr_ctx* ctx, vlr_grid* g, float half_width) {
@@ -577,38 +594,36 @@ int rebuild_narrow_band(vlr_ctx* ctx, vlr_grid* g, float half_width) {
     if (g->n == 0) return VLR_OK;
     float vs = (float)g->xf.voxel_size;
     float band = half_width * vs;
+    const bool window = std::isfinite(half_width) && vs > 0.0f && half_width <= 9.0f;
     CrossBufs b;
-    int rc = alloc_cross(ctx, g->n, b);
-    if (rc) return rc;
-    unsigned long long total = 0;
-    rc = crossings(ctx, g, b.xmask, b.xcount, b.total, &total);
-    if (rc) return rc;
-    if (total == 0) {  // no crossings: the grid is returned unchanged (level_set_track.rs:85-87)
-        VLR_CUDA(ctx, cudaFreeAsync(b.xmask, ctx->stream));
-        return VLR_OK;
-    }
-    GridView v = make_view(g);
-    bool window = std::isfinite(half_width) && vs > 0.0f && half_width <= 9.0f;
-    if (window) {
-        int R = std::max(0, (int)std::ceil(half_width) - 1);
-        VLR_TIMED(ctx, "k_rebuild_window",
-                  k_rebuild_window<<<g->n, 256, 0, ctx->stream>>>(v, (float*)g->values, g->mask, b.xmask, R, vs,
-                                                                 band, b.flags));
-    } else {
-        rc = scan_exclusive(ctx, b.xcount, b.pos, g->n, b.pos + g->n);
+    int* d_coords = nullptr;
+    auto run = [&]() -> int {
+        int rc = alloc_cross(ctx, g->n, !window, b);
+        if (!rc) rc = crossings(ctx, g, b);
+        int total = 0;
+        if (!rc) rc = read_int(ctx, window ? b.any : b.total, &total);
         if (rc) return rc;
-        int* d_coords = nullptr;
-        VLR_CUDA(ctx, cudaMallocFromPoolAsync(&d_coords, sizeof(int) * 3 * total, ctx->pool, ctx->stream));
-        k_emit_crossings<<<g->n, 512, 0, ctx->stream>>>(v, b.xmask, b.pos, d_coords);
-        k_rebuild_brute<<<g->n, 256, 0, ctx->stream>>>(v, (float*)g->values, g->mask, d_coords, (int)total, vs, band,
-                                                      b.flags);
-        VLR_CUDA(ctx, cudaFreeAsync(d_coords, ctx->stream));
-    }
-    VLR_CUDA(ctx, cudaGetLastError());
-    rc = grid_compact(ctx, g, b.flags);
-    if (rc) return rc;
-    VLR_CUDA(ctx, cudaFreeAsync(b.xmask, ctx->stream));
-    return consume_device_errors(ctx, "rebuild_narrow_band");
+        if (total == 0) return VLR_OK;  // no crossings: the grid is returned unchanged (level_set_track.rs:85-87)
+        GridView v = make_view(g);
+        if (window) {
+            int R = std::max(0, (int)std::ceil(half_width) - 1);
+            VLR_TIMED(ctx, "k_rebuild_window",
+                      k_rebuild_window<<<g->n, 256, 0, ctx->stream>>>(v, (float*)g->values, g->mask, b.xmask, R, vs,
+                                                                     band, b.flags));
+        } else {
+            VLR_CUDA(ctx, cudaMallocFromPoolAsync(&d_coords, sizeof(int) * 3 * (size_t)total, ctx->pool, ctx->stream));
+            emit_crossings(ctx, g, b, d_coords);
+            k_rebuild_brute<<<g->n, 256, 0, ctx->stream>>>(v, (float*)g->values, g->mask, d_coords, total, vs, band,
+                                                          b.flags);
+        }
+        VLR_CUDA(ctx, cudaGetLastError());
+        rc = grid_compact(ctx, g, b.flags);
+        return rc ? rc : consume_device_errors(ctx, "rebuild_narrow_band");
+    };
+    const int rc = run();
+    if (d_coords) cudaFreeAsync(d_coords, ctx->stream);
+    if (b.block) cudaFreeAsync(b.block, ctx->stream);
+    return rc;
 }
 
 static int32_t sat_i32(double v) {

@@ -125,8 +125,8 @@ int choose_base(vlr_ctx* ctx, const int32_t* origins, size_t n, long long base[3
 int grid_compact(vlr_ctx* ctx, vlr_grid* g, const int* d_flags);
 // Scratch memory owned by the context (valid until the next call that grows it).
 int ctx_scratch(vlr_ctx* ctx, size_t bytes, void** out);
-// Exclusive scan of n ints on the context stream; writes total to *d_total (device).
-int scan_exclusive(vlr_ctx* ctx, const int* d_in, int* d_out, int n, int* d_total);
+// Exclusive scan of n ints on the context stream (d_out may be d_in); writes total to *d_total (device).
+int scan_exclusive(vlr_ctx* ctx, const int* d_in, int* d_out, long long n, int* d_total);
 // Read the device error word, clear it, and map it to a status.
 int consume_device_errors(vlr_ctx* ctx, const char* what);
 // Device-to-host copy of `bytes` on the context stream, returning after it.

@@ -1,0 +1,37 @@
+"""The bit-mask forms of the crate's band tools where masks could go wrong:
+values whose products underflow, infinities, NaN, signed zeros and denormals,
+leaves far apart, and half-empty neighbourhoods; bit-exact against the oracle."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+SPECIAL = np.array([0.0, -0.0, 1e-40, -1e-40, 1e-30, -1e-30, 3e-23, -3e-23, 2.0 ** -62, -2.0 ** -62, 2.0 ** -63, 0.5,
+                    -0.5, 3e38, -3e38, np.inf, -np.inf, np.nan], np.float32)
+
+
+def special_grid(seed, n, spread, fill, mix):
+    """Random leaves; `mix` of the values are drawn from SPECIAL, the rest normal."""
+    from sharc.volrus_b200 import Grid
+    rng = np.random.default_rng(seed)
+    o = np.unique(rng.integers(-spread, spread, (n, 3)), axis=0).astype(np.int32) * 8
+    n = len(o)
+    on = rng.random((n, 512)) < fill
+    v = np.where(rng.random((n, 512)) < mix, rng.choice(SPECIAL, (n, 512)), rng.normal(0, 1, (n, 512)))
+    m = np.packbits(on, axis=1, bitorder="little").view(np.uint64)
+    return Grid.from_arrays(o, m, v.astype(np.float32), 2.0, None)
+
+
+def to_oracle(oracle, g):
+    o, m, v = g.to_arrays()
+    return oracle.OGrid.from_arrays(o, m, v, g.background, g.transform.voxel_size, g.transform.origin, g.affine.mat,
+                                    g.affine.voxel_size)
+
+
+@pytest.mark.parametrize("seed,n,spread,fill,mix", [(1, 40, 2, 0.7, 0.0), (2, 40, 2, 0.7, 0.4), (3, 60, 3, 0.5, 1.0),
+                                                    (4, 1, 1, 0.9, 0.3), (5, 300, 100000, 0.2, 0.1),
+                                                    (6, 33, 40, 1.0, 0.05)])
+def test_crossings_match_oracle(oracle, seed, n, spread, fill, mix):
+    from sharc.volrus_b200 import find_zero_crossings
+    g = special_grid(seed, n, spread, fill, mix)
+    assert np.array_equal(find_zero_crossings(g), to_oracle(oracle, g).zero_crossings())
