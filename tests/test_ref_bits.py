@@ -35,3 +35,18 @@ def test_crossings_match_oracle(oracle, seed, n, spread, fill, mix):
     from sharc.volrus_b200 import find_zero_crossings
     g = special_grid(seed, n, spread, fill, mix)
     assert np.array_equal(find_zero_crossings(g), to_oracle(oracle, g).zero_crossings())
+
+
+@pytest.mark.parametrize("hw", [0.4, 1.0, 1.7, 2.0, 2.6, 3.0, 3.2, 4.0])
+@pytest.mark.parametrize("seed,n,spread,fill,mix", [(7, 40, 2, 0.7, 0.02), (8, 25, 2, 1.0, 0.3), (9, 5, 50, 0.1, 0.0)])
+def test_rebuild_rows_match_oracle(oracle, hw, seed, n, spread, fill, mix):
+    """Windows of half size 0 to 3: whole rows up to 2, voxel windows above; sparse and crowded crossings."""
+    from sharc.volrus_b200 import rebuild_narrow_band
+    g = special_grid(seed, n, spread, fill, mix)
+    og = to_oracle(oracle, g)
+    rebuild_narrow_band(g, hw)
+    og.rebuild(hw, brute=True)
+    o1, m1, v1 = g.to_arrays()
+    o2, m2, v2 = og.arrays()
+    assert np.array_equal(o1, o2) and np.array_equal(m1, m2)
+    assert np.array_equal(v1.view(np.uint32), v2.view(np.uint32))
