@@ -131,11 +131,8 @@ int d2h_copy(vlr_ctx* ctx, void* dst, const void* src, size_t bytes) {
     return VLR_OK;
 }
 
-int consume_device_errors(vlr_ctx* ctx, const char* what) {
-    unsigned* h = (unsigned*)ctx->pinned;
-    VLR_CUDA(ctx, cudaMemcpyAsync(h, ctx->d_errword, sizeof(unsigned), cudaMemcpyDeviceToHost, ctx->stream));
-    VLR_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-    unsigned e = *h;
+// The status of error word e, reported as `what`; clears the word on the device.
+static int map_device_errors(vlr_ctx* ctx, unsigned e, const char* what) {
     if (!e) return VLR_OK;
     VLR_CUDA(ctx, cudaMemsetAsync(ctx->d_errword, 0, sizeof(unsigned), ctx->stream));
     std::string m = std::string(what) + ": device reported";
@@ -151,6 +148,22 @@ int consume_device_errors(vlr_ctx* ctx, const char* what) {
         code = VLR_ERR_INVALID;
     }
     return set_error(ctx, code, m);
+}
+
+int consume_device_errors(vlr_ctx* ctx, const char* what) {
+    unsigned* h = (unsigned*)ctx->pinned;
+    VLR_CUDA(ctx, cudaMemcpyAsync(h, ctx->d_errword, sizeof(unsigned), cudaMemcpyDeviceToHost, ctx->stream));
+    VLR_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    return map_device_errors(ctx, *h, what);
+}
+
+int read_int_checked(vlr_ctx* ctx, const int* d_ptr, int* out, const char* what) {
+    unsigned* h = (unsigned*)ctx->pinned;
+    VLR_CUDA(ctx, cudaMemcpyAsync(h + 1, d_ptr, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
+    VLR_CUDA(ctx, cudaMemcpyAsync(h, ctx->d_errword, sizeof(unsigned), cudaMemcpyDeviceToHost, ctx->stream));
+    VLR_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    *out = (int)h[1];
+    return map_device_errors(ctx, h[0], what);
 }
 
 void grid_free_arrays(vlr_grid* g) {
@@ -229,11 +242,14 @@ int choose_base(vlr_ctx* ctx, const int32_t* origins, size_t n, long long base[3
 
 // ---------------------------------------------------------------- kernels
 
-__global__ void k_hash_clear(uint64_t* key, int* val, int cap) {
+// Empty keys, values that every inserted slot is below (atomicMin), and the
+// duplicate flag.
+__global__ void k_hash_clear(uint64_t* key, int* val, int cap, int* dup) {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < cap; i += gridDim.x * blockDim.x) {
         key[i] = kEmptyKey;
-        val[i] = -1;
+        val[i] = INT_MAX;
     }
+    if (blockIdx.x == 0 && threadIdx.x == 0) *dup = 0;
 }
 
 __global__ void k_hash_insert(const int4* origin, int n, uint64_t* hkey, int* hval, int hcap, long long b0,
@@ -262,12 +278,6 @@ __global__ void k_hash_insert(const int4* origin, int n, uint64_t* hkey, int* hv
     atomicOr(err, kErrHashFull);
 }
 
-// hval starts at -1 after clear; atomicMin(-1, i) would keep -1, so inserts
-// first turn -1 into INT_MAX.
-__global__ void k_hash_prep_vals(int* val, int cap) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < cap; i += gridDim.x * blockDim.x) val[i] = INT_MAX;
-}
-
 __global__ void k_nbr_build(const int4* origin, int n, const uint64_t* hkey, const int* hval, int hcap, long long b0,
                             long long b1, long long b2, int* nbr, int* dup_flag) {
     int t = blockIdx.x * blockDim.x + threadIdx.x;
@@ -285,28 +295,24 @@ int grid_index(vlr_ctx* ctx, vlr_grid* g) {
     int hc = g->hcap;
     int thr = 256;
     int blocks = std::min((hc + thr - 1) / thr, ctx->sm_count * 8);
-    k_hash_clear<<<blocks, thr, 0, ctx->stream>>>(g->hkey, g->hval, hc);
-    k_hash_prep_vals<<<blocks, thr, 0, ctx->stream>>>(g->hval, hc);
+    void* sp;
+    int rc = ctx_scratch(ctx, sizeof(int), &sp);
+    if (rc) return rc;
+    int* dup = (int*)sp;
+    k_hash_clear<<<blocks, thr, 0, ctx->stream>>>(g->hkey, g->hval, hc, dup);
     if (g->n > 0) {
         k_hash_insert<<<(g->n + thr - 1) / thr, thr, 0, ctx->stream>>>(g->origin, g->n, g->hkey, g->hval, hc,
                                                                      g->base[0], g->base[1], g->base[2],
                                                                      ctx->d_errword);
-        void* sp;
-        int rc = ctx_scratch(ctx, sizeof(int), &sp);
-        if (rc) return rc;
-        int* dup = (int*)sp;
-        VLR_CUDA(ctx, cudaMemsetAsync(dup, 0, sizeof(int), ctx->stream));
         long long tot = (long long)g->n * kNbr;
         k_nbr_build<<<(unsigned)((tot + thr - 1) / thr), thr, 0, ctx->stream>>>(
             g->origin, g->n, g->hkey, g->hval, hc, g->base[0], g->base[1], g->base[2], g->nbr, dup);
-        VLR_CUDA(ctx, cudaGetLastError());
-        int h_dup = 0;
-        int r2 = read_int(ctx, dup, &h_dup);
-        if (r2) return r2;
-        if (h_dup) return set_error(ctx, VLR_ERR_INVALID, "duplicate leaf origin");
     }
     VLR_CUDA(ctx, cudaGetLastError());
-    return consume_device_errors(ctx, "grid index");
+    int h_dup = 0;
+    rc = read_int_checked(ctx, dup, &h_dup, "grid index");
+    if (h_dup) return set_error(ctx, VLR_ERR_INVALID, "duplicate leaf origin");
+    return rc;
 }
 
 // ------------------------------------------------------------------ scan
@@ -421,36 +427,48 @@ __global__ void k_compact_leaves(int n, const int* flags, const int* pos, const 
     for (int t = threadIdx.x; t < kVec; t += blockDim.x) dst[t] = src[t];
 }
 
-int grid_compact(vlr_ctx* ctx, vlr_grid* g, const int* d_flags) {
+int grid_compact(vlr_ctx* ctx, vlr_grid* g, const int* d_flags, const char* what, const vlr_grid* index) {
     if (g->n == 0) return VLR_OK;
     int* pos = nullptr;
     VLR_CUDA(ctx, cudaMallocFromPoolAsync(&pos, sizeof(int) * (g->n + 1), ctx->pool, ctx->stream));
-    int* d_total = pos + g->n;
-    int rc = scan_exclusive(ctx, d_flags, pos, g->n, d_total);
-    if (rc) return rc;
-    int total = 0;
-    rc = read_int(ctx, d_total, &total);
-    if (rc) return rc;
-    if (total == g->n) {
-        VLR_CUDA(ctx, cudaFreeAsync(pos, ctx->stream));
-        return VLR_OK;
-    }
     vlr_grid tmp;
     tmp.ctx = ctx;
     tmp.kind = g->kind;
-    rc = grid_alloc(ctx, &tmp, std::max(total, 1));
-    if (rc) return rc;
-    if (g->kind == VLR_KIND_F16_VOXEL)
-        k_compact_leaves<__half><<<g->n, 64, 0, ctx->stream>>>(g->n, d_flags, pos, g->origin, g->mask,
-                                                              (const __half*)g->values, tmp.origin, tmp.mask,
-                                                              (__half*)tmp.values);
-    else
-        k_compact_leaves<float><<<g->n, 128, 0, ctx->stream>>>(g->n, d_flags, pos, g->origin, g->mask,
-                                                              (const float*)g->values, tmp.origin, tmp.mask,
-                                                              (float*)tmp.values);
-    VLR_CUDA(ctx, cudaGetLastError());
-    VLR_CUDA(ctx, cudaFreeAsync(pos, ctx->stream));
-    VLR_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    int total = 0;
+    auto run = [&]() -> int {
+        int rc = scan_exclusive(ctx, d_flags, pos, g->n, pos + g->n);
+        if (!rc) rc = read_int_checked(ctx, pos + g->n, &total, what);
+        if (rc || total == g->n) return rc;
+        rc = grid_alloc(ctx, &tmp, std::max(total, 1));
+        if (rc) return rc;
+        if (g->kind == VLR_KIND_F16_VOXEL)
+            k_compact_leaves<__half><<<g->n, 64, 0, ctx->stream>>>(g->n, d_flags, pos, g->origin, g->mask,
+                                                                  (const __half*)g->values, tmp.origin, tmp.mask,
+                                                                  (__half*)tmp.values);
+        else
+            k_compact_leaves<float><<<g->n, 128, 0, ctx->stream>>>(g->n, d_flags, pos, g->origin, g->mask,
+                                                                  (const float*)g->values, tmp.origin, tmp.mask,
+                                                                  (float*)tmp.values);
+        VLR_CUDA(ctx, cudaGetLastError());
+        return VLR_OK;
+    };
+    const int rc = run();
+    cudaFreeAsync(pos, ctx->stream);
+    if (rc) {
+        grid_free_arrays(&tmp);
+        return rc;
+    }
+    if (total == g->n) {
+        if (!index) return VLR_OK;
+        if (index->hcap != g->hcap) return grid_index(ctx, g);
+        VLR_CUDA(ctx, cudaMemcpyAsync(g->nbr, index->nbr, sizeof(int) * kNbr * (size_t)g->n, cudaMemcpyDeviceToDevice,
+                                      ctx->stream));
+        VLR_CUDA(ctx, cudaMemcpyAsync(g->hkey, index->hkey, sizeof(uint64_t) * g->hcap, cudaMemcpyDeviceToDevice,
+                                      ctx->stream));
+        VLR_CUDA(ctx, cudaMemcpyAsync(g->hval, index->hval, sizeof(int) * g->hcap, cudaMemcpyDeviceToDevice,
+                                      ctx->stream));
+        return VLR_OK;
+    }
     std::swap(g->block, tmp.block);
     std::swap(g->origin, tmp.origin);
     std::swap(g->mask, tmp.mask);
@@ -460,7 +478,7 @@ int grid_compact(vlr_ctx* ctx, vlr_grid* g, const int* d_flags) {
     std::swap(g->hval, tmp.hval);
     std::swap(g->hcap, tmp.hcap);
     std::swap(g->cap, tmp.cap);
-    grid_free_arrays(&tmp);
+    grid_free_arrays(&tmp);  // stream-ordered: after the copy
     g->n = total;
     return grid_index(ctx, g);
 }

@@ -121,8 +121,10 @@ void grid_free_arrays(vlr_grid* g);
 int grid_index(vlr_ctx* ctx, vlr_grid* g);
 // Choose the hash-key base from the leaf-coordinate bounding box (host origins).
 int choose_base(vlr_ctx* ctx, const int32_t* origins, size_t n, long long base[3]);
-// Keep slots whose flag is non-zero (order preserved); rebuilds the index.
-int grid_compact(vlr_ctx* ctx, vlr_grid* g, const int* d_flags);
+// Keep slots whose flag is non-zero (order preserved); rebuilds the index when
+// some are dropped, else copies it from `index` when one is given (a grid with
+// the same leaves in the same slots).  Reports device errors as `what`.
+int grid_compact(vlr_ctx* ctx, vlr_grid* g, const int* d_flags, const char* what, const vlr_grid* index = nullptr);
 // Scratch memory owned by the context (valid until the next call that grows it).
 int ctx_scratch(vlr_ctx* ctx, size_t bytes, void** out);
 // Exclusive scan of n ints on the context stream (d_out may be d_in); writes total to *d_total (device).
@@ -135,6 +137,8 @@ int consume_device_errors(vlr_ctx* ctx, const char* what);
 // driver's own pageable rate here; small or pinned destinations take one copy.
 int d2h_copy(vlr_ctx* ctx, void* dst, const void* src, size_t bytes);
 int read_int(vlr_ctx* ctx, const int* d_ptr, int* out);
+// read_int and consume_device_errors in one round trip.
+int read_int_checked(vlr_ctx* ctx, const int* d_ptr, int* out, const char* what);
 
 // Kernel timing: bracket a launch with timer_begin/timer_end (no-ops unless
 // profiling is enabled); timer_collect folds finished event pairs into totals.

@@ -50,3 +50,28 @@ def test_rebuild_rows_match_oracle(oracle, hw, seed, n, spread, fill, mix):
     o2, m2, v2 = og.arrays()
     assert np.array_equal(o1, o2) and np.array_equal(m1, m2)
     assert np.array_equal(v1.view(np.uint32), v2.view(np.uint32))
+
+
+@pytest.mark.parametrize("same", [True, False], ids=["one-transform", "own-transforms"])
+@pytest.mark.parametrize("dt", [0.0, 0.37, 30.0])
+@pytest.mark.parametrize("seed,n,fill", [(11, 1, 1.0), (12, 3, 0.01), (13, 120, 0.3), (14, 40, 0.9)])
+def test_advect_sampled_fields_match_oracle(oracle, same, dt, seed, n, fill):
+    """Velocity grids over part of the level set's leaves, with one transform or three; samples inside the hinted
+    neighbourhood, across its faces and far outside it; leaves without active voxels."""
+    from sharc.volrus_b200 import VelocityField, VoxelTransform, advect_level_set
+    g = special_grid(seed, n, 2, fill, 0.02)
+    g._m[::5] = 0
+    comps = []
+    for a in range(3):
+        v = special_grid(seed + 20 + a, n, 2, 0.8, 0.0)
+        if not same:
+            v.set_transform(VoxelTransform.uniform((1.0, 0.75, 1.5)[a]))
+        comps.append(v)
+    out = advect_level_set(g, VelocityField(*comps), dt)
+    og = to_oracle(oracle, g).advect(*[to_oracle(oracle, c) for c in comps], dt)
+    o1, m1, v1 = out.to_arrays()
+    o2, m2, v2 = og.arrays()
+    assert np.array_equal(o1, o2) and np.array_equal(m1, m2)
+    assert np.array_equal(np.isnan(v1), np.isnan(v2))
+    keep = ~np.isnan(v1)
+    assert np.array_equal(v1.view(np.uint32)[keep], v2.view(np.uint32)[keep])
