@@ -304,7 +304,7 @@ class RefLargeSample:
 
 # ---------------------------------------------------------------- GPU legs
 
-STEP_KERNELS = ("k_m_advect", "k_m_reinit", "k_t_scanalloc", "k_t_finalize", "k_t_nbr")
+STEP_KERNELS = ("k_m_advect", "k_m_reinit", "k_t_scanalloc", "k_t_nbr")
 
 
 # DRAM bytes (read + write) per leaf of one launch of the stencil kernels,

@@ -4,32 +4,39 @@
 // set keep flags (a leaf survives if it, or a neighbour within one voxel,
 // has an active voxel: dilate26 of the band) and proposed missing leaves in
 // a hash table where atomicMin keeps the proposer whose direction, seen from
-// the new leaf, comes first.  Three kernels finish the step:
+// the new leaf, comes first.  Two kernels finish the step:
 //
 //   k_t_scanalloc  per list position: survive flag + owned proposals; an
 //                  exclusive scan in list order (single pass, decoupled
 //                  look-back over 256-position chunks taken by ticket) gives
 //                  each survivor its new position, followed by the new leaves
-//                  it owns; new leaves take slots from the free stack, slots
-//                  of dropped leaves go to a recycle list
-//   k_t_finalize   new list, fill of new leaves (clamped-sign rule from the
-//                  owner), hash insertion, recycled slots back on the stack
-//   k_t_nbr        27-neighbour rows updated where a neighbour was dropped or
-//                  is new (the rows of an upload are built whole by k_nbr);
-//                  publishes counts
+//                  it owns; every listed leaf's hash key is inserted, new
+//                  leaves take slots from the free stack and are filled from
+//                  their owners (clamped-sign rule), slots of dropped leaves
+//                  go to a recycle list
+//   k_t_nbr        the new list in place, 27-neighbour rows updated where a
+//                  neighbour was dropped or is new (the rows of an upload are
+//                  built whole by k_nbr), recycled slots back on the free
+//                  stack; publishes counts
+//
+// A third kernel between them (list copy, hash insertion and fills from the
+// scanned positions) cost a step one more launch and re-read what the scan
+// held: 64.8 -> 63.4 us a step at 3.0k leaves, 32.6 -> 32.2 at 62.
 //
 // The reference's counterparts are dilate (src/tools/morphology.rs:20-35),
 // trim_narrow_band's deactivation (src/tools/level_set_track.rs:53-68) and
 // remove_empty_leaves (src/tree/internal.rs:231-247).
 #include <algorithm>
+#include <type_traits>
 
 #include "method_state.hpp"
 
 namespace vlr {
 
-// scalars: [0] count  [1] step  [2] free top  [3] spare
-//          [4] new count  [5] recycled count  [6] new free top  [7] chunk ticket
+// scalars: [0] count  [1] step  [2] free top
+//          [3] finished CTAs of k_t_nbr  [4] new count  [5] recycled count  [7] chunk ticket
 constexpr int kChunk = 256;
+constexpr int kFillQueue = 512;  // new leaves of a chunk filled by whole warps (more: by their own thread)
 constexpr long long kSpinLimit = 1ll << 22;  // default bound of the look-back wait (about half a second)
 
 __device__ __forceinline__ void dir_of(int d, int& dx, int& dy, int& dz) {
@@ -50,9 +57,45 @@ __device__ __forceinline__ unsigned long long pack_status(unsigned tag, unsigned
     return ((unsigned long long)(tag & 0x3fffffffu) << 34) | ((unsigned long long)flag << 32) | value;
 }
 
-__global__ void __launch_bounds__(kChunk) k_t_scanalloc(MLeafArrays A, int4* origin, const int* keep,
+// Inserts a listed leaf's key (every key is listed once).
+__device__ __forceinline__ void hash_put(uint64_t key, int slot, uint64_t* hkey, int* hval, int hcap, unsigned* err) {
+    if (key == kEmptyKey) {
+        atomicOr(err, kErrExtent);
+        return;
+    }
+    const uint32_t m = (uint32_t)hcap - 1u;
+    uint32_t q = (uint32_t)mix64(key) & m;
+    for (int probe = 0; probe < hcap; ++probe) {
+        const unsigned long long prev =
+            atomicCAS((unsigned long long*)&hkey[q], (unsigned long long)kEmptyKey, (unsigned long long)key);
+        if (prev == kEmptyKey) {
+            hval[q] = slot;
+            return;
+        }
+        q = (q + 1u) & m;
+    }
+    atomicOr(err, kErrHashFull);
+}
+
+// Values of new leaf ns in direction d of its owner, voxels first, first +
+// step, ...: copysign(hw, the owner's value at the clamped position).
+template <typename T>
+__device__ __forceinline__ void fill_leaf(T* vals, int ns, int owner, int d, float hw, int first, int step) {
+    int dx, dy, dz;
+    dir_of(d, dx, dy, dz);
+    for (int off = first; off < kLeafVoxels; off += step) {
+        const int x = 8 * dx + (off >> 6), y = 8 * dy + ((off >> 3) & 7), z = 8 * dz + (off & 7);
+        const int cx = min(max(x, 0), 7), cy = min(max(y, 0), 7), cz = min(max(z, 0), 7);
+        const float v = to_f(vals[(size_t)owner * kLeafVoxels + ((cx << 6) | (cy << 3) | cz)]);
+        vals[(size_t)ns * kLeafVoxels + off] = from_f<T>(copysignf(hw, v));
+    }
+}
+
+template <typename T>
+__global__ void __launch_bounds__(kChunk) k_t_scanalloc(MLeafArrays A, int4* origin, T* vals, const int* keep,
                                                        const uint64_t* __restrict__ pkey, const int* __restrict__ pval,
-                                                       int hcap, const MGridParams* __restrict__ params, int bits,
+                                                       uint64_t* hkey, int* hval, int hcap,
+                                                       const MGridParams* __restrict__ params, int bits,
                                                        int* free_stack, int* recycled, int* list_new,
                                                        int* newinfo, unsigned long long* status, int* scalars,
                                                        int cap, unsigned* err) {
@@ -62,14 +105,20 @@ __global__ void __launch_bounds__(kChunk) k_t_scanalloc(MLeafArrays A, int4* ori
     __shared__ int s_ticket;
     __shared__ int s_warp[kChunk / 32];
     __shared__ int s_prefix;
+    __shared__ int2 s_fill[kFillQueue];  // new leaf's slot, owner slot * 32 + direction
+    __shared__ int s_nfill;
     const long long spin_limit = wait_limit(err, kSpinLimit);
     const bool hold_first = test_stall(err);
     const int count = scalars[0];
     const unsigned tag = (unsigned)scalars[1] + 1u;
     const int nchunks = (count + kChunk - 1) / kChunk;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    if ((int)blockIdx.x >= nchunks) return;  // no chunk is left for it; keeps the ticket off its path
     for (;;) {
-        if (threadIdx.x == 0) s_ticket = atomicAdd(&scalars[7], 1);
+        if (threadIdx.x == 0) {
+            s_ticket = atomicAdd(&scalars[7], 1);
+            s_nfill = 0;
+        }
         __syncthreads();
         const int chunk = s_ticket;
         __syncthreads();
@@ -167,6 +216,7 @@ __global__ void __launch_bounds__(kChunk) k_t_scanalloc(MLeafArrays A, int4* ori
                 if (pos < cap) {
                     list_new[pos] = s;
                     newinfo[pos] = -1;
+                    hash_put(leaf_key(o, 0, 0, 0, params, bits), s, hkey, hval, hcap, err);
                 }
                 ++pos;
             }
@@ -189,6 +239,10 @@ __global__ void __launch_bounds__(kChunk) k_t_scanalloc(MLeafArrays A, int4* ori
                 origin[ns] = make_int4(o.x + 8 * dx, o.y + 8 * dy, o.z + 8 * dz, o.w);
                 list_new[pos] = ns;
                 newinfo[pos] = s * 32 + d;  // owner slot and direction
+                hash_put(leaf_key(o, dx, dy, dz, params, bits), ns, hkey, hval, hcap, err);
+                const int f = atomicAdd(&s_nfill, 1);
+                if (f < kFillQueue) s_fill[f] = make_int2(ns, s * 32 + d);
+                else fill_leaf(vals, ns, s, d, params[o.w].hw, 0, 1);
                 A.spill[ns] = 0;
                 A.nonempty[ns] = 0;
 #pragma unroll
@@ -199,80 +253,15 @@ __global__ void __launch_bounds__(kChunk) k_t_scanalloc(MLeafArrays A, int4* ori
                 ++pos;
             }
         }
-    }
-}
-
-// One thread per new-list position, a block's 256 positions at a time: copy
-// the list and insert the leaf's hash key; the block's new leaves, queued in
-// shared memory, are then filled from their owners one warp each (coalesced
-// stores).  The dropped slots go back on the free stack.
-template <typename T>
-__global__ void __launch_bounds__(256) k_t_finalize(const int* list_new, const int* newinfo, int* list, const int4* origin,
-                                                   T* vals, uint64_t* hkey, int* hval, int hcap,
-                                                   const MGridParams* __restrict__ params, int bits, int* free_stack,
-                                                   const int* recycled, int* scalars, int cap, unsigned* err) {
-    dep_wait();
-    dep_launch();
-    if (step_aborted(err)) return;
-    __shared__ int s_q[256];
-    __shared__ int s_nq;
-    const int n = min(scalars[4], cap);
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    if (threadIdx.x == 0) s_nq = 0;
-    __syncthreads();
-    for (int base = blockIdx.x * 256; base < n; base += gridDim.x * 256) {
-        const int p = base + threadIdx.x;
-        if (p < n) {
-            const int s = list_new[p];
-            const int info = newinfo[p];
-            list[p] = s;
-            if (info != -2) {
-                const uint64_t key = leaf_key(origin[s], 0, 0, 0, params, bits);
-                bool done = false;
-                if (key != kEmptyKey) {
-                    uint32_t m = (uint32_t)hcap - 1u, q = (uint32_t)mix64(key) & m;
-                    for (int probe = 0; probe < hcap; ++probe) {
-                        const unsigned long long prev = atomicCAS((unsigned long long*)&hkey[q],
-                                                                  (unsigned long long)kEmptyKey,
-                                                                  (unsigned long long)key);
-                        if (prev == kEmptyKey) {
-                            hval[q] = s;
-                            done = true;
-                            break;
-                        }
-                        q = (q + 1u) & m;
-                    }
-                }
-                if (!done) atomicOr(err, key == kEmptyKey ? kErrExtent : kErrHashFull);
-            }
-            if (info >= 0) s_q[atomicAdd(&s_nq, 1)] = p;
+        __syncthreads();
+        // the chunk's new leaves, one warp each (coalesced stores)
+        const int nf = min(s_nfill, kFillQueue);
+        for (int f = w; f < nf; f += kChunk / 32) {
+            const int ns = s_fill[f].x, owner = s_fill[f].y >> 5;
+            fill_leaf(vals, ns, owner, s_fill[f].y & 31, params[origin[owner].w].hw, lane, 32);
         }
-        __syncthreads();
-        const int nq = s_nq;
-        for (int j = warp; j < nq; j += 256 / 32) {
-            const int q = s_q[j];
-            const int s = list_new[q], info = newinfo[q];
-            const int owner = info >> 5, d = info & 31;
-            int dx, dy, dz;
-            dir_of(d, dx, dy, dz);
-            const float hw = params[origin[owner].w].hw;
-            for (int off = lane; off < kLeafVoxels; off += 32) {
-                const int x = 8 * dx + (off >> 6), y = 8 * dy + ((off >> 3) & 7), z = 8 * dz + (off & 7);
-                const int cx = min(max(x, 0), 7), cy = min(max(y, 0), 7), cz = min(max(z, 0), 7);
-                const float v = to_f(vals[(size_t)owner * kLeafVoxels + ((cx << 6) | (cy << 3) | cz)]);
-                vals[(size_t)s * kLeafVoxels + off] = from_f<T>(copysignf(hw, v));
-            }
-        }
-        __syncthreads();
-        if (threadIdx.x == 0) s_nq = 0;
-        __syncthreads();
+        __syncthreads();  // the queue is read before the next chunk clears it
     }
-    // dropped slots go back on the free stack above the remaining free slots
-    const int top = max(scalars[2], 0);
-    const int nrec = scalars[5];
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nrec; i += gridDim.x * blockDim.x)
-        if (top + i < cap) free_stack[top + i] = recycled[i];
-    if (blockIdx.x == 0 && threadIdx.x == 0) scalars[6] = min(top + nrec, cap);
 }
 
 // Neighbour rows carried from step to step.  A survivor keeps its slot and
@@ -282,13 +271,17 @@ __global__ void __launch_bounds__(256) k_t_finalize(const int* list_new, const i
 // old row names its listed neighbours, and those that survive clear the
 // entry that points back at it.  One warp per new leaf (found by a ballot
 // over 32 list positions): lane d looks neighbour d up in the hash rebuilt
-// by k_t_finalize, writes the new leaf's row and, for a present neighbour,
+// by k_t_scanalloc, writes the new leaf's row and, for a present neighbour,
 // the entry that points back at the new leaf (two adjacent new leaves write
-// each other's entries with the same values).  Publishes the counts; the
-// dropped count is cleared by the next step's advect.
-__global__ void k_t_nbr(const int* list, const int* newinfo, const int* recycled, const int* keep, int* scalars,
-                        const int4* origin, const uint64_t* hkey, const int* hval, int hcap,
-                        const MGridParams* __restrict__ params, int bits, int* nbr, int cap, const unsigned* err) {
+// each other's entries with the same values).  The new list moves to its
+// place, the dropped slots go back on the free stack above the remaining free
+// ones, and the last CTA to finish publishes the counts and the stack's top
+// (which the others read); the dropped count is cleared by the next step's
+// advect.
+__global__ void k_t_nbr(const int* __restrict__ list_new, int* __restrict__ list, const int* newinfo,
+                        const int* recycled, const int* keep, int* free_stack, int* scalars, const int4* origin,
+                        const uint64_t* hkey, const int* hval, int hcap, const MGridParams* __restrict__ params,
+                        int bits, int* nbr, int cap, const unsigned* err) {
     dep_wait();
     dep_launch();
     if (step_aborted(err)) return;
@@ -296,8 +289,13 @@ __global__ void k_t_nbr(const int* list, const int* newinfo, const int* recycled
     const int nrec = min(scalars[5], cap);
     const int lane = threadIdx.x & 31;
     const int gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nw = (gridDim.x * blockDim.x) >> 5;
+    const int top = max(scalars[2], 0);
+    // CTAs that have a dropped leaf or list positions of their own
+    const int active = min((int)gridDim.x, max(max((count + 255) / 256, (nrec + 7) / 8), 1));
+    if ((int)blockIdx.x >= active) return;
     for (int i = gw; i < nrec; i += nw) {
         const int D = recycled[i];
+        if (lane == 0 && top + i < cap) free_stack[top + i] = D;
         if (lane < kNbr && lane != 13) {
             const int M = nbr[(size_t)D * kNbr + lane];
             if (M >= 0 && keep[M]) nbr[(size_t)M * kNbr + (kNbr - 1 - lane)] = -1;
@@ -305,11 +303,13 @@ __global__ void k_t_nbr(const int* list, const int* newinfo, const int* recycled
     }
     for (int base = gw * 32; base < count; base += nw * 32) {
         const int p = base + lane;
+        const int sp = p < count ? list_new[p] : 0;
+        if (p < count) list[p] = sp;
         unsigned b = __ballot_sync(0xffffffffu, p < count && newinfo[p] >= 0);
         while (b) {
             const int j = __ffs(b) - 1;
             b &= b - 1u;
-            const int N = list[base + j];
+            const int N = __shfl_sync(0xffffffffu, sp, j);
             if (lane < kNbr) {
                 int M = N;
                 if (lane != 13) {
@@ -322,10 +322,12 @@ __global__ void k_t_nbr(const int* list, const int* newinfo, const int* recycled
             }
         }
     }
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
+    __syncthreads();  // the CTA's reads of the stack's top are done
+    if (threadIdx.x == 0 && atomicAdd(&scalars[3], 1) == active - 1) {
+        scalars[3] = 0;
         scalars[0] = count;
         scalars[1] += 1;
-        scalars[2] = scalars[6];
+        scalars[2] = min(top + nrec, cap);
     }
 }
 
@@ -437,30 +439,24 @@ int ls_enqueue_retrack(vlr_ctx* ctx, vlr_level_set* ls) {
     MLeafArrays A = ls->arrays();
     // status words of the look-back scan live after the scan positions in `pos`
     unsigned long long* status = reinterpret_cast<unsigned long long*>(ls->pos);
-    VLR_TIMED(ctx, "k_t_scanalloc",
-              VLR_CUDA(ctx, pdl_launch(k_t_scanalloc, B, kChunk, 0, st, A, ls->origin, (const int*)ls->keep,
-                                       (const uint64_t*)ls->pkey, (const int*)ls->pval, ls->hcap,
-                                       (const MGridParams*)ls->d_params, ls->key_bits, ls->free_stack, ls->owned,
-                                       ls->list_new, ls->newinfo, status, ls->scalars, ls->cap, ctx->d_errword)));
-    if (ls->precision == VLR_PREC_F16)
-        VLR_TIMED(ctx, "k_t_finalize",
-                  VLR_CUDA(ctx, pdl_launch(k_t_finalize<__half>, B, 256, 0, st, (const int*)ls->list_new,
-                                           (const int*)ls->newinfo, ls->list, (const int4*)ls->origin,
-                                           (__half*)ls->vals[0], ls->hkey, ls->hval, ls->hcap,
-                                           (const MGridParams*)ls->d_params, ls->key_bits, ls->free_stack,
-                                           (const int*)ls->owned, ls->scalars, ls->cap, ctx->d_errword)));
-    else
-        VLR_TIMED(ctx, "k_t_finalize",
-                  VLR_CUDA(ctx, pdl_launch(k_t_finalize<float>, B, 256, 0, st, (const int*)ls->list_new,
-                                           (const int*)ls->newinfo, ls->list, (const int4*)ls->origin,
-                                           (float*)ls->vals[0], ls->hkey, ls->hval, ls->hcap,
-                                           (const MGridParams*)ls->d_params, ls->key_bits, ls->free_stack,
-                                           (const int*)ls->owned, ls->scalars, ls->cap, ctx->d_errword)));
+    auto scan = [&](auto* vals) -> int {
+        using T = std::remove_pointer_t<decltype(vals)>;
+        VLR_TIMED(ctx, "k_t_scanalloc",
+                  VLR_CUDA(ctx, pdl_launch(k_t_scanalloc<T>, B, kChunk, 0, st, A, ls->origin, vals,
+                                           (const int*)ls->keep, (const uint64_t*)ls->pkey, (const int*)ls->pval,
+                                           ls->hkey, ls->hval, ls->hcap, (const MGridParams*)ls->d_params,
+                                           ls->key_bits, ls->free_stack, ls->owned, ls->list_new, ls->newinfo, status,
+                                           ls->scalars, ls->cap, ctx->d_errword)));
+        return VLR_OK;
+    };
+    const int rc = ls->precision == VLR_PREC_F16 ? scan((__half*)ls->vals[0]) : scan((float*)ls->vals[0]);
+    if (rc) return rc;
     VLR_TIMED(ctx, "k_t_nbr",
-              VLR_CUDA(ctx, pdl_launch(k_t_nbr, B, 256, 0, st, (const int*)ls->list, (const int*)ls->newinfo,
-                                       (const int*)ls->owned, (const int*)ls->keep, ls->scalars,
-                                       (const int4*)ls->origin, (const uint64_t*)ls->hkey, (const int*)ls->hval,
-                                       ls->hcap, (const MGridParams*)ls->d_params, ls->key_bits, ls->nbr, ls->cap,
+              VLR_CUDA(ctx, pdl_launch(k_t_nbr, B, 256, 0, st, (const int*)ls->list_new, ls->list,
+                                       (const int*)ls->newinfo, (const int*)ls->owned, (const int*)ls->keep,
+                                       ls->free_stack, ls->scalars, (const int4*)ls->origin,
+                                       (const uint64_t*)ls->hkey, (const int*)ls->hval, ls->hcap,
+                                       (const MGridParams*)ls->d_params, ls->key_bits, ls->nbr, ls->cap,
                                        (const unsigned*)ctx->d_errword)));
     VLR_CUDA(ctx, cudaGetLastError());
     return VLR_OK;
