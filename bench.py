@@ -1020,7 +1020,7 @@ def bench_mesh(args, ctx, peak, peak_kind):
     ctx.profile(True)  # kernel times from a separate pass (the events would perturb the timed calls)
     for _ in range(args.steps):
         call()
-    names = ("k_mc_classify", "k_mc_emit", "k_rs_hist", "k_rs_scatter")
+    names = ("k_mc_classify", "k_mc_emit")
     kern = {k: ctx.kernel_time(k) for k in names}
     ctx.profile(False)
     kms = {k: v[0] / max(args.steps, 1) for k, v in kern.items()}

@@ -175,6 +175,16 @@ int vlr_flood_fill_sign(vlr_ctx* ctx, vlr_grid* g);
  * cap_triangles triangles are copied (pass null buffers to count only).  World-unit f32 grids only. */
 int vlr_volume_to_mesh(vlr_ctx* ctx, const vlr_grid* g, float isovalue, double* vertices, size_t cap_vertices,
                        uint32_t* triangles, size_t cap_triangles, size_t* n_vertices, size_t* n_triangles);
+/* The same in one marching: vlr_mesh_create leaves the mesh on the device and
+ * returns its counts, vlr_mesh_read copies up to the capacities (null: skip),
+ * vlr_mesh_destroy frees it (stream-ordered), so buffers of the exact size
+ * need no second pass over the grid. */
+typedef struct vlr_mesh vlr_mesh;
+int vlr_mesh_create(vlr_ctx* ctx, const vlr_grid* g, float isovalue, vlr_mesh** out, size_t* n_vertices,
+                    size_t* n_triangles);
+int vlr_mesh_read(vlr_ctx* ctx, const vlr_mesh* mesh, double* vertices, size_t cap_vertices, uint32_t* triangles,
+                  size_t cap_triangles);
+void vlr_mesh_destroy(vlr_mesh* mesh);
 /* The triangulation table used by vlr_volume_to_mesh: 256 cases (bit i set:
  * corner i below the isovalue) x 16 edge indices, three per triangle, -1
  * padded: the crate's TRI_TABLE (src/tools/volume_to_mesh.rs:246-503).

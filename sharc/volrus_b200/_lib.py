@@ -109,6 +109,9 @@ SIGNATURES = {
     "vlr_flood_fill_sign": (C.c_int, [P, P]),
     "vlr_volume_to_mesh": (C.c_int, [P, P, C.c_float, dbl_p, C.c_size_t, C.POINTER(C.c_uint32), C.c_size_t, size_p,
                                      size_p]),
+    "vlr_mesh_create": (C.c_int, [P, P, C.c_float, PP, size_p, size_p]),
+    "vlr_mesh_read": (C.c_int, [P, P, dbl_p, C.c_size_t, C.POINTER(C.c_uint32), C.c_size_t]),
+    "vlr_mesh_destroy": (None, [P]),
     "vlr_mc_triangle_table": (C.c_int, [C.POINTER(C.c_int8)]),
     "vlr_grid_from_vol": (C.c_int, [P, P, C.c_size_t, PP, C.POINTER(C.c_int)]),
     "vlr_grid_to_vol": (C.c_int, [P, P, C.c_int, P, C.c_size_t, size_p]),

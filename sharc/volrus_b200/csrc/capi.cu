@@ -31,7 +31,7 @@ int upload_leaves(vlr_ctx* ctx, vlr_grid* g, const int32_t* origins, const uint6
     for (size_t i = 1; i < n; ++i)
         if (!lex_less(origins + 3 * order[i - 1], origins + 3 * order[i]))
             return set_error(ctx, VLR_ERR_INVALID, "duplicate leaf origin");
-    int rc = choose_base(ctx, origins, n, g->base);
+    int rc = choose_base(ctx, origins, n, g->base, g->box);
     if (rc) return rc;
     rc = grid_alloc(ctx, g, (int)std::max<size_t>(n, 1));
     if (rc) return rc;
@@ -298,7 +298,7 @@ int vlr_grid_create_device(vlr_ctx* ctx, const vlr_transform* xf, float backgrou
     g->kind = VLR_KIND_F32_WORLD;
     g->background = background;
     g->xf = *xf;
-    int rc = choose_base(ctx, o.data(), n_leaves, g->base);
+    int rc = choose_base(ctx, o.data(), n_leaves, g->base, g->box);
     if (!rc) rc = grid_alloc(ctx, g, (int)std::max<size_t>(n_leaves, 1));
     if (!rc && n_leaves) {
         g->n = (int)n_leaves;

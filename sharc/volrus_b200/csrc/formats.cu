@@ -133,7 +133,7 @@ int grid_from_records(vlr_ctx* ctx, vlr_grid* g, const unsigned char* block, siz
                       int o_off, int m_off, int v_off, const std::vector<int>& order,
                       const std::vector<int32_t>& origins, bool drop_inactive) {
     const size_t n = order.size();
-    int rc = choose_base(ctx, origins.data(), n, g->base);
+    int rc = choose_base(ctx, origins.data(), n, g->base, g->box);
     if (rc) return rc;
     rc = grid_alloc(ctx, g, (int)std::max<size_t>(n, 1));
     if (rc) return rc;

@@ -221,8 +221,9 @@ int grid_alloc(vlr_ctx* ctx, vlr_grid* g, int cap) {
     return VLR_OK;
 }
 
-int choose_base(vlr_ctx* ctx, const int32_t* origins, size_t n, long long base[3]) {
+int choose_base(vlr_ctx* ctx, const int32_t* origins, size_t n, long long base[3], int* box) {
     if (n == 0) {
+        if (box) std::fill(box, box + 6, 0);
         base[0] = base[1] = base[2] = -kKeyHalf;
         return VLR_OK;
     }
@@ -236,6 +237,10 @@ int choose_base(vlr_ctx* ctx, const int32_t* origins, size_t n, long long base[3
         if (hi - lo >= (1ll << kKeyBits) - 2)
             return set_error(ctx, VLR_ERR_EXTENT, "grid spans more than 2^24 voxels along an axis");
         base[a] = (lo + hi) / 2 - kKeyHalf;
+        if (box) {
+            box[a] = (int)lo;
+            box[3 + a] = (int)hi;
+        }
     }
     return VLR_OK;
 }

@@ -228,7 +228,8 @@ int grid_add_leaves(vlr_ctx* ctx, vlr_grid* g, const std::vector<int32_t>& origi
         }
     }
     long long base[3];
-    int rc = choose_base(ctx, all.data(), (size_t)(n + m), base);
+    int box[6];
+    int rc = choose_base(ctx, all.data(), (size_t)(n + m), base, box);
     if (rc) return rc;
     vlr_grid tmp;
     tmp.ctx = ctx;
@@ -262,6 +263,7 @@ int grid_add_leaves(vlr_ctx* ctx, vlr_grid* g, const std::vector<int32_t>& origi
     grid_free_arrays(&tmp);
     g->n = n + m;
     std::memcpy(g->base, base, sizeof(base));
+    std::memcpy(g->box, box, sizeof(box));
     return grid_index(ctx, g);
 }
 

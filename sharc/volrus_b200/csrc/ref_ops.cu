@@ -603,6 +603,7 @@ int advect_ref(vlr_ctx* ctx, const vlr_grid* g, const vlr_grid* vx, const vlr_gr
     out->xf.voxel_size = g->xf.affine_voxel_size;
     out->xf.origin[0] = out->xf.origin[1] = out->xf.origin[2] = 0.0;
     for (int a = 0; a < 3; ++a) out->base[a] = g->base[a];
+    std::memcpy(out->box, g->box, sizeof(g->box));
     int rc = grid_alloc(ctx, out, std::max(g->n, 1));
     if (rc) return rc;
     out->n = g->n;
@@ -822,7 +823,7 @@ int make_sphere(vlr_ctx* ctx, double radius, const double c[3], double vs, doubl
     if (n_cand > (1ll << 26)) return set_error(ctx, VLR_ERR_CAPACITY, "sphere bounding box too large");
     int32_t corner[6] = {imin, jmin, kmin, imax, jmax, kmax};
     int32_t bb[6] = {corner[0], corner[1], corner[2], corner[3], corner[4], corner[5]};
-    int rc = choose_base(ctx, bb, 2, out->base);
+    int rc = choose_base(ctx, bb, 2, out->base, out->box);
     if (rc) return rc;
     rc = grid_alloc(ctx, out, (int)n_cand);
     if (rc) return rc;

@@ -52,6 +52,7 @@ struct vlr_grid {
     float background = 0.0f;
     vlr_transform xf{};
     long long base[3] = {0, 0, 0};
+    int box[6] = {0, 0, 0, 0, 0, 0};  // leaf coordinates: a box that holds every leaf (lower, upper corner)
     void* block = nullptr;  // one stream-ordered allocation (ctx->pool) holding the arrays below
     int4* origin = nullptr;
     uint64_t* mask = nullptr;
@@ -120,7 +121,8 @@ void grid_free_arrays(vlr_grid* g);
 // (Re)build hash table and neighbour table for slots 0..n-1.
 int grid_index(vlr_ctx* ctx, vlr_grid* g);
 // Choose the hash-key base from the leaf-coordinate bounding box (host origins).
-int choose_base(vlr_ctx* ctx, const int32_t* origins, size_t n, long long base[3]);
+// and, when box is given, the bounding box itself (lower, then upper corner).
+int choose_base(vlr_ctx* ctx, const int32_t* origins, size_t n, long long base[3], int* box = nullptr);
 // Keep slots whose flag is non-zero (order preserved); rebuilds the index when
 // some are dropped, else copies it from `index` when one is given (a grid with
 // the same leaves in the same slots).  Reports device errors as `what`.

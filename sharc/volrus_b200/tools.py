@@ -322,15 +322,16 @@ def volume_to_mesh(grid, isovalue: float = 0.0, ctx: Context | None = None) -> M
     d, created = _as_device(grid, ctx)
     try:
         nv, nt = C.c_size_t(), C.c_size_t()
-        ctx.check(ctx.lib.vlr_volume_to_mesh(ctx.handle, d.handle, C.c_float(isovalue), None, 0, None, 0,
-                                             C.byref(nv), C.byref(nt)), "vlr_volume_to_mesh")
-        v = np.zeros((nv.value, 3), np.float64)
-        t = np.zeros((nt.value, 3), np.uint32)
-        if nv.value or nt.value:
-            ctx.check(ctx.lib.vlr_volume_to_mesh(ctx.handle, d.handle, C.c_float(isovalue),
-                                                 v.ctypes.data_as(C.POINTER(C.c_double)), nv.value,
-                                                 t.ctypes.data_as(C.POINTER(C.c_uint32)), nt.value,
-                                                 C.byref(nv), C.byref(nt)), "vlr_volume_to_mesh")
+        mesh = C.c_void_p()
+        ctx.check(ctx.lib.vlr_mesh_create(ctx.handle, d.handle, C.c_float(isovalue), C.byref(mesh), C.byref(nv),
+                                          C.byref(nt)), "vlr_mesh_create")
+        try:
+            v = np.empty((nv.value, 3), np.float64)
+            t = np.empty((nt.value, 3), np.uint32)
+            ctx.check(ctx.lib.vlr_mesh_read(ctx.handle, mesh, v.ctypes.data_as(C.POINTER(C.c_double)), nv.value,
+                                            t.ctypes.data_as(C.POINTER(C.c_uint32)), nt.value), "vlr_mesh_read")
+        finally:
+            ctx.lib.vlr_mesh_destroy(mesh)
         return Mesh(v, t)
     finally:
         if created:

@@ -75,3 +75,29 @@ def test_advect_sampled_fields_match_oracle(oracle, same, dt, seed, n, fill):
     assert np.array_equal(np.isnan(v1), np.isnan(v2))
     keep = ~np.isnan(v1)
     assert np.array_equal(v1.view(np.uint32)[keep], v2.view(np.uint32)[keep])
+
+
+@pytest.mark.parametrize("iso", [0.0, 0.25])
+@pytest.mark.parametrize("seed,n,spread,fill,mix", [(31, 30, 2, 1.0, 0.0), (32, 30, 2, 1.0, 0.3), (33, 1, 1, 1.0, 0.0),
+                                                    (34, 40, 100000, 0.5, 0.0), (35, 200, 12, 0.3, 0.02)])
+def test_mesh_tile_lists_match_oracle(oracle, iso, seed, n, spread, fill, mix):
+    """Tiles from a bit per tile of the leaves' box, and from the sort where leaves lie far apart; crowded and empty
+    tiles, infinities and NaN."""
+    import ctypes as C
+    from sharc.volrus_b200 import DeviceGrid, volume_to_mesh
+    g = special_grid(seed, n, spread, fill, mix)
+    m = volume_to_mesh(g, iso)
+    v2, t2 = to_oracle(oracle, g).volume_to_mesh(iso)
+    assert np.array_equal(m.triangles, t2)
+    assert np.array_equal(np.isnan(m.vertices), np.isnan(v2))
+    ok = ~np.isnan(v2)
+    assert np.array_equal(m.vertices.view(np.uint64)[ok], v2.view(np.uint64)[ok])
+    # the one-call form: counts, then as much as fits
+    d = DeviceGrid.upload(g)
+    nv, nt = C.c_size_t(), C.c_size_t()
+    k = max(len(t2) // 2, 1)
+    t = np.zeros((k, 3), np.uint32)
+    d.ctx.check(d.ctx.lib.vlr_volume_to_mesh(d.ctx.handle, d.handle, C.c_float(iso), None, 0,
+                                             t.ctypes.data_as(C.POINTER(C.c_uint32)), k, C.byref(nv), C.byref(nt)))
+    assert (nv.value, nt.value) == (len(v2), len(t2))
+    assert np.array_equal(t[:len(t2)], t2[:k])
