@@ -13,16 +13,19 @@
 // origin order, so with particles handed in that binned order the re-binned
 // grid is a stable sort of the particles by their new leaf.  On the GPU:
 //   k_points_move    position update, then the new leaf per particle as three
-//                    order-preserving 29-bit keys (one per axis)
-//   (sort)           three stable radix sorts of (key, particle index): z,
-//                    then y, then x, the keys of each pass gathered in the
-//                    order the previous pass left (k_gather_keys)
+//                    order-preserving 29-bit keys (one per axis) and their
+//                    bounding box
+//   k_points_keys    one key per particle with just the bits of that box
+//   (sort)           stable radix sort of (key, particle index)
 //   k_points_emit    particles gathered into sorted order; a flag where the
 //                    leaf changes
 //   (scan)           leaf ranks; k_points_leaves writes each leaf's origin and
 //                    first particle
+// A box of more than 64 bits takes three stable sorts instead: z, then y, then
+// x, the keys of each pass gathered in the order the previous pass left.
 #include <algorithm>
 
+#include "box_reduce.cuh"
 #include "ref_ops.hpp"
 #include "sort_reduce.hpp"
 
@@ -33,10 +36,34 @@ struct V3 {
     double x, y, z;
 };
 
-__device__ __forceinline__ V3 vsample(const GridView& vx, const GridView& vy, const GridView& vz, const V3& p) {
-    return V3{(double)sample_trilinear_ref(vx, p.x, p.y, p.z), (double)sample_trilinear_ref(vy, p.x, p.y, p.z),
-              (double)sample_trilinear_ref(vz, p.x, p.y, p.z)};
-}
+// The velocity grids and, per particle, the leaf of each that the particle
+// starts in: one hash search per grid, after which its samples (a step moves
+// it little) come from the leaf's neighbour row.  SAME: the grids share their
+// transform, so position and fractions are computed once for the three.
+template <bool SAME>
+struct Field {
+    const GridView& vx;
+    const GridView& vy;
+    const GridView& vz;
+    Hint hx, hy, hz;
+
+    __device__ __forceinline__ Field(const GridView& x, const GridView& y, const GridView& z, const V3& p)
+        : vx(x), vy(y), vz(z) {
+        const Cell a = cell_of(vx, p.x, p.y, p.z);
+        hx = hint_at(vx, a.i, a.j, a.k);
+        const Cell b = SAME ? a : cell_of(vy, p.x, p.y, p.z);
+        hy = hint_at(vy, b.i, b.j, b.k);
+        const Cell c = SAME ? a : cell_of(vz, p.x, p.y, p.z);
+        hz = hint_at(vz, c.i, c.j, c.k);
+    }
+
+    __device__ __forceinline__ V3 operator()(const V3& p) const {
+        const Cell a = cell_of(vx, p.x, p.y, p.z);
+        return V3{(double)read_cell(vx, a, hx),
+                  (double)read_cell(vy, SAME ? a : cell_of(vy, p.x, p.y, p.z), hy),
+                  (double)read_cell(vz, SAME ? a : cell_of(vz, p.x, p.y, p.z), hz)};
+    }
+};
 
 __device__ __forceinline__ V3 scale(double s, const V3& v) {
     return V3{__dmul_rn(s, v.x), __dmul_rn(s, v.y), __dmul_rn(s, v.z)};
@@ -54,27 +81,38 @@ __device__ __forceinline__ double rk4_comb(double p, double k1, double k2, doubl
     return __dadd_rn(p, __ddiv_rn(s, 6.0));
 }
 
+// One RK4 or forward Euler step of a position.
+template <bool SAME>
+__device__ __forceinline__ V3 move_point(const GridView& vx, const GridView& vy, const GridView& vz, const V3& p,
+                                         double dt, int rk4) {
+    const Field<SAME> v(vx, vy, vz, p);
+    const V3 v1 = v(p);
+    if (!rk4)
+        return V3{__dadd_rn(p.x, __dmul_rn(dt, v1.x)), __dadd_rn(p.y, __dmul_rn(dt, v1.y)),
+                  __dadd_rn(p.z, __dmul_rn(dt, v1.z))};
+    const V3 k1 = scale(dt, v1);
+    const V3 k2 = scale(dt, v(axpy(p, k1, 0.5)));
+    const V3 k3 = scale(dt, v(axpy(p, k2, 0.5)));
+    const V3 k4 = scale(dt, v(axpy(p, k3, 1.0)));
+    return V3{rk4_comb(p.x, k1.x, k2.x, k3.x, k4.x), rk4_comb(p.y, k1.y, k2.y, k3.y, k4.y),
+              rk4_comb(p.z, k1.z, k2.z, k3.z, k4.z)};
+}
+
+template <bool SAME>
 __global__ void k_advect_particles(GridView vx, GridView vy, GridView vz, double* __restrict__ pos, int n, double dt,
                                    int rk4) {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const V3 p{pos[3 * i], pos[3 * i + 1], pos[3 * i + 2]};
-        V3 out;
-        if (rk4) {
-            const V3 k1 = scale(dt, vsample(vx, vy, vz, p));
-            const V3 k2 = scale(dt, vsample(vx, vy, vz, axpy(p, k1, 0.5)));
-            const V3 k3 = scale(dt, vsample(vx, vy, vz, axpy(p, k2, 0.5)));
-            const V3 k4 = scale(dt, vsample(vx, vy, vz, axpy(p, k3, 1.0)));
-            out = V3{rk4_comb(p.x, k1.x, k2.x, k3.x, k4.x), rk4_comb(p.y, k1.y, k2.y, k3.y, k4.y),
-                     rk4_comb(p.z, k1.z, k2.z, k3.z, k4.z)};
-        } else {
-            const V3 v = vsample(vx, vy, vz, p);
-            out = V3{__dadd_rn(p.x, __dmul_rn(dt, v.x)), __dadd_rn(p.y, __dmul_rn(dt, v.y)),
-                     __dadd_rn(p.z, __dmul_rn(dt, v.z))};
-        }
+        const V3 out = move_point<SAME>(vx, vy, vz, V3{pos[3 * i], pos[3 * i + 1], pos[3 * i + 2]}, dt, rk4);
         pos[3 * i] = out.x;
         pos[3 * i + 1] = out.y;
         pos[3 * i + 2] = out.z;
     }
+}
+
+// Whether the three grids sample at the same index position.
+bool same_transform(const GridView& a, const GridView& b) {
+    return a.inv_vs == b.inv_vs && a.t_origin[0] == b.t_origin[0] && a.t_origin[1] == b.t_origin[1] &&
+           a.t_origin[2] == b.t_origin[2];
 }
 
 // f64::round (half away from zero) then Rust's saturating `as i32`.
@@ -94,25 +132,19 @@ struct InvRows {
 __device__ __forceinline__ unsigned leaf_key(int32_t v) { return ((unsigned)v >> 3) ^ (1u << 28); }
 __device__ __forceinline__ int32_t key_leaf(unsigned k) { return (int32_t)((k ^ (1u << 28)) << 3); }
 
-__global__ void k_points_move(GridView vx, GridView vy, GridView vz, vlr_particle* __restrict__ pts, int n,
-                              double dt, int rk4, InvRows inv, unsigned* __restrict__ kx, unsigned* __restrict__ ky,
-                              unsigned* __restrict__ kz, unsigned* __restrict__ idx) {
+// Bound: load latency and the f64 and conversion instructions of 12 samples a
+// particle (RK4).  300k particles in a 64^3 field: 124 us with up to 8 hash
+// searches a sample, 46 us from the particle's leaf.
+template <bool SAME>
+__global__ void __launch_bounds__(256) k_points_move(GridView vx, GridView vy, GridView vz,
+                                                    vlr_particle* __restrict__ pts, int n, double dt, int rk4,
+                                                    InvRows inv, unsigned* __restrict__ kx,
+                                                    unsigned* __restrict__ ky, unsigned* __restrict__ kz,
+                                                    unsigned* __restrict__ idx, int* __restrict__ box) {
+    int lo[3] = {INT_MAX, INT_MAX, INT_MAX}, hi[3] = {INT_MIN, INT_MIN, INT_MIN};
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         double* pp = pts[i].position;
-        const V3 p{pp[0], pp[1], pp[2]};
-        V3 out;
-        if (rk4) {
-            const V3 k1 = scale(dt, vsample(vx, vy, vz, p));
-            const V3 k2 = scale(dt, vsample(vx, vy, vz, axpy(p, k1, 0.5)));
-            const V3 k3 = scale(dt, vsample(vx, vy, vz, axpy(p, k2, 0.5)));
-            const V3 k4 = scale(dt, vsample(vx, vy, vz, axpy(p, k3, 1.0)));
-            out = V3{rk4_comb(p.x, k1.x, k2.x, k3.x, k4.x), rk4_comb(p.y, k1.y, k2.y, k3.y, k4.y),
-                     rk4_comb(p.z, k1.z, k2.z, k3.z, k4.z)};
-        } else {
-            const V3 v = vsample(vx, vy, vz, p);
-            out = V3{__dadd_rn(p.x, __dmul_rn(dt, v.x)), __dadd_rn(p.y, __dmul_rn(dt, v.y)),
-                     __dadd_rn(p.z, __dmul_rn(dt, v.z))};
-        }
+        const V3 out = move_point<SAME>(vx, vy, vz, V3{pp[0], pp[1], pp[2]}, dt, rk4);
         pp[0] = out.x;
         pp[1] = out.y;
         pp[2] = out.z;
@@ -124,10 +156,27 @@ __global__ void k_points_move(GridView vx, GridView vy, GridView vz, vlr_particl
             const double f = __dadd_rn(__dadd_rn(__dadd_rn(__dmul_rn(r[0], out.x), __dmul_rn(r[1], out.y)),
                                                  __dmul_rn(r[2], out.z)),
                                        r[3]);
-            keys[a][i] = leaf_key(round_to_i32(f) & ~7);
+            const unsigned k = leaf_key(round_to_i32(f) & ~7);
+            keys[a][i] = k;
+            lo[a] = min(lo[a], (int)k);
+            hi[a] = max(hi[a], (int)k);
         }
         idx[i] = (unsigned)i;
     }
+    block_box(lo, hi, box);
+}
+
+// Lower corner of the box and the bits of y and z in a packed key.
+struct KeyBox {
+    unsigned lo[3];
+    int by, bz;
+};
+
+__global__ void k_points_keys(const unsigned* __restrict__ kx, const unsigned* __restrict__ ky,
+                              const unsigned* __restrict__ kz, int n, KeyBox b, uint64_t* __restrict__ keys) {
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+        keys[i] = ((uint64_t)(kx[i] - b.lo[0]) << (b.by + b.bz)) | ((uint64_t)(ky[i] - b.lo[1]) << b.bz) |
+                  (uint64_t)(kz[i] - b.lo[2]);
 }
 
 __global__ void k_gather_keys(const unsigned* __restrict__ keys, const unsigned* __restrict__ perm, int n,
@@ -184,8 +233,10 @@ int vlr_advect_particles(vlr_ctx* ctx, const vlr_grid* vx, const vlr_grid* vy, c
     VLR_CUDA(ctx, cudaMallocFromPoolAsync(&d, sizeof(double) * 3 * n, ctx->pool, ctx->stream));
     VLR_CUDA(ctx, cudaMemcpyAsync(d, positions, sizeof(double) * 3 * n, cudaMemcpyHostToDevice, ctx->stream));
     const int blocks = (int)std::min<size_t>((n + 255) / 256, (size_t)ctx->sm_count * 16);
-    k_advect_particles<<<blocks, 256, 0, ctx->stream>>>(make_view(vx), make_view(vy), make_view(vz), d, (int)n, dt,
-                                                        rk4 ? 1 : 0);
+    const GridView gx = make_view(vx), gy = make_view(vy), gz = make_view(vz);
+    auto* kernel = same_transform(gx, gy) && same_transform(gx, gz) ? k_advect_particles<true>
+                                                                   : k_advect_particles<false>;
+    kernel<<<blocks, 256, 0, ctx->stream>>>(gx, gy, gz, d, (int)n, dt, rk4 ? 1 : 0);
     VLR_CUDA(ctx, cudaGetLastError());
     VLR_CUDA(ctx, cudaMemcpyAsync(positions, d, sizeof(double) * 3 * n, cudaMemcpyDeviceToHost, ctx->stream));
     VLR_CUDA(ctx, cudaFreeAsync(d, ctx->stream));
@@ -213,9 +264,9 @@ int vlr_advect_points(vlr_ctx* ctx, const vlr_grid* vx, const vlr_grid* vy, cons
     for (int i = 0; i < 12; ++i) inv.r[i] = world_to_index[i];
     // one stream-ordered block: particles in and out, keys, permutation, flags, ranks, sort scratch
     const size_t pb = sizeof(vlr_particle) * n, wb = sizeof(unsigned) * n;
-    const size_t sb = radix_scratch_bytes(nn, 4);
+    const size_t sb = radix_scratch_bytes(nn, 8);
     auto al = [](size_t b) { return (b + 255) & ~(size_t)255; };
-    const size_t total = 2 * al(pb) + 8 * al(wb) + al(sizeof(int) * 2) + al(sb) + al(sizeof(int32_t) * 3 * n) +
+    const size_t total = 2 * al(pb) + 10 * al(wb) + al(sizeof(int) * 8) + al(sb) + al(sizeof(int32_t) * 3 * n) +
                          al(sizeof(uint32_t) * (n + 1));
     char* blk = nullptr;
     if (cudaMallocFromPoolAsync((void**)&blk, total, ctx->pool, st) != cudaSuccess) {
@@ -238,7 +289,9 @@ int vlr_advect_points(vlr_ctx* ctx, const vlr_grid* vx, const vlr_grid* vy, cons
     unsigned* pbuf = (unsigned*)take(wb);
     int* head = (int*)take(wb);
     int* rank = (int*)take(wb);
-    int* d_total = (int*)take(sizeof(int) * 2);
+    uint64_t* keys = (uint64_t*)take(2 * wb);
+    int* d_total = (int*)take(sizeof(int) * 8);
+    int* d_box = d_total + 2;
     void* scratch = take(sb);
     int32_t* d_org = (int32_t*)take(sizeof(int32_t) * 3 * n);
     uint32_t* d_start = (uint32_t*)take(sizeof(uint32_t) * (n + 1));
@@ -250,25 +303,48 @@ int vlr_advect_points(vlr_ctx* ctx, const vlr_grid* vx, const vlr_grid* vy, cons
     const int blocks = (int)std::min<size_t>((n + 255) / 256, (size_t)ctx->sm_count * 16);
     if (cudaMemcpyAsync(d_in, particles, pb, cudaMemcpyHostToDevice, st) != cudaSuccess)
         return fail(check_cuda(ctx, cudaGetLastError(), "particle upload"));
+    const GridView gx = make_view(vx), gy = make_view(vy), gz = make_view(vz);
+    auto* move = same_transform(gx, gy) && same_transform(gx, gz) ? k_points_move<true> : k_points_move<false>;
+    if (cudaMemsetAsync(d_box, kBoxClear, 6 * sizeof(int), st) != cudaSuccess)
+        return fail(check_cuda(ctx, cudaGetLastError(), "box"));
     VLR_TIMED(ctx, "k_points_move",
-              k_points_move<<<blocks, 256, 0, st>>>(make_view(vx), make_view(vy), make_view(vz), d_in, nn, dt,
-                                                    rk4 ? 1 : 0, inv, kx, ky, kz, idx));
-    // stable sorts by z, then y, then x: lexicographic (x, y, z), ties in input
-    // order.  A sort may leave its result in its scratch, which the next sort
-    // reuses, so each pass's permutation is first moved to pbuf.
-    const int bits = 29;
-    unsigned *ko = nullptr, *perm = nullptr;
-    if (cudaMemcpyAsync(kbuf, kz, wb, cudaMemcpyDeviceToDevice, st) != cudaSuccess)
-        return fail(check_cuda(ctx, cudaGetLastError(), "key copy"));
-    rc = radix_sort(ctx, kbuf, idx, nn, bits, scratch, &ko, &perm);
-    if (rc) return fail(rc);
-    const unsigned* axis_keys[2] = {ky, kx};
-    for (int pass = 0; pass < 2; ++pass) {
-        if (perm != pbuf && cudaMemcpyAsync(pbuf, perm, wb, cudaMemcpyDeviceToDevice, st) != cudaSuccess)
-            return fail(check_cuda(ctx, cudaGetLastError(), "permutation copy"));
-        k_gather_keys<<<blocks, 256, 0, st>>>(axis_keys[pass], pbuf, nn, kbuf);
-        rc = radix_sort(ctx, kbuf, pbuf, nn, bits, scratch, &ko, &perm);
+              move<<<blocks, 256, 0, st>>>(gx, gy, gz, d_in, nn, dt, rk4 ? 1 : 0, inv, kx, ky, kz, idx, d_box));
+    int* hb = static_cast<int*>(ctx->pinned) + 32;
+    if (cudaMemcpyAsync(hb, d_box, 6 * sizeof(int), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
+        cudaStreamSynchronize(st) != cudaSuccess)
+        return fail(check_cuda(ctx, cudaGetLastError(), "particle update"));
+    KeyBox kb;
+    int kbits[3];
+    for (int a = 0; a < 3; ++a) {
+        kb.lo[a] = (unsigned)~hb[a];
+        kbits[a] = bits_for((long long)hb[3 + a] - (long long)~hb[a]);
+    }
+    kb.by = kbits[1];
+    kb.bz = kbits[2];
+    const int bits = kbits[0] + kbits[1] + kbits[2];
+    unsigned* perm = nullptr;
+    if (bits <= 64) {
+        k_points_keys<<<blocks, 256, 0, st>>>(kx, ky, kz, nn, kb, keys);
+        uint64_t* ko = nullptr;
+        rc = radix_sort(ctx, keys, idx, nn, bits, scratch, &ko, &perm);
         if (rc) return fail(rc);
+    } else {
+        // stable sorts by z, then y, then x: lexicographic (x, y, z), ties in
+        // input order.  A sort may leave its result in its scratch, which the
+        // next sort reuses, so each pass's permutation is first moved to pbuf.
+        unsigned* ko = nullptr;
+        if (cudaMemcpyAsync(kbuf, kz, wb, cudaMemcpyDeviceToDevice, st) != cudaSuccess)
+            return fail(check_cuda(ctx, cudaGetLastError(), "key copy"));
+        rc = radix_sort(ctx, kbuf, idx, nn, 29, scratch, &ko, &perm);
+        if (rc) return fail(rc);
+        const unsigned* axis_keys[2] = {ky, kx};
+        for (int pass = 0; pass < 2; ++pass) {
+            if (perm != pbuf && cudaMemcpyAsync(pbuf, perm, wb, cudaMemcpyDeviceToDevice, st) != cudaSuccess)
+                return fail(check_cuda(ctx, cudaGetLastError(), "permutation copy"));
+            k_gather_keys<<<blocks, 256, 0, st>>>(axis_keys[pass], pbuf, nn, kbuf);
+            rc = radix_sort(ctx, kbuf, pbuf, nn, 29, scratch, &ko, &perm);
+            if (rc) return fail(rc);
+        }
     }
     VLR_TIMED(ctx, "k_points_emit",
               k_points_emit<<<blocks, 256, 0, st>>>(d_in, perm, kx, ky, kz, nn, d_out, head));

@@ -101,3 +101,22 @@ def test_mesh_tile_lists_match_oracle(oracle, iso, seed, n, spread, fill, mix):
                                              t.ctypes.data_as(C.POINTER(C.c_uint32)), k, C.byref(nv), C.byref(nt)))
     assert (nv.value, nt.value) == (len(v2), len(t2))
     assert np.array_equal(t[:len(t2)], t2[:k])
+
+
+@pytest.mark.parametrize("same", [True, False], ids=["one-transform", "own-transforms"])
+@pytest.mark.parametrize("rk4", [True, False])
+def test_particles_hinted_samples_match_oracle(oracle, same, rk4):
+    """Particles inside and outside the velocity grids' leaves, steps within and beyond a leaf, far positions."""
+    from sharc.volrus_b200 import VelocityField, VoxelTransform, advect_particles, advect_particles_euler
+    comps = []
+    for a in range(3):
+        v = special_grid(40 + a, 30, 2, 0.8, 0.0)
+        v.set_transform(VoxelTransform.uniform(0.5 if same else (0.5, 0.375, 0.75)[a]))
+        comps.append(v)
+    rng = np.random.default_rng(4)
+    p = np.concatenate([rng.uniform(-9, 9, (5000, 3)), rng.uniform(-1e6, 1e6, (50, 3)), [[1e12, -1e12, 3.0]]])
+    og = [to_oracle(oracle, c) for c in comps]
+    for dt in (0.1, 9.0):
+        got = (advect_particles if rk4 else advect_particles_euler)(p, VelocityField(*comps), dt)
+        want = oracle.advect_particles(*og, p, dt, rk4)
+        assert np.array_equal(got.view(np.uint64), want.view(np.uint64))
