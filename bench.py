@@ -507,10 +507,10 @@ def e2e_method(args, ctx, ls, precision, steps=None):
     one_pass_s = timed(1)
     e2e_s = timed(0)
     return {"value": a / e2e_s, "unit": "voxels/s", "h2d_bytes_per_step": int(h2d), "d2h_bytes_per_step": int(d2h),
-            "seconds_per_step": e2e_s, "steps": steps, "slabs": min(16, n >> 17) if n >= 1 << 18 else 1,
+            "seconds_per_step": e2e_s, "steps": steps, "slabs": min(16, 2 + (n >> 15)) if n >= 1 << 14 else 1,
             "one_pass_seconds_per_step": one_pass_s,
             "path": "vlr_ls_step_host (upload, one step, sorted download), pinned host buffers, f32 values on the "
-                    "host; states of 2^18 leaves or more step as a pipeline of x-slabs whose copies overlap"}
+                    "host; states of 2^14 leaves or more step as a pipeline of x-slabs whose copies overlap"}
 
 
 def roofline_of(r, value_bytes, peak, peak_kind, workload):

@@ -429,7 +429,7 @@ int vlr_ls_edit_device(vlr_ctx* ctx, vlr_level_set* ls, const uint8_t* d_drop, s
  * before the leaf count is known, so records past *n_out (up to that bound)
  * may be overwritten; the call then waits once for the count, the device
  * errors and those copies, and copies any records beyond them.
- * One step of a large single-grid state (at least 2^18 leaves by default)
+ * One step of a large single-grid state (at least 2^14 leaves by default)
  * whose host leaves are sorted by x and whose six host buffers are pinned
  * runs as a pipeline over slabs of consecutive x instead: each slab steps its
  * leaves with the input leaves within 16 voxels beside it and keeps the
@@ -437,10 +437,12 @@ int vlr_ls_edit_device(vlr_ctx* ctx, vlr_level_set* ls, const uint8_t* d_drop, s
  * input goes up and its outputs, sorted (x, y, z), go down on copy streams
  * while other slabs step, so the two copy directions overlap.  The result and
  * the level set's state afterwards are those of the one-pass call, and no
- * record past *n_out is written; an error (the output buffers or the pool
- * too small, a device error) leaves the state undefined until the next
- * upload.  vlr_ls_set_host_slabs sets the slab count: 0 automatic (one slab
- * per 2^17 leaves, at most 16), 1 always one pass, k >= 2 at most k slabs
+ * record past *n_out is written; with 2^18 leaves or more, or a slab count
+ * set, the leaves are then listed sorted, and an error (the output buffers or
+ * the pool too small, a device error) leaves the state undefined until the
+ * next upload; smaller states keep the one pass's list order and errors.
+ * vlr_ls_set_host_slabs sets the slab count: 0 automatic (two slabs and one
+ * more per 2^15 leaves, at most 16), 1 always one pass, k >= 2 at most k slabs
  * (fewer when the leaves have fewer distinct x).  No counterpart in the
  * reference (its step is serial Rust). */
 int vlr_ls_set_host_slabs(vlr_ctx* ctx, vlr_level_set* ls, int slabs);

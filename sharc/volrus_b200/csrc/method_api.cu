@@ -822,24 +822,52 @@ int download_n(vlr_ctx* ctx, const vlr_level_set* ls, size_t n, int grid, int32_
 // steps.  At the end the sorted result is loaded back into the pool, so the
 // level set holds the stepped state as after a one-pass host step.
 constexpr int kSlabRing = 16;                   // voxels: two leaves of input beside a slab
-constexpr size_t kSlabLeavesAuto = 1u << 17;    // automatic count: one slab per this many leaves
-constexpr uint64_t kSlabOther = 0x7fffffffffffffffull;  // key of a leaf the slab does not keep
+// Automatic count: one pass below 2^14 leaves, else 2 slabs and one more per
+// 2^15 leaves.  A slab costs about 0.2 ms of launches and round trips and
+// hides a share of the copies (2.1 KB a leaf each way).  One pass against the
+// best count and its time: 7.1k leaves 0.85 ms (2 slabs 0.94), 19.5k 2.39 (2:
+// 1.90), 38k 4.12 (3: 3.24), 84k 8.3 (4: 6.0), 194k 19.0 (4 to 8: 12.6), 2.5M
+// 239 (8 to 20: 135).
+//
+// Below kSlabLeavesSorted leaves the pipeline is not told from the one pass by
+// what it leaves behind either: the pool keeps the one pass's list order (the
+// larger states list their leaves sorted), and an error runs the one pass for
+// its status and state.
+constexpr size_t kSlabLeavesMin = 1u << 14;
+constexpr size_t kSlabLeavesSorted = 1u << 18;
+constexpr size_t kSlabLeavesPer = 1u << 15;
 
-// 63-bit keys of the listed leaves (leaf coordinates relative to the hash base) for those with x in [xlo, xhi),
-// kSlabOther for the others (sorted after every kept leaf), and the number
-// of kept leaves added to *kept.
+// Key layout of a slab's kept leaves: leaf coordinates relative to a corner
+// below every leaf that the step can leave in the slab, by and bz bits for y
+// and z; bits in all, and the key of the leaves it does not keep (sorted last).
+struct SlabKeys {
+    int x0, y0, z0, by, bz, bits;
+    uint64_t other;
+};
+
+// Keys of the listed leaves with x in [xlo, xhi), K.other for the others, and
+// the number of kept leaves added to *kept.  ord (when not null): each leaf's
+// place in the one pass's list, the input index (first + slot, the slab's
+// input filling the slots in order) of a survivor or of a new leaf's owner,
+// then the owner's direction.
 __global__ void k_slab_keys(const int* __restrict__ list, const int* __restrict__ count,
-                            const int4* __restrict__ origin, long long b0, long long b1, long long b2, int bits,
-                            long long xlo, long long xhi, uint64_t* __restrict__ keys, unsigned* __restrict__ idx,
-                            int* __restrict__ kept) {
+                            const int4* __restrict__ origin, SlabKeys K, long long xlo, long long xhi,
+                            uint64_t* __restrict__ keys, unsigned* __restrict__ idx, int* __restrict__ kept,
+                            const int* __restrict__ newinfo, unsigned first, uint64_t* __restrict__ ord) {
     const int n = *count;
     int c = 0;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const int4 o = origin[list[i]];
-        uint64_t k = kSlabOther;
+        const int slot = list[i];
+        const int4 o = origin[slot];
+        if (ord) {
+            const int info = newinfo[i];
+            ord[i] = info < 0 ? (uint64_t)(first + (unsigned)slot) << 5
+                              : ((uint64_t)(first + (unsigned)(info >> 5)) << 5 | (unsigned)((info & 31) + 1));
+        }
+        uint64_t k = K.other;
         if (o.x >= xlo && o.x < xhi) {
-            k = ((unsigned long long)((o.x >> 3) - b0) << (2 * bits)) |
-                ((unsigned long long)((o.y >> 3) - b1) << bits) | (unsigned long long)((o.z >> 3) - b2);
+            k = ((uint64_t)(unsigned)((o.x >> 3) - K.x0) << (K.by + K.bz)) |
+                ((uint64_t)(unsigned)((o.y >> 3) - K.y0) << K.bz) | (uint64_t)(unsigned)((o.z >> 3) - K.z0);
             ++c;
         }
         keys[i] = k;
@@ -855,7 +883,8 @@ template <typename T>
 __global__ void k_gather_slab(const int* __restrict__ list, const unsigned* __restrict__ sel,
                               const int* __restrict__ kept, int room, const int4* __restrict__ origin,
                               const uint64_t* __restrict__ mask, const T* __restrict__ vals, int32_t* __restrict__ o3,
-                              uint64_t* __restrict__ m_out, float* __restrict__ v_out) {
+                              uint64_t* __restrict__ m_out, float* __restrict__ v_out,
+                              const uint64_t* __restrict__ ord, uint64_t* __restrict__ ord_out) {
     const int k = min(*kept, room), lane = threadIdx.x & 31;
     const bool vec = aligned16(v_out);
     for (int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < k; i += (gridDim.x * blockDim.x) >> 5) {
@@ -864,8 +893,13 @@ __global__ void k_gather_slab(const int* __restrict__ list, const unsigned* __re
             const int4 o = origin[s];
             o3[3 * (size_t)i + lane] = lane == 0 ? o.x : (lane == 1 ? o.y : o.z);
         }
+        if (ord && lane == 3) ord_out[i] = ord[sel[i]];
         record_out(s, (size_t)i, mask, vals, m_out, v_out, vec, lane);
     }
+}
+
+__global__ void k_iota_u(unsigned* a, int n) {
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) a[i] = (unsigned)i;
 }
 
 __global__ void k_set_step(int* scalars, const int* step) { scalars[1] = *step; }
@@ -901,17 +935,44 @@ struct SlabPlan {
     std::vector<size_t> first;    // owned leaves of slab s: [first[s], first[s + 1])
     std::vector<long long> x;     // owned x range of slab s: [x[s], x[s + 1])
     std::vector<size_t> lo, hi;   // stepped input of slab s: [lo[s], hi[s])
+    int box[6];                   // leaf coordinates of the input: lower, upper corner
 };
+
+SlabKeys slab_keys(const SlabPlan& P, int s) {
+    // a step adds only leaves next to listed ones, so the outputs lie within
+    // one leaf of the input's box
+    const int ns = (int)P.first.size() - 1;
+    SlabKeys K;
+    const long long xa = s == 0 ? P.box[0] - 1 : P.x[s] >> 3, xb = s == ns - 1 ? P.box[3] + 1 : (P.x[s + 1] >> 3) - 1;
+    K.x0 = (int)xa;
+    K.y0 = P.box[1] - 1;
+    K.z0 = P.box[2] - 1;
+    K.by = bits_for((long long)P.box[4] - P.box[1] + 2);
+    K.bz = bits_for((long long)P.box[5] - P.box[2] + 2);
+    K.bits = bits_for(xb - xa) + K.by + K.bz;
+    K.other = 1ull << K.bits;
+    return K;
+}
 
 bool plan_slabs(const vlr_level_set* ls, const int32_t* origins, size_t n, SlabPlan* p) {
     int S = ls->host_slabs;
     if (S == 1 || n < 2 || n > (size_t)ls->cap) return false;
-    if (S == 0) S = (int)std::min<size_t>(kHostSlabsMax, n / kSlabLeavesAuto);
+    if (S == 0) S = n < kSlabLeavesMin ? 1 : (int)std::min<size_t>(kHostSlabsMax, 2 + n / kSlabLeavesPer);
     S = std::min(S, kHostSlabsMax);
     if (S < 2) return false;
+    int lo[3] = {INT_MAX, INT_MAX, INT_MAX}, hi[3] = {INT_MIN, INT_MIN, INT_MIN};
     for (size_t i = 0; i < n; ++i) {
-        if ((origins[3 * i] | origins[3 * i + 1] | origins[3 * i + 2]) & 7) return false;  // the one pass reports it
-        if (i && origins[3 * i] < origins[3 * i - 3]) return false;
+        const int32_t* o = origins + 3 * i;
+        if ((o[0] | o[1] | o[2]) & 7) return false;  // the one pass reports it
+        if (i && o[0] < o[-3]) return false;
+        for (int a = 0; a < 3; ++a) {
+            lo[a] = std::min(lo[a], o[a]);
+            hi[a] = std::max(hi[a], o[a]);
+        }
+    }
+    for (int a = 0; a < 3; ++a) {
+        p->box[a] = lo[a] >> 3;
+        p->box[3 + a] = hi[a] >> 3;
     }
     auto xat = [&](size_t i) { return (long long)origins[3 * i]; };
     auto lower = [&](long long x) {  // first leaf with x at or above
@@ -951,7 +1012,7 @@ int cuda_rc(vlr_ctx* ctx, cudaError_t e, const char* what) {
 
 int step_host_slabs(vlr_ctx* ctx, vlr_level_set* ls, const SlabPlan& P, const int32_t* origins,
                     const uint64_t* masks, const float* phi, size_t n, int32_t* out_o, uint64_t* out_m,
-                    float* out_v, size_t cap_leaves, size_t* n_out) {
+                    float* out_v, size_t cap_leaves, size_t* n_out, bool keep_order, int* entry_step) {
     cudaStream_t st = ctx->stream;
     const int ns = (int)P.first.size() - 1;
     for (cudaStream_t& s : ls->slab_stream)
@@ -967,8 +1028,8 @@ int step_host_slabs(vlr_ctx* ctx, vlr_level_set* ls, const SlabPlan& P, const in
     const size_t cmax = (size_t)ls->cap;
     const size_t rec = sizeof(float) * kLeafVoxels + 64 + 12;
     const size_t sort_bytes = radix_scratch_bytes((int)cmax, 8);
-    const size_t bytes = n * rec + cap_out * rec + cmax * (8 + 4) + sort_bytes + 2 * kHostSlabsMax * sizeof(int) +
-                         16 * 256;  // each of the 12 pieces below starts on a 256-byte boundary
+    const size_t bytes = n * rec + cap_out * rec + cmax * (8 + 4) + (keep_order ? 8 * (cmax + cap_out) : 0) + sort_bytes +
+                         2 * kHostSlabsMax * sizeof(int) + 16 * 256;  // each of the 12 pieces below starts on a 256-byte boundary
     char* buf = nullptr;
     VLR_CUDA(ctx, cudaMallocFromPoolAsync((void**)&buf, bytes, ctx->pool, st));
     char* q = buf;
@@ -985,12 +1046,16 @@ int step_host_slabs(vlr_ctx* ctx, vlr_level_set* ls, const SlabPlan& P, const in
     int32_t* out_so = (int32_t*)take(cap_out * 12);
     uint64_t* keys = (uint64_t*)take(cmax * 8);
     unsigned* kidx = (unsigned*)take(cmax * 4);
+    uint64_t* ord = keep_order ? (uint64_t*)take(cmax * 8) : nullptr;         // by list position of a slab
+    uint64_t* out_ord = keep_order ? (uint64_t*)take(cap_out * 8) : nullptr;  // by sorted output
     // [0, ns) kept per slab, [kHostSlabsMax] step at entry
     int* d_small = (int*)take(2 * kHostSlabsMax * sizeof(int));
     void* scratch = take(sort_bytes);
     int* h_count = static_cast<int*>(ctx->pinned) + 64;                  // pool count after slab s's step
     int* h_kept = static_cast<int*>(ctx->pinned) + 64 + kHostSlabsMax;   // outputs slab s keeps
     unsigned* h_err = static_cast<unsigned*>(ctx->pinned) + 64 + 2 * kHostSlabsMax;
+    int* h_step = static_cast<int*>(ctx->pinned) + 66 + 2 * kHostSlabsMax;
+    *h_step = -1;
 
     int rc = VLR_OK;
     auto finish = [&](int code) {
@@ -1002,6 +1067,7 @@ int step_host_slabs(vlr_ctx* ctx, vlr_level_set* ls, const SlabPlan& P, const in
         cudaFreeAsync(buf, st);
         if (code) {
             cudaStreamSynchronize(st);
+            *entry_step = *h_step;
             ls->state_lost = true;
         }
         return code;
@@ -1009,6 +1075,8 @@ int step_host_slabs(vlr_ctx* ctx, vlr_level_set* ls, const SlabPlan& P, const in
     if ((rc = cuda_rc(ctx, cudaMemsetAsync(d_small, 0, 2 * kHostSlabsMax * sizeof(int), st), "cudaMemsetAsync")) ||
         (rc = cuda_rc(ctx, cudaMemcpyAsync(d_small + kHostSlabsMax, ls->scalars + 1, sizeof(int),
                                            cudaMemcpyDeviceToDevice, st), "cudaMemcpyAsync")) ||
+        (rc = cuda_rc(ctx, cudaMemcpyAsync(h_step, ls->scalars + 1, sizeof(int), cudaMemcpyDeviceToHost, st),
+                      "step read-back")) ||
         (rc = cuda_rc(ctx, cudaEventRecord(ev_ready, st), "cudaEventRecord")) ||
         (rc = cuda_rc(ctx, cudaStreamWaitEvent(up, ev_ready, 0), "cudaStreamWaitEvent")) ||
         (rc = cuda_rc(ctx, cudaStreamWaitEvent(down, ev_ready, 0), "cudaStreamWaitEvent")))
@@ -1031,7 +1099,6 @@ int step_host_slabs(vlr_ctx* ctx, vlr_level_set* ls, const SlabPlan& P, const in
         }
         if ((rc = cuda_rc(ctx, cudaEventRecord(ev_up[s], up), "cudaEventRecord"))) return finish(rc);
     }
-    const vlr::MGridParams& G = ls->h_params[0];
     const int B = ctx->sm_count * 8;
     size_t off = 0;  // kept outputs of the slabs before
     std::vector<size_t> offs(ns, 0);
@@ -1077,21 +1144,22 @@ int step_host_slabs(vlr_ctx* ctx, vlr_level_set* ls, const SlabPlan& P, const in
         // its kept outputs, sorted by (x, y, z), gathered after those of the slabs before
         offs[s] = off;
         if (c) {
-            k_slab_keys<<<B, 256, 0, st>>>(ls->list, ls->scalars, ls->origin, G.base[0], G.base[1], G.base[2],
-                                           ls->key_bits, P.x[s], P.x[s + 1], keys, kidx, d_small + s);
+            const SlabKeys K = slab_keys(P, s);
+            k_slab_keys<<<B, 256, 0, st>>>(ls->list, ls->scalars, ls->origin, K, P.x[s], P.x[s + 1], keys, kidx,
+                                           d_small + s, ls->newinfo, (unsigned)P.lo[s], ord);
             uint64_t* k2;
             unsigned* v2;
-            if ((rc = radix_sort(ctx, keys, kidx, c, 63, scratch, &k2, &v2))) return finish(rc);
+            if ((rc = radix_sort(ctx, keys, kidx, c, K.bits + 1, scratch, &k2, &v2))) return finish(rc);
             const size_t o = std::min(off, cap_out);
             const int room = (int)(cap_out - o);
             if (ls->precision == VLR_PREC_F16)
                 k_gather_slab<__half><<<B, 256, 0, st>>>(ls->list, v2, d_small + s, room, ls->origin, ls->mask,
                                                          (const __half*)ls->vals[0], out_so + 3 * o, out_sm + 8 * o,
-                                                         out_sv + kLeafVoxels * o);
+                                                         out_sv + kLeafVoxels * o, ord, ord ? out_ord + o : nullptr);
             else
                 k_gather_slab<float><<<B, 256, 0, st>>>(ls->list, v2, d_small + s, room, ls->origin, ls->mask,
                                                         (const float*)ls->vals[0], out_so + 3 * o, out_sm + 8 * o,
-                                                        out_sv + kLeafVoxels * o);
+                                                        out_sv + kLeafVoxels * o, ord, ord ? out_ord + o : nullptr);
             if ((rc = cuda_rc(ctx, cudaGetLastError(), "slab gather"))) return finish(rc);
         }
         if ((rc = cuda_rc(ctx, cudaMemcpyAsync(h_kept + s, d_small + s, sizeof(int), cudaMemcpyDeviceToHost, st),
@@ -1106,6 +1174,17 @@ int step_host_slabs(vlr_ctx* ctx, vlr_level_set* ls, const SlabPlan& P, const in
     // the stepped state back into the pool (its step counter is already one
     // past the entry value), while the last outputs go down
     if ((rc = load_pool(ctx, ls, out_so, out_sm, out_sv, total))) return finish(rc);
+    if (ord && total) {
+        // slots are in sorted order; the list takes them in the one pass's
+        unsigned* perm;
+        uint64_t* sorted;
+        k_iota_u<<<B, 256, 0, st>>>(kidx, (int)total);
+        if ((rc = radix_sort(ctx, out_ord, kidx, (int)total, bits_for(32ll * (long long)n + 31), scratch, &sorted,
+                             &perm)) ||
+            (rc = cuda_rc(ctx, cudaMemcpyAsync(ls->list, perm, 4 * total, cudaMemcpyDeviceToDevice, st),
+                          "list order")))
+            return finish(rc);
+    }
     rc = finish(VLR_OK);
     if (rc) return rc;
     rc = consume_device_errors(ctx, "vlr_ls_step_host");
@@ -1273,9 +1352,15 @@ int vlr_ls_step_host(vlr_ctx* ctx, vlr_level_set* ls, const int32_t* origins, co
     SlabPlan plan;
     if (n_steps == 1 && 3 * ls->key_bits <= 63 && out_origins && out_masks && out_phi && host_pinned(origins) &&
         host_pinned(masks) && host_pinned(phi) && host_pinned(out_origins) && host_pinned(out_masks) &&
-        host_pinned(out_phi) && plan_slabs(ls, origins, n_leaves, &plan))
-        return step_host_slabs(ctx, ls, plan, origins, masks, phi, n_leaves, out_origins, out_masks, out_phi,
-                               cap_leaves, n_out);
+        host_pinned(out_phi) && plan_slabs(ls, origins, n_leaves, &plan)) {
+        const bool like_one_pass = ls->host_slabs == 0 && n_leaves < kSlabLeavesSorted;
+        int entry_step = -1;  // set once the pipeline may have changed the counter
+        int rc = step_host_slabs(ctx, ls, plan, origins, masks, phi, n_leaves, out_origins, out_masks, out_phi,
+                                 cap_leaves, n_out, like_one_pass, &entry_step);
+        if (rc == VLR_OK || !like_one_pass) return rc;
+        // the one pass reports what is wrong and leaves its state
+        if (entry_step >= 0 && (rc = vlr_ls_set_step(ctx, ls, entry_step))) return rc;
+    }
     // staging for the device-sorted download (sized first, so the upload
     // never regrows it while its copies are in flight)
     const size_t kv = (size_t)kDevSortLeaves;

@@ -120,3 +120,49 @@ def test_slabs_on_library_pinned_buffers(grid):
     cap = 2 * len(inp[0]) + 64
     out = tuple(ctx.pinned((cap,) + a.shape[1:], a.dtype) for a in inp)
     assert _same(_host_step(ls, tuple(lib_in), 4, out=out), ref)
+
+
+@pytest.mark.parametrize("precision", [1, 0], ids=["f16", "f32"])
+@pytest.mark.parametrize("spheres", [75, 140])
+def test_middling_states_leave_what_one_pass_leaves(precision, spheres):
+    """From 2^14 leaves the automatic count pipelines; below 2^18 the level set afterwards lists its leaves in the one
+    pass's order, and buffers too small fail as the one pass does, with a stepped state that steps on."""
+    import torch
+    from sharc.volrus_b200 import VolrusError
+    from sharc.volrus_b200.method import LevelSet, large_sphere_grid
+    sph, vel = large_sphere_grid(spheres, seed=3, extent=1600.0)
+    ls = LevelSet.spheres([(sph, vel)], 1.0, half_width=3.0, precision=precision, integrator=3, reinit_iters=2)
+    try:
+        inp = tuple(_pinned(a) for a in ls.arrays())
+        n = len(inp[0])
+        assert 1 << 14 <= n < 1 << 18
+        dev = torch.device("cuda")
+
+        def listed():
+            cap = 2 * n
+            t = [torch.zeros((cap, k), dtype=d, device=dev)
+                 for k, d in ((3, torch.int32), (8, torch.int64), (512, torch.float32))]
+            torch.cuda.synchronize()
+            k = ls.download_device(*(x.data_ptr() for x in t), cap)
+            return [x[:k].cpu() for x in t]
+        runs = []
+        for slabs in (1, 0):
+            got = _host_step(ls, inp, slabs)
+            state = listed()
+            ls.step(2)
+            runs.append((got, state, listed()))
+        assert _same(runs[0][0], runs[1][0])
+        for a, b in zip(runs[0][1] + runs[0][2], runs[1][1] + runs[1][2]):
+            assert torch.equal(a, b)
+        after = []
+        for slabs in (1, 0):
+            with pytest.raises(VolrusError) as e:
+                _host_step(ls, inp, slabs, out=_out(n // 2))
+            state = listed()
+            ls.step(1)
+            after.append((e.value.code, state, listed()))
+        assert after[0][0] == after[1][0]
+        for a, b in zip(after[0][1] + after[0][2], after[1][1] + after[1][2]):
+            assert torch.equal(a, b)
+    finally:
+        ls.close()
