@@ -518,26 +518,61 @@ int upload_enqueue(vlr_ctx* ctx, vlr_level_set* ls, const int32_t* origins, cons
     return rc;
 }
 
-// Device-resident leaves: origins i32[3] -> the pool's int4 origins (origins
-// not on the 8-voxel lattice flag kErrInput), f32 values -> the pool's type.
-__global__ void k_upload_dev_origins(const int32_t* o3, int n, int4* origin, unsigned* err) {
+// A round trip to the host costs about 12 us beside kernels of 1-3 us, so a
+// device exchange makes one per call and no more: origins are checked with the
+// index that is built from them, the read-out bounds itself by the count it
+// reads, and the step counter rides on its launch.  A 62-leaf frame (load,
+// counter, step, read-out: 8 waits before, 3 now) went from 133 to 96 us.
+//
+// Device-resident leaves, part 1: origins i32[3] -> the pool's int4 origins
+// (origins not on the 8-voxel lattice flag kErrInput), the list and the free
+// stack of n leaves in slots 0..n-1, an empty hash.
+__global__ void k_load_lists(const int32_t* __restrict__ o3, int n, int4* __restrict__ origin, int* __restrict__ list,
+                             int* __restrict__ free_stack, int* __restrict__ scalars, int cap,
+                             uint64_t* __restrict__ hkey, int* __restrict__ hval, int hcap, unsigned* err) {
     unsigned bad = 0;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const int x = o3[3 * i], y = o3[3 * i + 1], z = o3[3 * i + 2];
-        bad |= (unsigned)((x | y | z) & 7);
-        origin[i] = make_int4(x, y, z, 0);
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < max(cap, hcap); i += gridDim.x * blockDim.x) {
+        if (i < n) {
+            const int x = o3[3 * (size_t)i], y = o3[3 * (size_t)i + 1], z = o3[3 * (size_t)i + 2];
+            bad |= (unsigned)((x | y | z) & 7);
+            origin[i] = make_int4(x, y, z, 0);
+            list[i] = i;
+        }
+        if (i < cap - n) free_stack[i] = cap - 1 - i;
+        if (i < hcap) {
+            hkey[i] = kEmptyKey;
+            hval[i] = -1;
+        }
     }
     if (bad) atomicOr(err, kErrInput);
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        scalars[0] = n;
+        scalars[2] = cap - n;
+        for (int q = 3; q < 8; ++q) scalars[q] = 0;
+    }
+}
+
+// Part 2: masks (where given), and f32 values in the pool's type, one warp per leaf.
+template <typename T>
+__global__ void __launch_bounds__(256) k_load_records(const uint64_t* __restrict__ masks, const float* __restrict__ phi,
+                                                     int n, uint64_t* __restrict__ mask, T* __restrict__ vals) {
+    const int lane = threadIdx.x & 31;
+    const bool vec = aligned16(phi);
+    for (int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < n; i += (gridDim.x * blockDim.x) >> 5) {
+        if (masks && lane < 8) mask[(size_t)i * 8 + lane] = masks[(size_t)i * 8 + lane];
+        leaf_in(phi + (size_t)i * kLeafVoxels, vals + (size_t)i * kLeafVoxels, vec, lane);
+    }
 }
 
 // The listed leaves in list order into device buffers (origins i32[3], masks,
 // f32 values), one warp per leaf (312k f16 leaves: 466 us one CTA per leaf
 // and one value per thread, 166 us this way, 5.9 TB/s).
 template <typename T>
-__global__ void __launch_bounds__(256) k_export_dev(const int* list, const int* count, const int4* origin,
+__global__ void __launch_bounds__(256) k_export_dev(const int* list, const int* count, int cap, const int4* origin,
                                                    const uint64_t* mask, const T* vals, int32_t* o3,
                                                    uint64_t* m_out, float* v_out) {
     const int n = *count, lane = threadIdx.x & 31;
+    if (n > cap) return;  // the buffers are too small: nothing is written
     const bool vec = aligned16(v_out);
     for (int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < n; i += (gridDim.x * blockDim.x) >> 5) {
         const int s = list[i];
@@ -904,6 +939,12 @@ __global__ void k_iota_u(unsigned* a, int n) {
 
 __global__ void k_set_step(int* scalars, const int* step) { scalars[1] = *step; }
 
+// The step counter, and the look-back scan's n status words cleared.
+__global__ void k_set_step_value(int* scalars, int step, int* status, int n) {
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) status[i] = 0;
+    if (blockIdx.x == 0 && threadIdx.x == 0) scalars[1] = step;
+}
+
 bool host_pinned(const void* p) {
     cudaPointerAttributes at{};
     const bool ok = cudaPointerGetAttributes(&at, p) == cudaSuccess && at.type == cudaMemoryTypeHost;
@@ -1247,8 +1288,7 @@ int vlr_ls_enqueue(vlr_ctx* ctx, vlr_level_set* ls, int n_steps) {
 
 int vlr_ctx_check(vlr_ctx* ctx) {
     if (!ctx) return VLR_ERR_INVALID;
-    VLR_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-    return consume_device_errors(ctx, "vlr_ctx_check");
+    return consume_device_errors(ctx, "vlr_ctx_check");  // waits for the stream
 }
 
 int vlr_ls_step(vlr_ctx* ctx, vlr_level_set* ls, int n_steps) {
@@ -1257,8 +1297,7 @@ int vlr_ls_step(vlr_ctx* ctx, vlr_level_set* ls, int n_steps) {
         int rc = enqueue_one_step(ctx, ls);
         if (rc) return rc;
     }
-    VLR_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-    const int rc = consume_device_errors(ctx, "vlr_ls_step");
+    const int rc = consume_device_errors(ctx, "vlr_ls_step");  // waits for the stream
     if (rc == VLR_ERR_TIMEOUT || rc == VLR_ERR_CAPACITY) ls->state_lost = true;
     return rc;
 }
@@ -1453,21 +1492,33 @@ int vlr_ls_upload_device(vlr_ctx* ctx, vlr_level_set* ls, const int32_t* d_origi
     if (ls->n_grids != 1) return set_error(ctx, VLR_ERR_UNSUPPORTED, "upload replaces single-grid states only");
     if (n_leaves > (size_t)ls->cap) return set_error(ctx, VLR_ERR_CAPACITY, "more leaves than the level set's capacity");
     const int n = (int)n_leaves;
+    k_load_lists<<<ls->grid_blocks, 256, 0, ctx->stream>>>(d_origins, n, ls->origin, ls->list, ls->free_stack,
+                                                           ls->scalars, ls->cap, ls->hkey, ls->hval, ls->hcap,
+                                                           ctx->d_errword);
     if (n) {
-        k_upload_dev_origins<<<ls->grid_blocks, 256, 0, ctx->stream>>>(d_origins, n, ls->origin, ctx->d_errword);
-        VLR_CUDA(ctx, cudaMemcpyAsync(ls->mask, d_masks, 64 * n_leaves, cudaMemcpyDeviceToDevice, ctx->stream));
-        if (ls->precision == VLR_PREC_F16)
-            k_from_f32<__half><<<leaf_warp_blocks(ctx, n_leaves), 256, 0, ctx->stream>>>(
-                d_phi, (__half*)ls->vals[0], n_leaves);
-        else
+        const int B = leaf_warp_blocks(ctx, n_leaves);
+        // packed buffers may start at any byte: what the kernel cannot read goes by plain copies
+        const uint64_t* masks = (uintptr_t)d_masks & 7 ? nullptr : d_masks;
+        if (!masks)
+            VLR_CUDA(ctx, cudaMemcpyAsync(ls->mask, d_masks, 64 * n_leaves, cudaMemcpyDeviceToDevice, ctx->stream));
+        if (ls->precision == VLR_PREC_F16) {
+            k_load_records<__half><<<B, 256, 0, ctx->stream>>>(masks, d_phi, n, ls->mask, (__half*)ls->vals[0]);
+        } else if ((uintptr_t)d_phi & 3) {
+            if (masks)
+                VLR_CUDA(ctx, cudaMemcpyAsync(ls->mask, masks, 64 * n_leaves, cudaMemcpyDeviceToDevice, ctx->stream));
             VLR_CUDA(ctx, cudaMemcpyAsync(ls->vals[0], d_phi, sizeof(float) * kLeafVoxels * n_leaves,
                                           cudaMemcpyDeviceToDevice, ctx->stream));
-        VLR_CUDA(ctx, cudaGetLastError());
+        } else {
+            k_load_records<float><<<B, 256, 0, ctx->stream>>>(masks, d_phi, n, ls->mask, (float*)ls->vals[0]);
+        }
     }
-    // origins are checked before the index is built from them
-    int rc = consume_device_errors(ctx, "vlr_ls_upload_device");
-    if (rc) return rc;
-    return ls_init_lists(ctx, ls, n, false);
+    VLR_CUDA(ctx, cudaGetLastError());
+    int rc = ls_enqueue_index(ctx, ls, true);
+    // one round trip for the origins' check and the index's (an index built
+    // from origins off the lattice is never used: the call fails)
+    if (!rc) rc = consume_device_errors(ctx, "vlr_ls_upload_device");
+    if (!rc) ls->state_lost = false;  // a complete new state
+    return rc;
 }
 
 int vlr_ls_download_device(vlr_ctx* ctx, const vlr_level_set* ls, int32_t* d_origins, uint64_t* d_masks,
@@ -1475,22 +1526,22 @@ int vlr_ls_download_device(vlr_ctx* ctx, const vlr_level_set* ls, int32_t* d_ori
     if (!ctx || !ls || !n_out || !d_origins || !d_masks || !d_phi)
         return set_error(ctx, VLR_ERR_INVALID, "null argument");
     *n_out = 0;
-    size_t n = 0;
-    int rc = vlr_ls_info(ctx, ls, &n, nullptr, nullptr);
+    // the kernel reads the leaf count itself and writes nothing past the
+    // buffers, so the count comes back with its completion
+    const int cap = (int)std::min<size_t>(cap_leaves, (size_t)ls->cap);
+    const int B = leaf_warp_blocks(ctx, (size_t)cap);
+    if (ls->precision == VLR_PREC_F16)
+        k_export_dev<__half><<<B, 256, 0, ctx->stream>>>(ls->list, ls->scalars, cap, ls->origin, ls->mask,
+                                                         (const __half*)ls->vals[0], d_origins, d_masks, d_phi);
+    else
+        k_export_dev<float><<<B, 256, 0, ctx->stream>>>(ls->list, ls->scalars, cap, ls->origin, ls->mask,
+                                                        (const float*)ls->vals[0], d_origins, d_masks, d_phi);
+    VLR_CUDA(ctx, cudaGetLastError());
+    int n = 0;
+    int rc = read_int(ctx, ls->scalars, &n);
     if (rc) return rc;
-    if (n > cap_leaves) return set_error(ctx, VLR_ERR_CAPACITY, "output buffers too small");
-    if (n) {
-        const int B = leaf_warp_blocks(ctx, n);
-        if (ls->precision == VLR_PREC_F16)
-            k_export_dev<__half><<<B, 256, 0, ctx->stream>>>(ls->list, ls->scalars, ls->origin, ls->mask,
-                                                             (const __half*)ls->vals[0], d_origins, d_masks, d_phi);
-        else
-            k_export_dev<float><<<B, 256, 0, ctx->stream>>>(ls->list, ls->scalars, ls->origin, ls->mask,
-                                                            (const float*)ls->vals[0], d_origins, d_masks, d_phi);
-        VLR_CUDA(ctx, cudaGetLastError());
-        VLR_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-    }
-    *n_out = n;
+    if (n > cap) return set_error(ctx, VLR_ERR_CAPACITY, "output buffers too small");
+    *n_out = (size_t)n;
     return VLR_OK;
 }
 
@@ -1523,9 +1574,10 @@ int vlr_ls_set_step(vlr_ctx* ctx, vlr_level_set* ls, int step) {
     if (!ls->scalars) return set_error(ctx, VLR_ERR_INVALID, "level set has no state");
     // the look-back scan tags its status words with step + 1: clear them so no
     // word of an earlier step can carry the tag of a step to come
-    VLR_CUDA(ctx, cudaMemsetAsync(ls->pos, 0, sizeof(int) * (ls->cap + 1 + scan_scratch_ints(ls->cap)), ctx->stream));
-    VLR_CUDA(ctx, cudaMemcpyAsync(ls->scalars + 1, &step, sizeof(int), cudaMemcpyHostToDevice, ctx->stream));
-    VLR_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    const int words = (int)scan_scratch_ints(ls->cap);
+    k_set_step_value<<<std::min((words + 255) / 256, ls->grid_blocks), 256, 0, ctx->stream>>>(ls->scalars, step, ls->pos,
+                                                                                             words);
+    VLR_CUDA(ctx, cudaGetLastError());
     return VLR_OK;
 }
 

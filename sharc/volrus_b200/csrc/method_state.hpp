@@ -105,8 +105,8 @@ int ls_alloc(vlr_ctx* ctx, vlr_level_set* ls, int cap);
 void ls_free(vlr_level_set* ls);
 // Enqueue one step (no host synchronisation; capturable).
 int ls_enqueue_step(vlr_ctx* ctx, vlr_level_set* ls);
-// Rebuild hash and neighbour table from the list (enqueued).
-int ls_enqueue_index(vlr_ctx* ctx, vlr_level_set* ls);
+// Rebuild hash and neighbour table from the list (enqueued); cleared: the hash is empty already.
+int ls_enqueue_index(vlr_ctx* ctx, vlr_level_set* ls, bool cleared = false);
 int ls_enqueue_retrack(vlr_ctx* ctx, vlr_level_set* ls);
 // One step whose stencil kernels are launched at every candidate shape (timed,
 // synchronising); keeps the fastest shape of each kernel.  The step's result

@@ -421,10 +421,10 @@ MTopo topo_of(vlr_level_set* ls) {
     return t;
 }
 
-int ls_enqueue_index(vlr_ctx* ctx, vlr_level_set* ls) {
+int ls_enqueue_index(vlr_ctx* ctx, vlr_level_set* ls, bool cleared) {
     cudaStream_t st = ctx->stream;
     const int B = ls->grid_blocks;
-    k_h_clear<<<B, 256, 0, st>>>(ls->hkey, ls->hval, ls->hcap);
+    if (!cleared) k_h_clear<<<B, 256, 0, st>>>(ls->hkey, ls->hval, ls->hcap);
     k_h_insert<<<B, 256, 0, st>>>(ls->list, ls->scalars, ls->origin, ls->hkey, ls->hval, ls->hcap, ls->d_params,
                                   ls->key_bits, ctx->d_errword);
     k_nbr<<<B, 256, 0, st>>>(ls->list, ls->scalars, ls->origin, ls->hkey, ls->hval, ls->hcap, ls->d_params,
