@@ -149,6 +149,13 @@ typedef struct vlr_particle {
 int vlr_advect_points(vlr_ctx* ctx, const vlr_grid* vx, const vlr_grid* vy, const vlr_grid* vz,
                       const double world_to_index[12], vlr_particle* particles, size_t n, double dt, int rk4,
                       int32_t* leaf_origins, uint32_t* leaf_start, size_t cap_leaves, size_t* n_leaves);
+/* vlr_advect_points with the result in `out` (n records; it may be
+ * `particles`, and must not overlap it otherwise): the given particles stay
+ * as they are, and the caller needs no copy of them. */
+int vlr_advect_points_to(vlr_ctx* ctx, const vlr_grid* vx, const vlr_grid* vy, const vlr_grid* vz,
+                         const double world_to_index[12], const vlr_particle* particles, vlr_particle* out, size_t n,
+                         double dt, int rk4, int32_t* leaf_origins, uint32_t* leaf_start, size_t cap_leaves,
+                         size_t* n_leaves);
 /* Replaces dilate(&mut Grid<f32>, iterations) (src/tools/morphology.rs:20-35):
  * every inactive voxel with an active 6-neighbour becomes active with the
  * value of the neighbour that comes first in the tree's iteration order

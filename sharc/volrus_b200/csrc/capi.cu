@@ -166,6 +166,7 @@ void vlr_ctx_destroy(vlr_ctx* ctx) {
     cudaFree(ctx->scratch);
     cudaFree(ctx->d_errword);
     cudaFreeHost(ctx->pinned);
+    vlr::copy_threads_stop(ctx);
     if (ctx->stage) cudaFreeHost(ctx->stage);
     for (auto& e : ctx->stage_ev)
         if (e) cudaEventDestroy(e);

@@ -231,23 +231,33 @@ int vlr_advect_particles(vlr_ctx* ctx, const vlr_grid* vx, const vlr_grid* vy, c
     if (n > (size_t)INT32_MAX / 3) return set_error(ctx, VLR_ERR_CAPACITY, "too many particles");
     double* d = nullptr;
     VLR_CUDA(ctx, cudaMallocFromPoolAsync(&d, sizeof(double) * 3 * n, ctx->pool, ctx->stream));
-    VLR_CUDA(ctx, cudaMemcpyAsync(d, positions, sizeof(double) * 3 * n, cudaMemcpyHostToDevice, ctx->stream));
+    int rc = h2d_copy(ctx, d, positions, sizeof(double) * 3 * n);
     const int blocks = (int)std::min<size_t>((n + 255) / 256, (size_t)ctx->sm_count * 16);
     const GridView gx = make_view(vx), gy = make_view(vy), gz = make_view(vz);
     auto* kernel = same_transform(gx, gy) && same_transform(gx, gz) ? k_advect_particles<true>
                                                                    : k_advect_particles<false>;
-    kernel<<<blocks, 256, 0, ctx->stream>>>(gx, gy, gz, d, (int)n, dt, rk4 ? 1 : 0);
-    VLR_CUDA(ctx, cudaGetLastError());
-    VLR_CUDA(ctx, cudaMemcpyAsync(positions, d, sizeof(double) * 3 * n, cudaMemcpyDeviceToHost, ctx->stream));
-    VLR_CUDA(ctx, cudaFreeAsync(d, ctx->stream));
-    VLR_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-    return consume_device_errors(ctx, "vlr_advect_particles");
+    if (!rc) {
+        kernel<<<blocks, 256, 0, ctx->stream>>>(gx, gy, gz, d, (int)n, dt, rk4 ? 1 : 0);
+        const cudaError_t e = cudaGetLastError();
+        if (e != cudaSuccess) rc = check_cuda(ctx, e, "k_advect_particles");
+    }
+    if (!rc) rc = d2h_copy(ctx, positions, d, sizeof(double) * 3 * n);
+    cudaFreeAsync(d, ctx->stream);
+    return rc ? rc : consume_device_errors(ctx, "vlr_advect_particles");
 }
 
 int vlr_advect_points(vlr_ctx* ctx, const vlr_grid* vx, const vlr_grid* vy, const vlr_grid* vz,
                       const double world_to_index[12], vlr_particle* particles, size_t n, double dt, int rk4,
                       int32_t* leaf_origins, uint32_t* leaf_start, size_t cap_leaves, size_t* n_leaves) {
-    if (!ctx || !vx || !vy || !vz || !world_to_index || !n_leaves || (n && !particles) || !leaf_start ||
+    return vlr_advect_points_to(ctx, vx, vy, vz, world_to_index, particles, particles, n, dt, rk4, leaf_origins,
+                                leaf_start, cap_leaves, n_leaves);
+}
+
+int vlr_advect_points_to(vlr_ctx* ctx, const vlr_grid* vx, const vlr_grid* vy, const vlr_grid* vz,
+                         const double world_to_index[12], const vlr_particle* particles, vlr_particle* out, size_t n,
+                         double dt, int rk4, int32_t* leaf_origins, uint32_t* leaf_start, size_t cap_leaves,
+                         size_t* n_leaves) {
+    if (!ctx || !vx || !vy || !vz || !world_to_index || !n_leaves || (n && (!particles || !out)) || !leaf_start ||
         (cap_leaves && !leaf_origins))
         return set_error(ctx, VLR_ERR_INVALID, "null argument");
     if (vx->kind != VLR_KIND_F32_WORLD || vy->kind != VLR_KIND_F32_WORLD || vz->kind != VLR_KIND_F32_WORLD)
@@ -301,8 +311,7 @@ int vlr_advect_points(vlr_ctx* ctx, const vlr_grid* vx, const vlr_grid* vy, cons
         return code;
     };
     const int blocks = (int)std::min<size_t>((n + 255) / 256, (size_t)ctx->sm_count * 16);
-    if (cudaMemcpyAsync(d_in, particles, pb, cudaMemcpyHostToDevice, st) != cudaSuccess)
-        return fail(check_cuda(ctx, cudaGetLastError(), "particle upload"));
+    if ((rc = h2d_copy(ctx, d_in, particles, pb))) return fail(rc);
     const GridView gx = make_view(vx), gy = make_view(vy), gz = make_view(vz);
     auto* move = same_transform(gx, gy) && same_transform(gx, gz) ? k_points_move<true> : k_points_move<false>;
     if (cudaMemsetAsync(d_box, kBoxClear, 6 * sizeof(int), st) != cudaSuccess)
@@ -361,10 +370,10 @@ int vlr_advect_points(vlr_ctx* ctx, const vlr_grid* vx, const vlr_grid* vy, cons
         return set_error(ctx, VLR_ERR_CAPACITY,
                          "vlr_advect_points: " + std::to_string(leaves) + " leaves exceed cap_leaves");
     }
-    VLR_CUDA(ctx, cudaMemcpyAsync(particles, d_out, pb, cudaMemcpyDeviceToHost, st));
-    VLR_CUDA(ctx, cudaMemcpyAsync(leaf_origins, d_org, sizeof(int32_t) * 3 * leaves, cudaMemcpyDeviceToHost, st));
-    VLR_CUDA(ctx, cudaMemcpyAsync(leaf_start, d_start, sizeof(uint32_t) * leaves, cudaMemcpyDeviceToHost, st));
-    VLR_CUDA(ctx, cudaStreamSynchronize(st));
+    if ((rc = d2h_copy(ctx, out, d_out, pb)) ||
+        (rc = d2h_copy(ctx, leaf_origins, d_org, sizeof(int32_t) * 3 * leaves)) ||
+        (rc = d2h_copy(ctx, leaf_start, d_start, sizeof(uint32_t) * leaves)))
+        return fail(rc);
     leaf_start[leaves] = (uint32_t)n;
     cudaFreeAsync(blk, st);
     return consume_device_errors(ctx, "vlr_advect_points");

@@ -632,17 +632,17 @@ int advect_ref(vlr_ctx* ctx, const vlr_grid* g, const vlr_grid* vx, const vlr_gr
 int sample_points(vlr_ctx* ctx, const vlr_grid* g, const double* h_pts, size_t n, float* h_out) {
     if (n == 0) return VLR_OK;
     double* d_pts = nullptr;
-    float* d_out = nullptr;
-    VLR_CUDA(ctx, cudaMallocFromPoolAsync(&d_pts, sizeof(double) * 3 * n, ctx->pool, ctx->stream));
-    VLR_CUDA(ctx, cudaMallocFromPoolAsync(&d_out, sizeof(float) * n, ctx->pool, ctx->stream));
-    VLR_CUDA(ctx, cudaMemcpyAsync(d_pts, h_pts, sizeof(double) * 3 * n, cudaMemcpyHostToDevice, ctx->stream));
-    k_sample_points<<<(unsigned)((n + 255) / 256), 256, 0, ctx->stream>>>(make_view(g), d_pts, (int)n, d_out);
-    VLR_CUDA(ctx, cudaGetLastError());
-    VLR_CUDA(ctx, cudaMemcpyAsync(h_out, d_out, sizeof(float) * n, cudaMemcpyDeviceToHost, ctx->stream));
-    VLR_CUDA(ctx, cudaFreeAsync(d_pts, ctx->stream));
-    VLR_CUDA(ctx, cudaFreeAsync(d_out, ctx->stream));
-    VLR_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-    return VLR_OK;
+    VLR_CUDA(ctx, cudaMallocFromPoolAsync(&d_pts, (sizeof(double) * 3 + sizeof(float)) * n, ctx->pool, ctx->stream));
+    float* d_out = reinterpret_cast<float*>(d_pts + 3 * n);
+    int rc = h2d_copy(ctx, d_pts, h_pts, sizeof(double) * 3 * n);
+    if (!rc) {
+        k_sample_points<<<(unsigned)((n + 255) / 256), 256, 0, ctx->stream>>>(make_view(g), d_pts, (int)n, d_out);
+        const cudaError_t e = cudaGetLastError();
+        if (e != cudaSuccess) rc = check_cuda(ctx, e, "k_sample_points");
+    }
+    if (!rc) rc = d2h_copy(ctx, h_out, d_out, sizeof(float) * n);
+    cudaFreeAsync(d_pts, ctx->stream);
+    return rc;
 }
 
 // Device buffers of a crossing search over n leaves, in one block.

@@ -1,6 +1,7 @@
 // Host-side context and grid handles behind the C ABI (include/volrus_b200.h).
 #pragma once
 #include <cstdint>
+#include <memory>
 #include <string>
 #include <vector>
 #include <cuda_runtime.h>
@@ -21,6 +22,10 @@ struct vlr_kernel_timer {
     std::vector<std::pair<std::string, std::pair<double, long long>>> totals;  // name -> (ms, launches)
 };
 
+namespace vlr {
+struct CopyThreads;
+}
+
 struct vlr_ctx {
     int device = 0;
     int sm_count = 148;
@@ -32,8 +37,9 @@ struct vlr_ctx {
     void* scratch = nullptr;
     size_t scratch_bytes = 0;
     void* pinned = nullptr;             // small pinned host buffer for scalar read-backs
-    void* stage = nullptr;              // pinned double buffer for large copies into pageable memory
-    cudaEvent_t stage_ev[2] = {nullptr, nullptr};
+    void* stage = nullptr;              // pinned buffers for large copies from and into pageable memory
+    cudaEvent_t stage_ev[8] = {};
+    std::shared_ptr<vlr::CopyThreads> copy_threads;  // the threads that move those copies
     vlr_kernel_timer timer;
 };
 
@@ -134,10 +140,12 @@ int scan_exclusive(vlr_ctx* ctx, const int* d_in, int* d_out, long long n, int* 
 // Read the device error word, clear it, and map it to a status.
 int consume_device_errors(vlr_ctx* ctx, const char* what);
 // Device-to-host copy of `bytes` on the context stream, returning after it.
-// Large copies into pageable memory go through a pinned double buffer (the
-// DMA of one chunk overlaps the host copy of the previous one), twice the
-// driver's own pageable rate here; small or pinned destinations take one copy.
+// Large copies into or from pageable memory go through pinned buffers, in
+// shares that a few threads move at once; small or pinned ones take one copy.
+// h2d_copy has read the source when it returns; the device side is stream-ordered.
 int d2h_copy(vlr_ctx* ctx, void* dst, const void* src, size_t bytes);
+void copy_threads_stop(vlr_ctx* ctx);
+int h2d_copy(vlr_ctx* ctx, void* dst, const void* src, size_t bytes);
 int read_int(vlr_ctx* ctx, const int* d_ptr, int* out);
 // read_int and consume_device_errors in one round trip.
 int read_int_checked(vlr_ctx* ctx, const int* d_ptr, int* out, const char* what);

@@ -146,7 +146,7 @@ def sample_trilinear(grid, world_pos, ctx: Context | None = None):
     p = np.ascontiguousarray(world_pos, np.float64)
     single = p.ndim == 1
     p = p.reshape(-1, 3)
-    out = np.zeros(len(p), np.float32)
+    out = np.empty(len(p), np.float32)
     ctx.check(ctx.lib.vlr_sample_trilinear(ctx.handle, g.handle, ptr(p, C.c_double), len(p), ptr(out, C.c_float)),
               "vlr_sample_trilinear")
     return float(out[0]) if single else out
@@ -162,7 +162,8 @@ def find_zero_crossings(grid, ctx: Context | None = None) -> np.ndarray:
     out = np.empty((max(cap, 1), 3), np.int32)
     ctx.check(ctx.lib.vlr_find_zero_crossings(ctx.handle, g.handle, ptr(out, C.c_int32), cap, C.byref(cnt)),
               "vlr_find_zero_crossings")
-    return out[: cnt.value].copy()
+    out.resize((cnt.value, 3), refcheck=False)  # gives the room that was not needed back; no copy
+    return out
 
 
 def trim_narrow_band(grid, half_width: float, ctx: Context | None = None):
@@ -221,18 +222,20 @@ def _advect_points(points, velocity: VelocityField, dt: float, rk4: bool, ctx):
     update and the closing PointDataGrid::rebin, in one C-ABI call."""
     from .points import PARTICLE
     ctx = ctx or Context.default()
-    parts = np.ascontiguousarray(points.particles, PARTICLE).copy()
-    n = len(parts)
+    given = np.ascontiguousarray(points.particles, PARTICLE)
+    n = len(given)
+    parts = np.empty(n, PARTICLE)  # written by the call alone: the given particles stay as they are
     inv = points.inverse_rows()
     origins = np.zeros((max(n, 1), 3), np.int32)
     start = np.zeros(n + 1, np.uint32)
     nl = C.c_size_t()
     made = [_as_device(g, ctx) for g in (velocity.vx, velocity.vy, velocity.vz)]
     try:
-        ctx.check(ctx.lib.vlr_advect_points(ctx.handle, made[0][0].handle, made[1][0].handle, made[2][0].handle,
-                                            ptr(inv, C.c_double), parts.ctypes.data_as(C.c_void_p), n, float(dt),
-                                            1 if rk4 else 0, ptr(origins, C.c_int32), ptr(start, C.c_uint32),
-                                            max(n, 1), C.byref(nl)), "vlr_advect_points")
+        ctx.check(ctx.lib.vlr_advect_points_to(ctx.handle, made[0][0].handle, made[1][0].handle, made[2][0].handle,
+                                               ptr(inv, C.c_double), given.ctypes.data_as(C.c_void_p),
+                                               parts.ctypes.data_as(C.c_void_p), n, float(dt), 1 if rk4 else 0,
+                                               ptr(origins, C.c_int32), ptr(start, C.c_uint32), max(n, 1),
+                                               C.byref(nl)), "vlr_advect_points_to")
     finally:
         for d, created in made:
             if created:
