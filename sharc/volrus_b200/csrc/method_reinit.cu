@@ -18,20 +18,20 @@
 //              work in the common case (see godunov_update_raw).
 //   phase 1    warp 0 compacts the box voxels of D for iteration 1 (the
 //              10^3 box around the leaf without its edges and corners, which
-//              iteration 2 never reads) and keeps their bit words; warp 1
-//              compacts the leaf's voxels of D; warps 1-3 issue the next
-//              leaf's copies and write every voxel's outside-D result
-//              copysign(hw, value) to global memory (coalesced).
+//              iteration 2 never reads); warp 1 compacts the leaf's voxels
+//              of D; warps 1-3 issue the next leaf's copies, write every
+//              voxel's outside-D result copysign(hw, value) to global memory
+//              (coalesced) and copy phi1 on the box into phi2.
 //   phase 2    iteration 1 on the box list, consecutive voxels on
 //              consecutive lanes (bank-conflict-free stage reads), into phi2.
 //   phase 3    iteration 2 (or the only one) on the leaf list, its
-//              neighbours from phi2 where the box bit is set and from the
-//              stage (phi1) elsewhere; trim, stores over the outside-D
-//              results, activity bits into a shared mask.
+//              neighbours from phi2 (iteration 1's result on the box voxels
+//              of D, phi1 elsewhere); trim, stores over the outside-D
+//              results, activity bytes.
 //   phase 4    mask out, spill toward absent neighbours, keep flags and
 //              proposals (hash of the missing leaf, atomicMin of the
 //              proposer's direction), by warp 3 during the next leaf's
-//              phase 1 (its mask words, neighbour row, slot and origin kept
+//              phase 1 (its activity, neighbour row, slot and origin kept
 //              in shared memory), after the loop for the CTA's last leaf.
 //
 // Three CTA barriers per leaf (two without iteration 1).  Neighbour rows
@@ -138,18 +138,20 @@ __device__ __forceinline__ const T* at(const T* stage, int x, int y, int z) {
 // differences are u = max(sg (p - phi_-), 0) and w = max(sg (p - phi_+), 0),
 // sg = +-1 the sign of s, and the axis term is max(u, w)^2, the same value as
 // the sign-split form max(max(a-, 0)^2, min(a+, 0)^2) for s >= 0 and its
-// mirror for s < 0, without the sign branch.  max(u, w) is evaluated as
-// max(sg p - min(sg phi_-, sg phi_+), 0): negation is exact and rounding is
-// monotone, so this is the same value, and fminf drops a NaN neighbour just
-// as fmaxf drops its NaN difference.  The correctly rounded sqrtf keeps a
+// mirror for s < 0, without the sign branch.  With q = sg p the differences are
+// q - sg phi: the product is exact, so one FMA rounds each as the subtraction
+// would, and one three-input max joins them (fmaxf drops a NaN neighbour's
+// difference).  Min and max run at half the FMA rate and this kernel is bound
+// by instructions: two FMAs and one max per axis for two products, a min, a
+// subtraction and a max.  The correctly rounded sqrtf keeps a
 // full deformation period's FP32 topology equal to the FP64 run's (an
 // rsqrtf-based magnitude measured two voxels flipping at the band's edge).
 __device__ __forceinline__ float godunov_g(float p, float xm, float xp, float ym, float yp, float zm, float zp, float s) {
     const float sg = (s >= 0.f) ? 1.f : -1.f;
     const float q = sg * p;
-    const float mx = fmaxf(q - fminf(sg * xm, sg * xp), 0.f);
-    const float my = fmaxf(q - fminf(sg * ym, sg * yp), 0.f);
-    const float mz = fmaxf(q - fminf(sg * zm, sg * zp), 0.f);
+    const float mx = fmaxf(fmaxf(__fmaf_rn(-sg, xm, q), __fmaf_rn(-sg, xp, q)), 0.f);
+    const float my = fmaxf(fmaxf(__fmaf_rn(-sg, ym, q), __fmaf_rn(-sg, yp, q)), 0.f);
+    const float mz = fmaxf(fmaxf(__fmaf_rn(-sg, zm, q), __fmaf_rn(-sg, zp, q)), 0.f);
     // squares rounded before the sums (no contraction)
     float g2 = __fmul_rn(mx, mx) + __fmul_rn(my, my);
     g2 += __fmul_rn(mz, mz);
@@ -159,6 +161,14 @@ __device__ __forceinline__ float godunov_g(float p, float xm, float xp, float ym
 // NaN marks a voxel of an unallocated leaf; a 6-neighbour stencil reads it as
 // copysign(hw, phi(centre)).
 __device__ __forceinline__ float nbv(float v, float centre, float hw) { return (v != v) ? copysignf(hw, centre) : v; }
+
+// p / sqrt(p^2 + 1), the smoothed sign; p^2 + 1 is never subnormal, so the
+// flush-to-zero form of the reciprocal root gives rsqrtf's value without its scaling.
+__device__ __forceinline__ float smooth_sign(float p) {
+    float r;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(p * p + 1.0f));
+    return p * r;
+}
 
 struct Nb6 {
     float xm, xp, ym, yp, zm, zp;
@@ -283,17 +293,57 @@ __device__ __forceinline__ void write_outside(const T* stage, T* __restrict__ ou
     }
 }
 
-// Phase 4 of a leaf, by one warp: its mask words to global memory, the
+// phi1 on box row r = bx * 10 + by, bx, by in [0, 10), into phi2 as f32: what
+// iteration 2 reads of a voxel outside D.  (Ten values by five loads or fewer;
+// choosing per neighbour between phi2 and the stage instead cost six bit tests
+// per voxel and 8% of the kernel.)
+template <typename T>
+__device__ __forceinline__ void copy_box_row(const T* __restrict__ row, float* __restrict__ p2) {
+    // row: the stage at z = -1, one value before a 16-byte boundary
+    float v[kF];
+    v[0] = to_f(row[0]);
+    if constexpr (sizeof(T) == 2) {
+        const uint4 c = *reinterpret_cast<const uint4*>(row + 1);
+        const unsigned w[4] = {c.x, c.y, c.z, c.w};
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&w[i]));
+            v[1 + 2 * i] = f.x;
+            v[2 + 2 * i] = f.y;
+        }
+    } else {
+        const float4 a = *reinterpret_cast<const float4*>(row + 1), c = *reinterpret_cast<const float4*>(row + 5);
+        v[1] = a.x, v[2] = a.y, v[3] = a.z, v[4] = a.w, v[5] = c.x, v[6] = c.y, v[7] = c.z, v[8] = c.w;
+    }
+    v[9] = to_f(row[9]);
+    float2* o = reinterpret_cast<float2*>(p2);
+#pragma unroll
+    for (int i = 0; i < kF / 2; ++i) o[i] = make_float2(v[2 * i], v[2 * i + 1]);
+}
+
+// Bit i of the result: byte i of the 16 activity bytes at a (each 0 or 1),
+// which are cleared for the next leaf.
+__device__ __forceinline__ unsigned take_activity(unsigned char* a) {
+    const uint4 c = *reinterpret_cast<const uint4*>(a);
+    *reinterpret_cast<uint4*>(a) = make_uint4(0u, 0u, 0u, 0u);
+    // bytes 0..3 of a word to bits 28..31: the four products of byte i that land there do not overlap
+    auto nib = [](unsigned w) { return (w * 0x10204080u) >> 28; };
+    return nib(c.x) | (nib(c.y) << 4) | (nib(c.z) << 8) | (nib(c.w) << 12);
+}
+
+// Phase 4 of a leaf, by one warp: its mask to global memory, the
 // spill toward absent neighbours, keep flags and re-tracking proposals.
-// sM: the leaf's 16 mask words in shared memory; nb: the leaf's neighbour
-// slot for the lane's direction (-1 absent).
-__device__ __forceinline__ void spill_and_propose(const unsigned* sM, int slot, int4 o, int nb, int lane,
+// act: the leaf's 512 activity bytes; nb: the leaf's neighbour slot for the
+// lane's direction (-1 absent).
+__device__ __forceinline__ void spill_and_propose(unsigned char* act, int slot, int4 o, int nb, int lane,
                                                   const MLeafArrays& A, const MTopo& topo,
                                                   const MGridParams* __restrict__ params, unsigned* err) {
-    if (lane < 16) reinterpret_cast<unsigned*>(A.mask + (size_t)slot * 8)[lane] = sM[lane];
+    // rows r = x * 8 + y: lane l packs rows 2l and 2l + 1
+    const unsigned two = take_activity(act + 16 * lane);
+    reinterpret_cast<unsigned short*>(A.mask + (size_t)slot * 8)[lane] = (unsigned short)two;
     // spill mask from 64-bit (x*8+y) plane masks of z = 0, z = 7 and any z
-    const unsigned char* B = (const unsigned char*)sM;
-    const unsigned b0 = B[lane], b1 = B[lane + 32];
+    const unsigned pair0 = __shfl_sync(0xffffffffu, two, lane >> 1), pair1 = __shfl_sync(0xffffffffu, two, 16 + (lane >> 1));
+    const unsigned b0 = (pair0 >> (8 * (lane & 1))) & 0xffu, b1 = (pair1 >> (8 * (lane & 1))) & 0xffu;
     const uint64_t z0 = (uint64_t)__ballot_sync(0xffffffffu, b0 & 1u) |
                         ((uint64_t)__ballot_sync(0xffffffffu, b1 & 1u) << 32);
     const uint64_t z7 = (uint64_t)__ballot_sync(0xffffffffu, b0 & 0x80u) |
@@ -377,9 +427,15 @@ __global__ void __launch_bounds__(kNT, 8) k_m_reinit(MLeafArrays A, const T* __r
     __shared__ unsigned short s_list2[kLeafVoxels];
     __shared__ int s_nbr[3][32];   // neighbour rows of the previous, current and next leaf
     __shared__ int s_n1, s_n2;
-    __shared__ unsigned s_bx[32];  // the box voxels of D, one bit per flat index
     __shared__ short s_roff[kF * kF];  // stage offset of box row (bx, by) at bz = 0
-    __shared__ __align__(16) unsigned s_M2[2][16];  // new mask words (this leaf, the previous one)
+    // activity of the new values, a byte per voxel: plain stores, packed once
+    // per leaf and cleared by the warp that packs it (phase 4), in place of an
+    // atomic OR per voxel
+    // (One buffer, not two: in the step's chain of launches the SM keeps the
+    // shared-memory split it has, and at 35.6 KB instead of 35.1 KB per CTA the
+    // f32 kernel with the subcell fix had five CTAs resident, not six, and a
+    // second wave: 28,680-leaf frame 1045 us against 910.)
+    __shared__ __align__(16) unsigned char s_act[kLeafVoxels];
     __shared__ int s_pslot[2];
     __shared__ int4 s_po[2];
 
@@ -391,6 +447,7 @@ __global__ void __launch_bounds__(kNT, 8) k_m_reinit(MLeafArrays A, const T* __r
 
     for (int r = threadIdx.x; r < kF * kF; r += kNT)
         s_roff[r] = (short)(((r / kF - 1 + kH) * kE + (r % kF - 1 + kH)) * RP + Row<T>::Z0 - 1);
+    if (threadIdx.x < kLeafVoxels / 16) reinterpret_cast<uint4*>(s_act)[threadIdx.x] = make_uint4(0u, 0u, 0u, 0u);
     int slot = A.list[li];
     int4 o = A.origin[slot];
     if (warp == 0) s_nbr[0][lane] = (lane < kNbr) ? A.nbr[(size_t)slot * kNbr + lane] : -1;
@@ -437,7 +494,6 @@ __global__ void __launch_bounds__(kNT, 8) k_m_reinit(MLeafArrays A, const T* __r
             // by) * 10 + bz, ascending); without iteration 1 the leaf list
             if (NIT == 2) {
                 unsigned bw = box_word(s_m, lane);
-                s_bx[lane] = bw;
                 const int c = __popc(bw);
                 const int incl = warp_incl_scan(c, lane);
                 int pos = incl - c;
@@ -457,16 +513,17 @@ __global__ void __launch_bounds__(kNT, 8) k_m_reinit(MLeafArrays A, const T* __r
             if (slot_n >= 0)
                 issue_stage<T>(s_nbr[nx], src, A.dmask, stage_of(b ^ 1), masks_of(b ^ 1), t, kNT - 32);
             write_outside<T>(stage, out, hw, t);
-            if (t < 16) s_M2[b][t] = 0u;
+            if (NIT == 2)
+                for (int r = kF * kF - 1 - t; r >= 0; r -= kNT - 32) copy_box_row<T>(stage + s_roff[r], s_p2 + r * kF);
             if (warp == kNW - 1) {
-                // phase 4 of the previous leaf, whose mask words are complete
+                // phase 4 of the previous leaf, whose activity is complete
                 // since barrier A; this warp has the least phase-1 work
                 if (lane == 0) {
                     s_pslot[b] = slot;
                     s_po[b] = o;
                 }
                 if (it > 0)
-                    spill_and_propose(s_M2[b ^ 1], s_pslot[b ^ 1], s_po[b ^ 1], s_nbr[pv][lane], lane, A, topo, params,
+                    spill_and_propose(s_act, s_pslot[b ^ 1], s_po[b ^ 1], s_nbr[pv][lane], lane, A, topo, params,
                                       err);
             }
         }
@@ -483,9 +540,9 @@ __global__ void __launch_bounds__(kNT, 8) k_m_reinit(MLeafArrays A, const T* __r
                     const Nb6 n = load_nb6<T, kE * RP, RP>(c1, p, hw);
                     const float d = cut_distance(p, n);
                     s_dist[t] = d;
-                    s_p2[t] = (d == d) ? cut_relax(p, p, d) : godunov_update(p, n, p * rsqrtf(p * p + 1.0f));
+                    s_p2[t] = (d == d) ? cut_relax(p, p, d) : godunov_update(p, n, smooth_sign(p));
                 } else {
-                    s_p2[t] = godunov_update_raw(p, load_nb6_raw<T, kE * RP, RP>(c1), p * rsqrtf(p * p + 1.0f), hw);
+                    s_p2[t] = godunov_update_raw(p, load_nb6_raw<T, kE * RP, RP>(c1), smooth_sign(p), hw);
                 }
             }
             __syncthreads();  // barrier C: phi2 complete on the box
@@ -505,9 +562,9 @@ __global__ void __launch_bounds__(kNT, 8) k_m_reinit(MLeafArrays A, const T* __r
                     if (FIX) {
                         const Nb6 n = load_nb6<T, kE * RP, RP>(c1, p1, hw);
                         const float d = cut_distance(p1, n);
-                        v = (d == d) ? cut_relax(p1, p1, d) : godunov_update(p1, n, p1 * rsqrtf(p1 * p1 + 1.0f));
+                        v = (d == d) ? cut_relax(p1, p1, d) : godunov_update(p1, n, smooth_sign(p1));
                     } else {
-                        v = godunov_update_raw(p1, load_nb6_raw<T, kE * RP, RP>(c1), p1 * rsqrtf(p1 * p1 + 1.0f), hw);
+                        v = godunov_update_raw(p1, load_nb6_raw<T, kE * RP, RP>(c1), smooth_sign(p1), hw);
                     }
                 } else {
                     const int t10 = ((x + 1) * kF + (y + 1)) * kF + (z + 1);
@@ -517,20 +574,14 @@ __global__ void __launch_bounds__(kNT, 8) k_m_reinit(MLeafArrays A, const T* __r
                         v = cut_relax(p2, p1, d);
                     } else {
                         // a neighbour's phi2 is iteration 1's result on the box voxels
-                        // of D and phi1 (the stage) elsewhere
-                        auto nb = [&](int dt, int ds) {
-                            const int u = t10 + dt;
-                            return ((s_bx[u >> 5] >> (u & 31)) & 1u) ? s_p2[u] : to_f(c1[ds]);
-                        };
-                        const Nb6 n{nb(-kF * kF, -kE * RP), nb(kF * kF, kE * RP), nb(-kF, -RP),
-                                    nb(kF, RP),             nb(-1, -1),           nb(1, 1)};
-                        v = godunov_update_raw(p2, n, p1 * rsqrtf(p1 * p1 + 1.0f), hw);
+                        // of D and phi1 elsewhere (copy_box)
+                        v = godunov_update_raw(p2, load_nb6_raw<float, kF * kF, kF>(s_p2 + t10), smooth_sign(p1), hw);
                     }
                 }
                 const bool on = fabsf(v) < hw;
                 if (!on) v = copysignf(hw, v);
                 out[off] = from_f<T>(v);
-                if (on) atomicOr(&s_M2[b][off >> 5], 1u << (off & 31));
+                if (on) s_act[off] = 1;
             }
         }
         if (slot_n < 0) break;
@@ -542,8 +593,8 @@ __global__ void __launch_bounds__(kNT, 8) k_m_reinit(MLeafArrays A, const T* __r
         slot_nn = slot_nnn;
         nb_next = nb_after;
     }
-    __syncthreads();  // the last leaf's mask words are complete
-    if (warp == kNW - 1) spill_and_propose(s_M2[it & 1u], slot, o, s_nbr[it % 3u][lane], lane, A, topo, params, err);
+    __syncthreads();  // the last leaf's activity is complete
+    if (warp == kNW - 1) spill_and_propose(s_act, slot, o, s_nbr[it % 3u][lane], lane, A, topo, params, err);
 }
 
 #define VLR_REINIT_ARGS(T) MLeafArrays, const T*, T*, const MGridParams*, MTopo, unsigned*
