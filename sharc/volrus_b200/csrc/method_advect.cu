@@ -291,7 +291,6 @@ __global__ void __launch_bounds__(kNT, 8) k_m_advect(MLeafArrays A, const T* __r
                                                      const float2* __restrict__ tab, MStepParams sp, MTopo topo,
                                                      unsigned* __restrict__ err) {
     dep_wait();
-    dep_launch();
     if (step_aborted(err)) return;
     // clear this step's re-tracking state (keep flags, proposal table, leaf hash)
     for (int i = blockIdx.x * kNT + threadIdx.x; i < max(topo.cap, topo.hcap); i += gridDim.x * kNT) {
@@ -327,6 +326,7 @@ __global__ void __launch_bounds__(kNT, 8) k_m_advect(MLeafArrays A, const T* __r
     const int Gs = gridDim.x;
     int li = blockIdx.x;
     if (li >= count) return;
+    if (count <= Gs) dep_launch();  // else when the CTA is done (method.cuh)
     const int step = *A.step;
     const float t1 = sp.t0 + (float)(step + 1) * sp.dt;
     const float dt = sp.dt;
@@ -436,6 +436,7 @@ __global__ void __launch_bounds__(kNT, 8) k_m_advect(MLeafArrays A, const T* __r
         slot_nn = slot_nnn;
         nb_next = nb_after;
     }
+    if (count > Gs) dep_launch();
     if (bad) atomicOr(err, kErrReach);
 }
 

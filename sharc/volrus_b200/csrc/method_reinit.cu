@@ -413,7 +413,6 @@ __global__ void __launch_bounds__(kNT, 8) k_m_reinit(MLeafArrays A, const T* __r
                                                      const MGridParams* __restrict__ params, MTopo topo,
                                                      unsigned* __restrict__ err) {
     dep_wait();
-    dep_launch();
     if (step_aborted(err)) return;
     using Lay = ReinitLayout<T, NIT, FIX>;
     constexpr int RP = Row<T>::RP;
@@ -443,6 +442,7 @@ __global__ void __launch_bounds__(kNT, 8) k_m_reinit(MLeafArrays A, const T* __r
     const int Gs = gridDim.x;
     int li = blockIdx.x;
     if (li >= count) return;
+    if (count <= Gs) dep_launch();  // else when the CTA is done (method.cuh)
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 
     for (int r = threadIdx.x; r < kF * kF; r += kNT)
@@ -594,6 +594,7 @@ __global__ void __launch_bounds__(kNT, 8) k_m_reinit(MLeafArrays A, const T* __r
         nb_next = nb_after;
     }
     __syncthreads();  // the last leaf's activity is complete
+    if (count > Gs) dep_launch();
     if (warp == kNW - 1) spill_and_propose(s_act, slot, o, s_nbr[it % 3u][lane], lane, A, topo, params, err);
 }
 
