@@ -209,45 +209,57 @@ __device__ __forceinline__ void advect_list(const LeafVel& L, const float2 (*s_t
         const int x = off >> 6, y = (off >> 3) & 7, z = off & 7;
         const float3 f = backtrace<VK, OC, SER>(L.V, s_tab, x, y, z, dt, integrator, L.ct1, L.ct2, L.ct3);
         const float px = (float)(x + H) + f.x, py = (float)(y + H) + f.y, pz = (float)(z + H) + f.z;
-        const float bxf = floorf(px), byf = floorf(py), bzf = floorf(pz);
-        float wx = px - bxf, wy = py - byf, wz = pz - bzf;
-        int ii = (int)bxf, jj = (int)byf, kk = (int)bzf;
-        if ((unsigned)ii > (unsigned)(E - 2) || (unsigned)jj > (unsigned)(E - 2) || (unsigned)kk > (unsigned)(E - 2) ||
-            !(px == px) || !(py == py) || !(pz == pz)) {
+        // floor by adding 2^23 rounded down: the low bits of the sum are the
+        // integer part of a position in the tile, and anything outside it
+        // (negative, large, NaN) has them above E - 2
+        constexpr float kBig = 8388608.f;
+        const float tx = __fadd_rd(px, kBig), ty = __fadd_rd(py, kBig), tz = __fadd_rd(pz, kBig);
+        float wx = px - (tx - kBig), wy = py - (ty - kBig), wz = pz - (tz - kBig);
+        unsigned ii = __float_as_uint(tx) - 0x4b000000u, jj = __float_as_uint(ty) - 0x4b000000u,
+                 kk = __float_as_uint(tz) - 0x4b000000u;
+        if (max(max(ii, jj), kk) > (unsigned)(E - 2)) {
             bad = 1u;
-            ii = min(max(ii, 0), E - 2);
-            jj = min(max(jj, 0), E - 2);
-            kk = min(max(kk, 0), E - 2);
-            wx = fminf(fmaxf(wx, 0.f), 1.f);
-            wy = fminf(fmaxf(wy, 0.f), 1.f);
-            wz = fminf(fmaxf(wz, 0.f), 1.f);
+            auto clamped = [](float c, float& w, unsigned& i) {
+                const float f = floorf(c);
+                w = fminf(fmaxf(c - f, 0.f), 1.f);
+                i = (unsigned)min(max((int)f, 0), E - 2);
+            };
+            clamped(px, wx, ii);
+            clamped(py, wy, jj);
+            clamped(pz, wz, kk);
         }
         // tile (ii, jj, kk) = row (ii, jj), element kk - H + Z0
-        const T* q = stage + (ii * E + jj) * RP + (Z0 - H) + kk;
+        const T* q = stage + (int)((ii * E + jj) * RP + kk) + (Z0 - H);
         float c000 = to_f(q[0]), c001 = to_f(q[1]), c010 = to_f(q[RP]), c011 = to_f(q[RP + 1]);
         float c100 = to_f(q[E * RP]), c101 = to_f(q[E * RP + 1]), c110 = to_f(q[E * RP + RP]),
               c111 = to_f(q[E * RP + RP + 1]);
-        const float sum = ((c000 + c001) + (c010 + c011)) + ((c100 + c101) + (c110 + c111));
-        if (sum != sum) {
-            // a corner in an absent leaf (NaN): the missing-leaf rule,
-            // copysign(hw, the leaf's own value at the clamped position)
+        auto sample = [&]() {
+            const float c00 = c000 * (1.f - wx) + c100 * wx, c01 = c001 * (1.f - wx) + c101 * wx;
+            const float c10 = c010 * (1.f - wx) + c110 * wx, c11 = c011 * (1.f - wx) + c111 * wx;
+            const float c0 = c00 * (1.f - wy) + c10 * wy, c1 = c01 * (1.f - wy) + c11 * wy;
+            return c0 * (1.f - wz) + c1 * wz;
+        };
+        float v = sample();
+        if (v != v) {
+            // a corner in an absent leaf (NaN, which every weight lets through):
+            // the missing-leaf rule, copysign(hw, the leaf's own value at the
+            // clamped position)
             auto own = [&](int ti, int tj, int tk) {
                 const int cx = min(max(ti - H, 0), 7), cy = min(max(tj - H, 0), 7), cz = min(max(tk - H, 0), 7);
                 return copysignf(hwT, to_f(stage[((cx + H) * E + (cy + H)) * RP + Z0 + cz]));
             };
-            if (c000 != c000) c000 = own(ii, jj, kk);
-            if (c001 != c001) c001 = own(ii, jj, kk + 1);
-            if (c010 != c010) c010 = own(ii, jj + 1, kk);
-            if (c011 != c011) c011 = own(ii, jj + 1, kk + 1);
-            if (c100 != c100) c100 = own(ii + 1, jj, kk);
-            if (c101 != c101) c101 = own(ii + 1, jj, kk + 1);
-            if (c110 != c110) c110 = own(ii + 1, jj + 1, kk);
-            if (c111 != c111) c111 = own(ii + 1, jj + 1, kk + 1);
+            const int i0 = (int)ii, j0 = (int)jj, k0 = (int)kk;
+            if (c000 != c000) c000 = own(i0, j0, k0);
+            if (c001 != c001) c001 = own(i0, j0, k0 + 1);
+            if (c010 != c010) c010 = own(i0, j0 + 1, k0);
+            if (c011 != c011) c011 = own(i0, j0 + 1, k0 + 1);
+            if (c100 != c100) c100 = own(i0 + 1, j0, k0);
+            if (c101 != c101) c101 = own(i0 + 1, j0, k0 + 1);
+            if (c110 != c110) c110 = own(i0 + 1, j0 + 1, k0);
+            if (c111 != c111) c111 = own(i0 + 1, j0 + 1, k0 + 1);
+            v = sample();
         }
-        const float c00 = c000 * (1.f - wx) + c100 * wx, c01 = c001 * (1.f - wx) + c101 * wx;
-        const float c10 = c010 * (1.f - wx) + c110 * wx, c11 = c011 * (1.f - wx) + c111 * wx;
-        const float c0 = c00 * (1.f - wy) + c10 * wy, c1 = c01 * (1.f - wy) + c11 * wy;
-        out[off] = from_f<T>(c0 * (1.f - wz) + c1 * wz);
+        out[off] = from_f<T>(v);
     }
 }
 
