@@ -136,20 +136,25 @@ __device__ __forceinline__ const T* at(const T* stage, int x, int y, int z) {
 
 // Godunov upwind |grad phi| for the sign of s.  Per axis the upwind one-sided
 // differences are u = max(sg (p - phi_-), 0) and w = max(sg (p - phi_+), 0),
-// sg = +-1 the sign of s, and the axis term is max(u, w)^2, the same value as
-// the sign-split form max(max(a-, 0)^2, min(a+, 0)^2) for s >= 0 and its
-// mirror for s < 0, without the sign branch.  With q = sg p the differences are
-// q - sg phi: the product is exact, so one FMA rounds each as the subtraction
-// would, and one three-input max joins them (fmaxf drops a NaN neighbour's
-// difference).  Min and max run at half the FMA rate and this kernel is bound
-// by instructions: two FMAs and one max per axis for two products, a min, a
-// subtraction and a max.  The correctly rounded sqrtf keeps a
-// full deformation period's FP32 topology equal to the FP64 run's (an
-// rsqrtf-based magnitude measured two voxels flipping at the band's edge).
+// sg = +-1 the sign bit of s (for s = 0 the update is zero whatever G is), and
+// the axis term is max(u, w)^2, the same value as the sign-split form
+// max(max(a-, 0)^2, min(a+, 0)^2) for s >= 0 and its mirror for s < 0, without
+// the sign branch.  With q = sg p the differences are q - sg phi: the product
+// is exact, so one FMA rounds each as the subtraction would, and one
+// three-input max joins them (fmaxf drops a NaN neighbour's difference).  Min
+// and max run at half the FMA rate and this kernel is bound by instructions:
+// two FMAs and one max per axis for two products, a min, a subtraction and a
+// max.  The correctly rounded sqrtf keeps a full deformation period's FP32
+// topology equal to the FP64 run's (an rsqrtf-based magnitude measured two
+// voxels flipping at the band's edge).
+// Only G - 1 is used, which is -1 for every G below 2^-25: kFlat for 0 in one
+// axis changes G below 1e-11 alone and keeps sqrtf off its path for a zero or
+// subnormal argument, which flat stretches of the field would take.
+constexpr float kFlat = 1e-15f;
 __device__ __forceinline__ float godunov_g(float p, float xm, float xp, float ym, float yp, float zm, float zp, float s) {
-    const float sg = (s >= 0.f) ? 1.f : -1.f;
+    const float sg = copysignf(1.f, s);
     const float q = sg * p;
-    const float mx = fmaxf(fmaxf(__fmaf_rn(-sg, xm, q), __fmaf_rn(-sg, xp, q)), 0.f);
+    const float mx = fmaxf(fmaxf(__fmaf_rn(-sg, xm, q), __fmaf_rn(-sg, xp, q)), kFlat);
     const float my = fmaxf(fmaxf(__fmaf_rn(-sg, ym, q), __fmaf_rn(-sg, yp, q)), 0.f);
     const float mz = fmaxf(fmaxf(__fmaf_rn(-sg, zm, q), __fmaf_rn(-sg, zp, q)), 0.f);
     // squares rounded before the sums (no contraction)
@@ -195,11 +200,13 @@ __device__ __forceinline__ float godunov_update(float p, const Nb6& n, float s) 
 
 // godunov_update with raw neighbours, NaN marking an unallocated leaf.  The
 // missing-leaf value copysign(hw, p) gives an upwind term max(<= 0, 0) = 0
-// whenever |p| <= hw and p's sign bit matches the upwind sign of s, and
-// fmaxf gives the same 0 for the NaN itself, so the NaNs are resolved only
-// outside that case: bit for bit the update of the resolved neighbours.
+// whenever |p| <= hw and p's sign bit is that of s, and fmaxf gives the same 0
+// for the NaN itself, so the NaNs are resolved only outside that case: bit for
+// bit the update of the resolved neighbours.  OWN: s is p's own smoothed sign,
+// which has its sign bit.
+template <bool OWN>
 __device__ __forceinline__ float godunov_update_raw(float p, Nb6 n, float s, float hw) {
-    if (!(fabsf(p) <= hw && (signbit(p) != 0) == (s < 0.f)))
+    if (!(fabsf(p) <= hw && (OWN || (__float_as_int(p) ^ __float_as_int(s)) >= 0)))
         n = Nb6{nbv(n.xm, p, hw), nbv(n.xp, p, hw), nbv(n.ym, p, hw),
                 nbv(n.yp, p, hw), nbv(n.zm, p, hw), nbv(n.zp, p, hw)};
     return godunov_update(p, n, s);
@@ -426,7 +433,7 @@ __global__ void __launch_bounds__(kNT, 8) k_m_reinit(MLeafArrays A, const T* __r
     __shared__ unsigned short s_list2[kLeafVoxels];
     __shared__ int s_nbr[3][32];   // neighbour rows of the previous, current and next leaf
     __shared__ int s_n1, s_n2;
-    __shared__ short s_roff[kF * kF];  // stage offset of box row (bx, by) at bz = 0
+    __shared__ short s_roff[kF * kF];  // stage offset of box row r = bx * 10 + by at bz = 0, less 10 r
     // activity of the new values, a byte per voxel: plain stores, packed once
     // per leaf and cleared by the warp that packs it (phase 4), in place of an
     // atomic OR per voxel
@@ -446,7 +453,7 @@ __global__ void __launch_bounds__(kNT, 8) k_m_reinit(MLeafArrays A, const T* __r
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 
     for (int r = threadIdx.x; r < kF * kF; r += kNT)
-        s_roff[r] = (short)(((r / kF - 1 + kH) * kE + (r % kF - 1 + kH)) * RP + Row<T>::Z0 - 1);
+        s_roff[r] = (short)(((r / kF - 1 + kH) * kE + (r % kF - 1 + kH)) * RP + Row<T>::Z0 - 1 - kF * r);
     if (threadIdx.x < kLeafVoxels / 16) reinterpret_cast<uint4*>(s_act)[threadIdx.x] = make_uint4(0u, 0u, 0u, 0u);
     int slot = A.list[li];
     int4 o = A.origin[slot];
@@ -514,7 +521,7 @@ __global__ void __launch_bounds__(kNT, 8) k_m_reinit(MLeafArrays A, const T* __r
                 issue_stage<T>(s_nbr[nx], src, A.dmask, stage_of(b ^ 1), masks_of(b ^ 1), t, kNT - 32);
             write_outside<T>(stage, out, hw, t);
             if (NIT == 2)
-                for (int r = kF * kF - 1 - t; r >= 0; r -= kNT - 32) copy_box_row<T>(stage + s_roff[r], s_p2 + r * kF);
+                for (int r = kF * kF - 1 - t; r >= 0; r -= kNT - 32) copy_box_row<T>(stage + s_roff[r] + r * kF, s_p2 + r * kF);
             if (warp == kNW - 1) {
                 // phase 4 of the previous leaf, whose activity is complete
                 // since barrier A; this warp has the least phase-1 work
@@ -533,8 +540,7 @@ __global__ void __launch_bounds__(kNT, 8) k_m_reinit(MLeafArrays A, const T* __r
             const int n1 = s_n1;
             for (int i = threadIdx.x; i < n1; i += kNT) {
                 const int t = s_list1[i];
-                const int r = t / kF;
-                const T* c1 = stage + s_roff[r] + (t - r * kF);
+                const T* c1 = stage + s_roff[t / kF] + t;
                 const float p = to_f(c1[0]);
                 if (FIX) {
                     const Nb6 n = load_nb6<T, kE * RP, RP>(c1, p, hw);
@@ -542,7 +548,7 @@ __global__ void __launch_bounds__(kNT, 8) k_m_reinit(MLeafArrays A, const T* __r
                     s_dist[t] = d;
                     s_p2[t] = (d == d) ? cut_relax(p, p, d) : godunov_update(p, n, smooth_sign(p));
                 } else {
-                    s_p2[t] = godunov_update_raw(p, load_nb6_raw<T, kE * RP, RP>(c1), smooth_sign(p), hw);
+                    s_p2[t] = godunov_update_raw<true>(p, load_nb6_raw<T, kE * RP, RP>(c1), smooth_sign(p), hw);
                 }
             }
             __syncthreads();  // barrier C: phi2 complete on the box
@@ -564,7 +570,7 @@ __global__ void __launch_bounds__(kNT, 8) k_m_reinit(MLeafArrays A, const T* __r
                         const float d = cut_distance(p1, n);
                         v = (d == d) ? cut_relax(p1, p1, d) : godunov_update(p1, n, smooth_sign(p1));
                     } else {
-                        v = godunov_update_raw(p1, load_nb6_raw<T, kE * RP, RP>(c1), smooth_sign(p1), hw);
+                        v = godunov_update_raw<true>(p1, load_nb6_raw<T, kE * RP, RP>(c1), smooth_sign(p1), hw);
                     }
                 } else {
                     const int t10 = ((x + 1) * kF + (y + 1)) * kF + (z + 1);
@@ -575,7 +581,7 @@ __global__ void __launch_bounds__(kNT, 8) k_m_reinit(MLeafArrays A, const T* __r
                     } else {
                         // a neighbour's phi2 is iteration 1's result on the box voxels
                         // of D and phi1 elsewhere (copy_box)
-                        v = godunov_update_raw(p2, load_nb6_raw<float, kF * kF, kF>(s_p2 + t10), smooth_sign(p1), hw);
+                        v = godunov_update_raw<false>(p2, load_nb6_raw<float, kF * kF, kF>(s_p2 + t10), smooth_sign(p1), hw);
                     }
                 }
                 const bool on = fabsf(v) < hw;
