@@ -101,6 +101,24 @@ struct vlr_level_set {
 
 namespace vlr {
 
+// Launch one kernel of a chain with programmatic stream serialization (its
+// CTAs may be scheduled while the previous kernel drains; the kernel itself
+// waits for that kernel's results with dep_wait()).
+template <typename... KArgs, typename... Args>
+cudaError_t pdl_launch(void (*kernel)(KArgs...), int grid, int block, size_t smem, cudaStream_t st, Args... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)grid);
+    cfg.blockDim = dim3((unsigned)block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
 int ls_alloc(vlr_ctx* ctx, vlr_level_set* ls, int cap);
 void ls_free(vlr_level_set* ls);
 // Enqueue one step (no host synchronisation; capturable).

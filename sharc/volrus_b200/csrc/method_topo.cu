@@ -388,25 +388,6 @@ size_t scan_scratch_ints(int n) { return (size_t)((n + kChunk - 1) / kChunk) * 2
 
 // ----------------------------------------------------------- orchestration
 
-// Launch one kernel of the step with programmatic stream serialization (its
-// CTAs may be scheduled while the previous kernel drains; the kernel itself
-// waits for that kernel's results with dep_wait()).
-template <typename... KArgs, typename... Args>
-static cudaError_t pdl_launch(void (*kernel)(KArgs...), int grid, int block, size_t smem, cudaStream_t st,
-                              Args... args) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)grid);
-    cfg.blockDim = dim3((unsigned)block);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kernel, args...);
-}
-
 MTopo topo_of(vlr_level_set* ls) {
     MTopo t;
     t.keep = ls->keep;
