@@ -200,6 +200,7 @@ __device__ __forceinline__ void chain_wait() {
 
 // Resident CTAs of 256 threads per SM of the chunk kernels.
 constexpr int kChunkCtas = 6;
+constexpr int kWideCtas = 4;  // k_adj_lambda with three candidate rows in flight
 
 // The chain header -> voxel, foot, neighbour slots -> corners is three trips
 // to memory per chunk, and a band beyond L2 pays DRAM latency for each.  So
@@ -479,7 +480,7 @@ __device__ __forceinline__ void add_corner(float& acc, unsigned t, const float4&
 //
 // One warp per chunk of a leaf's band voxels: the window is uniform, a
 // neighbour slot costs a shuffle, and the words of up to three candidates
-// along z are loaded before the first is tested.  Where the neighbourhood has
+// along z, on ROWS rows, are loaded before the first is tested.  Where the neighbourhood has
 // one foot offset (floor(s u) equal at both ends of its range on every axis,
 // the common case of a smooth field), candidate and corner correspond one to
 // one, so no candidate word is read or tested; voxels off the band hold
@@ -491,8 +492,8 @@ __device__ __forceinline__ void add_corner(float& acc, unsigned t, const float4&
 // set: 373 us one thread per voxel with its own gradient term, 313 us in
 // chunks without it (770 instructions a chunk), 197 us with the untested
 // path, 166 us with the prefetch.
-template <bool LAM>
-__global__ void __launch_bounds__(256, kChunkCtas)
+template <bool LAM, int ROWS>
+__global__ void __launch_bounds__(256, ROWS == 1 ? kChunkCtas : kWideCtas)
     k_adj_lambda(const int2* __restrict__ chunks, int n_chunks, int ahead, const int* __restrict__ bvox,
                  const int* __restrict__ nbr, const float* __restrict__ nrange, const unsigned* foot_pk,
                  const float4* foot_w, const float* lam_in, int R, BackOut o) {
@@ -551,23 +552,22 @@ __global__ void __launch_bounds__(256, kChunkCtas)
     for (int dx = x0; dx <= x1; ++dx) {
         const int x = cx + dx;
         float plane = 0.f;
-        for (int dy = y0; dy <= y1; ++dy) {
-            const int y = cy + dy;
-            const int nb2 = leaf_of(x) * 9 + leaf_of(y) * 3;
-            const int o2 = ((x & 7) << 6) | ((y & 7) << 3);
+        for (int dy = y0; dy <= y1; dy += ROWS) {
             for (int dz = z0; dz <= z1; dz += 3) {
-                unsigned t[3], e[3];
+                unsigned t[3 * ROWS], e[3 * ROWS];
 #pragma unroll
-                for (int q = 0; q < 3; ++q) {
-                    const int z = cz + dz + q;
-                    // offsets past the window (up to z1 + 2 <= R + 2 < 9 from the voxel) test nothing
-                    const int ns = __shfl_sync(0xffffffffu, k.row, nb2 + min(leaf_of(z), 2));
-                    e[q] = (unsigned)ns * kLeafVoxels + (unsigned)(o2 | (z & 7));
+                for (int q = 0; q < 3 * ROWS; ++q) {
+                    const int ry = q / 3, rz = q % 3, y = cy + dy + ry, z = cz + dz + rz;
+                    // offsets past the window (up to y1 + 2, z1 + 2 <= R + 2 < 9 from the voxel) test nothing
+                    const int ns = __shfl_sync(0xffffffffu, k.row,
+                                               leaf_of(x) * 9 + min(leaf_of(y), 2) * 3 + min(leaf_of(z), 2));
+                    e[q] = (unsigned)ns * kLeafVoxels + (unsigned)voxel_off(x, y, z);
                     t[q] = ~0u;
-                    if (ns >= 0 && dz + q <= z1) t[q] = cell_key(dx, dy, dz + q) - foot_pk[e[q]];
+                    if (ns >= 0 && dy + ry <= y1 && dz + rz <= z1)
+                        t[q] = cell_key(dx, dy + ry, dz + rz) - foot_pk[e[q]];
                 }
 #pragma unroll
-                for (int q = 0; q < 3; ++q)
+                for (int q = 0; q < 3 * ROWS; ++q)
                     if (!(t[q] & ~kCorner)) {
                         const float4 w = foot_w[e[q]];
                         add_corner(plane, t[q], w, LAM ? lam_in[e[q]] : w.w);
@@ -852,11 +852,11 @@ int enqueue_lambda_step(vlr_ctx* ctx, vlr_adjoint* a, int cur, const BackOut& o)
     const int nb = a->n_band;
     const unsigned* pk = a->foot_pk[a->disp ? 0 : cur];
     const float4* w = a->foot_w[a->disp ? 0 : cur];
-    // The quad wins while its voxels fit one wave (4 CTAs of 64 voxels per SM,
-    // 37,888 here): 10.7 against 14.7 us a launch at 30,368 band voxels, even
-    // at 47,354 (14.5, 14.7), behind from there (16.8, 14.7 at 77,406; 65, 31
-    // at 644,824).  It covers a reach of one voxel only.
-    if (a->gather == 2 || (a->gather == 0 && a->reach == 1 && nb <= ctx->sm_count * 4 * 64)) {
+    // The quad wins while its voxels fit one wave (3 CTAs of 64 voxels per SM,
+    // 28,416 here).  A pass of 64 steps, quad and windowed: 12,971 band voxels
+    // 514 and 619 us, 19,525 542 and 639, 30,368 710 and 641, 51,229 813 and
+    // 675.  It covers a reach of one voxel only.
+    if (a->gather == 2 || (a->gather == 0 && a->reach == 1 && nb <= ctx->sm_count * 3 * 64)) {
         const int B = blocks_for(ctx, 4ll * nb);
         if (a->disp)
             VLR_TIMED(ctx, "k_adj_lambda",
@@ -868,16 +868,22 @@ int enqueue_lambda_step(vlr_ctx* ctx, vlr_adjoint* a, int cur, const BackOut& o)
                                                (const float*)nullptr, o)));
     } else {
         const int B = chunk_blocks(a);
+        // Three candidate rows in flight shorten the chain of trips while the
+        // warps fit two waves (4 CTAs of 8 per SM); past that the one-row
+        // kernel's six CTAs cover it.  A pass of 64 steps, one row -> three:
+        // 51,229 band voxels 839 -> 675 us, 77,406 886 -> 813, 152,937 1188 ->
+        // 1054, 309,106 1818 -> 1802, 610,952 3052 -> 3180.
+        const bool wide = a->n_chunks <= 2 * ctx->sm_count * kWideCtas * 8;
+        auto launch = [&](auto* kernel, const float* lam) {
+            return pdl_launch(kernel, B, 256, 0, st, a->chunks, a->n_chunks, chunk_wave(ctx), a->bvox, a->nbr, a->nrange,
+                              pk, w, lam, a->reach, o);
+        };
         if (a->disp)
-            VLR_TIMED(ctx, "k_adj_lambda",
-                      VLR_CUDA(ctx, pdl_launch(k_adj_lambda<true>, B, 256, 0, st, a->chunks, a->n_chunks,
-                                               chunk_wave(ctx), a->bvox, a->nbr, a->nrange, pk, w, a->lam_pool[cur],
-                                               a->reach, o)));
+            VLR_TIMED(ctx, "k_adj_lambda", VLR_CUDA(ctx, launch(wide ? k_adj_lambda<true, 3> : k_adj_lambda<true, 1>,
+                                                                (const float*)a->lam_pool[cur])));
         else
-            VLR_TIMED(ctx, "k_adj_lambda",
-                      VLR_CUDA(ctx, pdl_launch(k_adj_lambda<false>, B, 256, 0, st, a->chunks, a->n_chunks,
-                                               chunk_wave(ctx), a->bvox, a->nbr, a->nrange, pk, w,
-                                               (const float*)nullptr, a->reach, o)));
+            VLR_TIMED(ctx, "k_adj_lambda", VLR_CUDA(ctx, launch(wide ? k_adj_lambda<false, 3> : k_adj_lambda<false, 1>,
+                                                                (const float*)nullptr)));
     }
     return VLR_OK;
 }
@@ -1402,8 +1408,7 @@ int vlr_adj_forward(vlr_ctx* ctx, vlr_adjoint* a, float* phi_k_band) {
     if (phi_k_band)
         VLR_CUDA(ctx, cudaMemcpyAsync(phi_k_band, a->lam[1], sizeof(float) * a->n_band, cudaMemcpyDeviceToHost,
                                       ctx->stream));
-    VLR_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-    return consume_device_errors(ctx, "vlr_adj_forward");
+    return consume_device_errors(ctx, "vlr_adj_forward");  // waits for the stream
 }
 
 // Backward pass (vlr_adj_forward must have run): grad_phik_band = dL/dphi_K
@@ -1448,8 +1453,7 @@ int vlr_adj_backward(vlr_ctx* ctx, vlr_adjoint* a, const float* grad_phik_band, 
     if (grad_vel)
         VLR_CUDA(ctx, cudaMemcpyAsync(grad_vel, a->gvel, sizeof(float) * 3ull * a->n_stag * a->n_stag * a->n_stag,
                                       cudaMemcpyDeviceToHost, st));
-    VLR_CUDA(ctx, cudaStreamSynchronize(st));
-    return consume_device_errors(ctx, "vlr_adj_backward");
+    return consume_device_errors(ctx, "vlr_adj_backward");  // waits for the stream
 }
 
 void vlr_adj_destroy(vlr_adjoint* a) {
