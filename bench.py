@@ -322,26 +322,26 @@ STEP_KERNELS = ("k_m_advect", "k_m_reinit", "k_t_scanalloc", "k_t_nbr")
 #   deformation512: `bench.py --workload deformation512 --steps 1 --warmup 3`,
 #     -s 6 (2,858 leaves, L2-resident).
 TRAFFIC_PER_LEAF: dict = {
-    ("large8192", "k_m_advect", 2): 2548.8,
-    ("large8192", "k_m_reinit", 2): 2342.5,
-    ("large8192", "k_m_advect", 4): 4864.1,
-    ("large8192", "k_m_reinit", 4): 4509.9,
-    ("batched256", "k_m_advect", 2): 2327.1,
-    ("batched256", "k_m_reinit", 2): 2081.1,
-    ("deformation512", "k_m_advect", 2): 1238.0,
-    ("deformation512", "k_m_reinit", 2): 1224.9,
+    ("large8192", "k_m_advect", 2): 2564.5,
+    ("large8192", "k_m_reinit", 2): 2296.8,
+    ("large8192", "k_m_advect", 4): 4877.3,
+    ("large8192", "k_m_reinit", 4): 4458.7,
+    ("batched256", "k_m_advect", 2): 2321.6,
+    ("batched256", "k_m_reinit", 2): 2075.1,
+    ("deformation512", "k_m_advect", 2): 1238.5,
+    ("deformation512", "k_m_reinit", 2): 1224.7,
 }
 
 
 # Warp instructions per leaf of one launch (smsp__inst_executed.sum over the
 # launch's leaves) from the same captures, FP16, 128-thread CTAs.
 INST_PER_LEAF: dict = {
-    ("large8192", "k_m_advect"): 4452.5,
-    ("large8192", "k_m_reinit"): 4198.8,
-    ("batched256", "k_m_advect"): 4768.3,
-    ("batched256", "k_m_reinit"): 4194.8,
-    ("deformation512", "k_m_advect"): 3003.1,
-    ("deformation512", "k_m_reinit"): 4440.2,
+    ("large8192", "k_m_advect"): 4403.3,
+    ("large8192", "k_m_reinit"): 3616.9,
+    ("batched256", "k_m_advect"): 4719.3,
+    ("batched256", "k_m_reinit"): 3616.9,
+    ("deformation512", "k_m_advect"): 2955.7,
+    ("deformation512", "k_m_reinit"): 3882.0,
 }
 SM_COUNT = 148
 ISSUE_PER_SM_PER_CYCLE = 4  # one warp instruction per scheduler per cycle

@@ -474,8 +474,7 @@ void vlr_ls_destroy(vlr_level_set* ls);
  * forward/backward follow the autograd-Function contract: forward(phi_0, V)
  * -> phi_K, backward(dL/dphi_K) -> (dL/dphi_0, dL/dV).  The backward pass
  * recomputes states from checkpoints taken every `checkpoint_every` steps and
- * scatters trilinear weights by stable radix sort + segmented sum (no float
- * atomics; deterministic).  Band arrays follow vlr_adj_band's order. */
+ * sums trilinear weights in a fixed order (no float atomics; deterministic).  Band arrays follow vlr_adj_band's order. */
 typedef struct vlr_adjoint vlr_adjoint;
 
 int vlr_adj_create(vlr_ctx* ctx, const int32_t* origins, const uint64_t* masks, const float* phi, size_t n_leaves,
