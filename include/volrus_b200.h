@@ -437,7 +437,8 @@ int vlr_ls_edit_device(vlr_ctx* ctx, vlr_level_set* ls, const uint8_t* d_drop, s
  * may be overwritten; the call then waits once for the count, the device
  * errors and those copies, and copies any records beyond them.
  * One step of a large single-grid state (at least 2^14 leaves by default)
- * whose host leaves are sorted by x and whose six host buffers are pinned
+ * whose host leaves are sorted by x and whose six host buffers are pinned and
+ * apart (a step in place takes the one pass)
  * runs as a pipeline over slabs of consecutive x instead: each slab steps its
  * leaves with the input leaves within 16 voxels beside it and keeps the
  * outputs in its own x range, which are bit for bit the one-pass step's; its

@@ -952,6 +952,25 @@ bool host_pinned(const void* p) {
     return ok;
 }
 
+// Whether n input records (origins, masks, values) and cap output records share
+// no byte.  The one pass has read its input before it writes; a pipeline's
+// first outputs come down while its last inputs are still on their way up, so
+// a step in place takes the one pass.
+struct HostRecords {
+    const void *o, *m, *v;
+};
+bool apart(const HostRecords& in, const HostRecords& out, size_t n, size_t cap) {
+    const size_t size[3] = {12, 64, sizeof(float) * kLeafVoxels};
+    const void* const a[3] = {in.o, in.m, in.v};
+    const void* const b[3] = {out.o, out.m, out.v};
+    for (int i = 0; i < 3; ++i)
+        for (int j = 0; j < 3; ++j) {
+            const uintptr_t x = (uintptr_t)a[i], y = (uintptr_t)b[j];
+            if (x < y + size[j] * cap && y < x + size[i] * n) return false;
+        }
+    return true;
+}
+
 // Leaves [n_first, n_first + n) of a device copy of host records (o3, masks,
 // f32 values) as the pool's state, index enqueued; no wait.
 int load_pool(vlr_ctx* ctx, vlr_level_set* ls, const int32_t* o3, const uint64_t* masks, const float* phi, size_t n) {
@@ -1391,7 +1410,9 @@ int vlr_ls_step_host(vlr_ctx* ctx, vlr_level_set* ls, const int32_t* origins, co
     SlabPlan plan;
     if (n_steps == 1 && 3 * ls->key_bits <= 63 && out_origins && out_masks && out_phi && host_pinned(origins) &&
         host_pinned(masks) && host_pinned(phi) && host_pinned(out_origins) && host_pinned(out_masks) &&
-        host_pinned(out_phi) && plan_slabs(ls, origins, n_leaves, &plan)) {
+        host_pinned(out_phi) &&
+        apart({origins, masks, phi}, {out_origins, out_masks, out_phi}, n_leaves, cap_leaves) &&
+        plan_slabs(ls, origins, n_leaves, &plan)) {
         const bool like_one_pass = ls->host_slabs == 0 && n_leaves < kSlabLeavesSorted;
         int entry_step = -1;  // set once the pipeline may have changed the counter
         int rc = step_host_slabs(ctx, ls, plan, origins, masks, phi, n_leaves, out_origins, out_masks, out_phi,

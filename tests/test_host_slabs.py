@@ -166,3 +166,22 @@ def test_middling_states_leave_what_one_pass_leaves(precision, spheres):
             assert torch.equal(a, b)
     finally:
         ls.close()
+
+
+@pytest.mark.parametrize("spheres", [75, 1100])
+def test_step_in_place(spheres):
+    """The input buffers as the output buffers: the one pass's result, at states that pipeline when the buffers are apart."""
+    from sharc.volrus_b200.method import LevelSet, large_sphere_grid
+    sph, vel = large_sphere_grid(spheres, seed=3, extent=1600.0 if spheres < 1000 else 4096.0)
+    ls = LevelSet.spheres([(sph, vel)], 1.0, half_width=3.0, precision=1, integrator=3, reinit_iters=2)
+    try:
+        o, m, v = ls.arrays()
+        n, cap = len(o), 2 * len(o)
+        assert n >= 1 << 14
+        want = _host_step(ls, tuple(_pinned(a) for a in (o, m, v)), 1)
+        buf = _out(cap)
+        for b, a in zip(buf, (o, m, v)):
+            b[:n] = a
+        assert _same(_host_step(ls, tuple(b[:n] for b in buf), 0, out=buf), want)
+    finally:
+        ls.close()
