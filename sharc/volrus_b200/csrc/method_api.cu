@@ -1114,6 +1114,7 @@ int step_host_slabs(vlr_ctx* ctx, vlr_level_set* ls, const SlabPlan& P, const in
     int* h_count = static_cast<int*>(ctx->pinned) + 64;                  // pool count after slab s's step
     int* h_kept = static_cast<int*>(ctx->pinned) + 64 + kHostSlabsMax;   // outputs slab s keeps
     unsigned* h_err = static_cast<unsigned*>(ctx->pinned) + 64 + 2 * kHostSlabsMax;
+    unsigned* h_entry_err = static_cast<unsigned*>(ctx->pinned) + 65 + 2 * kHostSlabsMax;  // error word at entry
     int* h_step = static_cast<int*>(ctx->pinned) + 66 + 2 * kHostSlabsMax;
     *h_step = -1;
 
@@ -1137,6 +1138,8 @@ int step_host_slabs(vlr_ctx* ctx, vlr_level_set* ls, const SlabPlan& P, const in
                                            cudaMemcpyDeviceToDevice, st), "cudaMemcpyAsync")) ||
         (rc = cuda_rc(ctx, cudaMemcpyAsync(h_step, ls->scalars + 1, sizeof(int), cudaMemcpyDeviceToHost, st),
                       "step read-back")) ||
+        (rc = cuda_rc(ctx, cudaMemcpyAsync(h_entry_err, ctx->d_errword, sizeof(unsigned), cudaMemcpyDeviceToHost, st),
+                      "error read-back")) ||
         (rc = cuda_rc(ctx, cudaEventRecord(ev_ready, st), "cudaEventRecord")) ||
         (rc = cuda_rc(ctx, cudaStreamWaitEvent(up, ev_ready, 0), "cudaStreamWaitEvent")) ||
         (rc = cuda_rc(ctx, cudaStreamWaitEvent(down, ev_ready, 0), "cudaStreamWaitEvent")))
@@ -1198,6 +1201,9 @@ int step_host_slabs(vlr_ctx* ctx, vlr_level_set* ls, const SlabPlan& P, const in
         if ((rc = cuda_rc(ctx, cudaStreamSynchronize(st), "cudaStreamSynchronize"))) return finish(rc);
         const int c = h_count[s];
         if (*h_err || c < 0 || c > ls->cap) {
+            // an error of an earlier call, or a wait that ran out: the word stays for the one pass to report
+            if (keep_order && (*h_entry_err || (*h_err & kErrTimeout)))
+                return finish(set_error(ctx, VLR_ERR_CUDA, "vlr_ls_step_host: device error"));
             rc = consume_device_errors(ctx, "vlr_ls_step_host");
             return finish(rc ? rc : set_error(ctx, VLR_ERR_CUDA, "slab step left an inconsistent leaf count"));
         }

@@ -1,0 +1,67 @@
+"""What vlr_ls_step_host reports where the automatic slab count pipelines (2^14
+leaves and more) is what the one pass reports, and so is the state it leaves."""
+import numpy as np
+import pytest
+
+from tests.test_errors import _codes, _sphere
+from tests.test_host_slabs import _host_step, _pinned, _same
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def state():
+    """About 20,000 leaves in pinned buffers."""
+    from sharc.volrus_b200.method import LevelSet, large_sphere_grid
+    sph, vel = large_sphere_grid(75, seed=3, extent=1600.0)
+    ls = LevelSet.spheres([(sph, vel)], 1.0, half_width=3.0, precision=1, integrator=3, reinit_iters=2)
+    inp = tuple(_pinned(a) for a in ls.arrays())
+    assert 1 << 14 <= len(inp[0]) < 1 << 18
+    yield ls, inp
+    ls.close()
+
+
+def _leave_reach_error(ctx):
+    from sharc.volrus_b200.method import curl_noise
+    vel = curl_noise(5, 256.0, 0.8, 3)
+    vel["domain"] = ((0, 0, 0), (256, 256, 256))  # the sphere reaches negative coordinates
+    other = _sphere(ctx, 1, vel=vel, radius=20.0)
+    other.enqueue(1)
+    return other
+
+
+def _leave_timeout(ctx):
+    other = _sphere(ctx, 1, radius=60.0)  # several chunks in the look-back scan
+    ctx.check(ctx.lib.vlr_ctx_set_wait_limit(ctx.handle, 2000), "vlr_ctx_set_wait_limit")
+    ctx.check(ctx.lib.vlr_ctx_test_stall(ctx.handle, 1), "vlr_ctx_test_stall")
+    try:
+        other.enqueue(1)
+    finally:
+        ctx.check(ctx.lib.vlr_ctx_test_stall(ctx.handle, 0), "vlr_ctx_test_stall")
+        ctx.check(ctx.lib.vlr_ctx_set_wait_limit(ctx.handle, 0), "vlr_ctx_set_wait_limit")
+    return other
+
+
+@pytest.mark.parametrize("leave,name", [(_leave_reach_error, "VLR_ERR_REACH"), (_leave_timeout, "VLR_ERR_TIMEOUT")])
+def test_error_of_an_earlier_call_is_reported(ctx, state, leave, name):
+    """An error that another level set's enqueued step left on the context."""
+    from sharc.volrus_b200 import VolrusError
+    ls, inp = state
+    after = []
+    for slabs in (1, 0):
+        _host_step(ls, inp, slabs)
+        other = leave(ctx)
+        with pytest.raises(VolrusError) as e:
+            _host_step(ls, inp, slabs)
+        assert e.value.code == _codes()[name], slabs
+        ctx.check_device()  # reported once
+        if name == "VLR_ERR_TIMEOUT":  # the step was abandoned: the state waits for an upload
+            with pytest.raises(VolrusError) as e:
+                ls.step(1)
+            assert e.value.code == _codes()["VLR_ERR_INVALID"]
+        else:
+            after.append((ls.info(), ls.arrays()))
+        other.close()
+    for a, b in zip(after, after[1:]):
+        assert a[0] == b[0] and _same(a[1], b[1])
+    assert _same(_host_step(ls, inp, 0), _host_step(ls, inp, 1))
