@@ -22,6 +22,7 @@ int set_error(vlr_ctx* ctx, int code, const std::string& msg) {
 }
 
 int check_cuda(vlr_ctx* ctx, cudaError_t e, const char* what) {
+    cudaGetLastError();  // reported here: the next launch's check must not find it again
     int code = (e == cudaErrorMemoryAllocation) ? VLR_ERR_NOMEM : VLR_ERR_CUDA;
     return set_error(ctx, code, std::string(what) + ": " + cudaGetErrorString(e));
 }

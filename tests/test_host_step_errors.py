@@ -65,3 +65,30 @@ def test_error_of_an_earlier_call_is_reported(ctx, state, leave, name):
     for a, b in zip(after, after[1:]):
         assert a[0] == b[0] and _same(a[1], b[1])
     assert _same(_host_step(ls, inp, 0), _host_step(ls, inp, 1))
+
+
+def test_little_device_memory_takes_the_one_pass(ctx, state):
+    """Device memory that holds the one pass's buffers but not the pipeline's."""
+    import torch
+    from sharc.volrus_b200 import Context
+    from sharc.volrus_b200.method import LevelSet, large_sphere_grid
+    ls, inp = state
+    want = _host_step(ls, inp, 1)
+    own = Context()  # its pool holds no memory of other tests
+    sph, vel = large_sphere_grid(75, seed=3, extent=1600.0)
+    other = LevelSet.spheres([(sph, vel)], 1.0, half_width=3.0, precision=1, integrator=3, reinit_iters=2, ctx=own)
+    fill = None
+    try:
+        _host_step(other, inp, 1)  # the one pass's staging stands
+        n = len(inp[0])
+        torch.cuda.synchronize()
+        free = torch.cuda.mem_get_info()[0]
+        fill = torch.empty(free - n * 2048 // 2, dtype=torch.uint8, device="cuda")  # the input's values alone do not fit
+        got = _host_step(other, inp, 0)
+        del fill
+        assert _same(got, want)
+    finally:
+        fill = None
+        torch.cuda.empty_cache()
+        other.close()
+        own.close()
