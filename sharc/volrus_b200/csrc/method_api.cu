@@ -1251,17 +1251,16 @@ int step_host_slabs(vlr_ctx* ctx, vlr_level_set* ls, const SlabPlan& P, const in
                           "list order")))
             return finish(rc);
     }
-    rc = finish(VLR_OK);
-    if (rc) return rc;
+    finish(VLR_OK);
     rc = consume_device_errors(ctx, "vlr_ls_step_host");
     if (rc) {
+        *entry_step = *h_step;
         ls->state_lost = true;
         return rc;
     }
     *n_out = total;
     return VLR_OK;
 }
-
 
 }  // namespace
 
