@@ -405,7 +405,9 @@ int vlr_ls_volume_partials(vlr_ctx* ctx, vlr_level_set* ls, const double ref[3],
  * 8-voxel lattice, masks u64[8], values f32[512] in voxel units.  The upload
  * replaces the state and keeps the time; the download writes the allocated
  * leaves in the level set's list order (unsorted) and sets *n_out, failing
- * with VLR_ERR_CAPACITY above cap_leaves.  Both return after their work. */
+ * with VLR_ERR_CAPACITY above cap_leaves.  Both return after their work.  An
+ * upload that fails its checks (origins off the lattice, repeated or out of
+ * extent) leaves no state: steps are refused until the next upload. */
 int vlr_ls_upload_device(vlr_ctx* ctx, vlr_level_set* ls, const int32_t* d_origins, const uint64_t* d_masks,
                          const float* d_phi, size_t n_leaves);
 int vlr_ls_download_device(vlr_ctx* ctx, const vlr_level_set* ls, int32_t* d_origins, uint64_t* d_masks,

@@ -644,7 +644,7 @@ int enqueue_one_step(vlr_ctx* ctx, vlr_level_set* ls) {
     if (ls->state_lost)
         return set_error(ctx, VLR_ERR_INVALID,
                          "the level set's state is undefined after a step failed with VLR_ERR_TIMEOUT or "
-                         "VLR_ERR_CAPACITY: upload a state first");
+                         "VLR_ERR_CAPACITY, or an upload was refused: upload a state first");
     if (ls->autotune && !ls->tuned) {
         const bool timing = ctx->timer.enabled;
         ctx->timer.enabled = false;
@@ -1518,6 +1518,7 @@ int vlr_ls_upload_device(vlr_ctx* ctx, vlr_level_set* ls, const int32_t* d_origi
     if (ls->n_grids != 1) return set_error(ctx, VLR_ERR_UNSUPPORTED, "upload replaces single-grid states only");
     if (n_leaves > (size_t)ls->cap) return set_error(ctx, VLR_ERR_CAPACITY, "more leaves than the level set's capacity");
     const int n = (int)n_leaves;
+    ls->state_lost = true;  // until the new state has passed its checks
     k_load_lists<<<ls->grid_blocks, 256, 0, ctx->stream>>>(d_origins, n, ls->origin, ls->list, ls->free_stack,
                                                            ls->scalars, ls->cap, ls->hkey, ls->hval, ls->hcap,
                                                            ctx->d_errword);
@@ -1541,7 +1542,7 @@ int vlr_ls_upload_device(vlr_ctx* ctx, vlr_level_set* ls, const int32_t* d_origi
     VLR_CUDA(ctx, cudaGetLastError());
     int rc = ls_enqueue_index(ctx, ls, true);
     // one round trip for the origins' check and the index's (an index built
-    // from origins off the lattice is never used: the call fails)
+    // from origins off the lattice is never used: the state stays lost)
     if (!rc) rc = consume_device_errors(ctx, "vlr_ls_upload_device");
     if (!rc) ls->state_lost = false;  // a complete new state
     return rc;

@@ -74,7 +74,8 @@ struct vlr_level_set {
     StencilShape adv_shape;  // launch shapes of the stencil kernels
     StencilShape re_shape;
     bool tuned = false;      // shapes chosen (by the autotuner or the caller)
-    bool state_lost = false; // a step failed with VLR_ERR_TIMEOUT or VLR_ERR_CAPACITY: the state is undefined
+    bool state_lost = false; // a step failed with VLR_ERR_TIMEOUT or VLR_ERR_CAPACITY, or an edit or a device upload
+                             // was refused: the state is undefined
     bool autotune = true;    // choose the shapes on the first step
     // host steps over x-slabs (vlr_ls_step_host): 0 automatic, 1 one pass,
     // k >= 2 at most k slabs; the copy streams and events, made on first use

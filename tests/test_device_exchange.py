@@ -110,3 +110,28 @@ def test_refused_upload_then_a_good_one(fault):
     out = Buffers(33)
     assert ls.download_device(*out.ptr(), 33) == 33 and same(out.get(33), a)
     ls.close()
+
+
+@pytest.mark.parametrize("fault", ["lattice", "twice", "extent"])
+def test_refused_upload_leaves_nothing_to_step(fault):
+    """Steps are refused until the next complete upload, which steps as in a level set that saw no refusal."""
+    from sharc.volrus_b200._lib import ERROR_NAMES, VolrusError
+    ls, ref = level_set(0), level_set(0)
+    a = ball(33, 33)  # steps within the pool of CAP leaves
+    bad = a[0].copy()
+    bad[7] = bad[7] + 1 if fault == "lattice" else bad[6] if fault == "twice" else (1 << 30, 0, 0)
+    b = Buffers(33)
+    b.put((bad, a[1], a[2]))
+    with pytest.raises(VolrusError):
+        ls.upload_device(*b.ptr(), 33)
+    for call in (lambda: ls.step(1), lambda: ls.enqueue(1)):
+        with pytest.raises(VolrusError) as e:
+            call()
+        assert ERROR_NAMES[e.value.code] == "VLR_ERR_INVALID"
+    b.put(a)
+    for s in (ls, ref):
+        s.upload_device(*b.ptr(), 33)
+        s.step(1)
+    assert same(ls.arrays(), ref.arrays())
+    ls.close()
+    ref.close()
