@@ -1030,10 +1030,13 @@ bool plan_slabs(const vlr_level_set* ls, const int32_t* origins, size_t n, SlabP
             hi[a] = std::max(hi[a], o[a]);
         }
     }
+    int bits = 1;  // the key of the leaves a slab does not keep
     for (int a = 0; a < 3; ++a) {
         p->box[a] = lo[a] >> 3;
         p->box[3 + a] = hi[a] >> 3;
+        bits += bits_for((long long)p->box[3 + a] - p->box[a] + 2);
     }
+    if (bits > 64) return false;  // no slab's keys (slab_keys) need more than the box's
     auto xat = [&](size_t i) { return (long long)origins[3 * i]; };
     auto lower = [&](long long x) {  // first leaf with x at or above
         size_t a = 0, b = n;

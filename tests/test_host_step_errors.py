@@ -92,3 +92,32 @@ def test_little_device_memory_takes_the_one_pass(ctx, state):
         torch.cuda.empty_cache()
         other.close()
         own.close()
+
+
+@pytest.mark.parametrize("width", [1 << 20, (1 << 21) - 2, (1 << 21) - 1, 1 << 21, 1 << 27])
+def test_states_as_wide_as_the_hash(ctx, width):
+    """Leaves at the corners of a box of `width` leaves an axis (the hash holds 2^21): keys of that box and its
+    margin need up to 67 bits, and a wider state is refused as the one pass refuses it."""
+    from sharc.volrus_b200 import VolrusError
+    from sharc.volrus_b200.method import LevelSet
+    lo = -((width + 1) // 2)
+    c = np.stack(np.unravel_index(np.arange(8), (2, 2, 2)), 1) * width + lo
+    o = (np.concatenate([c, [[0, 0, 0]]])[[0, 1, 2, 3, 8, 4, 5, 6, 7]] * 8).astype(np.int32)
+    phi = np.full((9, 8, 8, 8), 3.0, np.float32)
+    phi[:, 3:5, 3:5, 3:5] = np.random.default_rng(5).uniform(-2, 2, (9, 2, 2, 2))
+    phi = phi.reshape(9, 512)
+    m = np.ascontiguousarray(np.packbits(np.abs(phi) < 3, axis=1, bitorder="little")).view(np.uint64)
+    ls = LevelSet.from_leaves(o[4:5], m[4:5], phi[4:5], {"kind": "constant", "c": (0.25, -0.5, 0.125)}, 1.0,
+                              capacity=256, ctx=ctx)
+    inp = tuple(_pinned(a) for a in (o, m, phi))
+    res = []
+    for slabs in (1, 2):
+        try:
+            res.append(_host_step(ls, inp, slabs))
+        except VolrusError as e:
+            res.append(e.code)
+    if width < 1 << 21:
+        assert len(res[0][0]) == 9 and _same(res[0], res[1])
+    else:
+        assert res[0] == res[1] == _codes()["VLR_ERR_EXTENT"]
+    ls.close()
