@@ -468,6 +468,31 @@ __device__ __forceinline__ void add_corner(float& acc, unsigned t, const float4&
     acc += lam * wx * wy * wz;
 }
 
+// The candidates (dy.., dz..) of Y rows of Z offsets at x offset dx, added to
+// plane in (y, z) order; their words are loaded before the first is tested.
+// Offsets past the window (y1, z1) test nothing; they lie within R + 8 < 16 of
+// the voxel, and their leaf offset is held to the neighbourhood.
+template <bool LAM, int Y, int Z>
+__device__ __forceinline__ void add_candidates(float& plane, int row, int x, int cy, int cz, int dx, int dy, int dz,
+                                               int y1, int z1, const unsigned* foot_pk, const float4* foot_w,
+                                               const float* lam_in) {
+    unsigned t[Y * Z], e[Y * Z];
+#pragma unroll
+    for (int q = 0; q < Y * Z; ++q) {
+        const int ry = q / Z, rz = q % Z, y = cy + dy + ry, z = cz + dz + rz;
+        const int ns = __shfl_sync(0xffffffffu, row, leaf_of(x) * 9 + min(leaf_of(y), 2) * 3 + min(leaf_of(z), 2));
+        e[q] = (unsigned)ns * kLeafVoxels + (unsigned)voxel_off(x, y, z);
+        t[q] = ~0u;
+        if (ns >= 0 && dy + ry <= y1 && dz + rz <= z1) t[q] = cell_key(dx, dy + ry, dz + rz) - foot_pk[e[q]];
+    }
+#pragma unroll
+    for (int q = 0; q < Y * Z; ++q)
+        if (!(t[q] & ~kCorner)) {
+            const float4 w = foot_w[e[q]];
+            add_corner(plane, t[q], w, LAM ? lam_in[e[q]] : w.w);
+        }
+}
+
 // Adjoint of step k as a gather:
 //   lambda'(b) = sum over band voxels x of lambda(x) w_b(p(x))  (b as a corner)
 // A step moves a voxel by at most R = reach voxels per axis, so b is a corner
@@ -481,8 +506,10 @@ __device__ __forceinline__ void add_corner(float& acc, unsigned t, const float4&
 // nor their order; smooth fields leave 2-3 offsets per axis, against 2R + 2.
 //
 // One warp per chunk of a leaf's band voxels: the window is uniform, a
-// neighbour slot costs a shuffle, and the words of up to three candidates
-// along z, on ROWS rows, are loaded before the first is tested.  Where the neighbourhood has
+// neighbour slot costs a shuffle, and the words of three candidates along z
+// (WIDE: of nine or ten, on as many rows as the window's depth in z leaves, so
+// that both kernels add in the same order) are loaded before the first is
+// tested.  Where the neighbourhood has
 // one foot offset (floor(s u) equal at both ends of its range on every axis,
 // the common case of a smooth field), candidate and corner correspond one to
 // one, so no candidate word is read or tested; voxels off the band hold
@@ -493,9 +520,12 @@ __device__ __forceinline__ void add_corner(float& acc, unsigned t, const float4&
 // hits per voxel (32 bytes a voxel from HBM).  7.67M band voxels of a level
 // set: 373 us one thread per voxel with its own gradient term, 313 us in
 // chunks without it (770 instructions a chunk), 197 us with the untested
-// path, 166 us with the prefetch.
-template <bool LAM, int ROWS>
-__global__ void __launch_bounds__(256, ROWS == 1 ? kChunkCtas : kWideCtas)
+// path, 166 us with the prefetch.  WIDE, 77k band voxels, 16 steps back in a
+// rough field: 629 us by three rows of three whatever the depth (which adds
+// windows deeper than three out of order), 541 us by two rows of five at a
+// depth of five; 1.94 and 1.93 ms by rows of nine at a depth of nine.
+template <bool LAM, bool WIDE>
+__global__ void __launch_bounds__(256, WIDE ? kWideCtas : kChunkCtas)
     k_adj_lambda(const int2* __restrict__ chunks, int n_chunks, int ahead, const int* __restrict__ bvox,
                  const int* __restrict__ nbr, const float* __restrict__ nrange, const unsigned* foot_pk,
                  const float4* foot_w, const float* lam_in, int R, BackOut o) {
@@ -554,27 +584,17 @@ __global__ void __launch_bounds__(256, ROWS == 1 ? kChunkCtas : kWideCtas)
     for (int dx = x0; dx <= x1; ++dx) {
         const int x = cx + dx;
         float plane = 0.f;
-        for (int dy = y0; dy <= y1; dy += ROWS) {
-            for (int dz = z0; dz <= z1; dz += 3) {
-                unsigned t[3 * ROWS], e[3 * ROWS];
-#pragma unroll
-                for (int q = 0; q < 3 * ROWS; ++q) {
-                    const int ry = q / 3, rz = q % 3, y = cy + dy + ry, z = cz + dz + rz;
-                    // offsets past the window (up to y1 + 2, z1 + 2 <= R + 2 < 9 from the voxel) test nothing
-                    const int ns = __shfl_sync(0xffffffffu, k.row,
-                                               leaf_of(x) * 9 + min(leaf_of(y), 2) * 3 + min(leaf_of(z), 2));
-                    e[q] = (unsigned)ns * kLeafVoxels + (unsigned)voxel_off(x, y, z);
-                    t[q] = ~0u;
-                    if (ns >= 0 && dy + ry <= y1 && dz + rz <= z1)
-                        t[q] = cell_key(dx, dy + ry, dz + rz) - foot_pk[e[q]];
-                }
-#pragma unroll
-                for (int q = 0; q < 3 * ROWS; ++q)
-                    if (!(t[q] & ~kCorner)) {
-                        const float4 w = foot_w[e[q]];
-                        add_corner(plane, t[q], w, LAM ? lam_in[e[q]] : w.w);
-                    }
-            }
+        if (WIDE && z1 - z0 < 3) {
+            for (int dy = y0; dy <= y1; dy += 3)
+                add_candidates<LAM, 3, 3>(plane, k.row, x, cy, cz, dx, dy, z0, y1, z1, foot_pk, foot_w, lam_in);
+        } else if (WIDE && z1 - z0 < 5) {
+            for (int dy = y0; dy <= y1; dy += 2)
+                add_candidates<LAM, 2, 5>(plane, k.row, x, cy, cz, dx, dy, z0, y1, z1, foot_pk, foot_w, lam_in);
+        } else {
+            constexpr int Z = WIDE ? 9 : 3;
+            for (int dy = y0; dy <= y1; ++dy)
+                for (int dz = z0; dz <= z1; dz += Z)
+                    add_candidates<LAM, 1, Z>(plane, k.row, x, cy, cz, dx, dy, dz, y1, z1, foot_pk, foot_w, lam_in);
         }
         acc += plane;
     }
@@ -881,10 +901,10 @@ int enqueue_lambda_step(vlr_ctx* ctx, vlr_adjoint* a, int cur, const BackOut& o)
                               pk, w, lam, a->reach, o);
         };
         if (a->disp)
-            VLR_TIMED(ctx, "k_adj_lambda", VLR_CUDA(ctx, launch(wide ? k_adj_lambda<true, 3> : k_adj_lambda<true, 1>,
+            VLR_TIMED(ctx, "k_adj_lambda", VLR_CUDA(ctx, launch(wide ? k_adj_lambda<true, true> : k_adj_lambda<true, false>,
                                                                 (const float*)a->lam_pool[cur])));
         else
-            VLR_TIMED(ctx, "k_adj_lambda", VLR_CUDA(ctx, launch(wide ? k_adj_lambda<false, 3> : k_adj_lambda<false, 1>,
+            VLR_TIMED(ctx, "k_adj_lambda", VLR_CUDA(ctx, launch(wide ? k_adj_lambda<false, true> : k_adj_lambda<false, false>,
                                                                 (const float*)nullptr)));
     }
     return VLR_OK;
