@@ -55,6 +55,9 @@ typedef struct vlr_transform {
 } vlr_transform;
 
 /* ---- context ---------------------------------------------------------- */
+/* Copies of 3 MB and more between pageable host memory and the device are
+ * shared with three threads of the context's own, started by its first such
+ * copy and joined by vlr_ctx_destroy: none is in the library's code after it. */
 int vlr_ctx_create(int device, vlr_ctx** out);
 void vlr_ctx_destroy(vlr_ctx* ctx);
 const char* vlr_last_error(const vlr_ctx* ctx);

@@ -4,13 +4,16 @@
 // src/tree/root.rs:55-72, src/tree/internal.rs:88-143) with flat device
 // arrays that the stencil kernels index directly.
 #include <algorithm>
+#include <pthread.h>
+#include <unistd.h>
+
 #include <condition_variable>
 #include <cstdlib>
 #include <cstring>
-#include <memory>
 #include <mutex>
 #include <string>
 #include <thread>
+#include <vector>
 
 #include "vlr_host.hpp"
 
@@ -155,9 +158,9 @@ static cudaError_t copy_share(char* host, char* dev, size_t bytes, bool up, char
 // The threads beside the caller, kept with the context from its first large
 // copy: started and joined per copy they cost 30-50 us, and what they allocate
 // in the caller's heap made glibc give its top back to the system and fault it
-// in again on each call (meshing 2.1 -> 2.9 ms).  They are detached and share
-// the state, which the last of them frees, so nothing waits for them when the
-// context goes.
+// in again on each call (meshing 2.1 -> 2.9 ms).  They are joined when the
+// context goes (idle by then), so none of them is in the library's code after
+// that; a forked child, which has no such threads, leaves the state be.
 struct CopyThreads {
     std::mutex m;
     std::condition_variable go, idle;
@@ -165,11 +168,13 @@ struct CopyThreads {
     void* arg = nullptr;
     unsigned long turn = 0;
     int running = 0;  // threads still at the current job
-    int count = 0;    // threads started
     bool quit = false;
+    const pid_t owner = getpid();
+    std::vector<std::thread> threads;
 };
 
-static void copy_thread(std::shared_ptr<CopyThreads> s, int t, int device) {
+static void copy_thread(CopyThreads* s, int t, int device) {
+    pthread_setname_np(pthread_self(), "vlr-copy");
     const bool ok = cudaSetDevice(device) == cudaSuccess;
     std::unique_lock<std::mutex> lock(s->m);
     for (unsigned long seen = 0;;) {
@@ -184,13 +189,16 @@ static void copy_thread(std::shared_ptr<CopyThreads> s, int t, int device) {
 }
 
 void copy_threads_stop(vlr_ctx* ctx) {
-    if (!ctx->copy_threads) return;
+    CopyThreads* s = ctx->copy_threads;
+    ctx->copy_threads = nullptr;
+    if (!s || s->owner != getpid()) return;
     {
-        std::lock_guard<std::mutex> lock(ctx->copy_threads->m);
-        ctx->copy_threads->quit = true;
+        std::lock_guard<std::mutex> lock(s->m);
+        s->quit = true;
     }
-    ctx->copy_threads->go.notify_all();
-    ctx->copy_threads.reset();
+    s->go.notify_all();
+    for (std::thread& t : s->threads) t.join();
+    delete s;
 }
 
 static int staged_copy(vlr_ctx* ctx, char* host, char* dev, size_t bytes, bool up) {
@@ -201,10 +209,9 @@ static int staged_copy(vlr_ctx* ctx, char* host, char* dev, size_t bytes, bool u
     }
     if (!ctx->copy_threads) {
         try {
-            auto s = std::make_shared<CopyThreads>();
-            ctx->copy_threads = s;
-            for (; s->count + 1 < kCopyShares; ++s->count)
-                std::thread(copy_thread, s, s->count + 1, ctx->device).detach();
+            CopyThreads* s = ctx->copy_threads = new CopyThreads;
+            s->threads.reserve(kCopyShares - 1);
+            for (int t = 1; t < kCopyShares; ++t) s->threads.emplace_back(copy_thread, s, t, ctx->device);
         } catch (...) {  // no more threads: the caller takes the shares that are left
         }
     }
@@ -217,8 +224,8 @@ static int staged_copy(vlr_ctx* ctx, char* host, char* dev, size_t bytes, bool u
             err[t] = copy_share(host + a, dev + a, z - a, up, static_cast<char*>(ctx->stage) + 2 * t * kCopyChunk,
                                 ctx->stage_ev + 2 * t, st);
     };
-    CopyThreads* pool = ctx->copy_threads.get();
-    const int others = pool ? pool->count : 0;
+    CopyThreads* pool = ctx->copy_threads;
+    const int others = pool ? (int)pool->threads.size() : 0;
     if (others) {
         std::lock_guard<std::mutex> lock(pool->m);
         pool->job = [](void* f, int t) { (*static_cast<decltype(share)*>(f))(t); };

@@ -1,7 +1,6 @@
 // Host-side context and grid handles behind the C ABI (include/volrus_b200.h).
 #pragma once
 #include <cstdint>
-#include <memory>
 #include <string>
 #include <vector>
 #include <cuda_runtime.h>
@@ -39,7 +38,7 @@ struct vlr_ctx {
     void* pinned = nullptr;             // small pinned host buffer for scalar read-backs
     void* stage = nullptr;              // pinned buffers for large copies from and into pageable memory
     cudaEvent_t stage_ev[8] = {};
-    std::shared_ptr<vlr::CopyThreads> copy_threads;  // the threads that move those copies
+    vlr::CopyThreads* copy_threads = nullptr;  // the threads that move those copies
     vlr_kernel_timer timer;
 };
 
@@ -144,7 +143,7 @@ int consume_device_errors(vlr_ctx* ctx, const char* what);
 // shares that a few threads move at once; small or pinned ones take one copy.
 // h2d_copy has read the source when it returns; the device side is stream-ordered.
 int d2h_copy(vlr_ctx* ctx, void* dst, const void* src, size_t bytes);
-void copy_threads_stop(vlr_ctx* ctx);
+void copy_threads_stop(vlr_ctx* ctx);  // joins them
 int h2d_copy(vlr_ctx* ctx, void* dst, const void* src, size_t bytes);
 int read_int(vlr_ctx* ctx, const int* d_ptr, int* out);
 // read_int and consume_device_errors in one round trip.

@@ -78,3 +78,34 @@ def test_contexts_side_by_side():
     [t.start() for t in ts]
     [t.join() for t in ts]
     assert all(np.array_equal(got[s], want[s]) for s in want)
+
+
+def test_threads_end_with_their_context():
+    """The threads of large copies start with a context's first one and are joined by its destruction."""
+    import os
+    import time
+    from sharc.volrus_b200._lib import Context
+    from sharc.volrus_b200.tools import advect_particles_euler, make_uniform_velocity
+
+    def names():
+        n = 0
+        for t in os.listdir("/proc/self/task"):
+            try:
+                n += open(f"/proc/self/task/{t}/comm").read().strip() == "vlr-copy"
+            except OSError:
+                pass  # gone since the listing
+        return n
+    vel = make_uniform_velocity(1.0, (0.0, 0.0, 0.0))
+    pos = np.random.default_rng(0).uniform(-8, 8, (200000, 3))
+    base = names()
+    ctx = Context()
+    advect_particles_euler(pos[:1000], vel, 0.5, ctx=ctx)
+    assert names() == base
+    for _ in range(2):
+        advect_particles_euler(pos, vel, 0.5, ctx=ctx)
+        assert names() == base + 3
+    ctx.close()
+    until = time.monotonic() + 1.0  # the system may list a joined thread for an instant
+    while names() != base and time.monotonic() < until:
+        time.sleep(0.001)
+    assert names() == base
