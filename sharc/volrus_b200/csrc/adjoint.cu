@@ -808,6 +808,16 @@ void adj_free(vlr_adjoint* a) {
     for (void* p : ptrs) cudaFree(p);
 }
 
+// Steps between checkpoints for the caller's wish: results do not depend on
+// them, memory does, 12 C bytes a band voxel for the gradients of a segment
+// and 4 steps / C for the checkpoints.  A wish up to 40 stands (the 8 C bytes
+// that gradients take beyond values are then less than the sort buffers that a
+// plan no longer holds), and is never more than the steps; a longer segment is
+// cut to where both together are least.
+int checkpoint_steps(int wish, int steps) {
+    return std::min({wish, steps, std::max(40, (int)std::ceil(std::sqrt(steps / 3.0)))});
+}
+
 // Per-axis displacement bound of one step in whole voxels: |s_k u| <= dt max|V|
 // (the upsample is a convex combination of V and |cos| <= 1).
 int reach_of(const float* vel, size_t nvel, double dt) {
@@ -992,15 +1002,21 @@ int make_chunks(vlr_ctx* ctx, vlr_adjoint* a) {
     return rc || e == cudaSuccess ? rc : check_cuda(ctx, e, "adjoint chunk list");
 }
 
+// Temporaries up to this size come from the context's pool, which keeps them
+// for the next plan; larger ones (576 bytes a band voxel) go back to the device.
+constexpr size_t kPoolTemp = 32u << 20;
+
 // The sorted entries of upsample^T (synchronises; allocates them).
 int make_vel_entries(vlr_ctx* ctx, vlr_adjoint* a) {
     cudaStream_t st = ctx->stream;
     const int ne = a->n_band * 24, n = a->n_stag, B = blocks_for(ctx, ne);
     const float H = (float)a->H;
-    // temporaries in one block of the context's pool
+    // temporaries in one block
     const size_t sb = (radix_scratch_bytes(ne, 4) + 255) & ~(size_t)255;
+    const size_t bytes = sb + sizeof(int) * (4 * (size_t)ne + 1);
     char* blk = nullptr;
-    VLR_CUDA(ctx, cudaMallocFromPoolAsync((void**)&blk, sb + sizeof(int) * (4 * (size_t)ne + 1), ctx->pool, st));
+    if (bytes > kPoolTemp) VLR_CUDA(ctx, cudaMalloc((void**)&blk, bytes));
+    else VLR_CUDA(ctx, cudaMallocFromPoolAsync((void**)&blk, bytes, ctx->pool, st));
     unsigned* keys = (unsigned*)(blk + sb);
     unsigned* ids = keys + ne;
     int* head = (int*)(ids + ne);
@@ -1024,7 +1040,8 @@ int make_vel_entries(vlr_ctx* ctx, vlr_adjoint* a) {
         return VLR_OK;
     };
     const int rc = make();
-    cudaFreeAsync(blk, st);
+    if (bytes > kPoolTemp) cudaFree(blk);  // waits for the device
+    else cudaFreeAsync(blk, st);
     return rc;
 }
 
@@ -1277,7 +1294,7 @@ int vlr_adj_create(vlr_ctx* ctx, const int32_t* origins, const uint64_t* masks, 
     a->period = period;
     a->t0 = t0;
     a->steps = steps;
-    a->chk_every = checkpoint_every;
+    a->chk_every = checkpoint_steps(checkpoint_every, steps);
     auto fail = [&](int rc) {
         adj_free(a);
         delete a;
@@ -1304,7 +1321,7 @@ int vlr_adj_create(vlr_ctx* ctx, const int32_t* origins, const uint64_t* masks, 
     std::vector<int4> o4(n_leaves);
     for (size_t i = 0; i < n_leaves; ++i) o4[i] = make_int4(origins[3 * i], origins[3 * i + 1], origins[3 * i + 2], 0);
     size_t nvel = 3ull * n_stag * n_stag * n_stag;
-    int n_chk = steps / checkpoint_every + 1;
+    const size_t n_chk = (size_t)(steps / a->chk_every) + 1;
     if (nb > (size_t)INT32_MAX / 24) return fail(set_error(ctx, VLR_ERR_CAPACITY, "band too large for a staggered adjoint"));
 #define ADJ_MALLOC(p, bytes) \
     do { cudaError_t e_ = cudaMalloc(&(p), (bytes)); if (e_ != cudaSuccess) return fail(check_cuda(ctx, e_, "cudaMalloc")); } while (0)
@@ -1319,25 +1336,13 @@ int vlr_adj_create(vlr_ctx* ctx, const int32_t* origins, const uint64_t* masks, 
     ADJ_MALLOC(a->bvox, sizeof(int) * nb);
     ADJ_MALLOC(a->ub, sizeof(float3) * nb);
     ADJ_MALLOC(a->vel, sizeof(float) * nvel);
-    ADJ_MALLOC(a->checkpoints, sizeof(float) * nb * n_chk);
-    ADJ_MALLOC(a->segment, sizeof(float3) * nb * checkpoint_every);
     ADJ_MALLOC(a->lam[0], sizeof(float) * nb);
     ADJ_MALLOC(a->lam[1], sizeof(float) * nb);
     ADJ_MALLOC(a->gvel, sizeof(float) * nvel);
-    for (int q = 0; q < 2; ++q) {
-        ADJ_MALLOC(a->foot_pk[q], sizeof(unsigned) * 512 * n_leaves);
-        ADJ_MALLOC(a->foot_w[q], sizeof(float4) * 512 * n_leaves);
-    }
     ADJ_MALLOC(a->lstart, sizeof(int) * (n_leaves + 1));
     ADJ_MALLOC(a->urange, sizeof(float) * 6 * n_leaves);
     ADJ_MALLOC(a->nrange, sizeof(float) * 6 * n_leaves);
-    ADJ_MALLOC(a->G, sizeof(float3) * nb);
-#undef ADJ_MALLOC
     cudaStream_t st = ctx->stream;
-    for (int q = 0; q < 2; ++q) {  // off the band: no foot, weight 0, lambda 0
-        VLR_CUDA(ctx, cudaMemsetAsync(a->foot_pk[q], 0, sizeof(unsigned) * 512 * n_leaves, st));
-        VLR_CUDA(ctx, cudaMemsetAsync(a->foot_w[q], 0, sizeof(float4) * 512 * n_leaves, st));
-    }
     VLR_CUDA(ctx, cudaMemcpyAsync(a->lstart, lstart.data(), sizeof(int) * (n_leaves + 1), cudaMemcpyHostToDevice, st));
     VLR_CUDA(ctx, cudaMemcpyAsync(a->origin, o4.data(), sizeof(int4) * n_leaves, cudaMemcpyHostToDevice, st));
     VLR_CUDA(ctx, cudaMemcpyAsync(a->phi_init, phi, sizeof(float) * 512 * n_leaves, cudaMemcpyHostToDevice, st));
@@ -1361,6 +1366,18 @@ int vlr_adj_create(vlr_ctx* ctx, const int32_t* origins, const uint64_t* masks, 
     if (!rc) rc = make_chunks(ctx, a);
     if (!rc) rc = make_vel_entries(ctx, a);
     if (rc) return fail(rc);
+    // the passes' own buffers, when the temporaries of the entries are gone
+    ADJ_MALLOC(a->checkpoints, sizeof(float) * nb * n_chk);
+    ADJ_MALLOC(a->segment, sizeof(float3) * nb * a->chk_every);
+    ADJ_MALLOC(a->G, sizeof(float3) * nb);
+    for (int q = 0; q < 2; ++q) {
+        ADJ_MALLOC(a->foot_pk[q], sizeof(unsigned) * 512 * n_leaves);
+        ADJ_MALLOC(a->foot_w[q], sizeof(float4) * 512 * n_leaves);
+        // off the band: no foot, weight 0, lambda 0
+        VLR_CUDA(ctx, cudaMemsetAsync(a->foot_pk[q], 0, sizeof(unsigned) * 512 * n_leaves, st));
+        VLR_CUDA(ctx, cudaMemsetAsync(a->foot_w[q], 0, sizeof(float4) * 512 * n_leaves, st));
+    }
+#undef ADJ_MALLOC
     cudaError_t e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) return fail(check_cuda(ctx, e, "adjoint setup"));
     rc = consume_device_errors(ctx, "vlr_adj_create");
