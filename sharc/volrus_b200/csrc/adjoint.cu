@@ -506,10 +506,11 @@ __device__ __forceinline__ void add_candidates(float& plane, int row, int x, int
 // nor their order; smooth fields leave 2-3 offsets per axis, against 2R + 2.
 //
 // One warp per chunk of a leaf's band voxels: the window is uniform, a
-// neighbour slot costs a shuffle, and the words of three candidates along z
-// (WIDE: of nine or ten, on as many rows as the window's depth in z leaves, so
-// that both kernels add in the same order) are loaded before the first is
-// tested.  Where the neighbourhood has
+// neighbour slot costs a shuffle, and the words of several candidates are
+// loaded before the first is tested: kNarrow three along z; kThreeRows three
+// rows of three, the whole depth of a window at a reach of one voxel; kDeep
+// three rows of three, or one row of five or nine where the window is deeper,
+// so that every instance adds in the same order.  Where the neighbourhood has
 // one foot offset (floor(s u) equal at both ends of its range on every axis,
 // the common case of a smooth field), candidate and corner correspond one to
 // one, so no candidate word is read or tested; voxels off the band hold
@@ -520,12 +521,14 @@ __device__ __forceinline__ void add_candidates(float& plane, int row, int x, int
 // hits per voxel (32 bytes a voxel from HBM).  7.67M band voxels of a level
 // set: 373 us one thread per voxel with its own gradient term, 313 us in
 // chunks without it (770 instructions a chunk), 197 us with the untested
-// path, 166 us with the prefetch.  WIDE, 77k band voxels, 16 steps back in a
-// rough field: 629 us by three rows of three whatever the depth (which adds
-// windows deeper than three out of order), 541 us by two rows of five at a
-// depth of five; 1.94 and 1.93 ms by rows of nine at a depth of nine.
-template <bool LAM, bool WIDE>
-__global__ void __launch_bounds__(256, WIDE ? kWideCtas : kChunkCtas)
+// path, 166 us with the prefetch.  16 steps back on 77k band voxels in a rough
+// field, windows five and nine deep: 629 us and 1.95 ms cut into threes (which
+// adds them out of order), 469 us and 1.92 ms by kDeep; 64 steps on a 256^3
+// sphere, reach one: 849 us by kDeep, 822 us by kThreeRows.
+enum Rows { kNarrow, kThreeRows, kDeep };
+
+template <bool LAM, Rows ROWS>
+__global__ void __launch_bounds__(256, ROWS == kNarrow ? kChunkCtas : kWideCtas)
     k_adj_lambda(const int2* __restrict__ chunks, int n_chunks, int ahead, const int* __restrict__ bvox,
                  const int* __restrict__ nbr, const float* __restrict__ nrange, const unsigned* foot_pk,
                  const float4* foot_w, const float* lam_in, int R, BackOut o) {
@@ -584,14 +587,14 @@ __global__ void __launch_bounds__(256, WIDE ? kWideCtas : kChunkCtas)
     for (int dx = x0; dx <= x1; ++dx) {
         const int x = cx + dx;
         float plane = 0.f;
-        if (WIDE && z1 - z0 < 3) {
+        if (ROWS == kThreeRows || (ROWS == kDeep && z1 - z0 < 3)) {
             for (int dy = y0; dy <= y1; dy += 3)
                 add_candidates<LAM, 3, 3>(plane, k.row, x, cy, cz, dx, dy, z0, y1, z1, foot_pk, foot_w, lam_in);
-        } else if (WIDE && z1 - z0 < 5) {
-            for (int dy = y0; dy <= y1; dy += 2)
-                add_candidates<LAM, 2, 5>(plane, k.row, x, cy, cz, dx, dy, z0, y1, z1, foot_pk, foot_w, lam_in);
+        } else if (ROWS == kDeep && z1 - z0 < 5) {
+            for (int dy = y0; dy <= y1; ++dy)
+                add_candidates<LAM, 1, 5>(plane, k.row, x, cy, cz, dx, dy, z0, y1, z1, foot_pk, foot_w, lam_in);
         } else {
-            constexpr int Z = WIDE ? 9 : 3;
+            constexpr int Z = ROWS == kDeep ? 9 : 3;
             for (int dy = y0; dy <= y1; ++dy)
                 for (int dz = z0; dz <= z1; dz += Z)
                     add_candidates<LAM, 1, Z>(plane, k.row, x, cy, cz, dx, dy, dz, y1, z1, foot_pk, foot_w, lam_in);
@@ -910,12 +913,18 @@ int enqueue_lambda_step(vlr_ctx* ctx, vlr_adjoint* a, int cur, const BackOut& o)
             return pdl_launch(kernel, B, 256, 0, st, a->chunks, a->n_chunks, chunk_wave(ctx), a->bvox, a->nbr, a->nrange,
                               pk, w, lam, a->reach, o);
         };
+        // At a reach of one |s u| < 1 (reach_of), so foot offsets are -1 and 0
+        // and windows at most three deep.
+        const Rows rows = !wide ? kNarrow : a->reach == 1 ? kThreeRows : kDeep;
+        auto pick = [&](auto* narrow, auto* three, auto* deep) {
+            return rows == kNarrow ? narrow : rows == kThreeRows ? three : deep;
+        };
         if (a->disp)
-            VLR_TIMED(ctx, "k_adj_lambda", VLR_CUDA(ctx, launch(wide ? k_adj_lambda<true, true> : k_adj_lambda<true, false>,
-                                                                (const float*)a->lam_pool[cur])));
+            VLR_TIMED(ctx, "k_adj_lambda", VLR_CUDA(ctx, launch(pick(k_adj_lambda<true, kNarrow>, k_adj_lambda<true, kThreeRows>,
+                                                                     k_adj_lambda<true, kDeep>), (const float*)a->lam_pool[cur])));
         else
-            VLR_TIMED(ctx, "k_adj_lambda", VLR_CUDA(ctx, launch(wide ? k_adj_lambda<false, true> : k_adj_lambda<false, false>,
-                                                                (const float*)nullptr)));
+            VLR_TIMED(ctx, "k_adj_lambda", VLR_CUDA(ctx, launch(pick(k_adj_lambda<false, kNarrow>, k_adj_lambda<false, kThreeRows>,
+                                                                     k_adj_lambda<false, kDeep>), (const float*)nullptr)));
     }
     return VLR_OK;
 }
