@@ -455,8 +455,9 @@ int vlr_ls_edit_device(vlr_ctx* ctx, vlr_level_set* ls, const uint8_t* d_drop, s
  * the pool too small, a device error) leaves the state undefined until the
  * next upload; smaller states keep the one pass's list order and errors.
  * vlr_ls_set_host_slabs sets the slab count: 0 automatic (two slabs and one
- * more per 2^15 leaves, at most 16), 1 always one pass, k >= 2 at most k slabs
- * (fewer when the leaves have fewer distinct x).  No counterpart in the
+ * more per 2^15 leaves, at most 16, fewer or one pass where the state is thin
+ * in x), 1 always one pass, k >= 2 at most k slabs (fewer when the leaves have
+ * fewer distinct x).  No counterpart in the
  * reference (its step is serial Rust). */
 int vlr_ls_set_host_slabs(vlr_ctx* ctx, vlr_level_set* ls, int slabs);
 int vlr_ls_step_host(vlr_ctx* ctx, vlr_level_set* ls, const int32_t* origins, const uint64_t* masks, const float* phi,

@@ -862,7 +862,12 @@ constexpr int kSlabRing = 16;                   // voxels: two leaves of input b
 // hides a share of the copies (2.1 KB a leaf each way).  One pass against the
 // best count and its time: 7.1k leaves 0.85 ms (2 slabs 0.94), 19.5k 2.39 (2:
 // 1.90), 38k 4.12 (3: 3.24), 84k 8.3 (4: 6.0), 194k 19.0 (4 to 8: 12.6), 2.5M
-// 239 (8 to 20: 135).
+// 239 (8 to 20: 135).  Each slab also steps two leaves of x beside it, which
+// states thin in x pay for: the automatic count is the largest with fewer than
+// twice the leaves stepped in all (one pass against the count above and the
+// one taken: 3 leaves thick, 120k, 15.9, 17.2 and 15.9 ms; 6 thick, 135k, 15.9,
+// 19.0 and 14.5; 12 thick, 145k, 15.9, 14.7 and 12.2; 16 thick, 160k, 17.1,
+// 13.9 and 12.7).
 //
 // Below kSlabLeavesSorted leaves the pipeline is not told from the one pass by
 // what it leaves behind either: the pool keeps the one pass's list order (the
@@ -1047,23 +1052,29 @@ bool plan_slabs(const vlr_level_set* ls, const int32_t* origins, size_t n, SlabP
         }
         return a;
     };
-    p->first.assign(1, 0);
-    for (int s = 1; s < S; ++s) {
-        const size_t j = lower(xat((size_t)s * n / S));
-        if (j > p->first.back() && j < n) p->first.push_back(j);
-    }
-    p->first.push_back(n);
-    const int ns = (int)p->first.size() - 1;
-    if (ns < 2) return false;
-    p->x.assign(ns + 1, 0);
-    p->x[0] = LLONG_MIN;
-    p->x[ns] = LLONG_MAX;
-    for (int s = 1; s < ns; ++s) p->x[s] = xat(p->first[s]);
-    p->lo.resize(ns);
-    p->hi.resize(ns);
-    for (int s = 0; s < ns; ++s) {
-        p->lo[s] = s == 0 ? 0 : lower(p->x[s] - kSlabRing);
-        p->hi[s] = s == ns - 1 ? n : lower(p->x[s + 1] + kSlabRing);
+    for (;; --S) {
+        p->first.assign(1, 0);
+        for (int s = 1; s < S; ++s) {
+            const size_t j = lower(xat((size_t)s * n / S));
+            if (j > p->first.back() && j < n) p->first.push_back(j);
+        }
+        p->first.push_back(n);
+        const int ns = (int)p->first.size() - 1;
+        if (ns < 2) return false;
+        p->x.assign(ns + 1, 0);
+        p->x[0] = LLONG_MIN;
+        p->x[ns] = LLONG_MAX;
+        for (int s = 1; s < ns; ++s) p->x[s] = xat(p->first[s]);
+        p->lo.resize(ns);
+        p->hi.resize(ns);
+        size_t stepped = 0;
+        for (int s = 0; s < ns; ++s) {
+            p->lo[s] = s == 0 ? 0 : lower(p->x[s] - kSlabRing);
+            p->hi[s] = s == ns - 1 ? n : lower(p->x[s + 1] + kSlabRing);
+            stepped += p->hi[s] - p->lo[s];
+        }
+        if (ls->host_slabs != 0 || stepped < 2 * n) break;
+        S = ns;  // one less next
     }
     return true;
 }

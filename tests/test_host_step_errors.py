@@ -121,3 +121,32 @@ def test_states_as_wide_as_the_hash(ctx, width):
     else:
         assert res[0] == res[1] == _codes()["VLR_ERR_EXTENT"]
     ls.close()
+
+
+@pytest.mark.parametrize("dims,steps", [((2, 91, 91), 1), ((3, 74, 74), 1), ((4, 64, 64), 1), ((8, 66, 66), 2),
+                                        ((16, 64, 64), 4), ((64, 16, 16), 2)])
+def test_states_thin_in_x(ctx, dims, steps):
+    """The automatic count steps fewer than twice the leaves (a slab also steps two leaves of x beside it), and gives
+    the one pass's result at any count."""
+    from sharc.volrus_b200.method import LevelSet
+    from tests.test_host_slabs import _out
+    c = np.stack(np.unravel_index(np.arange(np.prod(dims)), dims), 1).astype(np.int32) * 8
+    p = [(c[:, a:a + 1] + w).astype(np.float32) for a, w in enumerate(np.unravel_index(np.arange(512), (8, 8, 8)))]
+    phi = (2.5 * np.sin(0.35 * p[0] + 0.1) * np.cos(0.3 * p[1] + 0.2) * np.cos(0.33 * p[2])).astype(np.float32)
+    m = np.ascontiguousarray(np.packbits(np.abs(phi) < 2, axis=1, bitorder="little")).view(np.uint64)
+    ls = LevelSet.from_leaves(c, m, phi, {"kind": "constant", "c": (0.5, 0.25, -0.3)}, 1.0, precision=1,
+                              capacity=3 * len(c) + 8192, ctx=ctx)
+    inp = tuple(_pinned(a) for a in (c, m, phi))
+    out = _out(3 * len(c) + 8192)
+    want = _host_step(ls, inp, 1, out)
+    got = _host_step(ls, inp, 0, out)
+    ctx.profile(True)  # counts launches
+    try:
+        before = ctx.kernel_time("k_m_advect")[1]
+        counted = _host_step(ls, inp, 0, out)
+        assert ctx.kernel_time("k_m_advect")[1] - before == steps
+    finally:
+        ctx.profile(False)
+    assert _same(want, got) and _same(want, counted)
+    assert _same(want, _host_step(ls, inp, 3, out))
+    ls.close()
