@@ -11,13 +11,13 @@
 //                  look-back over 256-position chunks taken by ticket) gives
 //                  each survivor its new position, followed by the new leaves
 //                  it owns; every listed leaf's hash key is inserted, new
-//                  leaves take slots from the free stack and are filled from
-//                  their owners (clamped-sign rule), slots of dropped leaves
-//                  go to a recycle list
+//                  leaves take slots from the free stack and (the first of a
+//                  chunk) are filled from their owners (clamped-sign rule),
+//                  slots of dropped leaves go to a recycle list
 //   k_t_nbr        the new list in place, 27-neighbour rows updated where a
 //                  neighbour was dropped or is new (the rows of an upload are
-//                  built whole by k_nbr), recycled slots back on the free
-//                  stack; publishes counts
+//                  built whole by k_nbr), new leaves not yet filled, recycled
+//                  slots back on the free stack; publishes counts
 //
 // A third kernel between them (list copy, hash insertion and fills from the
 // scanned positions) cost a step one more launch and re-read what the scan
@@ -36,7 +36,19 @@ namespace vlr {
 // scalars: [0] count  [1] step  [2] free top
 //          [3] finished CTAs of k_t_nbr  [4] new count  [5] recycled count  [7] chunk ticket
 constexpr int kChunk = 256;
-constexpr int kFillQueue = 512;  // new leaves of a chunk filled by whole warps (more: by their own thread)
+// New leaves of a chunk of the scan: the first kKeyQueue have their hash keys
+// inserted by a thread each (the others by their owner's thread, one after the
+// other), beside the fills of the first kFillHere by its warps; the others' are
+// left to k_t_nbr and the whole GPU.  A step adds a few leaves a chunk, but the
+// one after an upload may add 26 a leaf, and a chunk runs on one SM: the new
+// leaves of 343 isolated ones took 1.0 ms when their owners' threads filled
+// those beyond a queue of 512, and take 33 us; 8,000 in a cube (83 a chunk) 22
+// and 15 us.  64 against 16 and 256 here: 97, 91 and 103 us for six steps of
+// the cube; frames of few new leaves do not tell them apart.
+constexpr int kKeyQueue = 256;
+constexpr int kFillHere = 64;
+// newinfo of a new leaf, owner slot * 32 + direction, when its values are still to be filled
+__device__ __forceinline__ int unfilled(int info) { return -3 - info; }
 constexpr long long kSpinLimit = 1ll << 22;  // default bound of the look-back wait (about half a second)
 
 __device__ __forceinline__ void dir_of(int d, int& dx, int& dy, int& dz) {
@@ -77,13 +89,32 @@ __device__ __forceinline__ void hash_put(uint64_t key, int slot, uint64_t* hkey,
     atomicOr(err, kErrHashFull);
 }
 
-// Values of new leaf ns in direction d of its owner, voxels first, first +
-// step, ...: copysign(hw, the owner's value at the clamped position).
+// Values of new leaf ns in direction d of its owner, by one warp:
+// copysign(hw, the owner's value at the clamped position).
 template <typename T>
-__device__ __forceinline__ void fill_leaf(T* vals, int ns, int owner, int d, float hw, int first, int step) {
+__device__ __forceinline__ void fill_leaf(T* vals, int ns, int owner, int d, float hw, int lane) {
+    constexpr int N = kLeafVoxels / 32;
     int dx, dy, dz;
     dir_of(d, dx, dy, dz);
-    for (int off = first; off < kLeafVoxels; off += step) {
+    T v[N];  // every load is under way before the first store
+#pragma unroll
+    for (int q = 0; q < N; ++q) {
+        const int off = lane + 32 * q, x = 8 * dx + (off >> 6), y = 8 * dy + ((off >> 3) & 7), z = 8 * dz + (off & 7);
+        const int cx = min(max(x, 0), 7), cy = min(max(y, 0), 7), cz = min(max(z, 0), 7);
+        v[q] = vals[(size_t)owner * kLeafVoxels + ((cx << 6) | (cy << 3) | cz)];
+    }
+#pragma unroll
+    for (int q = 0; q < N; ++q) vals[(size_t)ns * kLeafVoxels + lane + 32 * q] = from_f<T>(copysignf(hw, to_f(v[q])));
+}
+
+// The same with a load and a store at a time, for the few of a chunk: with the
+// loads ahead of the stores the scan is slower (eight steps at 3.0k leaves
+// 484 -> 495 us).
+template <typename T>
+__device__ __forceinline__ void fill_leaf_few(T* vals, int ns, int owner, int d, float hw, int lane) {
+    int dx, dy, dz;
+    dir_of(d, dx, dy, dz);
+    for (int off = lane; off < kLeafVoxels; off += 32) {
         const int x = 8 * dx + (off >> 6), y = 8 * dy + ((off >> 3) & 7), z = 8 * dz + (off & 7);
         const int cx = min(max(x, 0), 7), cy = min(max(y, 0), 7), cz = min(max(z, 0), 7);
         const float v = to_f(vals[(size_t)owner * kLeafVoxels + ((cx << 6) | (cy << 3) | cz)]);
@@ -105,8 +136,9 @@ __global__ void __launch_bounds__(kChunk) k_t_scanalloc(MLeafArrays A, int4* ori
     __shared__ int s_ticket;
     __shared__ int s_warp[kChunk / 32];
     __shared__ int s_prefix;
-    __shared__ int2 s_fill[kFillQueue];  // new leaf's slot, owner slot * 32 + direction
-    __shared__ int s_nfill;
+    __shared__ uint64_t s_key[kKeyQueue];  // a new leaf's key, slot, and owner slot * 32 + direction
+    __shared__ int s_slot[kKeyQueue], s_info[kFillHere];
+    __shared__ int s_new;
     const long long spin_limit = wait_limit(err, kSpinLimit);
     const bool hold_first = test_stall(err);
     const int count = scalars[0];
@@ -117,7 +149,7 @@ __global__ void __launch_bounds__(kChunk) k_t_scanalloc(MLeafArrays A, int4* ori
     for (;;) {
         if (threadIdx.x == 0) {
             s_ticket = atomicAdd(&scalars[7], 1);
-            s_nfill = 0;
+            s_new = 0;
         }
         __syncthreads();
         const int chunk = s_ticket;
@@ -238,11 +270,16 @@ __global__ void __launch_bounds__(kChunk) k_t_scanalloc(MLeafArrays A, int4* ori
                 dir_of(d, dx, dy, dz);
                 origin[ns] = make_int4(o.x + 8 * dx, o.y + 8 * dy, o.z + 8 * dz, o.w);
                 list_new[pos] = ns;
-                newinfo[pos] = s * 32 + d;  // owner slot and direction
-                hash_put(leaf_key(o, dx, dy, dz, params, bits), ns, hkey, hval, hcap, err);
-                const int f = atomicAdd(&s_nfill, 1);
-                if (f < kFillQueue) s_fill[f] = make_int2(ns, s * 32 + d);
-                else fill_leaf(vals, ns, s, d, params[o.w].hw, 0, 1);
+                const int f = atomicAdd(&s_new, 1), info = s * 32 + d;
+                const uint64_t key = leaf_key(o, dx, dy, dz, params, bits);
+                newinfo[pos] = f < kFillHere ? info : unfilled(info);
+                if (f < kFillHere) s_info[f] = info;
+                if (f < kKeyQueue) {
+                    s_key[f] = key;
+                    s_slot[f] = ns;
+                } else {
+                    hash_put(key, ns, hkey, hval, hcap, err);
+                }
                 A.spill[ns] = 0;
                 A.nonempty[ns] = 0;
 #pragma unroll
@@ -254,11 +291,13 @@ __global__ void __launch_bounds__(kChunk) k_t_scanalloc(MLeafArrays A, int4* ori
             }
         }
         __syncthreads();
-        // the chunk's new leaves, one warp each (coalesced stores)
-        const int nf = min(s_nfill, kFillQueue);
-        for (int f = w; f < nf; f += kChunk / 32) {
-            const int ns = s_fill[f].x, owner = s_fill[f].y >> 5;
-            fill_leaf(vals, ns, owner, s_fill[f].y & 31, params[origin[owner].w].hw, lane, 32);
+        const int added = s_new;
+        const int h = kChunk - 1 - (int)threadIdx.x;
+        if (h < min(added, kKeyQueue)) hash_put(s_key[h], s_slot[h], hkey, hval, hcap, err);
+        // one warp a leaf (coalesced stores)
+        for (int f = w; f < min(added, kFillHere); f += kChunk / 32) {
+            const int info = s_info[f];
+            fill_leaf_few(vals, s_slot[f], info >> 5, info & 31, params[origin[info >> 5].w].hw, lane);
         }
         __syncthreads();  // the queue is read before the next chunk clears it
     }
@@ -278,7 +317,8 @@ __global__ void __launch_bounds__(kChunk) k_t_scanalloc(MLeafArrays A, int4* ori
 // ones, and the last CTA to finish publishes the counts and the stack's top
 // (which the others read); the dropped count is cleared by the next step's
 // advect.
-__global__ void k_t_nbr(const int* __restrict__ list_new, int* __restrict__ list, const int* newinfo,
+template <typename T>
+__global__ void k_t_nbr(const int* __restrict__ list_new, int* __restrict__ list, int* newinfo, T* vals,
                         const int* recycled, const int* keep, int* free_stack, int* scalars, const int4* origin,
                         const uint64_t* hkey, const int* hval, int hcap, const MGridParams* __restrict__ params,
                         int bits, int* nbr, int cap, const unsigned* err) {
@@ -305,7 +345,9 @@ __global__ void k_t_nbr(const int* __restrict__ list_new, int* __restrict__ list
         const int p = base + lane;
         const int sp = p < count ? list_new[p] : 0;
         if (p < count) list[p] = sp;
-        unsigned b = __ballot_sync(0xffffffffu, p < count && newinfo[p] >= 0);
+        const int info = p < count ? newinfo[p] : -1;
+        unsigned b = __ballot_sync(0xffffffffu, info >= 0 || info <= unfilled(0));
+        unsigned todo = __ballot_sync(0xffffffffu, info <= unfilled(0));
         while (b) {
             const int j = __ffs(b) - 1;
             b &= b - 1u;
@@ -319,6 +361,17 @@ __global__ void k_t_nbr(const int* __restrict__ list_new, int* __restrict__ list
                 }
                 nbr[(size_t)N * kNbr + lane] = M;
                 if (M >= 0 && M != N) nbr[(size_t)M * kNbr + (kNbr - 1 - lane)] = N;
+            }
+        }
+        if (todo) {
+            float hw = 0.f;
+            if (info <= unfilled(0)) {
+                newinfo[p] = unfilled(info);
+                hw = params[origin[sp].w].hw;
+            }
+            for (; todo; todo &= todo - 1u) {
+                const int j = __ffs(todo) - 1, own = unfilled(__shfl_sync(0xffffffffu, info, j));
+                fill_leaf(vals, __shfl_sync(0xffffffffu, sp, j), own >> 5, own & 31, __shfl_sync(0xffffffffu, hw, j), lane);
             }
         }
     }
@@ -420,7 +473,7 @@ int ls_enqueue_retrack(vlr_ctx* ctx, vlr_level_set* ls) {
     MLeafArrays A = ls->arrays();
     // status words of the look-back scan live after the scan positions in `pos`
     unsigned long long* status = reinterpret_cast<unsigned long long*>(ls->pos);
-    auto scan = [&](auto* vals) -> int {
+    auto launch = [&](auto* vals) -> int {
         using T = std::remove_pointer_t<decltype(vals)>;
         VLR_TIMED(ctx, "k_t_scanalloc",
                   VLR_CUDA(ctx, pdl_launch(k_t_scanalloc<T>, B, kChunk, 0, st, A, ls->origin, vals,
@@ -428,17 +481,16 @@ int ls_enqueue_retrack(vlr_ctx* ctx, vlr_level_set* ls) {
                                            ls->hkey, ls->hval, ls->hcap, (const MGridParams*)ls->d_params,
                                            ls->key_bits, ls->free_stack, ls->owned, ls->list_new, ls->newinfo, status,
                                            ls->scalars, ls->cap, ctx->d_errword)));
+        VLR_TIMED(ctx, "k_t_nbr",
+                  VLR_CUDA(ctx, pdl_launch(k_t_nbr<T>, B, 256, 0, st, (const int*)ls->list_new, ls->list, ls->newinfo,
+                                           vals, (const int*)ls->owned, (const int*)ls->keep, ls->free_stack,
+                                           ls->scalars, (const int4*)ls->origin, (const uint64_t*)ls->hkey,
+                                           (const int*)ls->hval, ls->hcap, (const MGridParams*)ls->d_params,
+                                           ls->key_bits, ls->nbr, ls->cap, (const unsigned*)ctx->d_errword)));
         return VLR_OK;
     };
-    const int rc = ls->precision == VLR_PREC_F16 ? scan((__half*)ls->vals[0]) : scan((float*)ls->vals[0]);
+    const int rc = ls->precision == VLR_PREC_F16 ? launch((__half*)ls->vals[0]) : launch((float*)ls->vals[0]);
     if (rc) return rc;
-    VLR_TIMED(ctx, "k_t_nbr",
-              VLR_CUDA(ctx, pdl_launch(k_t_nbr, B, 256, 0, st, (const int*)ls->list_new, ls->list,
-                                       (const int*)ls->newinfo, (const int*)ls->owned, (const int*)ls->keep,
-                                       ls->free_stack, ls->scalars, (const int4*)ls->origin,
-                                       (const uint64_t*)ls->hkey, (const int*)ls->hval, ls->hcap,
-                                       (const MGridParams*)ls->d_params, ls->key_bits, ls->nbr, ls->cap,
-                                       (const unsigned*)ctx->d_errword)));
     VLR_CUDA(ctx, cudaGetLastError());
     return VLR_OK;
 }

@@ -1,7 +1,6 @@
-"""More new leaves in a chunk of the re-tracking scan than its fill queue holds:
-343 isolated leaves, active throughout, each bring in their 26 neighbours, 6,656
-in the first chunk of 256 list positions against a queue of 512.  Leaf set and
-masks are the FP64 oracle's; every new leaf holds copysign(hw, its owner's value
+"""New leaves of a chunk of the re-tracking scan around and far beyond the 64 it
+fills itself and the 256 keys it queues: isolated leaves, active throughout,
+each bring in their 26 neighbours, 6,656 in a chunk of 256.  Leaf set and masks are the FP64 oracle's; every new leaf holds copysign(hw, its owner's value
 at the clamped position), bit for bit; a second step works from them.
 
 Bounds: those of the parity tests for a step from a common state."""
@@ -17,11 +16,12 @@ HW = 3.0
 
 
 @pytest.mark.parametrize("precision", [0, 1], ids=["f32", "f16"])
-def test_more_new_leaves_than_the_queue(oracle, precision):
+@pytest.mark.parametrize("leaves", [2, 3, 9, 10, 343])
+def test_many_new_leaves(oracle, leaves, precision):
     from sharc.volrus_b200.method import LevelSet
     side = 7
     c = np.stack(np.unravel_index(np.arange(side ** 3), (side,) * 3), 1)
-    o = (c * 32).astype(np.int32)
+    o = (c[:leaves] * 32).astype(np.int32)
     x, y, z = np.stack(np.unravel_index(np.arange(512), (8, 8, 8))).astype(np.float32)
     n = np.arange(len(o), dtype=np.float32)[:, None]
     v = (0.6 * np.sin(0.4 * x + 0.1 * n) + 0.5 * np.cos(0.35 * y - 0.2 * n) + 0.2 * np.sin(0.3 * z + n)).astype(np.float32)
