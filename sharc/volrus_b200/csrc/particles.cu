@@ -36,32 +36,35 @@ struct V3 {
     double x, y, z;
 };
 
-// The velocity grids and, per particle, the leaf of each that the particle
-// starts in: one hash search per grid, after which its samples (a step moves
-// it little) come from the leaf's neighbour row.  SAME: the grids share their
+// The velocity grids and, with HINT, the leaf of each that the particle starts
+// in: its samples (a step moves it little) come from that leaf's neighbour row,
+// without it every sample searches the hash.  SAME: the grids share their
 // transform, so position and fractions are computed once for the three.
-template <bool SAME>
+template <bool SAME, bool HINT>
 struct Field {
     const GridView& vx;
     const GridView& vy;
     const GridView& vz;
     Hint hx, hy, hz;
 
-    __device__ __forceinline__ Field(const GridView& x, const GridView& y, const GridView& z, const V3& p)
+    // h: the leaf of vx that holds p, a its cell there (HINT)
+    __device__ __forceinline__ Field(const GridView& x, const GridView& y, const GridView& z, const V3& p, const Cell& a,
+                                     const Hint& h)
         : vx(x), vy(y), vz(z) {
-        const Cell a = cell_of(vx, p.x, p.y, p.z);
-        hx = hint_at(vx, a.i, a.j, a.k);
-        const Cell b = SAME ? a : cell_of(vy, p.x, p.y, p.z);
-        hy = hint_at(vy, b.i, b.j, b.k);
-        const Cell c = SAME ? a : cell_of(vz, p.x, p.y, p.z);
-        hz = hint_at(vz, c.i, c.j, c.k);
+        if (HINT) {
+            hx = h;
+            const Cell b = SAME ? a : cell_of(vy, p.x, p.y, p.z);
+            hy = hint_at(vy, b.i, b.j, b.k);
+            const Cell c = SAME ? a : cell_of(vz, p.x, p.y, p.z);
+            hz = hint_at(vz, c.i, c.j, c.k);
+        }
     }
 
     __device__ __forceinline__ V3 operator()(const V3& p) const {
         const Cell a = cell_of(vx, p.x, p.y, p.z);
-        return V3{(double)read_cell(vx, a, hx),
-                  (double)read_cell(vy, SAME ? a : cell_of(vy, p.x, p.y, p.z), hy),
-                  (double)read_cell(vz, SAME ? a : cell_of(vz, p.x, p.y, p.z), hz)};
+        return V3{(double)read_cell(vx, a, HINT ? hx : Hint()),
+                  (double)read_cell(vy, SAME ? a : cell_of(vy, p.x, p.y, p.z), HINT ? hy : Hint()),
+                  (double)read_cell(vz, SAME ? a : cell_of(vz, p.x, p.y, p.z), HINT ? hz : Hint())};
     }
 };
 
@@ -81,11 +84,8 @@ __device__ __forceinline__ double rk4_comb(double p, double k1, double k2, doubl
     return __dadd_rn(p, __ddiv_rn(s, 6.0));
 }
 
-// One RK4 or forward Euler step of a position.
-template <bool SAME>
-__device__ __forceinline__ V3 move_point(const GridView& vx, const GridView& vy, const GridView& vz, const V3& p,
-                                         double dt, int rk4) {
-    const Field<SAME> v(vx, vy, vz, p);
+template <class F>
+__device__ __forceinline__ V3 move_in(const F& v, const V3& p, double dt, int rk4) {
     const V3 v1 = v(p);
     if (!rk4)
         return V3{__dadd_rn(p.x, __dmul_rn(dt, v1.x)), __dadd_rn(p.y, __dmul_rn(dt, v1.y)),
@@ -96,6 +96,21 @@ __device__ __forceinline__ V3 move_point(const GridView& vx, const GridView& vy,
     const V3 k4 = scale(dt, v(axpy(p, k3, 1.0)));
     return V3{rk4_comb(p.x, k1.x, k2.x, k3.x, k4.x), rk4_comb(p.y, k1.y, k2.y, k3.y, k4.y),
               rk4_comb(p.z, k1.z, k2.z, k3.z, k4.z)};
+}
+
+// One RK4 or forward Euler step of a position.  A warp goes by its particles'
+// leaves when all of them start in one: particles without a leaf search the
+// hash for every sample, and a warp that does both takes the time of both (RK4
+// of 100k particles, the kernel, both and this way: most outside 125 leaves 122
+// and 78 us, all outside 124 and 86, 9 % outside 20k leaves 114 and 98, all
+// inside 48 and 48; 1,000 particles there 9 % outside 35 and 58).
+template <bool SAME>
+__device__ __forceinline__ V3 move_point(const GridView& vx, const GridView& vy, const GridView& vz, const V3& p,
+                                         double dt, int rk4) {
+    const Cell a = cell_of(vx, p.x, p.y, p.z);
+    const Hint h = hint_at(vx, a.i, a.j, a.k);
+    if (__all_sync(__activemask(), h.slot >= 0)) return move_in(Field<SAME, true>(vx, vy, vz, p, a, h), p, dt, rk4);
+    return move_in(Field<SAME, false>(vx, vy, vz, p, a, h), p, dt, rk4);
 }
 
 template <bool SAME>
