@@ -256,11 +256,9 @@ int d2h_copy(vlr_ctx* ctx, void* dst, const void* src, size_t bytes) {
 
 int h2d_copy(vlr_ctx* ctx, void* dst, const void* src, size_t bytes) {
     if (!bytes) return VLR_OK;
-    const bool pageable = host_pageable(src);
-    if (bytes >= kCopyMin && pageable)
+    if (bytes >= kCopyMin && host_pageable(src))
         return staged_copy(ctx, static_cast<char*>(const_cast<void*>(src)), static_cast<char*>(dst), bytes, true);
     VLR_CUDA(ctx, cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, ctx->stream));
-    if (!pageable) VLR_CUDA(ctx, cudaStreamSynchronize(ctx->stream));  // the driver has not read it yet
     return VLR_OK;
 }
 

@@ -141,7 +141,7 @@ int consume_device_errors(vlr_ctx* ctx, const char* what);
 // Device-to-host copy of `bytes` on the context stream, returning after it.
 // Large copies into or from pageable memory go through pinned buffers, in
 // shares that a few threads move at once; small or pinned ones take one copy.
-// h2d_copy has read the source when it returns; the device side is stream-ordered.
+// h2d_copy is stream-ordered: a page-locked source is read until the stream gets there.
 int d2h_copy(vlr_ctx* ctx, void* dst, const void* src, size_t bytes);
 void copy_threads_stop(vlr_ctx* ctx);  // joins them
 int h2d_copy(vlr_ctx* ctx, void* dst, const void* src, size_t bytes);
