@@ -60,6 +60,7 @@ struct vlr_adjoint {
     double H = 1.0;                      // staggered cell size in voxels
     double dt = 0.0, t0 = 0.0, period = 1.0;
     int steps = 0, chk_every = 1;
+    char* block = nullptr;               // staggered: holds checkpoints, segment, G and the feet
     float* checkpoints = nullptr;        // (steps / chk_every + 1) x n_band
     float3* segment = nullptr;           // chk_every x n_band (gradients of the recomputed states at the feet)
     float* lam[2] = {nullptr, nullptr};  // band order: [1] lambda_K (and phi_K), [0] lambda_0
@@ -804,6 +805,13 @@ void adj_drop_graphs(vlr_adjoint* a) {
 
 void adj_free(vlr_adjoint* a) {
     adj_drop_graphs(a);
+    if (a->block) {  // holds these
+        a->checkpoints = nullptr;
+        a->segment = a->G = nullptr;
+        a->foot_pk[0] = a->foot_pk[1] = nullptr;
+        a->foot_w[0] = a->foot_w[1] = nullptr;
+        cudaFree(a->block);
+    }
     void* ptrs[] = {a->origin, a->nbr, a->hkey, a->hval, a->phi[0], a->phi[1], a->phi_init, a->bidx, a->bvox,
                     a->ub, a->vel, a->checkpoints, a->segment, a->lam[0], a->lam[1], a->G, a->gvel, a->lstart,
                     a->chunks, a->urange, a->nrange, a->foot_pk[0], a->foot_pk[1], a->foot_w[0], a->foot_w[1],
@@ -813,10 +821,10 @@ void adj_free(vlr_adjoint* a) {
 
 // Steps between checkpoints for the caller's wish: results do not depend on
 // them, memory does, 12 C bytes a band voxel for the gradients of a segment
-// and 4 steps / C for the checkpoints.  A wish up to 40 stands (the 8 C bytes
-// that gradients take beyond values are then less than the sort buffers that a
-// plan no longer holds), and is never more than the steps; a longer segment is
-// cut to where both together are least.
+// and 4 steps / C for the checkpoints.  A wish up to 40 stands (the plan then
+// takes about the memory that sorting its entries takes at creation), and is
+// never more than the steps; a longer segment is cut to where both together are
+// least.
 int checkpoint_steps(int wish, int steps) {
     return std::min({wish, steps, std::max(40, (int)std::ceil(std::sqrt(steps / 3.0)))});
 }
@@ -1011,47 +1019,38 @@ int make_chunks(vlr_ctx* ctx, vlr_adjoint* a) {
     return rc || e == cudaSuccess ? rc : check_cuda(ctx, e, "adjoint chunk list");
 }
 
-// Temporaries up to this size come from the context's pool, which keeps them
-// for the next plan; larger ones (576 bytes a band voxel) go back to the device.
-constexpr size_t kPoolTemp = 32u << 20;
+// Bytes of the temporaries of make_vel_entries for n_band voxels (576 each).
+size_t vel_temp_bytes(int n_band) {
+    const int ne = 24 * n_band;
+    return ((radix_scratch_bytes(ne, 4) + 255) & ~(size_t)255) + sizeof(int) * (4 * (size_t)ne + 1);
+}
 
-// The sorted entries of upsample^T (synchronises; allocates them).
-int make_vel_entries(vlr_ctx* ctx, vlr_adjoint* a) {
+// The sorted entries of upsample^T (synchronises; allocates them), by way of
+// vel_temp_bytes at blk.
+int make_vel_entries(vlr_ctx* ctx, vlr_adjoint* a, char* blk) {
     cudaStream_t st = ctx->stream;
     const int ne = a->n_band * 24, n = a->n_stag, B = blocks_for(ctx, ne);
     const float H = (float)a->H;
-    // temporaries in one block
-    const size_t sb = (radix_scratch_bytes(ne, 4) + 255) & ~(size_t)255;
-    const size_t bytes = sb + sizeof(int) * (4 * (size_t)ne + 1);
-    char* blk = nullptr;
-    if (bytes > kPoolTemp) VLR_CUDA(ctx, cudaMalloc((void**)&blk, bytes));
-    else VLR_CUDA(ctx, cudaMallocFromPoolAsync((void**)&blk, bytes, ctx->pool, st));
-    unsigned* keys = (unsigned*)(blk + sb);
+    unsigned* keys = (unsigned*)(blk + ((radix_scratch_bytes(ne, 4) + 255) & ~(size_t)255));
     unsigned* ids = keys + ne;
     int* head = (int*)(ids + ne);
     int* rank = head + ne;
     unsigned *ks = nullptr, *is = nullptr;
-    auto make = [&]() -> int {
-        VLR_CUDA(ctx, cudaMalloc(&a->ent_b, sizeof(int) * ne));
-        VLR_CUDA(ctx, cudaMalloc(&a->ent_w, sizeof(float) * ne));
-        k_adj_vel_keys<<<B, 256, 0, st>>>(a->bvox, a->origin, ne, n, H, keys, ids);
-        int rc = radix_sort(ctx, keys, ids, ne, bits_for(3ll * n * n * n - 1), blk, &ks, &is);
-        if (rc) return rc;
-        k_adj_vel_entries<<<B, 256, 0, st>>>(a->bvox, a->origin, ne, n, H, ks, is, a->ent_b, a->ent_w, head);
-        rc = scan_exclusive(ctx, head, rank, ne, rank + ne);
-        if (!rc) rc = read_int(ctx, rank + ne, &a->n_seg);
-        if (rc) return rc;
-        VLR_CUDA(ctx, cudaMalloc(&a->seg_start, sizeof(int) * ((size_t)a->n_seg + 1)));
-        VLR_CUDA(ctx, cudaMalloc(&a->seg_node, sizeof(unsigned) * a->n_seg));
-        k_adj_vel_segments<<<B, 256, 0, st>>>(ks, head, rank, ne, a->seg_start, a->seg_node);
-        VLR_CUDA(ctx, cudaMemcpyAsync(a->seg_start + a->n_seg, &ne, sizeof(int), cudaMemcpyHostToDevice, st));
-        VLR_CUDA(ctx, cudaGetLastError());
-        return VLR_OK;
-    };
-    const int rc = make();
-    if (bytes > kPoolTemp) cudaFree(blk);  // waits for the device
-    else cudaFreeAsync(blk, st);
-    return rc;
+    VLR_CUDA(ctx, cudaMalloc(&a->ent_b, sizeof(int) * ne));
+    VLR_CUDA(ctx, cudaMalloc(&a->ent_w, sizeof(float) * ne));
+    k_adj_vel_keys<<<B, 256, 0, st>>>(a->bvox, a->origin, ne, n, H, keys, ids);
+    int rc = radix_sort(ctx, keys, ids, ne, bits_for(3ll * n * n * n - 1), blk, &ks, &is);
+    if (rc) return rc;
+    k_adj_vel_entries<<<B, 256, 0, st>>>(a->bvox, a->origin, ne, n, H, ks, is, a->ent_b, a->ent_w, head);
+    rc = scan_exclusive(ctx, head, rank, ne, rank + ne);
+    if (!rc) rc = read_int(ctx, rank + ne, &a->n_seg);
+    if (rc) return rc;
+    VLR_CUDA(ctx, cudaMalloc(&a->seg_start, sizeof(int) * ((size_t)a->n_seg + 1)));
+    VLR_CUDA(ctx, cudaMalloc(&a->seg_node, sizeof(unsigned) * a->n_seg));
+    k_adj_vel_segments<<<B, 256, 0, st>>>(ks, head, rank, ne, a->seg_start, a->seg_node);
+    VLR_CUDA(ctx, cudaMemcpyAsync(a->seg_start + a->n_seg, &ne, sizeof(int), cudaMemcpyHostToDevice, st));
+    VLR_CUDA(ctx, cudaGetLastError());
+    return VLR_OK;
 }
 
 // Run `enqueue` through a CUDA graph captured on first use (or directly while
@@ -1330,7 +1329,6 @@ int vlr_adj_create(vlr_ctx* ctx, const int32_t* origins, const uint64_t* masks, 
     std::vector<int4> o4(n_leaves);
     for (size_t i = 0; i < n_leaves; ++i) o4[i] = make_int4(origins[3 * i], origins[3 * i + 1], origins[3 * i + 2], 0);
     size_t nvel = 3ull * n_stag * n_stag * n_stag;
-    const size_t n_chk = (size_t)(steps / a->chk_every) + 1;
     if (nb > (size_t)INT32_MAX / 24) return fail(set_error(ctx, VLR_ERR_CAPACITY, "band too large for a staggered adjoint"));
 #define ADJ_MALLOC(p, bytes) \
     do { cudaError_t e_ = cudaMalloc(&(p), (bytes)); if (e_ != cudaSuccess) return fail(check_cuda(ctx, e_, "cudaMalloc")); } while (0)
@@ -1373,20 +1371,34 @@ int vlr_adj_create(vlr_ctx* ctx, const int32_t* origins, const uint64_t* masks, 
                                                         a->ub);
     rc = enqueue_ranges(ctx, a);
     if (!rc) rc = make_chunks(ctx, a);
-    if (!rc) rc = make_vel_entries(ctx, a);
     if (rc) return fail(rc);
-    // the passes' own buffers, when the temporaries of the entries are gone
-    ADJ_MALLOC(a->checkpoints, sizeof(float) * nb * n_chk);
-    ADJ_MALLOC(a->segment, sizeof(float3) * nb * a->chk_every);
-    ADJ_MALLOC(a->G, sizeof(float3) * nb);
-    for (int q = 0; q < 2; ++q) {
-        ADJ_MALLOC(a->foot_pk[q], sizeof(unsigned) * 512 * n_leaves);
-        ADJ_MALLOC(a->foot_w[q], sizeof(float4) * 512 * n_leaves);
-        // off the band: no foot, weight 0, lambda 0
-        VLR_CUDA(ctx, cudaMemsetAsync(a->foot_pk[q], 0, sizeof(unsigned) * 512 * n_leaves, st));
-        VLR_CUDA(ctx, cudaMemsetAsync(a->foot_w[q], 0, sizeof(float4) * 512 * n_leaves, st));
-    }
+    // one block, first for the temporaries of the entries, then for the buffers of the passes
+    const size_t n_chk = (size_t)(steps / a->chk_every) + 1, pool = 512 * n_leaves;
+    const struct {
+        void** p;
+        size_t bytes;
+    } own[] = {{(void**)&a->checkpoints, sizeof(float) * nb * n_chk},
+               {(void**)&a->segment, sizeof(float3) * nb * a->chk_every},
+               {(void**)&a->G, sizeof(float3) * nb},
+               {(void**)&a->foot_pk[0], sizeof(unsigned) * pool},
+               {(void**)&a->foot_pk[1], sizeof(unsigned) * pool},
+               {(void**)&a->foot_w[0], sizeof(float4) * pool},
+               {(void**)&a->foot_w[1], sizeof(float4) * pool}};
+    size_t bytes = 0;
+    for (const auto& o : own) bytes += (o.bytes + 255) & ~(size_t)255;
+    ADJ_MALLOC(a->block, std::max(bytes, vel_temp_bytes(a->n_band)));
 #undef ADJ_MALLOC
+    rc = make_vel_entries(ctx, a, a->block);
+    if (rc) return fail(rc);
+    bytes = 0;
+    for (const auto& o : own) {
+        *o.p = a->block + bytes;
+        bytes += (o.bytes + 255) & ~(size_t)255;
+    }
+    for (int q = 0; q < 2; ++q) {  // off the band: no foot, weight 0, lambda 0
+        VLR_CUDA(ctx, cudaMemsetAsync(a->foot_pk[q], 0, sizeof(unsigned) * pool, st));
+        VLR_CUDA(ctx, cudaMemsetAsync(a->foot_w[q], 0, sizeof(float4) * pool, st));
+    }
     cudaError_t e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) return fail(check_cuda(ctx, e, "adjoint setup"));
     rc = consume_device_errors(ctx, "vlr_adj_create");
