@@ -25,7 +25,8 @@ and ``tools160``.
 
 Timing: W warm-up steps, then exactly K timed steps, each bracketed by CUDA
 events on the library's stream; a 256 MiB write flushes the L2 between
-steps, outside the events.  ``--impl reference`` times the crate's own step
+steps, outside the events.  ``--impl reference`` says why the crate itself
+cannot run here; ``--impl port`` times its step
 (a C++ restatement of advect_level_set + rebuild_narrow_band with its data
 structure, one thread as the crate runs it) on the host CPU, for large8192 on
 a box of the same grid with the whole-grid rate extrapolated (see
@@ -51,6 +52,8 @@ if str(ROOT) not in sys.path:
 L2_FLUSH_BYTES = 256 << 20
 FALLBACK_HBM_GBS = 6650.0
 METRIC = "active voxels/s per advection step"
+# the reference arm runs the unmodified crate or nothing
+REFERENCE_UNAVAILABLE = "the reference is a Rust crate and no Rust toolchain exists here (pip finds no Python project in it)"
 
 DEFORM = dict(radius=0.15, center=(0.35, 0.35, 0.35), voxel_size=1.0 / 512.0, half_width=3.0, period=3.0)
 REF_SPHERE = dict(radius=32.0, center=(64.0, 64.0, 64.0), voxel_size=1.0, half_width=3.0)
@@ -1339,7 +1342,7 @@ def main():
     ap.add_argument("--gpus", type=int, default=1)
     ap.add_argument("--steps", type=int, default=20)
     ap.add_argument("--warmup", type=int, default=3)
-    ap.add_argument("--impl", choices=["ours", "reference"], default="ours")
+    ap.add_argument("--impl", choices=["ours", "reference", "port"], default="ours")
     ap.add_argument("--workload", choices=["deformation512", "batched256", "large8192", "adjoint256",
                                            "reference-sphere128", "mesh96", "tools160"],
                     default="large8192")
@@ -1374,7 +1377,11 @@ def main():
     else:
         sphere, vel_world, ref_dt = REF_SPHERE, REF_VEL, 1.0
 
-    if args.impl == "reference" and args.workload == "mesh96":
+    if args.impl == "reference":
+        if rank == 0:
+            print(json.dumps({"impl": "reference", "unavailable": REFERENCE_UNAVAILABLE}))
+        return
+    if args.impl == "port" and args.workload == "mesh96":
         if rank != 0:
             return
         # the reference's volume_to_mesh restated on the host (its data structure, one thread)
@@ -1394,7 +1401,7 @@ def main():
             vals.append(cells / (time.perf_counter() - t0))
         value = statistics.median(vals)
         print(json.dumps({
-            "impl": "reference", "metric": "cells/s of volume_to_mesh", "value": value, "unit": "cells/s",
+            "impl": "port", "metric": "cells/s of volume_to_mesh", "value": value, "unit": "cells/s",
             "higher_is_better": True, "n_gpus": args.gpus, "steps": len(vals), "warmup": args.warmup,
             "dtype": "f32", "data": "synthetic", "config": {"workload": args.workload},
             "cpu_baseline": {"value": value, "unit": "cells/s", "cores": 1, "kind": "port",
@@ -1402,7 +1409,7 @@ def main():
             "e2e": {"value": value, "unit": "cells/s", "h2d_bytes_per_step": 0, "d2h_bytes_per_step": 0},
         }))
         return
-    if args.impl == "reference" and args.workload == "large8192":
+    if args.impl == "port" and args.workload == "large8192":
         if rank != 0:
             return
         ref = RefLargeSample(args)
@@ -1411,7 +1418,7 @@ def main():
         samples = [ref.step() for _ in range(args.steps)]
         value = statistics.median(x["value"] for x in samples)
         print(json.dumps({
-            "impl": "reference", "metric": METRIC, "value": value, "unit": "voxels/s", "higher_is_better": True,
+            "impl": "port", "metric": METRIC, "value": value, "unit": "voxels/s", "higher_is_better": True,
             "n_gpus": args.gpus, "steps": args.steps, "warmup": args.warmup, "dtype": "f32", "data": "synthetic",
             "config": large_config(args),
             "cpu_baseline": {"value": value, "unit": "voxels/s", "cores": 1, "kind": "port", "sample": ref.describe()},
@@ -1421,7 +1428,7 @@ def main():
                               "box_crossings", "grid_crossings_est")},
         }))
         return
-    if args.impl == "reference":
+    if args.impl == "port":
         if rank != 0:
             return
         vals, desc = [], ""
@@ -1432,7 +1439,7 @@ def main():
             vals.append(v)
         value = statistics.median(vals)
         print(json.dumps({
-            "impl": "reference", "metric": METRIC, "value": value, "unit": "voxels/s", "higher_is_better": True,
+            "impl": "port", "metric": METRIC, "value": value, "unit": "voxels/s", "higher_is_better": True,
             "n_gpus": args.gpus, "steps": args.steps, "warmup": args.warmup, "dtype": "f32", "data": "synthetic",
             "config": {"workload": args.workload},
             "cpu_baseline": {"value": value, "unit": "voxels/s", "cores": 1, "kind": "port", "sample": desc},
