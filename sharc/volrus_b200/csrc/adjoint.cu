@@ -61,6 +61,7 @@ struct vlr_adjoint {
     double dt = 0.0, t0 = 0.0, period = 1.0;
     int steps = 0, chk_every = 1;
     char* block = nullptr;               // staggered: holds checkpoints, segment, G and the feet
+    bool block_pooled = false;           // from the context's pool
     float* checkpoints = nullptr;        // (steps / chk_every + 1) x n_band
     float3* segment = nullptr;           // chk_every x n_band (gradients of the recomputed states at the feet)
     float* lam[2] = {nullptr, nullptr};  // band order: [1] lambda_K (and phi_K), [0] lambda_0
@@ -810,7 +811,8 @@ void adj_free(vlr_adjoint* a) {
         a->segment = a->G = nullptr;
         a->foot_pk[0] = a->foot_pk[1] = nullptr;
         a->foot_w[0] = a->foot_w[1] = nullptr;
-        cudaFree(a->block);
+        if (a->block_pooled) cudaFreeAsync(a->block, a->ctx->stream);
+        else cudaFree(a->block);
     }
     void* ptrs[] = {a->origin, a->nbr, a->hkey, a->hval, a->phi[0], a->phi[1], a->phi_init, a->bidx, a->bvox,
                     a->ub, a->vel, a->checkpoints, a->segment, a->lam[0], a->lam[1], a->G, a->gvel, a->lstart,
@@ -1018,6 +1020,10 @@ int make_chunks(vlr_ctx* ctx, vlr_adjoint* a) {
     cudaFreeAsync(cnt, ctx->stream);
     return rc || e == cudaSuccess ? rc : check_cuda(ctx, e, "adjoint chunk list");
 }
+
+// Blocks up to this size come from the context's pool, which keeps them for the
+// next plan; larger ones go back to the device.
+constexpr size_t kPoolBlock = 32u << 20;
 
 // Bytes of the temporaries of make_vel_entries for n_band voxels (576 each).
 size_t vel_temp_bytes(int n_band) {
@@ -1386,7 +1392,11 @@ int vlr_adj_create(vlr_ctx* ctx, const int32_t* origins, const uint64_t* masks, 
                {(void**)&a->foot_w[1], sizeof(float4) * pool}};
     size_t bytes = 0;
     for (const auto& o : own) bytes += (o.bytes + 255) & ~(size_t)255;
-    ADJ_MALLOC(a->block, std::max(bytes, vel_temp_bytes(a->n_band)));
+    bytes = std::max(bytes, vel_temp_bytes(a->n_band));
+    a->block_pooled = bytes <= kPoolBlock;
+    const cudaError_t eb = a->block_pooled ? cudaMallocFromPoolAsync((void**)&a->block, bytes, ctx->pool, st)
+                                           : cudaMalloc((void**)&a->block, bytes);
+    if (eb != cudaSuccess) return fail(check_cuda(ctx, eb, "adjoint buffers"));
 #undef ADJ_MALLOC
     rc = make_vel_entries(ctx, a, a->block);
     if (rc) return fail(rc);
