@@ -480,8 +480,10 @@ void vlr_ls_destroy(vlr_level_set* ls);
  * voxels, component a on the faces normal to axis a, index ((i*n)+j)*n+k.
  * forward/backward follow the autograd-Function contract: forward(phi_0, V)
  * -> phi_K, backward(dL/dphi_K) -> (dL/dphi_0, dL/dV).  The backward pass
- * recomputes states from checkpoints taken every `checkpoint_every` steps and
- * sums trilinear weights in a fixed order (no float atomics; deterministic).  Band arrays follow vlr_adj_band's order. */
+ * recomputes states from checkpoints taken every `checkpoint_every` steps (more
+ * often where that is over 40 and takes less memory; the results do not depend
+ * on it) and sums trilinear weights in a fixed order (no float atomics;
+ * deterministic).  Band arrays follow vlr_adj_band's order. */
 typedef struct vlr_adjoint vlr_adjoint;
 
 int vlr_adj_create(vlr_ctx* ctx, const int32_t* origins, const uint64_t* masks, const float* phi, size_t n_leaves,
@@ -505,11 +507,12 @@ int vlr_adj_displacement(vlr_ctx* ctx, const vlr_adjoint* a, float* out);
  * context stream (the target of an L2 loss against a translated copy). */
 int vlr_adj_shifted_phi0(vlr_ctx* ctx, const vlr_adjoint* a, int sx, int sy, int sz, float* d_out);
 /* The kernel of the backward pass's lambda transpose: 0 (default) the quad
- * gather for bands under 2^20 voxels at a reach of one voxel per step, the
- * windowed gather otherwise; 1 always the windowed gather; 2 always the quad
- * gather (reach 1 only, VLR_ERR_INVALID otherwise).  Both sum each voxel's
- * terms in a fixed order but associate them differently, so a grid divided
- * over ranks pins one kernel to reproduce the undivided sums bit for bit. */
+ * gather for bands of up to 192 voxels per SM (28,416 on a B200) at a reach of
+ * one voxel per step, the windowed gather otherwise; 1 always the windowed
+ * gather; 2 always the quad gather (reach 1 only, VLR_ERR_INVALID otherwise).
+ * Both sum each voxel's terms in a fixed order, whatever the size of the band,
+ * but associate them differently, so a grid divided over ranks pins one kernel
+ * to reproduce the undivided sums bit for bit. */
 int vlr_adj_set_gather(vlr_ctx* ctx, vlr_adjoint* a, int mode);
 /* Band voxel coordinates (int32[n][3]); coords may be null to query n. */
 int vlr_adj_band(vlr_ctx* ctx, const vlr_adjoint* a, int32_t* coords, size_t cap, size_t* n);

@@ -229,8 +229,9 @@ __device__ __forceinline__ int leaf_of(int c) { return (c + 8) >> 3; }
 // phi_K), when not null.  GRAD: the trilinear gradient of src at the foot, in
 // band order (the backward pass's recomputation); dst may then be null.
 //
-// Bound: the latency of header -> voxel, foot, slots -> eight corners (24
-// bytes a voxel from HBM, 28 us at 7.67M band voxels).  One thread per voxel
+// Bound: instruction issue (70 % of the slots at 7.67M band voxels) and the
+// latency of header -> voxel, foot, slots -> eight corners (24 bytes a voxel
+// from HBM, 28 us there).  One thread per voxel
 // with a neighbour-table load per corner took 121 us there, slots by shuffles
 // 110 us, and 96 us with the next wave's lines prefetched into L2; 2.5 against
 // 3.6 us at 77k voxels (launch-bound).

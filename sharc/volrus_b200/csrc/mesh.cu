@@ -39,8 +39,9 @@
 // Sphere of radius 96 (6,822 tiles, 337k vertices, 673k triangles): classify
 // 43 us and emit 46 us (one thread per cell of a 512-thread CTA, every tile
 // staged: 133 and 139), the tile list 28 us in 5 launches (the sort: 106 us in
-// 22).  Bound: the latency of the slot and rank lookups of a tile and of the
-// creators' words; the mesh's copy to the host is ten times either.
+// 22).  Bound: instruction issue (61 % of the slots), the barriers of a tile
+// (classify) and the loads of its slots and creators' words (emit); the mesh's
+// copy to the host is ten times either.
 // So the output order needs no sort and no atomics: every index is a prefix
 // count in visit order.
 //

@@ -65,7 +65,7 @@ template <> __device__ __forceinline__ __half from_f<__half>(float v) { return _
 //
 // The stencil kernels give that signal when a CTA is done, not when it begins,
 // once CTAs take several leaves (count > gridDim).  Given early, the next
-// kernel's larger CTAs (30-35 KB of shared memory against 17-25) were placed
+// kernel's larger CTAs (26-35 KB of shared memory against 21-25) were placed
 // one by one into the gaps that retiring CTAs left, one CTA per SM fewer fitted
 // than alone, and the missing ones ran as a second wave: 28,680 leaves in f32
 // 930 us per two steps against 799, 9,135 leaves 416 against 372, 2,975 leaves

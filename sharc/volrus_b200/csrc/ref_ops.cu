@@ -161,9 +161,10 @@ __device__ inline void local_get(const GridView& g, int slot, int x, int y, int 
 // zero, is flagged, and its candidates and its neighbours' are decided by the
 // products themselves.
 //
-// Bound: HBM, the one pass over the values (2.2 KB a leaf).  17.5k leaves
-// (L2-resident) take 12 us for the signs and 8 us for the bits; one thread per
-// voxel with a table lookup per neighbour took 83 us.
+// Bound: the ballots of the pass over the values (half the issue slots; 30 % of
+// HBM from a cold cache, 2.2 KB a leaf), then the latency of the neighbours'
+// words.  17.5k leaves (L2-resident) take 12 us for the signs and 8 us for the
+// bits; one thread per voxel with a table lookup per neighbour took 83 us.
 constexpr float kTinyValue = 2.16840434497100887e-19f;  // 2^-62
 
 // One warp per leaf: 16 coalesced rows of 32 values, a ballot each, lane w
@@ -398,8 +399,9 @@ __global__ void __launch_bounds__(256) k_rebuild_window(GridView g, float* __res
 // dz^2 (at most 10 different), so 8 voxels cost one pass over (2R + 1)^2 words
 // and a voxel's minimum is the smallest set that holds it.
 //
-// Bound: HBM (4.2 KB a leaf).  17.5k leaves, R = 2 (L2-resident): 34 us, against
-// 179 us one voxel and 25 row tests at a time.
+// Bound: instruction issue (60 % of the slots) and the staging's barrier.  17.5k
+// leaves, R = 2 (L2-resident, 4.2 KB a leaf): 34 us, against 179 us one voxel
+// and 25 row tests at a time.
 template <int R>
 __global__ void __launch_bounds__(256) k_rebuild_rows(GridView g, float* __restrict__ values,
                                                      unsigned char* __restrict__ mask,
