@@ -50,14 +50,15 @@ def _compare(small, whole):
     assert np.abs(g[0]).max() > 0
 
 
-@pytest.mark.parametrize("speed", [0.9, 1.0, 1.9, 3.9, 5.9])
+@pytest.mark.parametrize("speed", [0.9, 0.999999, 1.0, 1.9, 3.9, 5.9])
 def test_staggered(speed):
     from sharc.volrus_b200.adjoint import AdvectionFunction
     V = (np.random.default_rng(11).uniform(-1, 1, (3, 28, 28, 28)) * speed).astype(np.float32)
-    if speed == 1.0:  # whole voxels, which a reach of one just excludes: foot offsets -1 and 1 at an edge
+    if speed in (0.999999, 1.0):
+        # a whole voxel a step and the largest speed below it that has a reach of one: foot offsets at an edge
         V = np.where(np.random.default_rng(12).random((3, 7, 7, 7)) < 0.5, -1, 1).repeat(4, 1).repeat(4, 2).repeat(4, 3)
-        V = np.ascontiguousarray(V, np.float32)
-    fns = [AdvectionFunction(*leaves, V, 8.0, 1.0, 50.0, 3, 2) for leaves in _both()]
+        V = np.ascontiguousarray(V * speed, np.float32)
+    fns = [AdvectionFunction(*leaves, V, 8.0, 1.0, 1e12 if speed <= 1.0 else 50.0, 3, 2) for leaves in _both()]
     _compare(*fns)
     for f in fns:
         f.close()
