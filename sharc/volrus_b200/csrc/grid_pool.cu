@@ -225,7 +225,7 @@ static int staged_copy(vlr_ctx* ctx, char* host, char* dev, size_t bytes, bool u
                                 ctx->stage_ev + 2 * t, st);
     };
     CopyThreads* pool = ctx->copy_threads;
-    const int others = pool ? (int)pool->threads.size() : 0;
+    const int others = pool && pool->owner == getpid() ? (int)pool->threads.size() : 0;
     if (others) {
         std::lock_guard<std::mutex> lock(pool->m);
         pool->job = [](void* f, int t) { (*static_cast<decltype(share)*>(f))(t); };

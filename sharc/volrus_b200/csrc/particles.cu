@@ -148,8 +148,9 @@ __device__ __forceinline__ unsigned leaf_key(int32_t v) { return ((unsigned)v >>
 __device__ __forceinline__ int32_t key_leaf(unsigned k) { return (int32_t)((k ^ (1u << 28)) << 3); }
 
 // Bound: load latency, the instruction cache (45 % of the issue slots) and the f64
-// and conversion instructions of 12 samples a particle (RK4).  300k particles in a 64^3 field: 124 us with up to 8 hash
-// searches a sample, 46 us from the particle's leaf.
+// and conversion instructions of 12 samples a particle (RK4).  300k particles in
+// a 64^3 field: 124 us with up to 8 hash searches a sample, 49 us from the
+// particle's leaf.
 template <bool SAME>
 __global__ void __launch_bounds__(256) k_points_move(GridView vx, GridView vy, GridView vz,
                                                     vlr_particle* __restrict__ pts, int n, double dt, int rk4,
