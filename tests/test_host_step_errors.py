@@ -150,3 +150,25 @@ def test_states_thin_in_x(ctx, dims, steps):
     assert _same(want, got) and _same(want, counted)
     assert _same(want, _host_step(ls, inp, 3, out))
     ls.close()
+
+
+def test_wait_that_runs_out_in_a_slab(ctx, state):
+    """A bounded wait of the step gives up: reported, the state lost, and an upload brings it back."""
+    from sharc.volrus_b200 import VolrusError
+    ls, inp = state
+    want = _host_step(ls, inp, 1)
+    for slabs in (1, 0):
+        ctx.check(ctx.lib.vlr_ctx_set_wait_limit(ctx.handle, 2000), "vlr_ctx_set_wait_limit")
+        ctx.check(ctx.lib.vlr_ctx_test_stall(ctx.handle, 1), "vlr_ctx_test_stall")
+        try:
+            with pytest.raises(VolrusError) as e:
+                _host_step(ls, inp, slabs)
+            assert e.value.code == _codes()["VLR_ERR_TIMEOUT"]
+        finally:
+            ctx.check(ctx.lib.vlr_ctx_test_stall(ctx.handle, 0), "vlr_ctx_test_stall")
+            ctx.check(ctx.lib.vlr_ctx_set_wait_limit(ctx.handle, 0), "vlr_ctx_set_wait_limit")
+        with pytest.raises(VolrusError) as e:
+            ls.step(1)
+        assert e.value.code == _codes()["VLR_ERR_INVALID"]
+        ctx.check_device()
+        assert _same(_host_step(ls, inp, slabs), want)
